@@ -171,7 +171,7 @@ Engine::~Engine() {
                     d.ic_new, d.arr_count, d.arr_start, d.arr_list, d.work, d.new_count,
                     d.new_start, d.cell_atoms2, d.nlist, d.numn, d.posq, d.posq2, d.pos2, d.alist,
                     d.pair_cnt, d.olist, d.out_cnt, d.rlist, d.numr, d.xout, d.xhalf, d.mlist, d.mid_cnt, d.xbuild, d.tab_r4, d.tab_e2,
-                    d.tab_r4f, d.tab_e2f, d.tab_aux, d.partials, d.flags, d.revmask, d.box, d.scan_tmp, d.adj, d.rdf};
+                    d.tab_r4f, d.tab_e2f, d.tab_aux, d.partials, d.run_scratch, d.flags, d.revmask, d.box, d.scan_tmp, d.adj, d.rdf};
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (host_box_) cudaFreeHost(host_box_);
@@ -249,6 +249,7 @@ static int init_engine(Engine &E, int device) {
     CHECK(dev_alloc(&d.mid_cnt, nm, "mid_cnt"));
     CHECK(dev_alloc(&d.xbuild, nm, "xbuild"));
     CHECK(dev_alloc(&d.partials, 3 * (size_t)kMaxBlocks * kPartials, "partials"));
+    CHECK(dev_alloc(&d.run_scratch, run_scratch_bytes() / sizeof(double), "run scratch"));
     CHECK(dev_alloc(&d.flags, 16, "flags"));
     CHECK(dev_alloc(&d.revmask, (size_t)kRevPlanes * nm, "reverse-row masks"));
     CHECK(dev_alloc(&d.box, 1, "box"));
@@ -566,7 +567,7 @@ int Engine::get_linkcells(int32_t *l0, int32_t *link, int32_t *ic) {
 }
 
 int Engine::check_flags() {
-    int32_t f[12];
+    int32_t f[14];
     CUDA_CHECK(cudaMemcpyAsync(f, d.flags, sizeof(f), cudaMemcpyDeviceToHost, stream_), "flags");
     int32_t st = 0;
     CUDA_CHECK(cudaMemcpyAsync(&st, &d.box->status, sizeof(st), cudaMemcpyDeviceToHost, stream_), "flags");
@@ -583,6 +584,10 @@ int Engine::check_flags() {
     if (f[1]) {
         cudaMemsetAsync(d.flags, 0, sizeof(f), stream_);
         return fail(MOLDY_ERR_CAPACITY, "link-cell relink produced inconsistent cell counts");
+    }
+    if (f[13]) {
+        cudaMemsetAsync(d.flags, 0, sizeof(f), stream_);
+        return fail(MOLDY_ERR_CUDA, "a grid barrier of a fused run of steps gave up waiting; the state is not usable");
     }
     if (f[10]) {
         cudaMemsetAsync(d.flags, 0, sizeof(f), stream_);
@@ -817,6 +822,65 @@ int Engine::md_init(moldy_force_out *out) {
     return MOLDY_OK;
 }
 
+// Steps from here on that a fused run can take (at most left): none of them
+// builds the half list, and only the last may be followed by a relink or scalev.
+int Engine::run_length(int left) const {
+    if (!list_ready_ || !cells_ready_ || mid_dirty_) return 0;
+    int m = 0, ntc = ntc_;
+    double tt = thermotimer_;
+    while (m < left && m < kRunMaxSteps && ntc != 0) {
+        ++m;
+        ntc = ntc + 1;
+        tt = tt + prm.deltat;
+        bool sv = false;
+        if (tt >= kFemtosecond) {
+            tt = tt - kFemtosecond;
+            sv = nose_ > 0.0;
+        }
+        if (ntc == ntcm_ || sv) break;
+    }
+    return m;
+}
+
+// Queues a fused run of m steps and advances the host-side state; the pieces
+// are launched one by one while profiling (the same results bit for bit).
+int Engine::queue_run(int m, bool therm, double *rec, int rec0, bool last, bool &scalev, int *ntcs) {
+    const bool mixed = precision_ == MOLDY_PREC_MIXED;
+    cudaStream_t s = stream_;
+    int rc = 0;
+    auto pieces = [&](int id, int h0, int h1) {
+        LAUNCH(*this, id, 1, s,
+               if (!rc) rc = launch_run(d, prm, tab, mixed, rmid, rcut, rout, m, h0, h1, therm ? 1 : 0, rec, rec0,
+                                        last ? 1 : 0, s));
+    };
+    if (prof.on) {
+        pieces(K_DRIFT, 0, 0);
+        for (int q = 0; q < m; ++q) {
+            pieces(K_SCREEN, 2 * q + 1, 2 * q + 1);
+            pieces(K_PAIR, 2 * q + 2, 2 * q + 2);
+        }
+        pieces(K_FINALIZE, 2 * m + 1, 2 * m + 1);
+    } else {
+        pieces(K_PAIR, 0, 2 * m + 1);
+    }
+    if (rc) return cuda_fail((cudaError_t)rc, "fused run of steps");
+    for (int q = 0; q < m; ++q) {
+        ntc_ = ntc_ + 1;
+        if (ntc_ == ntcm_) ntc_ = 0;
+        ntcs[q] = ntc_;
+        thermotimer_ = thermotimer_ + prm.deltat;
+        scalev = false;
+        if (thermotimer_ >= kFemtosecond) {
+            thermotimer_ = thermotimer_ - kFemtosecond;
+            scalev = nose_ > 0.0;
+        }
+    }
+    therm_blocks = 0;
+    therm_rec = nullptr;
+    skip_rho = false;
+    return MOLDY_OK;
+}
+
 int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
     CHECK(check_ready());
     if (nsteps < 0) return fail(MOLDY_ERR_INVALID, "nsteps < 0");
@@ -851,8 +915,28 @@ int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
     cudaGraphExec_t step_graph = nullptr;
     bool graph_failed = prof.on || nsteps < 8, rec_synced = false;
     long long per_replay[K_COUNT] = {};
+    const bool mixed = precision_ == MOLDY_PREC_MIXED;
     for (int k = 0; k < nsteps; ++k) {
         bool rb = false;
+        // consecutive steps of a small system that need no half-list build, up
+        // to and including one that is followed by a relink or scalev: one launch
+        const int run = run_applies(prm, tab, mixed) ? run_length(nsteps - k) : 0;
+        if (run >= 2) {
+            CHECK(ensure_active_capacity(0));
+            bool scalev = false;
+            CHECK(queue_run(run, therm_pending, thermo ? d.thermo_rec : nullptr, k - 1, k + run == nsteps, scalev,
+                            &ntcs[k]));
+            for (int q = 0; q < run; ++q) rbs[k + q] = 0;
+            k += run - 1;
+            rec_synced = false;
+            therm_pending = !(scalev || k == nsteps - 1);
+            if (!therm_pending)
+                LAUNCH(*this, K_THERM, 2, stream_,
+                       launch_therm(d, prm, false, thermo ? d.thermo_rec + (size_t)kThermoRec * k : nullptr, stream_));
+            if (ntc_ == 0) LAUNCH(*this, K_RELINK, 6, stream_, launch_relink(d, prm, stream_));
+            if (scalev) LAUNCH(*this, K_SCALEV, 4, stream_, launch_scalev(d, prm, nose_, rqke_, stream_));
+            continue;
+        }
         {
             // this step's scalev decision, as made below
             double tt = thermotimer_ + prm.deltat;

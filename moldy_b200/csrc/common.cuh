@@ -38,6 +38,7 @@ struct BoxState {
     int32_t out_rebuild;           // 1: the outer list is rebuilt this step
     int32_t out_builds;            // number of outer-list builds so far
     int32_t rec_step;              // thermo record the next indexed k_mid_decide writes
+    double rec_b0[9], rec_b1[9];   // fused runs: the box of the step whose thermo record is next
 };
 
 // Per-launch constant parameters.

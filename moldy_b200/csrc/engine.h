@@ -78,12 +78,14 @@ struct DeviceState {
     int thermo_cap = 0;
     // reductions, flags and box state
     double *partials = nullptr;
+    double *run_scratch = nullptr; // partial sums and barrier counter of the fused runs (run.cu)
     int32_t *flags = nullptr;     // [0] neighbour overflow, [1] relink inconsistency,
                                   // [2] overflow atom, [3] active-list overflow, [4] its count,
                                   // [5] intermediate-row overflow, [6] its count,
                                   // [8] outer-row overflow, [9] its count,
                                   // [10] reverse half-row overflow, [11] its count,
-                                  // [12] a link cell too full for the reverse-row masks
+                                  // [12] a link cell too full for the reverse-row masks,
+                                  // [13] a grid barrier of a fused run gave up waiting
     // per (cell rank r of the half stencil, round of 32 home atoms, atom j):
     // the home atoms of j's source cell whose half-list rows hold j (one bit
     // per home atom of the round), written by the half-list build
@@ -226,6 +228,8 @@ class Engine {
     int force_device(bool *rebuilt);     // queue force on the stream
     int fetch_force_out(moldy_force_out *out);
     int check_flags();
+    int run_length(int left) const;
+    int queue_run(int m, bool therm, double *rec, int rec0, bool last, bool &scalev, int *ntcs);
 
     cudaStream_t stream_ = nullptr;
     int device_ = 0;
@@ -259,6 +263,8 @@ class Engine {
     int host_rec_cap_ = 0;
 };
 
+constexpr int kRunMaxAtoms = 150000;    // fused runs of steps (run.cu) up to this many atoms
+constexpr int kRunMaxSteps = 512;      // steps of one fused run
 constexpr int kAtomThreads = 256;
 constexpr int kMaxBlocks = 148 * 8;    // grid-stride kernels: 8 blocks per SM
 constexpr int kPairCapMin = 24;        // least compact-row entries per atom
@@ -331,6 +337,16 @@ int launch_kinetic(DeviceState &d, const Params &p, double *partials, cudaStream
 void launch_mid_decide(DeviceState &d, const Params &p, double rmid, double rcut, double rout, int force,
                        int half_build, int apply_box, int therm_nblk, double *rec, cudaStream_t s,
                        int rec_indexed = 0);
+// runs of steps in one launch (run.cu): whether they apply, their device
+// scratch, and the pieces h0..h1 (0: first drift, 2s+1 and 2s+2: the two
+// pieces of step s, 2m+1: the final box) of a run of m steps; therm: the step
+// before awaits its update_therm_avs; rec, rec0: thermo records and the index
+// of that step's; store: the last step stores rho and the forces.  Returns the
+// CUDA status of the launch.
+bool run_applies(const Params &p, const Tables &t, bool mixed);
+size_t run_scratch_bytes();
+int launch_run(DeviceState &d, const Params &p, const Tables &t, bool mixed, double rmid, double rcut, double rout,
+               int m, int h0, int h1, int therm, double *rec, int rec0, int store, cudaStream_t s);
 void launch_set_rec_step(DeviceState &d, int step, cudaStream_t s);
 // the outer list from the half list when k_mid_decide asked for it, then the
 // intermediate list from the outer list when it asked for that

@@ -38,6 +38,7 @@
 #include <type_traits>
 
 #include "engine.h"
+#include "pairs.cuh"
 
 namespace moldy {
 
@@ -70,86 +71,6 @@ static int one_wave(K kernel) {
 // inside an allocated buffer)
 __device__ __forceinline__ void prefetch_l2(const void *ptr) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr));
-}
-
-// Squared FP32 distance of an FP64 fractional difference (any box): the
-// difference rounded to FP32 (off by at most 2^-24 |dx|), the minimum image by
-// rintf in the periodic directions.
-__device__ __forceinline__ float sep2_f32(const float *bf, int ivol, double dxd, double dyd, double dzd) {
-    float dx = (float)dxd, dy = (float)dyd, dz = (float)dzd;
-    if (ivol == 0 || ivol == 1 || ivol == 4) {
-        dx -= rintf(dx); dy -= rintf(dy); dz -= rintf(dz);
-    } else if (ivol == 2) {
-        dx -= rintf(dx); dy -= rintf(dy);
-    } else if (ivol == 5) {
-        dz -= rintf(dz);
-    }
-    const float rx = fmaf(bf[6], dz, fmaf(bf[3], dy, bf[0] * dx));
-    const float ry = fmaf(bf[7], dz, fmaf(bf[4], dy, bf[1] * dx));
-    const float rz = fmaf(bf[8], dz, fmaf(bf[5], dy, bf[2] * dx));
-    return fmaf(rz, rz, fmaf(ry, ry, rx * rx));
-}
-
-// Separation of two atoms from their fixed-point coordinates (fully periodic
-// box): the 32-bit differences are the minimum image; bs is B0 per fixed-point
-// unit.  Returns r^2 and the Cartesian separation, all FP32.
-__device__ __forceinline__ float fix_sep(const float *bs, const int4 &qa, const int4 &qj, float &rx, float &ry,
-                                         float &rz, float &dx, float &dy, float &dz) {
-    dx = fix_to_float((int32_t)((uint32_t)qa.x - (uint32_t)qj.x));
-    dy = fix_to_float((int32_t)((uint32_t)qa.y - (uint32_t)qj.y));
-    dz = fix_to_float((int32_t)((uint32_t)qa.z - (uint32_t)qj.z));
-    rx = fmaf(bs[6], dz, fmaf(bs[3], dy, bs[0] * dx));
-    ry = fmaf(bs[7], dz, fmaf(bs[4], dy, bs[1] * dx));
-    rz = fmaf(bs[8], dz, fmaf(bs[5], dy, bs[2] * dx));
-    return fmaf(rz, rz, fmaf(ry, ry, rx * rx));
-}
-
-__device__ __forceinline__ float fix_sep(const float *bs, const int4 &qa, const int4 &qj, float &rx, float &ry,
-                                         float &rz) {
-    float dx, dy, dz;
-    return fix_sep(bs, qa, qj, rx, ry, rz, dx, dy, dz);
-}
-
-// --------------------------------------------------------------- screen --
-// Squared screening radius for the FP32 pre-selection.  The FP32 copy of a
-// fractional coordinate is off by at most 2^-24 |x|; for |x| < 5 (positions
-// are never wrapped) the FP32 distance is then within 2e-6 |B0|_F + 1e-4 A of
-// the FP64 one.  rintf and NINT pick different images only at |dx| = 1/2,
-// i.e. at half a box width; when half the narrowest width is not beyond the
-// screening radius every pair goes to the FP64 test.
-__device__ float screen_radius2(const double *b, double rcull2) {
-    double nf = 0.0;
-    for (int k = 0; k < 9; ++k) nf += b[k] * b[k];
-    double rs = sqrt(rcull2) + 2.0e-6 * sqrt(nf) + 1.0e-4;
-    double vol = fabs(b[0] * (b[4] * b[8] - b[7] * b[5]) - b[3] * (b[1] * b[8] - b[7] * b[2]) +
-                      b[6] * (b[1] * b[5] - b[4] * b[2]));
-    double wmin = 1e300;
-    for (int k = 0; k < 3; ++k) {   // width across the face spanned by the other two box vectors
-        const double *u = b + 3 * ((k + 1) % 3), *w = b + 3 * ((k + 2) % 3);
-        double cx = u[1] * w[2] - u[2] * w[1], cy = u[2] * w[0] - u[0] * w[2], cz = u[0] * w[1] - u[1] * w[0];
-        double a = sqrt(cx * cx + cy * cy + cz * cz);
-        if (a > 0.0) wmin = fmin(wmin, vol / a);
-    }
-    if (!(0.5 * wmin > rs * (1.0 + 1e-6))) return 3.0e38f;
-    return (float)(rs * rs);
-}
-
-
-constexpr int32_t kOwnBit = (int32_t)0x80000000u;
-constexpr int32_t kIdMask = 0x7fffffff;
-
-// The exact FP64 test r^2 <= rcull^2 for a pair whose FP32 distance lies in
-// the error band around the cut (rare: kept out of line, so its registers do
-// not count against the screening loop)
-__device__ __noinline__ bool inside_cut_fp64(const double4 *__restrict__ pos, int a, int j, const double *b,
-                                             int ivol, double rcull2) {
-    const double4 pa = pos[a], qd = pos[j];
-    double ex = pa.x - qd.x, ey = pa.y - qd.y, ez = pa.z - qd.z;
-    min_image(ivol, ex, ey, ez);
-    double sx = b[0] * ex + b[3] * ey + b[6] * ez;
-    double sy = b[1] * ex + b[4] * ey + b[7] * ez;
-    double sz = b[2] * ex + b[5] * ey + b[8] * ez;
-    return (sx * sx + sy * sy + sz * sz) <= rcull2;
 }
 
 // Keeps pair (a, j) iff its distance is inside the table range, sums rho_a,
@@ -270,17 +191,6 @@ k_screen_density(Params p, Tables t, const double4 *__restrict__ pos, const int4
 }
 
 // --------------------------------------------------------------- forces --
-// v[1..6] += s * sym(a (x) b) in the order xx, yy, zz, xy, xz, yz
-__device__ __forceinline__ void add_sym(double *v, double ax, double ay, double az, double bx, double by,
-                                        double bz, double s) {
-    v[1] += s * (ax * bx);
-    v[2] += s * (ay * by);
-    v[3] += s * (az * bz);
-    v[4] += (0.5 * s) * (ax * by + ay * bx);
-    v[5] += (0.5 * s) * (ax * bz + az * bx);
-    v[6] += (0.5 * s) * (ay * bz + az * by);
-}
-
 // f_i = sum_j g_ij over the compact row, g_ij = d_ij fp_ij; pe and the
 // virial moment D = sum over pairs d d^T fp (tp = B0 D, pairs with
 // m_i + m_j <= 0.1 left out, src/dynamics_m.F90:287); mode 1 adds the
@@ -521,13 +431,6 @@ k_forces(Params p, Tables t, const double4 *__restrict__ pos2, const int4 *__res
 // no atomics and every row is the same from run to run.  The intermediate
 // build filters each atom's outer row the same way.  Each kernel returns at
 // once when k_mid_decide asked for no build.
-
-// FP32 keep radius^2 of a list of radius r: r plus twice the FP32 distance
-// error bound, or every pair when the box is too small for the FP32 screen
-__device__ float keep_radius2(const double *sb, double r) {
-    const float keep = (float)(r + 2.0 * (2.0e-6 * frob(sb) + 1.0e-4));
-    return screen_radius2(sb, r * r) > 1e37f ? 3.0e38f : keep * keep;
-}
 
 // Appends to atom a's row (entries kept in [cnt, cap), entry-major with
 // stride nm) the entries of one source row (n entries, entry k at
