@@ -162,6 +162,7 @@ Engine::Engine(const moldy_params &p) {
     precision_ = p.precision;
     device_ = p.device;
     std::memset(&tab, 0, sizeof(tab));
+    variant[K_SCREEN] = variant[K_PAIR] = kAutoVariant;
 }
 
 Engine::~Engine() {
@@ -321,6 +322,16 @@ int upload_device_tables(const HostTables &h, double4 **r4d, float4 **r4fd, doub
         r4f[2 * (size_t)i + 1] = make_float4(b.x - a.x, b.y - a.y, b.z - a.z, b.w - a.w);
         phi2f[i].y = phi2f[i + 1].x - phi2f[i].x;
     }
+    // FP64 intervals as (node, step): (V', phi') and (V), (phi); the last stored
+    // node has no step, so it is what every distance beyond it takes
+    std::vector<double4> df4(nr);
+    std::vector<double2> dv2(nr), dp2(nr);
+    for (int i = 0; i < nr; ++i) {
+        const double4 a = r4[i], b = r4[i + 1 < nr ? i + 1 : i];
+        df4[i] = make_double4(a.y, a.w, b.y - a.y, b.w - a.w);
+        dv2[i] = make_double2(a.x, b.x - a.x);
+        dp2[i] = make_double2(a.z, b.z - a.z);
+    }
     std::vector<double2> e2(n + 1);
     std::vector<float2> e2f(n + 1);
     for (int i = 0; i <= n; ++i) {
@@ -333,23 +344,35 @@ int upload_device_tables(const HostTables &h, double4 **r4d, float4 **r4fd, doub
     *r4d = nullptr; *e2d = nullptr; *r4fd = nullptr; *e2fd = nullptr; *auxd = nullptr;
     CHECK(dev_alloc(r4d, nr, "tables"));
     CHECK(dev_alloc(r4fd, 2 * (size_t)nr, "tables"));
-    // phi2 (nr double2), then phi2f (nr float2)
+    // df4 (nr double4), phi2, dv2, dp2 (nr double2 each), then phi2f (nr float2), one copy
+    const size_t aux_bytes = (size_t)nr * (sizeof(double4) + 3 * sizeof(double2) + sizeof(float2));
+    std::vector<unsigned char> aux_h(aux_bytes);
+    size_t off = 0;
+    size_t at[5];
+    const void *parts[5] = {df4.data(), phi2.data(), dv2.data(), dp2.data(), phi2f.data()};
+    const size_t sizes[5] = {sizeof(double4), sizeof(double2), sizeof(double2), sizeof(double2), sizeof(float2)};
+    for (int k = 0; k < 5; ++k) {
+        at[k] = off;
+        std::memcpy(aux_h.data() + off, parts[k], nr * sizes[k]);
+        off += nr * sizes[k];
+    }
     unsigned char *aux = nullptr;
-    CHECK(dev_alloc(&aux, (size_t)nr * (sizeof(double2) + sizeof(float2)), "tables"));
+    CHECK(dev_alloc(&aux, aux_bytes, "tables"));
     *auxd = aux;
     CHECK(dev_alloc(e2d, n + 1, "tables"));
     CHECK(dev_alloc(e2fd, n + 1, "tables"));
     CUDA_CHECK(cudaMemcpy(*r4d, r4.data(), nr * sizeof(double4), cudaMemcpyHostToDevice), "tables");
     CUDA_CHECK(cudaMemcpy(*r4fd, r4f.data(), 2 * (size_t)nr * sizeof(float4), cudaMemcpyHostToDevice), "tables");
-    CUDA_CHECK(cudaMemcpy(aux, phi2.data(), nr * sizeof(double2), cudaMemcpyHostToDevice), "tables");
-    CUDA_CHECK(cudaMemcpy(aux + nr * sizeof(double2), phi2f.data(), nr * sizeof(float2), cudaMemcpyHostToDevice),
-               "tables");
+    CUDA_CHECK(cudaMemcpy(aux, aux_h.data(), aux_bytes, cudaMemcpyHostToDevice), "tables");
     CUDA_CHECK(cudaMemcpy(*e2d, e2.data(), (n + 1) * sizeof(double2), cudaMemcpyHostToDevice), "tables");
     CUDA_CHECK(cudaMemcpy(*e2fd, e2f.data(), (n + 1) * sizeof(float2), cudaMemcpyHostToDevice), "tables");
 
     t.r4 = *r4d; t.e2 = *e2d; t.r4f = *r4fd; t.e2f = *e2fd;
-    t.phi2 = reinterpret_cast<const double2 *>(aux);
-    t.phi2f = reinterpret_cast<const float2 *>(aux + nr * sizeof(double2));
+    t.df4 = reinterpret_cast<const double4 *>(aux + at[0]);
+    t.phi2 = reinterpret_cast<const double2 *>(aux + at[1]);
+    t.dv2 = reinterpret_cast<const double2 *>(aux + at[2]);
+    t.dp2 = reinterpret_cast<const double2 *>(aux + at[3]);
+    t.phi2f = reinterpret_cast<const float2 *>(aux + at[4]);
     t.nlookup = n;
     t.nr = nr;
     t.idx_cut = cut;
@@ -359,6 +382,7 @@ int upload_device_tables(const HostTables &h, double4 **r4d, float4 **r4fd, doub
     t.vp_reciprange = 1.0 / t.vp_range;
     t.vp_recipnlkp = 1.0 / (double)n;
     t.vp_recipstep = (double)n / t.vp_range;
+    t.vp_xoff = -h.rmin * t.vp_recipstep;
     t.e_rmin = h.rhomin; t.e_rmax = h.rhomax;
     t.e_range = h.rhomax - h.rhomin;
     t.e_reciprange = 1.0 / t.e_range;

@@ -58,11 +58,14 @@ struct Tables {
     const float4 *r4f;      // FP32 copy of r4 for the mixed path, node pairs: [2k] = node k, [2k+1] = node k+1
     const float2 *e2f;
     const double2 *phi2;    // per node k (phi_k, phi_k+1): one load per density lookup
+    const double4 *df4;     // per interval (dvee, dphi, their steps to the next node); the last has step zero
+    const double2 *dv2, *dp2;   // per interval (vee, step) and (phi, step)
     const float2 *phi2f;
     int nlookup;            // intervals
     int nr;                 // stored r nodes (culled tail removed)
     int idx_cut;            // first node from which all r tables are zero
     int exact;              // 1: evaluate *_src analytically, not from tables
+    double vp_xoff;         // node coordinate of r: r * vp_recipstep + vp_xoff
     double vp_rmin, vp_rmax, vp_range, vp_reciprange, vp_recipnlkp, vp_recipstep;
     double e_rmin, e_rmax, e_range, e_reciprange, e_recipnlkp, e_recipstep;
     double rcull2;          // pairs with r^2 above this contribute exactly zero
@@ -241,13 +244,13 @@ __device__ __forceinline__ float4 lookup_r4f(const Tables &t, float r) {
     return make_float4(fmaf(b.x, dr, a.x), fmaf(b.y, dr, a.y), fmaf(b.z, dr, a.z), fmaf(b.w, dr, a.w));
 }
 
-__device__ __forceinline__ float lookup_phif(const Tables &t, float r) {
+__device__ __forceinline__ float lookup_phif(const Tables &t, const float2 *__restrict__ phi2f, float r) {
     const float x = fmaf(r, t.recipstep_f, t.xoff_f);
     float fl;
     const int idx = floor_small(fmaxf(x, 0.f), fl);
     if (idx >= t.nr - 1) return t.tail_f.z;
     const float dr = x - fl;
-    const float2 v = __ldg(&t.phi2f[idx]);
+    const float2 v = phi2f[idx];
     return fmaf(v.y, dr, v.x);
 }
 

@@ -67,7 +67,7 @@ k_finalize_force(Params p, BoxState *__restrict__ box, const double *__restrict_
 void launch_finalize_force(DeviceState &d, const Params &p, const double *part_embed, int nblk_embed,
                            const double *part_force, int nblk_force, const double *part_kin, int nblk_kin,
                            int mode, cudaStream_t s) {
-    launch_pdl(k_finalize_force, 1, 256, s, p, d.box, part_embed, nblk_embed, part_force, nblk_force, part_kin, nblk_kin,
+    launch_pdl(k_finalize_force, 1, 256, 0, s, p, d.box, part_embed, nblk_embed, part_force, nblk_force, part_kin, nblk_kin,
                                         mode);
 }
 
@@ -137,7 +137,7 @@ k_mid_decide(Params p, BoxState *__restrict__ box, double rmid, double rcut, dou
 void launch_mid_decide(DeviceState &d, const Params &p, double rmid, double rcut, double rout, int force,
                        int half_build, int apply_box, int therm_nblk, double *rec, cudaStream_t s,
                        int rec_indexed) {
-    launch_pdl(k_mid_decide, 1, 256, s, p, d.box, rmid, rcut, rout, force, half_build, apply_box, d.partials,
+    launch_pdl(k_mid_decide, 1, 256, 0, s, p, d.box, rmid, rcut, rout, force, half_build, apply_box, d.partials,
                                    therm_nblk, rec, rec_indexed);
 }
 
@@ -230,10 +230,10 @@ k_drift(Params p, double4 *__restrict__ pos, int4 *__restrict__ posq,
 int launch_drift(DeviceState &d, const Params &p, double *kin_partials, bool therm, cudaStream_t s) {
     int nb = stream_blocks(p.nm);
     if (therm)
-        launch_pdl(k_drift<true>, nb, kAtomThreads, s, p, d.pos, d.posq, d.x1, d.x2, d.box, d.xbuild, d.mass, d.znum,
+        launch_pdl(k_drift<true>, nb, kAtomThreads, 0, s, p, d.pos, d.posq, d.x1, d.x2, d.box, d.xbuild, d.mass, d.znum,
                                                   kin_partials, d.partials);
     else
-        launch_pdl(k_drift<false>, nb, kAtomThreads, s, p, d.pos, d.posq, d.x1, d.x2, d.box, d.xbuild, d.mass, d.znum,
+        launch_pdl(k_drift<false>, nb, kAtomThreads, 0, s, p, d.pos, d.posq, d.x1, d.x2, d.box, d.xbuild, d.mass, d.znum,
                                                    kin_partials, nullptr);
     return nb;
 }

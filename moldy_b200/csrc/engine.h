@@ -263,7 +263,6 @@ class Engine {
     int host_rec_cap_ = 0;
 };
 
-constexpr int kRunMaxAtoms = 150000;    // fused runs of steps (run.cu) up to this many atoms
 constexpr int kRunMaxSteps = 512;      // steps of one fused run
 constexpr int kAtomThreads = 256;
 constexpr int kMaxBlocks = 148 * 8;    // grid-stride kernels: 8 blocks per SM
@@ -289,11 +288,11 @@ inline int grid_blocks(long long work, int threads) {
 // (the kernel calls grid_dep_wait before touching any data), which hides the
 // launch gap between the kernels of a step.
 template <typename... KArgs, typename... Args>
-inline void launch_pdl(void (*kernel)(KArgs...), int grid, int block, cudaStream_t s, Args &&...args) {
+inline void launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t s, Args &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -316,6 +315,7 @@ void launch_build_nlist(DeviceState &d, const Params &p, cudaStream_t s);
 void launch_export_nlist(const int32_t *rows, const int32_t *cnt, bool atom_major, const Params &p, int32_t *out,
                          cudaStream_t s);
 constexpr int kVariants = 8;           // compiled variants per tunable pass
+constexpr int kAutoVariant = -1;       // the pass chooses by precision and size (until set or tuned)
 // store_rho false: rho is not written (no caller reads it before the next
 // evaluation overwrites it: the inner steps of an md_steps call)
 int launch_screen_density(DeviceState &d, const Params &p, const Tables &t, bool mixed, int variant,

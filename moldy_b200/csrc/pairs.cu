@@ -42,15 +42,17 @@
 
 namespace moldy {
 
-// One wave of resident blocks for the kernel (at 256 threads): every block
-// then runs the same number of grid-stride iterations (to within one), and no
-// partly filled last wave idles the SMs.  Computed once per instantiation.
+// One wave of resident blocks for the kernel (nt threads, smem
+// bytes of dynamic shared memory): every block then runs the same number of
+// grid-stride iterations (to within one), and no partly filled last wave
+// idles the SMs.  Computed once per instantiation.
 template <typename K>
-static int one_wave(K kernel) {
+static int one_wave(K kernel, int nt = 256, size_t smem = 0) {
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0) != cudaSuccess) {
+    if (smem > 0) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, nt, smem) != cudaSuccess) {
         cudaGetLastError();
         per_sm = 0;
     }
@@ -62,10 +64,18 @@ static int one_wave(K kernel) {
     do {                                                     \
         static const int wave_ = one_wave(KERNEL);           \
         NB = NB < wave_ ? NB : wave_;                        \
-        launch_pdl(KERNEL, NB, 256, S, __VA_ARGS__);         \
+        launch_pdl(KERNEL, NB, 256, 0, S, __VA_ARGS__);      \
     } while (0)
 
-
+// NT threads per block and SMEM bytes of tables, at most MAXS (512 threads and
+// more fill an SM's registers: one block per SM whatever the tables take)
+#define LAUNCH_WAVE_SMEM(KERNEL, NT, SMEM, MAXS, NB, S, ...) \
+    do {                                                     \
+        static const int wave_ = one_wave(KERNEL, NT, MAXS); \
+        NB = (p.nm + NT - 1) / NT;                           \
+        NB = NB < wave_ ? NB : wave_;                        \
+        launch_pdl(KERNEL, NB, NT, SMEM, S, __VA_ARGS__);    \
+    } while (0)
 
 // L2 prefetch of one address (no register result; the address is always
 // inside an allocated buffer)
@@ -141,7 +151,7 @@ k_screen_density(Params p, Tables t, const double4 *__restrict__ pos, const int4
                     if (r2 > rscreen2) continue;
                     // inside the error band: the FP64 distance decides
                     if (!(r2 < rin2) && !inside_cut_fp64(pos, a, ee[u] & kIdMask, sb, p.ivol, t.rcull2)) continue;
-                    rho_a += (double)lookup_phif(t, r2 * rsqrt_ftz(r2));
+                    rho_a += (double)lookup_phif(t, t.phi2f, r2 * rsqrt_ftz(r2));
                     if (cnt < p.pair_cap) alist[(size_t)cnt * stride + a] = ee[u];
                     ++cnt;
                 }
@@ -191,6 +201,66 @@ k_screen_density(Params p, Tables t, const double4 *__restrict__ pos, const int4
 }
 
 // --------------------------------------------------------------- forces --
+// Fixed-point coordinates beyond which an atom may have a pair whose 32-bit
+// difference wraps (crosses a periodic boundary): a pair inside the cut spans
+// at most M_d = rcull |row d of B0^-1| box lengths in direction d; an atom
+// whose coordinates all lie within 2^31 - M_d of zero has none.
+static __device__ void wrap_limits(const double *b, double rcull2, int *lim) {
+    double bi[9];
+    const bool ok = mat_invert(b, bi);
+    for (int d = 0; d < 3; ++d) {
+        const double rn = sqrt(MAT(bi, d + 1, 1) * MAT(bi, d + 1, 1) + MAT(bi, d + 1, 2) * MAT(bi, d + 1, 2) +
+                               MAT(bi, d + 1, 3) * MAT(bi, d + 1, 3));
+        const double m = sqrt(rcull2) * rn * (1.0 + 1e-6) * kFixScale + 4.0;
+        lim[d] = (ok && m < 2147483000.0) ? (int)(2147483647.0 - m) : -1;
+    }
+}
+
+// The virial correction of a pair that crosses a periodic boundary (image m =
+// +-1 in the directions whose difference e = q_a - q_j wrapped) or that the
+// mass filter excludes; g the pair's force term.  False when there is none.
+__device__ __forceinline__ bool wrap_correction(double *v, const int4 &qa, const int4 &qj, int32_t ex, int32_t ey,
+                                                int32_t ez, bool excluded, double gx, double gy, double gz) {
+    // sign bit set: that difference wrapped
+    const int32_t wx = (qa.x ^ qj.x) & (qa.x ^ ex), wy = (qa.y ^ qj.y) & (qa.y ^ ey), wz = (qa.z ^ qj.z) & (qa.z ^ ez);
+    if ((wx | wy | wz) < 0 || excluded) {
+        // c = m 2^32 (the image), or q_a - q_j exactly when excluded
+        double cx = wx < 0 ? (qa.x >= 0 ? kFixScale : -kFixScale) : 0.0;
+        double cy = wy < 0 ? (qa.y >= 0 ? kFixScale : -kFixScale) : 0.0;
+        double cz = wz < 0 ? (qa.z >= 0 ? kFixScale : -kFixScale) : 0.0;
+        if (excluded) { cx += (double)ex; cy += (double)ey; cz += (double)ez; }
+        add_sym(v, cx, cy, cz, gx, gy, gz, -0.5);
+        return true;
+    }
+    return false;
+}
+
+// velocity Verlet second half of atom a (src/quench_m.F90:606-622), previous tgid
+__device__ __forceinline__ void second_half(const Params &p, const double *stg, int a, double ma,
+                                            const int32_t *__restrict__ znum, const double *__restrict__ del2,
+                                            double fxa, double fya, double fza, double *__restrict__ x1,
+                                            double *__restrict__ x2) {
+    const size_t nm = (size_t)p.nm;
+    double ux = x1[a], uy = x1[nm + a], uz = x1[2 * nm + a];
+    double wx = x2[a], wy = x2[nm + a], wz = x2[2 * nm + a];
+    double hx = ux + wx, hy = uy + wy, hz = uz + wz;
+    if (!(znum[a] == 0 || ma < 0.1)) {
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+        if (p.ivol == 0) {
+            s0 = stg[0] * ux + stg[3] * uy + stg[6] * uz;
+            s1 = stg[1] * ux + stg[4] * uy + stg[7] * uz;
+            s2 = stg[2] * ux + stg[5] * uy + stg[8] * uz;
+        }
+        if (p.ivol == 4) s2 = stg[8] * uz;
+        double d2 = del2[a];
+        wx = d2 * fxa - 0.5 * s0;
+        wy = d2 * fya - 0.5 * s1;
+        wz = d2 * fza - 0.5 * s2;
+        x2[a] = wx; x2[nm + a] = wy; x2[2 * nm + a] = wz;
+    }
+    x1[a] = hx + wx; x1[nm + a] = hy + wy; x1[2 * nm + a] = hz + wz;
+}
+
 // f_i = sum_j g_ij over the compact row, g_ij = d_ij fp_ij; pe and the
 // virial moment D = sum over pairs d d^T fp (tp = B0 D, pairs with
 // m_i + m_j <= 0.1 left out, src/dynamics_m.F90:287); mode 1 adds the
@@ -225,18 +295,7 @@ k_forces(Params p, Tables t, const double4 *__restrict__ pos2, const int4 *__res
     }
     __syncthreads();
     if (MIXED && threadIdx.x == 0) {
-        // a pair inside the cut spans at most M_d = rcull |row d of B0^-1|
-        // box lengths in direction d; an atom whose fixed-point coordinates
-        // all lie within 2^31 - M_d of zero has no pair whose 32-bit
-        // difference wraps (crosses a periodic boundary)
-        double bi[9];
-        const bool ok = mat_invert(sb, bi);
-        for (int d = 0; d < 3; ++d) {
-            const double rn = sqrt(MAT(bi, d + 1, 1) * MAT(bi, d + 1, 1) + MAT(bi, d + 1, 2) * MAT(bi, d + 1, 2) +
-                                   MAT(bi, d + 1, 3) * MAT(bi, d + 1, 3));
-            const double m = sqrt(t.rcull2) * rn * (1.0 + 1e-6) * kFixScale + 4.0;
-            slim[d] = (ok && m < 2147483000.0) ? (int)(2147483647.0 - m) : -1;
-        }
+        wrap_limits(sb, t.rcull2, slim);
     }
     __syncthreads();
     const int limx = slim[0], limy = slim[1], limz = slim[2];
@@ -311,18 +370,8 @@ k_forces(Params p, Tables t, const double4 *__restrict__ pos2, const int4 *__res
                         if (STRESS) { tx = fmaf(rx, fp, tx); ty = fmaf(ry, fp, ty); tz = fmaf(rz, fp, tz); }
                     }
                     if constexpr (CORR) {
-                        // sign bit set: that difference wrapped (a periodic image, m = +-1)
-                        const int32_t wx = (qa.x ^ qj.x) & (qa.x ^ ex), wy = (qa.y ^ qj.y) & (qa.y ^ ey),
-                                      wz = (qa.z ^ qj.z) & (qa.z ^ ez);
-                        const bool excluded = !(ma > 0.1 || ma + mass[j] > 0.1);
-                        if ((wx | wy | wz) < 0 || excluded) {
-                            // c = m 2^32 (the image), or q_a - q_j exactly when excluded
-                            double cx = wx < 0 ? (qa.x >= 0 ? kFixScale : -kFixScale) : 0.0;
-                            double cy = wy < 0 ? (qa.y >= 0 ? kFixScale : -kFixScale) : 0.0;
-                            double cz = wz < 0 ? (qa.z >= 0 ? kFixScale : -kFixScale) : 0.0;
-                            if (excluded) { cx += (double)ex; cy += (double)ey; cz += (double)ez; }
-                            add_sym(v, cx, cy, cz, (double)dfx, (double)dfy, (double)dfz, -0.5);
-                        }
+                        wrap_correction(v, qa, qj, ex, ey, ez, !(ma > 0.1 || ma + mass[j] > 0.1), (double)dfx,
+                                        (double)dfy, (double)dfz);
                     }
                 }
             }
@@ -379,25 +428,7 @@ k_forces(Params p, Tables t, const double4 *__restrict__ pos2, const int4 *__res
         f[a] = fxa; f[nm + a] = fya; f[2 * nm + a] = fza;
         if (STRESS) { stress[a] = sx; stress[nm + a] = sy; stress[2 * nm + a] = sz; }
         if (mode == 1) {
-            // velocity Verlet second half (src/quench_m.F90:606-622), previous tgid
-            double ux = x1[a], uy = x1[nm + a], uz = x1[2 * nm + a];
-            double wx = x2[a], wy = x2[nm + a], wz = x2[2 * nm + a];
-            double hx = ux + wx, hy = uy + wy, hz = uz + wz;
-            if (!(znum[a] == 0 || ma < 0.1)) {
-                double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-                if (p.ivol == 0) {
-                    s0 = stg[0] * ux + stg[3] * uy + stg[6] * uz;
-                    s1 = stg[1] * ux + stg[4] * uy + stg[7] * uz;
-                    s2 = stg[2] * ux + stg[5] * uy + stg[8] * uz;
-                }
-                if (p.ivol == 4) s2 = stg[8] * uz;
-                double d2 = del2[a];
-                wx = d2 * fxa - 0.5 * s0;
-                wy = d2 * fya - 0.5 * s1;
-                wz = d2 * fza - 0.5 * s2;
-                x2[a] = wx; x2[nm + a] = wy; x2[2 * nm + a] = wz;
-            }
-            x1[a] = hx + wx; x1[nm + a] = hy + wy; x1[2 * nm + a] = hz + wz;
+            second_half(p, stg, a, ma, znum, del2, fxa, fya, fza, x1, x2);
         }
     }
     if (MIXED) {   // the virial moments were summed in fixed-point units^2
@@ -406,6 +437,541 @@ k_forces(Params p, Tables t, const double4 *__restrict__ pos2, const int4 *__res
     }
     // v[1..6] is D; every directed pair entered half of it
     block_partials<7>(v, partials, 0);
+}
+
+// ------------------------------------- mixed passes of large systems --
+// The mixed passes above cost 103 (screening) and 124 (forces) warp
+// instructions per row entry: nested branches (entry valid, inside the
+// screening radius, inside the band, inside the table, room in the row), each
+// with its convergence bookkeeping, 64-bit index products, one FMA per
+// component, and table intervals fetched through L1 by 32 lanes from some 30
+// lines.  k_screen_st and k_forces_st do the same arithmetic, bit for bit per
+// pair and in the same order per atom, without branches: every entry of a
+// batch is evaluated, what does not count is not added or stored (predicates);
+// the FMAs of two entries go as one packed instruction (f32x2); the tables
+// sit in shared memory, one block of NT threads per SM.  The tables are loaded
+// before the wait for the previous kernel: they change between launches only.
+
+__device__ __forceinline__ unsigned long long pk2(float lo, float hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void up2(unsigned long long v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long v;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+
+// B0 per fixed-point unit; PACK: each element in both halves of a register
+// pair, for the packed FMAs (nine registers more, so not with 64 per thread)
+template <bool PACK>
+struct Box2 {
+    unsigned long long b[PACK ? 9 : 1];
+    float s[PACK ? 1 : 9];
+    __device__ __forceinline__ void set(int k, float v) {
+        if constexpr (PACK) b[k] = pk2(v, v);
+        else s[k] = v;
+    }
+};
+
+// fix_sep of two entries: the fixed-point differences (exact integers), their
+// FP32 values d and the squared distance, per entry the operations of fix_sep
+template <bool PACK>
+__device__ __forceinline__ void fix_sep2(const Box2<PACK> &B, const int4 &qa, const int4 &q0, const int4 &q1,
+                                         float (&dx)[2], float (&dy)[2], float (&dz)[2], float &r0, float &r1) {
+    dx[0] = fix_to_float((int32_t)((uint32_t)qa.x - (uint32_t)q0.x));
+    dx[1] = fix_to_float((int32_t)((uint32_t)qa.x - (uint32_t)q1.x));
+    dy[0] = fix_to_float((int32_t)((uint32_t)qa.y - (uint32_t)q0.y));
+    dy[1] = fix_to_float((int32_t)((uint32_t)qa.y - (uint32_t)q1.y));
+    dz[0] = fix_to_float((int32_t)((uint32_t)qa.z - (uint32_t)q0.z));
+    dz[1] = fix_to_float((int32_t)((uint32_t)qa.z - (uint32_t)q1.z));
+    if constexpr (PACK) {
+        const unsigned long long x = pk2(dx[0], dx[1]), y = pk2(dy[0], dy[1]), z = pk2(dz[0], dz[1]);
+        const unsigned long long rx = fma2(B.b[6], z, fma2(B.b[3], y, mul2(B.b[0], x)));
+        const unsigned long long ry = fma2(B.b[7], z, fma2(B.b[4], y, mul2(B.b[1], x)));
+        const unsigned long long rz = fma2(B.b[8], z, fma2(B.b[5], y, mul2(B.b[2], x)));
+        up2(fma2(rz, rz, fma2(ry, ry, mul2(rx, rx))), r0, r1);
+    } else {
+        float r[2];
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            const float rx = fmaf(B.s[6], dz[w], fmaf(B.s[3], dy[w], B.s[0] * dx[w]));
+            const float ry = fmaf(B.s[7], dz[w], fmaf(B.s[4], dy[w], B.s[1] * dx[w]));
+            const float rz = fmaf(B.s[8], dz[w], fmaf(B.s[5], dy[w], B.s[2] * dx[w]));
+            r[w] = fmaf(rz, rz, fmaf(ry, ry, rx * rx));
+        }
+        r0 = r[0]; r1 = r[1];
+    }
+}
+
+// Node interval and offset of r in the stored table; at and beyond the last
+// stored node, whose stored step is zero, that node (lookup_r4f's tail)
+__device__ __forceinline__ int interval(const Tables &t, float r, float &dr) {
+    const float x = fmaf(r, t.recipstep_f, t.xoff_f);
+    float fl;
+    const int idx = floor_small(fmaxf(x, 0.f), fl);
+    dr = x - fl;
+    return idx < t.nr - 1 ? idx : t.nr - 1;
+}
+
+// Half width of the band around the cut in which the FP64 distance decides,
+// for separations from fixed-point coordinates.  Against the FP64 distance of
+// the same positions such a separation is off by the rounding of two
+// coordinates to 2^-33 box lengths each (under 2^-31 |B0|_F in length), and by
+// the rounding of the conversion, of three products and two sums per
+// component and of the squared length, each under 2^-24 of |B0|_F |d| <=
+// |B0|_F |B0^-1|_F r: fewer than 16 of them.  (The band of the general pass,
+// 2e-6 |B0|_F + 1e-4 A, allows for FP32 positions; at 2 M atoms it holds a pair
+// of every row of a warp, 1.1e-3 against 1.1e-5 A.)
+__device__ float fix_band(const double *b, double rcut) {
+    double inv[9];
+    const double nb = frob(b);
+    if (!mat_invert(b, inv)) return 1.0e30f;
+    return (float)(4.7e-10 * nb + 16.0 * 6.0e-8 * nb * frob(inv) * rcut) * 1.01f;
+}
+
+template <int B, bool PF, int NT>
+__global__ void __launch_bounds__(NT, 1)
+k_screen_st(Params p, Tables t, const double4 *__restrict__ pos, const int4 *__restrict__ posq,
+            int4 *__restrict__ posq2, const BoxState *__restrict__ box, const int32_t *__restrict__ mlist,
+            const int32_t *__restrict__ mid_cnt, int32_t *__restrict__ alist, int32_t *__restrict__ pair_cnt,
+            double *__restrict__ rho, double *__restrict__ afrho, double *__restrict__ dafrho,
+            double *__restrict__ partials, int32_t *__restrict__ flags, int store_rho) {
+    extern __shared__ __align__(16) unsigned char dsm[];
+    float2 *sphi = reinterpret_cast<float2 *>(dsm);
+    for (int k = threadIdx.x; k < t.nr; k += NT) {
+        const float2 v = __ldg(&t.phi2f[k]);
+        sphi[k] = k < t.nr - 1 ? v : make_float2(t.tail_f.z, 0.f);
+    }
+    grid_dep_wait();   // launched dependent on the step's previous kernel
+    __shared__ double sb[9];
+    __shared__ float srs2, srin2;
+    if (threadIdx.x < 9) sb[threadIdx.x] = box->b0[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        // screen_radius2 tells whether the 32-bit difference is the image NINT
+        // picks for every pair inside the radius; else every pair goes to FP64
+        const float wide = screen_radius2(sb, t.rcull2);
+        const float rc = (float)sqrt(t.rcull2), d = fix_band(sb, sqrt(t.rcull2)) + 4.0e-7f * rc;
+        const bool ok = wide < 1e37f && d < 0.5f * rc;
+        srs2 = ok ? (rc + d) * (rc + d) : 3.0e38f;
+        srin2 = ok ? (rc - d) * (rc - d) : -1.f;
+    }
+    __syncthreads();
+    constexpr bool PACK = NT < 1024;
+    Box2<PACK> bx;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) bx.set(k, (float)(sb[k] * kFixUnit));
+    const float rscreen2 = srs2, rin2 = srin2;
+    double v[2] = {0.0, 0.0};   // embedding energy, directed pairs
+    const unsigned nm = (unsigned)p.nm, astride = gridDim.x * NT;
+    int over = 0, over_max = 0;
+    for (unsigned a = blockIdx.x * NT + threadIdx.x; a < nm; a += astride) {
+        if (PF && a + astride < nm) {   // next atom of this thread: its row and data into L2
+            const unsigned an = a + astride;
+#pragma unroll
+            for (unsigned u = 0; u < 16; ++u) prefetch_l2(&mlist[u * nm + an]);
+            prefetch_l2(&mid_cnt[an]);
+            prefetch_l2(&posq[an]);
+            prefetch_l2(&dafrho[an]);
+        }
+        const int mc = mid_cnt[a];
+        const int n = mc < p.mid_cap ? mc : p.mid_cap;
+        const int4 qa = posq[a];
+        double rho_a = 0.0;
+        int cnt = 0;
+        unsigned rd = a, wr = a;                       // next entry read, next entry written
+        for (int k0 = 0; k0 < n; k0 += B) {
+            int ee[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                ee[u] = k0 + u < n ? __ldg(&mlist[rd]) : (int)a;
+                rd += nm;
+            }
+            int4 qq[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) qq[u] = __ldg(&posq[ee[u] & kIdMask]);
+            float r2[B];
+            bool in[B], band = false;
+#pragma unroll
+            for (int u = 0; u < B; u += 2) {
+                float dx[2], dy[2], dz[2];
+                fix_sep2<PACK>(bx, qa, qq[u], qq[u + 1], dx, dy, dz, r2[u], r2[u + 1]);
+#pragma unroll
+                for (int w = u; w < u + 2; ++w) {
+                    in[w] = k0 + w < n && r2[w] <= rscreen2;
+                    band = band || (in[w] && !(r2[w] < rin2));
+                }
+            }
+            if (band) {                                // inside the error band: the FP64 distance decides
+#pragma unroll
+                for (int u = 0; u < B; ++u)
+                    if (in[u] && !(r2[u] < rin2))
+                        in[u] = inside_cut_fp64(pos, (int)a, ee[u] & kIdMask, sb, p.ivol, t.rcull2);
+            }
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                float dr;
+                const float2 q = sphi[interval(t, r2[u] * rsqrt_ftz(r2[u]), dr)];
+                const float ph = fmaf(q.y, dr, q.x);
+                if (in[u]) rho_a += (double)ph;
+                if (in[u] && cnt < p.pair_cap) alist[wr] = ee[u];
+                wr += in[u] ? nm : 0u;
+                cnt += in[u] ? 1 : 0;
+            }
+        }
+        pair_cnt[a] = cnt;
+        v[1] += (double)cnt;
+        if (cnt > p.pair_cap) { over = 1; over_max = max(over_max, cnt); }
+        if (mc > p.mid_cap) { over |= 2; over_max = max(over_max, mc); }
+        // embed (src/potential_m.F90:148-169): rho <= 1e-40 keeps the old values
+        double fd;
+        if (rho_a > 1e-40) {
+            const double2 e = lookup_e2(t, rho_a);
+            afrho[a] = e.x;
+            dafrho[a] = e.y;
+            fd = e.y;
+            v[0] += e.x;
+        } else {
+            fd = dafrho[a];
+        }
+        if (store_rho) rho[a] = rho_a;
+        posq2[a] = make_int4(qa.x, qa.y, qa.z, __float_as_int((float)fd));
+    }
+    if (over & 1) { atomicExch(&flags[3], 1); atomicMax(&flags[4], over_max); }
+    if (over & 2) { atomicExch(&flags[5], 1); atomicMax(&flags[6], over_max); }
+    block_partials<2>(v, partials, 0);
+}
+
+template <int B, bool PF, int NT>
+__global__ void __launch_bounds__(NT, 1)
+k_forces_st(Params p, Tables t, const int4 *__restrict__ posq2, const BoxState *__restrict__ box,
+            const int32_t *__restrict__ alist, const int32_t *__restrict__ pair_cnt, const double *__restrict__ mass,
+            const int32_t *__restrict__ znum, const double *__restrict__ del2, double *__restrict__ f,
+            double *__restrict__ x1, double *__restrict__ x2, double *__restrict__ partials, int mode) {
+    extern __shared__ __align__(16) unsigned char dsm[];
+    float4 *sdf = reinterpret_cast<float4 *>(dsm);                  // V', phi', their steps
+    float2 *sv = reinterpret_cast<float2 *>(sdf + t.nr);            // V, its step
+    for (int k = threadIdx.x; k < t.nr; k += NT) {
+        float4 lo, st;
+        ldg8f(&t.r4f[2 * k], lo, st);
+        if (k == t.nr - 1) { lo = t.tail_f; st = make_float4(0.f, 0.f, 0.f, 0.f); }
+        sdf[k] = make_float4(lo.y, lo.w, st.y, st.w);
+        sv[k] = make_float2(lo.x, st.x);
+    }
+    grid_dep_wait();   // launched dependent on the step's previous kernel
+    __shared__ double sb[9], stg[9];
+    __shared__ int slim[3];
+    if (threadIdx.x < 9) {
+        sb[threadIdx.x] = box->b0[threadIdx.x];
+        stg[threadIdx.x] = box->tgid[threadIdx.x];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) wrap_limits(sb, t.rcull2, slim);
+    __syncthreads();
+    const int limx = slim[0], limy = slim[1], limz = slim[2];
+    constexpr bool PACK = NT < 1024;
+    Box2<PACK> bx;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) bx.set(k, (float)(sb[k] * kFixUnit));
+    // the virial moments (one addition per atom, and the few corrections) are
+    // summed in shared memory, 12 registers less across the row
+    double *acc = reinterpret_cast<double *>(sv + ((t.nr + 1) & ~1)) + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) acc[k * NT] = 0.0;
+    double pe = 0.0;
+    const unsigned nm = (unsigned)p.nm, astride = gridDim.x * NT;
+    for (unsigned a = blockIdx.x * NT + threadIdx.x; a < nm; a += astride) {
+        if (PF && a + astride < nm) {
+            const unsigned an = a + astride;
+#pragma unroll
+            for (unsigned u = 0; u < 8; ++u) prefetch_l2(&alist[u * nm + an]);
+            prefetch_l2(&pair_cnt[an]); prefetch_l2(&posq2[an]); prefetch_l2(&mass[an]);
+            if (mode == 1) {
+                prefetch_l2(&x1[an]); prefetch_l2(&x1[(size_t)nm + an]); prefetch_l2(&x1[2 * (size_t)nm + an]);
+                prefetch_l2(&x2[an]); prefetch_l2(&x2[(size_t)nm + an]); prefetch_l2(&x2[2 * (size_t)nm + an]);
+                prefetch_l2(&del2[an]); prefetch_l2(&znum[an]);
+            }
+        }
+        int ne = pair_cnt[a];
+        ne = ne < p.pair_cap ? ne : p.pair_cap;
+        const double ma = mass[a];
+        const int4 qa = posq2[a];
+        const float fa = __int_as_float(qa.w);
+        double gx = 0.0, gy = 0.0, gz = 0.0;   // sum of g = d fp, fixed-point units
+        // CORR: the pairs that wrap or that the mass filter leaves out are
+        // corrected; a warp takes that path when one of its atoms lies near a
+        // face (wrap_limits) or has m <= 0.1
+        const bool slow = !(ma > 0.1) || qa.x > limx || qa.x < -limx || qa.y > limy || qa.y < -limy || qa.z > limz ||
+                          qa.z < -limz;
+        auto row = [&](auto corr) {
+            constexpr bool CORR = decltype(corr)::value;
+            unsigned rd = a;
+            for (int e0 = 0; e0 < ne; e0 += B) {
+                int ee[B];
+#pragma unroll
+                for (int u = 0; u < B; ++u) {
+                    ee[u] = e0 + u < ne ? alist[rd] : (int)a;
+                    rd += nm;
+                }
+                int4 qq[B];
+#pragma unroll
+                for (int u = 0; u < B; ++u) qq[u] = __ldg(&posq2[ee[u] & kIdMask]);
+#pragma unroll
+                for (int u = 0; u < B; u += 2) {
+                    float dx[2], dy[2], dz[2], r2[2], rr[2], fp[2];
+                    fix_sep2<PACK>(bx, qa, qq[u], qq[u + 1], dx, dy, dz, r2[0], r2[1]);
+#pragma unroll
+                    for (int w = 0; w < 2; ++w) {
+                        const bool live = e0 + u + w < ne;
+                        const float s = live ? r2[w] : 1.0f;
+                        rr[w] = rsqrt_ftz(s);
+                        float dr;
+                        const int idx = interval(t, s * rr[w], dr);
+                        const float4 q = sdf[idx];
+                        const float dvee = fmaf(q.z, dr, q.x), dphi = fmaf(q.w, dr, q.y);
+                        fp[w] = -(dvee + dphi * (fa + __int_as_float(qq[u + w].w))) * rr[w];
+                        if (live && (ee[u + w] & kOwnBit)) {   // the owner's copy carries the pair energy
+                            const float2 qv = sv[idx];
+                            pe += (double)fmaf(qv.y, dr, qv.x);
+                        }
+                        // an entry past the end is the atom itself: d = 0 and a finite fp add zero
+                    }
+#pragma unroll
+                    for (int w = 0; w < 2; ++w) {
+                        const float fx = dx[w] * fp[w], fy = dy[w] * fp[w], fz = dz[w] * fp[w];
+                        gx += (double)fx; gy += (double)fy; gz += (double)fz;
+                        if constexpr (CORR) {
+                            const int4 qj = qq[u + w];
+                            const int32_t ex = (int32_t)((uint32_t)qa.x - (uint32_t)qj.x);
+                            const int32_t ey = (int32_t)((uint32_t)qa.y - (uint32_t)qj.y);
+                            const int32_t ez = (int32_t)((uint32_t)qa.z - (uint32_t)qj.z);
+                            double c[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+                            if (wrap_correction(c, qa, qj, ex, ey, ez,
+                                                !(ma > 0.1 || ma + mass[ee[u + w] & kIdMask] > 0.1), (double)fx,
+                                                (double)fy, (double)fz))
+#pragma unroll
+                                for (int k = 0; k < 6; ++k) acc[k * NT] += c[k + 1];
+                        }
+                    }
+                }
+            }
+        };
+        if (__any_sync(__activemask(), slow)) row(std::true_type{});
+        else row(std::false_type{});
+        {
+            double c[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            add_sym(c, (double)qa.x, (double)qa.y, (double)qa.z, gx, gy, gz, 1.0);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) acc[k * NT] += c[k + 1];
+        }
+        const double fxa = gx * kFixUnit, fya = gy * kFixUnit, fza = gz * kFixUnit;
+        f[a] = fxa; f[(size_t)nm + a] = fya; f[2 * (size_t)nm + a] = fza;
+        if (mode == 1) second_half(p, stg, a, ma, znum, del2, fxa, fya, fza, x1, x2);
+    }
+    double v[7] = {pe};
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k + 1] = acc[k * NT] * (kFixUnit * kFixUnit);   // summed in fixed-point units^2
+    block_partials<7>(v, partials, 0);
+}
+
+// ------------------------------------------------- FP64 passes, lookup mode --
+// k_screen_density and k_forces took 170 and 200 warp instructions per row
+// entry in FP64: NINT three times per pair, a square root and a division, 64
+// bytes of table nodes interpolated for four functions, nested branches.  Here
+// NINT is evaluated only for pairs across a face, the root and its inverse
+// come from one reciprocal square root, an interval is one 32-byte load of
+// what the pair needs (V on the owner's copy alone), and entries that do not
+// count are predicated off.  432,000 atoms: see the variants' rule below.
+template <int B, bool PF, int MINB>
+__global__ void __launch_bounds__(256, MINB)
+k_screen_d(Params p, Tables t, const double4 *__restrict__ pos, double4 *__restrict__ pos2,
+           const BoxState *__restrict__ box, const int32_t *__restrict__ mlist, const int32_t *__restrict__ mid_cnt,
+           int32_t *__restrict__ alist, int32_t *__restrict__ pair_cnt, double *__restrict__ rho,
+           double *__restrict__ afrho, double *__restrict__ dafrho, double *__restrict__ partials,
+           int32_t *__restrict__ flags, int store_rho) {
+    grid_dep_wait();   // launched dependent on the step's previous kernel
+    __shared__ double sb[9];
+    if (threadIdx.x < 9) sb[threadIdx.x] = box->b0[threadIdx.x];
+    __syncthreads();
+    double b[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) b[k] = sb[k];
+    double v[2] = {0.0, 0.0};   // embedding energy, directed pairs
+    const int nm = p.nm;
+    const size_t stride = (size_t)nm;
+    const int astride = gridDim.x * blockDim.x;
+    int over = 0, over_max = 0;
+    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < nm; a += astride) {
+        if (PF && a + astride < nm) {   // next atom of this thread: its row and data into L2
+            const int an = a + astride;
+#pragma unroll
+            for (int u = 0; u < 16; ++u) prefetch_l2(&mlist[(size_t)u * stride + an]);
+            prefetch_l2(&mid_cnt[an]);
+            prefetch_l2(&pos[an]);
+            prefetch_l2(&dafrho[an]);
+        }
+        const int mc = mid_cnt[a];
+        const int n = mc < p.mid_cap ? mc : p.mid_cap;
+        const double4 pa = pos[a];
+        double rho_a = 0.0;
+        int cnt = 0;
+        const int32_t *rd = mlist + a;
+        int32_t *wr = alist + a;
+        for (int k0 = 0; k0 < n; k0 += B) {
+            int ee[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                ee[u] = k0 + u < n ? __ldg(rd) : a;
+                rd += stride;
+            }
+            double4 qq[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) qq[u] = ldg4(&pos[ee[u] & kIdMask]);
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                double dx = pa.x - qq[u].x, dy = pa.y - qq[u].y, dz = pa.z - qq[u].z;
+                if (outside_half(dx, dy, dz)) min_image(p.ivol, dx, dy, dz);
+                const double rx = b[0] * dx + b[3] * dy + b[6] * dz;
+                const double ry = b[1] * dx + b[4] * dy + b[7] * dz;
+                const double rz = b[2] * dx + b[5] * dy + b[8] * dz;
+                const double r2 = rx * rx + ry * ry + rz * rz;
+                const bool in = k0 + u < n && r2 <= t.rcull2;
+                double rr, dr;
+                const double r = root_and_inverse(in ? r2 : 1.0, rr);
+                const double2 q = __ldg(&t.dp2[interval_d(t, r, dr)]);
+                if (in) {
+                    rho_a += fma(q.y, dr, q.x);
+                    if (cnt < p.pair_cap) *wr = ee[u];
+                    wr += stride;
+                    ++cnt;
+                }
+            }
+        }
+        pair_cnt[a] = cnt;
+        v[1] += (double)cnt;
+        if (cnt > p.pair_cap) { over = 1; over_max = max(over_max, cnt); }
+        if (mc > p.mid_cap) { over |= 2; over_max = max(over_max, mc); }
+        // embed (src/potential_m.F90:148-169): rho <= 1e-40 keeps the old values
+        double fd;
+        if (rho_a > 1e-40) {
+            const double2 e = lookup_e2(t, rho_a);
+            afrho[a] = e.x;
+            dafrho[a] = e.y;
+            fd = e.y;
+            v[0] += e.x;
+        } else {
+            fd = dafrho[a];
+        }
+        if (store_rho) rho[a] = rho_a;
+        pos2[a] = make_double4(pa.x, pa.y, pa.z, fd);
+    }
+    if (over & 1) { atomicExch(&flags[3], 1); atomicMax(&flags[4], over_max); }
+    if (over & 2) { atomicExch(&flags[5], 1); atomicMax(&flags[6], over_max); }
+    block_partials<2>(v, partials, 0);
+}
+
+template <int B, bool PF, bool STRESS, int MINB>
+__global__ void __launch_bounds__(256, MINB)
+k_forces_d(Params p, Tables t, const double4 *__restrict__ pos2, const BoxState *__restrict__ box,
+           const int32_t *__restrict__ alist, const int32_t *__restrict__ pair_cnt, const double *__restrict__ mass,
+           const int32_t *__restrict__ znum, const double *__restrict__ del2, double *__restrict__ f,
+           double *__restrict__ x1, double *__restrict__ x2, double *__restrict__ stress,
+           double *__restrict__ partials, int mode) {
+    grid_dep_wait();   // launched dependent on the step's previous kernel
+    __shared__ double sb[9], stg[9];
+    if (threadIdx.x < 9) {
+        sb[threadIdx.x] = box->b0[threadIdx.x];
+        stg[threadIdx.x] = box->tgid[threadIdx.x];
+    }
+    __syncthreads();
+    double b[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) b[k] = sb[k];
+    double v[7];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) v[k] = 0.0;
+    const int nm = p.nm;
+    const size_t stride = (size_t)nm;
+    const int astride = gridDim.x * blockDim.x;
+    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < nm; a += astride) {
+        if (PF && a + astride < nm) {
+            const int an = a + astride;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) prefetch_l2(&alist[(size_t)u * nm + an]);
+            prefetch_l2(&pair_cnt[an]); prefetch_l2(&pos2[an]); prefetch_l2(&mass[an]);
+            if (mode == 1) {
+                prefetch_l2(&x1[an]); prefetch_l2(&x1[stride + an]); prefetch_l2(&x1[2 * stride + an]);
+                prefetch_l2(&x2[an]); prefetch_l2(&x2[stride + an]); prefetch_l2(&x2[2 * stride + an]);
+                prefetch_l2(&del2[an]); prefetch_l2(&znum[an]);
+            }
+        }
+        int ne = pair_cnt[a];
+        ne = ne < p.pair_cap ? ne : p.pair_cap;
+        const double ma = mass[a];
+        const double4 pa = pos2[a];
+        double fxa = 0.0, fya = 0.0, fza = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
+        const int32_t *rd = alist + a;
+        for (int e0 = 0; e0 < ne; e0 += B) {
+            int ee[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                ee[u] = e0 + u < ne ? *rd : a;
+                rd += stride;
+            }
+            double4 qq[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) qq[u] = ldg4(&pos2[ee[u] & kIdMask]);
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                const bool live = e0 + u < ne;
+                const double4 q = qq[u];
+                const double ux = pa.x - q.x, uy = pa.y - q.y, uz = pa.z - q.z;
+                double dx = ux, dy = uy, dz = uz;
+                // across a face, or left out by the mass filter: the virial's correction
+                const bool image = outside_half(ux, uy, uz), special = image || !(ma > 0.1);
+                if (image) min_image(p.ivol, dx, dy, dz);
+                const double rx = b[0] * dx + b[3] * dy + b[6] * dz;
+                const double ry = b[1] * dx + b[4] * dy + b[7] * dz;
+                const double rz = b[2] * dx + b[5] * dy + b[8] * dz;
+                const double r2 = rx * rx + ry * ry + rz * rz;
+                double rr, dr;
+                const double r = root_and_inverse(live ? r2 : 1.0, rr);
+                const int idx = interval_d(t, r, dr);
+                const double4 w = ldg4(&t.df4[idx]);
+                const double dvee = fma(w.z, dr, w.x), dphi = fma(w.w, dr, w.y);
+                const double fp = -dvee * rr - (dphi * pa.w + dphi * q.w) * rr;
+                const double gx = dx * fp, gy = dy * fp, gz = dz * fp;   // zero past the end (d = 0)
+                fxa += gx; fya += gy; fza += gz;
+                if (live && (ee[u] & kOwnBit)) {   // the owner's copy carries the pair energy
+                    const double2 qv = __ldg(&t.dv2[idx]);
+                    v[0] += fma(qv.y, dr, qv.x);
+                    if (STRESS) { sx += rx * fp; sy += ry * fp; sz += rz * fp; }
+                }
+                if (special && live) {
+                    const bool excluded = !(ma > 0.1 || ma + mass[ee[u] & kIdMask] > 0.1);
+                    const double mx = ux - dx, my = uy - dy, mz = uz - dz;   // the image (exact)
+                    if (mx != 0.0 || my != 0.0 || mz != 0.0 || excluded)
+                        // c = m, or x_a - x_j when excluded
+                        add_sym(v, excluded ? ux : mx, excluded ? uy : my, excluded ? uz : mz, gx, gy, gz, -0.5);
+                }
+            }
+        }
+        add_sym(v, pa.x, pa.y, pa.z, fxa, fya, fza, 1.0);
+        f[a] = fxa; f[stride + a] = fya; f[2 * stride + a] = fza;
+        if (STRESS) { stress[a] = sx; stress[stride + a] = sy; stress[2 * stride + a] = sz; }
+        if (mode == 1) second_half(p, stg, a, ma, znum, del2, fxa, fya, fza, x1, x2);
+    }
+    block_partials<7>(v, partials, 0);   // v[1..6] is D; every directed pair entered half of it
 }
 
 // ------------------------------------------------ outer and intermediate --
@@ -577,9 +1143,26 @@ void launch_mid_build(DeviceState &d, const Params &p, double rmid, double rout,
 // ------------------------------------------------------------ launchers --
 // Variant v (0..7): bit 0 selects the batch of list entries whose gathers are
 // issued before any is used (screen-density {4, 8}, forces {2, 4}); bit 1 adds
-// L2 prefetches of the next atom's rows and per-atom data; bit 2 asks for 3
-// resident blocks per SM instead of 2 (fewer registers per thread, more warps
-// to hide the gather latency).
+// L2 prefetches of the next atom's rows and per-atom data; bit 2 asks for 768
+// resident threads per SM instead of 512 (variants 0 and 1: 1024), fewer
+// registers each and more warps to hide the gather latency.
+//
+// The mixed passes of at least kStAtoms atoms in lookup mode keep their tables
+// in shared memory (ST: one block per SM); smaller systems, whose atoms would
+// fill few such blocks, tables above kStNodes nodes and the FP64 passes read
+// them through L1 with blocks of 256.
+constexpr int kStAtoms = 100000;
+constexpr int kStNodes = 6000;           // 24 bytes per node: 144 KB beside 48 bytes per thread
+
+constexpr size_t force_smem(int nodes, int nt) {
+    return (size_t)nodes * sizeof(float4) + (size_t)((nodes + 1) & ~1) * sizeof(float2) + (size_t)nt * 6 * sizeof(double);
+}
+
+static bool st_applies(const Params &p, const Tables &t) {
+    const long long cap = p.mid_cap > p.pair_cap ? p.mid_cap : p.pair_cap;
+    return p.nm >= kStAtoms && t.nr <= kStNodes && p.nm * (cap + 16) < (1LL << 32);   // 32-bit row offsets
+}
+
 template <int B, bool PF, int MINB>
 static int sd_variant(DeviceState &d, const Params &p, const Tables &t, bool mixed, double *partials,
                       int store_rho, cudaStream_t s) {
@@ -587,8 +1170,13 @@ static int sd_variant(DeviceState &d, const Params &p, const Tables &t, bool mix
                 d.rho, d.afrho, d.dafrho, partials, d.flags, store_rho
     int nb = grid_blocks(p.nm, 256);
     if (t.exact) LAUNCH_WAVE((k_screen_density<false, true, B, PF, MINB>), nb, s, SD_ARGS);
+    else if (mixed && st_applies(p, t))
+        LAUNCH_WAVE_SMEM((k_screen_st<B, PF, 256 * MINB>), 256 * MINB, (size_t)t.nr * sizeof(float2),
+                         kStNodes * sizeof(float2), nb, s, p, t, d.pos, d.posq, d.posq2, d.box, d.mlist, d.mid_cnt,
+                         d.alist, d.pair_cnt, d.rho, d.afrho, d.dafrho, partials, d.flags, store_rho);
     else if (mixed) LAUNCH_WAVE((k_screen_density<true, false, B, PF, MINB>), nb, s, SD_ARGS);
-    else LAUNCH_WAVE((k_screen_density<false, false, B, PF, MINB>), nb, s, SD_ARGS);
+    else LAUNCH_WAVE((k_screen_d<B, PF, MINB>), nb, s, p, t, d.pos, d.pos2, d.box, d.mlist, d.mid_cnt, d.alist,
+                     d.pair_cnt, d.rho, d.afrho, d.dafrho, partials, d.flags, store_rho);
 #undef SD_ARGS
     return nb;
 }
@@ -600,6 +1188,7 @@ static inline bool mixed_applies(const Params &p) { return p.ivol == 0 || p.ivol
 int launch_screen_density(DeviceState &d, const Params &p, const Tables &t, bool mixed, int variant,
                           double *partials, cudaStream_t s, bool store_rho) {
     mixed = mixed && mixed_applies(p);
+    if (variant < 0) variant = t.exact ? 1 : (mixed ? (st_applies(p, t) ? 6 : 7) : 6);
     switch (variant) {
     case 0: return sd_variant<4, true, 4>(d, p, t, mixed, partials, store_rho ? 1 : 0, s);
     case 1: return sd_variant<8, true, 4>(d, p, t, mixed, partials, store_rho ? 1 : 0, s);
@@ -619,8 +1208,13 @@ static int forces_variant(DeviceState &d, const Params &p, const Tables &t, bool
                    d.stress, partials, mode
     int nb = grid_blocks(p.nm, 256);
     if (t.exact) LAUNCH_WAVE((k_forces<false, true, B, PF, STRESS, MINB>), nb, s, FORCE_ARGS);
+    else if (mixed && !STRESS && st_applies(p, t))
+        LAUNCH_WAVE_SMEM((k_forces_st<B, PF, 256 * MINB>), 256 * MINB,
+                         force_smem(t.nr, 256 * MINB), force_smem(kStNodes, 256 * MINB), nb, s, p, t, d.posq2, d.box, d.alist, d.pair_cnt,
+                         d.mass, d.znum, d.del2, d.f, d.x1, d.x2, partials, mode);
     else if (mixed) LAUNCH_WAVE((k_forces<true, false, B, PF, STRESS, MINB>), nb, s, FORCE_ARGS);
-    else LAUNCH_WAVE((k_forces<false, false, B, PF, STRESS, MINB>), nb, s, FORCE_ARGS);
+    else LAUNCH_WAVE((k_forces_d<B, PF, STRESS, MINB>), nb, s, p, t, d.pos2, d.box, d.alist, d.pair_cnt, d.mass,
+                     d.znum, d.del2, d.f, d.x1, d.x2, d.stress, partials, mode);
 #undef FORCE_ARGS
     return nb;
 }
@@ -628,6 +1222,7 @@ static int forces_variant(DeviceState &d, const Params &p, const Tables &t, bool
 int launch_forces(DeviceState &d, const Params &p, const Tables &t, bool mixed, int mode,
                   int variant, double *partials, cudaStream_t s) {
     mixed = mixed && mixed_applies(p);
+    if (variant < 0) variant = t.exact ? 1 : (mixed ? 7 : 3);
     if (p.atomstress) return forces_variant<2, false, true, 2>(d, p, t, mixed, mode, partials, s);
     switch (variant) {
     case 0: return forces_variant<2, true, false, 4>(d, p, t, mixed, mode, partials, s);

@@ -104,4 +104,33 @@ static __device__ float keep_radius2(const double *sb, double r) {
     return screen_radius2(sb, r * r) > 1e37f ? 3.0e38f : keep * keep;
 }
 
+// ------------------------------------------------------- FP64 pair terms --
+// r = sqrt(r2) and 1/r of a positive r2 from one reciprocal square root: the
+// product r2 y is corrected by half its residual times y and then 1/r by its
+// own residual (one Newton step each), which leaves both within an ulp, in 6
+// operations where a square root and a division took two full routines.
+__device__ __forceinline__ double root_and_inverse(double r2, double &rr) {
+    const double y = rsqrt(r2);
+    double r = r2 * y;
+    r = fma(fma(-r, r, r2), 0.5 * y, r);
+    rr = fma(fma(-r, y, 1.0), y, y);
+    return r;
+}
+
+// Interval of r in the stored nodes and the offset in it; beyond the last
+// stored node, that node (its step is zero).  floor by a round-down addition.
+__device__ __forceinline__ int interval_d(const Tables &t, double r, double &dr) {
+    const double x = fma(r, t.vp_recipstep, t.vp_xoff);
+    const double b = __dadd_rd(fmin(fmax(x, 0.0), (double)(t.nr - 1)), 4503599627370496.0);   // + 2^52
+    dr = x - (b - 4503599627370496.0);
+    return __double2loint(b);
+}
+
+// The minimum image of min_image: u - NINT(u) in the periodic directions, m =
+// NINT(u).  Nearly every difference lies inside (-1/2, 1/2), where NINT is
+// zero: true when one does not (the caller's rare case).
+__device__ __forceinline__ bool outside_half(double ux, double uy, double uz) {
+    return !(fabs(ux) < 0.5 && fabs(uy) < 0.5 && fabs(uz) < 0.5);
+}
+
 }  // namespace moldy

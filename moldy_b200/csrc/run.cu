@@ -936,8 +936,15 @@ static void run_shape(int nm, int &lanes, int &threads, int &blocks) {
     blocks = (int)(nb < kRunBlocks ? nb : kRunBlocks);
 }
 
+// A run keeps one block of at most 512 threads per SM (its box algebra, list
+// builds and both pair pieces share the registers), the launched passes up to
+// 1024.  Against those passes (us per step, NPT, launched / run): mixed 54,000
+// atoms 45.7 / 31.0, 78,608 51.4 / 52.9, 128,000 69.6 / 54.9, 170,368 74.1 /
+// 76.2; FP64 54,000 51.7 / 42.7, 101,306 68.4 / 78.4.  So runs are taken while
+// every atom has a thread of its own, and in mixed precision, whose pair terms
+// are shorter, up to two atoms per thread.
 bool run_applies(const Params &p, const Tables &t, bool mixed) {
-    return p.nm <= kRunMaxAtoms && !t.exact && !p.atomstress && (p.ivol == 0 || p.ivol == 1 || p.ivol == 4) &&
+    return p.nm <= (mixed ? 2 : 1) * kRunBlocks * kRunThreads && !t.exact && !p.atomstress && (p.ivol == 0 || p.ivol == 1 || p.ivol == 4) &&
            run_smem(t, mixed) <= 200 * 1024;
 }
 
