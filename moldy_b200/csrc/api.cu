@@ -824,7 +824,7 @@ int Engine::velocityverlet(moldy_force_out *out) {
 
 int Engine::update_therm_avs(double *s123) {
     CHECK(check_ready());
-    LAUNCH(*this, K_THERM, 3, stream_, launch_therm(d, prm, true, nullptr, stream_));   // prep, sums, finish
+    LAUNCH(*this, K_THERM, 2, stream_, launch_therm(d, prm, true, nullptr, stream_));   // prep, sums
     if (!host_box_) {
         CUDA_CHECK(cudaMallocHost((void **)&host_box_, sizeof(BoxState) * 4), "pinned staging");
         host_box_cap_ = 4;
@@ -905,6 +905,15 @@ int Engine::queue_run(int m, bool therm, double *rec, int rec0, bool last, bool 
     return MOLDY_OK;
 }
 
+// update_therm_avs of a step whose sums the next drift does not take, and the
+// scalev that ends it; the scaling of x1 is left to the next drift unless the
+// step is the call's last
+void Engine::finish_step(bool scalev, bool last, double *rec) {
+    LAUNCH(*this, K_THERM, 1, stream_, launch_therm(d, prm, false, rec, stream_, scalev));
+    if (scalev)
+        LAUNCH(*this, K_SCALEV, last ? 2 : 1, stream_, launch_scalev(d, prm, nose_, rqke_, false, last, stream_));
+}
+
 int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
     CHECK(check_ready());
     if (nsteps < 0) return fail(MOLDY_ERR_INVALID, "nsteps < 0");
@@ -929,6 +938,7 @@ int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
     // deferred into the drift kernel of step k + 1, which reads both anyway,
     // and finished by the k_mid_decide that follows it.
     bool therm_pending = false;
+    bool scale_pending = false;   // the next drift scales x1 for the scalev that ended its step
     // An ordinary step (the thermo sums of the step before deferred into its
     // drift, no half-list build or relink, no scalev, not the last step) makes
     // the same launches with the same arguments throughout a call: it is
@@ -944,7 +954,7 @@ int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
         bool rb = false;
         // consecutive steps of a small system that need no half-list build, up
         // to and including one that is followed by a relink or scalev: one launch
-        const int run = run_applies(prm, tab, mixed) ? run_length(nsteps - k) : 0;
+        const int run = !scale_pending && run_applies(prm, tab, mixed) ? run_length(nsteps - k) : 0;
         if (run >= 2) {
             CHECK(ensure_active_capacity(0));
             bool scalev = false;
@@ -954,11 +964,9 @@ int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
             k += run - 1;
             rec_synced = false;
             therm_pending = !(scalev || k == nsteps - 1);
-            if (!therm_pending)
-                LAUNCH(*this, K_THERM, 2, stream_,
-                       launch_therm(d, prm, false, thermo ? d.thermo_rec + (size_t)kThermoRec * k : nullptr, stream_));
+            if (!therm_pending) finish_step(scalev, k == nsteps - 1, thermo ? d.thermo_rec + (size_t)kThermoRec * k : nullptr);
+            scale_pending = scalev && k < nsteps - 1;
             if (ntc_ == 0) LAUNCH(*this, K_RELINK, 6, stream_, launch_relink(d, prm, stream_));
-            if (scalev) LAUNCH(*this, K_SCALEV, 4, stream_, launch_scalev(d, prm, nose_, rqke_, stream_));
             continue;
         }
         {
@@ -1040,7 +1048,7 @@ int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
         }
         LAUNCH(*this, K_DRIFT, 1, stream_,
                kin_blocks = launch_drift(d, prm, d.partials + 2 * (size_t)kMaxBlocks * kPartials, therm_pending,
-                                         stream_));
+                                         stream_, scale_pending));
         if (therm_pending) {
             therm_blocks = kin_blocks;
             therm_rec = thermo ? d.thermo_rec + (size_t)kThermoRec * (k - 1) : nullptr;
@@ -1058,11 +1066,9 @@ int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
         ntcs[k] = ntc_;
         rbs[k] = rb ? 1 : 0;
         therm_pending = !(scalev || k == nsteps - 1);
-        if (!therm_pending)
-            LAUNCH(*this, K_THERM, 2, stream_,
-                   launch_therm(d, prm, false, thermo ? d.thermo_rec + (size_t)kThermoRec * k : nullptr, stream_));
+        if (!therm_pending) finish_step(scalev, k == nsteps - 1, thermo ? d.thermo_rec + (size_t)kThermoRec * k : nullptr);
+        scale_pending = scalev && k < nsteps - 1;
         if (ntc_ == 0) LAUNCH(*this, K_RELINK, 6, stream_, launch_relink(d, prm, stream_));
-        if (scalev) LAUNCH(*this, K_SCALEV, 4, stream_, launch_scalev(d, prm, nose_, rqke_, stream_));
     }
     if (step_graph) cudaGraphExecDestroy(step_graph);
     CUDA_CHECK(cudaGetLastError(), "md_steps launch");
@@ -1257,7 +1263,7 @@ int Engine::get_thermostat(double *out4) {
 // one scalev call (src/thermostat_m.F90:317-395), whatever the timer
 int Engine::scalev() {
     CHECK(check_ready());
-    if (nose_ > 0.0) LAUNCH(*this, K_SCALEV, 4, stream_, launch_scalev(d, prm, nose_, rqke_, stream_));
+    if (nose_ > 0.0) LAUNCH(*this, K_SCALEV, 3, stream_, launch_scalev(d, prm, nose_, rqke_, true, true, stream_));
     CUDA_CHECK(cudaStreamSynchronize(stream_), "scalev");
     CUDA_CHECK(cudaGetLastError(), "scalev");
     return MOLDY_OK;

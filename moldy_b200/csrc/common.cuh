@@ -24,6 +24,7 @@ struct BoxState {
     double npairs;                 // directed interacting pairs in the last density pass
     double bbuild[9];              // B0 when the intermediate list was built
     double snhv, snhf, scalev_ke;  // Nose-Hoover scaling state of scalev and its last KE
+    double sc_mean[3];             // the mean of x1 that its scaling removes
     double th_tgid[9], th_cof[9];  // tg^-1 tgdot and cof(B0)/vol of the box k_therm sees
     double bout[9];                // B0 when the outer list was built
     double dmax_mid, dmax_out;     // rnear |B_build^-1|_F of those builds (0: none)

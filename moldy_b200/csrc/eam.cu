@@ -93,14 +93,20 @@ __global__ void k_therm_prep(Params p, BoxState *__restrict__ box) {
     therm_prep(p, b0, b1, *box);
 }
 
-// Every block's three partial sums of update_therm_avs, in block order, and
-// the quantities derived from them (one block)
-__global__ void __launch_bounds__(256)
-k_therm_finish(Params p, BoxState *__restrict__ box, const double *__restrict__ partials, int nblk,
-               double *__restrict__ rec) {
-    __shared__ double s3[3];
-    reduce_partials<3>(partials, nblk, s3);
-    if (threadIdx.x == 0) therm_store(p, *box, s3, rec);
+// True in every thread of the block that finishes last of the grid, once the
+// partials of all blocks are visible to it; the ticket is left at zero for the
+// next launch.
+__device__ __forceinline__ bool last_block(int32_t *ticket) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+        if (last) *ticket = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last != 0;
 }
 
 // ------------------------------------------------ intermediate-list check --
@@ -156,10 +162,14 @@ void launch_set_rec_step(DeviceState &d, int step, cudaStream_t s) { k_set_rec_s
 // box has not yet moved, and the grid is k_therm's, so the sums are k_therm's
 // to the last bit.  The block partials go to therm_partials; k_mid_decide,
 // which runs next, finishes them.
-template <bool THERM>
+//
+// SCALE: the scalev that ended the previous step left its mean and scaling in
+// the box; x1 = (x1 - mean) (1 + snhv) of the movable atoms is formed and stored
+// here, as k_scalev_scale would have.
+template <bool THERM, bool SCALE>
 __global__ void __launch_bounds__(256, 4)   // the grid is 4 blocks per SM (stream_blocks): one wave
 k_drift(Params p, double4 *__restrict__ pos, int4 *__restrict__ posq,
-        const double *__restrict__ x1, const double *__restrict__ x2, BoxState *__restrict__ box,
+        double *__restrict__ x1, const double *__restrict__ x2, BoxState *__restrict__ box,
         const int4 *__restrict__ xbuild, const double *__restrict__ mass, const int32_t *__restrict__ znum,
         double *__restrict__ kin_partials, double *__restrict__ therm_partials) {
     grid_dep_wait();   // launched dependent on the step's previous kernel
@@ -171,6 +181,9 @@ k_drift(Params p, double4 *__restrict__ pos, int4 *__restrict__ posq,
         sh[9 + threadIdx.x] = box->b0[threadIdx.x];
         sh[18 + threadIdx.x] = box->th_cof[threadIdx.x];
     }
+    __shared__ double scale[SCALE ? 4 : 1];
+    if (SCALE && threadIdx.x >= 32 && threadIdx.x < 36)
+        scale[threadIdx.x - 32] = threadIdx.x < 35 ? box->sc_mean[threadIdx.x - 32] : 1.0 + box->snhv;
     if (threadIdx.x == 0) {
         const BoxState &B = *box;
         double b1[9], b0[9];
@@ -191,9 +204,13 @@ k_drift(Params p, double4 *__restrict__ pos, int4 *__restrict__ posq,
     double vt[3] = {0.0, 0.0, 0.0};
     const int nm = p.nm;
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < nm; a += gridDim.x * blockDim.x) {
-        const double ex = x1[a], ey = x1[nm + a], ez = x1[2 * nm + a];
+        double ex = x1[a], ey = x1[nm + a], ez = x1[2 * nm + a];
         const double wx = x2[a], wy = x2[nm + a], wz = x2[2 * nm + a];
-    double4 q = pos[a];
+        double4 q = pos[a];
+        if (SCALE && !(znum[a] == 0 || mass[a] < 0.1)) {
+            ex = (ex - scale[0]) * scale[3]; ey = (ey - scale[1]) * scale[3]; ez = (ez - scale[2]) * scale[3];
+            x1[a] = ex; x1[nm + a] = ey; x1[2 * nm + a] = ez;
+        }
         q.x = q.x + (ex + wx);
         q.y = q.y + (ey + wy);
         q.z = q.z + (ez + wz);
@@ -227,14 +244,12 @@ k_drift(Params p, double4 *__restrict__ pos, int4 *__restrict__ posq,
     // here can read a box another block has already moved
 }
 
-int launch_drift(DeviceState &d, const Params &p, double *kin_partials, bool therm, cudaStream_t s) {
+int launch_drift(DeviceState &d, const Params &p, double *kin_partials, bool therm, cudaStream_t s, bool scale) {
     int nb = stream_blocks(p.nm);
-    if (therm)
-        launch_pdl(k_drift<true>, nb, kAtomThreads, 0, s, p, d.pos, d.posq, d.x1, d.x2, d.box, d.xbuild, d.mass, d.znum,
-                                                  kin_partials, d.partials);
-    else
-        launch_pdl(k_drift<false>, nb, kAtomThreads, 0, s, p, d.pos, d.posq, d.x1, d.x2, d.box, d.xbuild, d.mass, d.znum,
-                                                   kin_partials, nullptr);
+    // a step that scalev ended has taken its thermo sums already
+    auto k = therm ? k_drift<true, false> : (scale ? k_drift<false, true> : k_drift<false, false>);
+    launch_pdl(k, nb, kAtomThreads, 0, s, p, d.pos, d.posq, d.x1, d.x2, d.box, d.xbuild, d.mass, d.znum, kin_partials,
+               therm ? d.partials : nullptr);
     return nb;
 }
 
@@ -263,12 +278,16 @@ void launch_md_init_x2(DeviceState &d, const Params &p, cudaStream_t s) {
 }
 
 // update_therm_avs over the atoms with a species, after a force evaluation
-// (therm_prep has left tgid and cof(B0)/vol in the box state); block partials
-// only, finished by k_therm_finish
-__global__ void __launch_bounds__(256)
+// (therm_prep has left tgid and cof(B0)/vol in the box state).  MEAN: also the
+// mean of x1 over all atoms, for the scalev that follows.  The last block to
+// finish sums the block partials in order and stores what follows from them.
+template <bool MEAN>
+__global__ void __launch_bounds__(256, 4)
 k_therm(Params p, BoxState *__restrict__ box, const double *__restrict__ x1,
         const double *__restrict__ x2, const double *__restrict__ mass,
-        const int32_t *__restrict__ znum, double *__restrict__ partials) {
+        const int32_t *__restrict__ znum, double *__restrict__ partials, double *__restrict__ rec,
+        int32_t *__restrict__ ticket) {
+    grid_dep_wait();   // launched dependent on the step's previous kernel
     __shared__ double sh[9 + 9 + 9];   // tgid, b0, cof(b0)/vol
     if (threadIdx.x < 9) {
         sh[threadIdx.x] = box->th_tgid[threadIdx.x];
@@ -276,7 +295,7 @@ k_therm(Params p, BoxState *__restrict__ box, const double *__restrict__ x1,
         sh[18 + threadIdx.x] = box->th_cof[threadIdx.x];
     }
     __syncthreads();
-    double v[3] = {0.0, 0.0, 0.0};
+    double v[3] = {0.0, 0.0, 0.0}, m[3] = {0.0, 0.0, 0.0};
     const int nm = p.nm;
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < nm; a += gridDim.x * blockDim.x) {
         // every load issued before the species test, so none waits on it
@@ -284,19 +303,29 @@ k_therm(Params p, BoxState *__restrict__ box, const double *__restrict__ x1,
         const double ux = x1[a], uy = x1[nm + a], uz = x1[2 * nm + a];
         const double wx = x2[a], wy = x2[nm + a], wz = x2[2 * nm + a];
         const double ma = mass[a];
+        if (MEAN) { m[0] += ux; m[1] += uy; m[2] += uz; }
         if (z == 0) continue;
         therm_terms(v, sh, sh + 9, sh + 18, ma, ux, uy, uz, wx, wy, wz);
     }
     block_partials<3>(v, partials, 0);
+    if (MEAN) block_partials<3>(m, partials, 3);
+    if (!last_block(ticket)) return;
+    __shared__ double s3[MEAN ? 6 : 3];
+    reduce_partials<MEAN ? 6 : 3, true>(partials, gridDim.x, s3);
+    if (threadIdx.x == 0) {
+        therm_store(p, *box, s3, rec);
+        if (MEAN)
+            for (int k = 0; k < 3; ++k) box->sc_mean[k] = s3[3 + k] / (double)(float)nm;   // float(nm): default REAL
+    }
 }
 
 // prep: compute the box quantities first (the call does not follow a force
-// evaluation that left them)
-int launch_therm(DeviceState &d, const Params &p, bool prep, double *rec, cudaStream_t s) {
+// evaluation that left them); mean: for a scalev that follows
+int launch_therm(DeviceState &d, const Params &p, bool prep, double *rec, cudaStream_t s, bool mean) {
     if (prep) k_therm_prep<<<1, 1, 0, s>>>(p, d.box);
     int nblocks = stream_blocks(p.nm);
-    k_therm<<<nblocks, kAtomThreads, 0, s>>>(p, d.box, d.x1, d.x2, d.mass, d.znum, d.partials);
-    k_therm_finish<<<1, kAtomThreads, 0, s>>>(p, d.box, d.partials, nblocks, rec);
+    launch_pdl(mean ? k_therm<true> : k_therm<false>, nblocks, kAtomThreads, 0, s, p, d.box, d.x1, d.x2, d.mass, d.znum,
+               d.partials, rec, d.flags + 14);
     return nblocks;
 }
 
@@ -305,43 +334,55 @@ int launch_therm(DeviceState &d, const Params &p, bool prep, double *rec, cudaSt
 // remove the mean of x1 (over all atoms) from the movable atoms, measure their
 // kinetic energy, update snhv -= (ke - rqke) / (nose nm) and scale their x1
 // by 1 + snhv.  Atoms with Z = 0 or mass < 0.1 are not movable.
-__global__ void __launch_bounds__(256)
-k_scalev_mean(int nm, const double *__restrict__ x1, double *__restrict__ partials) {
+//
+// In an MD step the mean comes with the thermo sums (k_therm), k_scalev_ke
+// measures the energy without writing x1, its last block updates snhv, and the
+// next step's drift, which streams x1 anyway, removes the mean and scales: two
+// passes over x1 and three launches fewer than mean, removal, finish and
+// scaling one after the other (1,024,000 atoms: 84 us per step with the thermo
+// sums, of which 35 us for every block of the removal pass summing 1,184
+// blocks' partials).
+__global__ void __launch_bounds__(256, 4)
+k_scalev_mean(int nm, BoxState *__restrict__ box, const double *__restrict__ x1, double *__restrict__ partials,
+              int32_t *__restrict__ ticket) {
     double v[3] = {0.0, 0.0, 0.0};
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < nm; a += gridDim.x * blockDim.x) {
         v[0] += x1[a]; v[1] += x1[nm + a]; v[2] += x1[2 * nm + a];
     }
     block_partials<3>(v, partials, 0);
+    if (!last_block(ticket)) return;
+    __shared__ double s[3];
+    reduce_partials<3, true>(partials, gridDim.x, s);
+    if (threadIdx.x < 3) box->sc_mean[threadIdx.x] = s[threadIdx.x] / (double)(float)nm;
 }
 
-__global__ void __launch_bounds__(256)
-k_scalev_ke(Params p, const BoxState *__restrict__ box, const double *__restrict__ mean_part, int nblk,
-            double *__restrict__ x1, const double *__restrict__ mass, const int32_t *__restrict__ znum,
-            double *__restrict__ partials) {
-    __shared__ double s[3];
-    reduce_partials<3>(mean_part, nblk, s);
+__global__ void __launch_bounds__(256, 4)
+k_scalev_ke(Params p, BoxState *__restrict__ box, const double *__restrict__ x1, const double *__restrict__ mass,
+            const int32_t *__restrict__ znum, double *__restrict__ partials, double nose, double rqke,
+            int32_t *__restrict__ ticket) {
+    grid_dep_wait();   // launched dependent on the step's previous kernel
+    __shared__ double sh[12];   // B0, the mean
+    if (threadIdx.x < 9) sh[threadIdx.x] = box->b0[threadIdx.x];
+    else if (threadIdx.x < 12) sh[threadIdx.x] = box->sc_mean[threadIdx.x - 9];
+    __syncthreads();
     const int nm = p.nm;
-    const double fnm = (double)(float)nm;      // float(nm): default REAL
-    const double sx = s[0] / fnm, sy = s[1] / fnm, sz = s[2] / fnm;
-    const double *b = box->b0;
+    const double *b = sh;
+    const double sx = sh[9], sy = sh[10], sz = sh[11];
     double v[1] = {0.0};
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < nm; a += gridDim.x * blockDim.x) {
-        if (znum[a] == 0 || mass[a] < 0.1) continue;
-        double ux = x1[a] - sx, uy = x1[nm + a] - sy, uz = x1[2 * nm + a] - sz;
-        x1[a] = ux; x1[nm + a] = uy; x1[2 * nm + a] = uz;
-        double rx = b[0] * ux + b[3] * uy + b[6] * uz;
-        double ry = b[1] * ux + b[4] * uy + b[7] * uz;
-        double rz = b[2] * ux + b[5] * uy + b[8] * uz;
-        v[0] += mass[a] * (rx * rx + ry * ry + rz * rz);
+        const int z = znum[a];
+        const double ma = mass[a];
+        const double ux = x1[a] - sx, uy = x1[nm + a] - sy, uz = x1[2 * nm + a] - sz;
+        if (z == 0 || ma < 0.1) continue;
+        const double rx = b[0] * ux + b[3] * uy + b[6] * uz;
+        const double ry = b[1] * ux + b[4] * uy + b[7] * uz;
+        const double rz = b[2] * ux + b[5] * uy + b[8] * uz;
+        v[0] += ma * (rx * rx + ry * ry + rz * rz);
     }
     block_partials<1>(v, partials, 0);
-}
-
-__global__ void __launch_bounds__(256)
-k_scalev_finish(Params p, BoxState *__restrict__ box, const double *__restrict__ partials, int nblk, double nose,
-                double rqke) {
+    if (!last_block(ticket)) return;
     __shared__ double s[1];
-    reduce_partials<1>(partials, nblk, s);
+    reduce_partials<1, true>(partials, gridDim.x, s);
     if (threadIdx.x != 0) return;
     BoxState &B = *box;
     double ke = s[0] / (p.deltat * p.deltat) / 2.0;
@@ -354,20 +395,23 @@ k_scalev_finish(Params p, BoxState *__restrict__ box, const double *__restrict__
 __global__ void __launch_bounds__(256)
 k_scalev_scale(int nm, const BoxState *__restrict__ box, double *__restrict__ x1, const double *__restrict__ mass,
                const int32_t *__restrict__ znum) {
-    const double f = 1.0 + box->snhv;
+    const double f = 1.0 + box->snhv, sx = box->sc_mean[0], sy = box->sc_mean[1], sz = box->sc_mean[2];
     for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < nm; a += gridDim.x * blockDim.x) {
         if (znum[a] == 0 || mass[a] < 0.1) continue;
-        x1[a] = x1[a] * f; x1[nm + a] = x1[nm + a] * f; x1[2 * nm + a] = x1[2 * nm + a] * f;
+        x1[a] = (x1[a] - sx) * f;
+        x1[nm + a] = (x1[nm + a] - sy) * f;
+        x1[2 * nm + a] = (x1[2 * nm + a] - sz) * f;
     }
 }
 
-void launch_scalev(DeviceState &d, const Params &p, double nose, double rqke, cudaStream_t s) {
-    const int nb = grid_blocks(p.nm, kAtomThreads);
-    double *mean_part = d.partials, *ke_part = d.partials + (size_t)kMaxBlocks * kPartials;
-    k_scalev_mean<<<nb, kAtomThreads, 0, s>>>(p.nm, d.x1, mean_part);
-    k_scalev_ke<<<nb, kAtomThreads, 0, s>>>(p, d.box, mean_part, nb, d.x1, d.mass, d.znum, ke_part);
-    k_scalev_finish<<<1, kAtomThreads, 0, s>>>(p, d.box, ke_part, nb, nose, rqke);
-    k_scalev_scale<<<nb, kAtomThreads, 0, s>>>(p.nm, d.box, d.x1, d.mass, d.znum);
+// mean: the mean is not in the box yet; scale: scale x1 now (else the next
+// drift does)
+void launch_scalev(DeviceState &d, const Params &p, double nose, double rqke, bool mean, bool scale, cudaStream_t s) {
+    const int nb = stream_blocks(p.nm);
+    double *part = d.partials + (size_t)kMaxBlocks * kPartials;
+    if (mean) k_scalev_mean<<<nb, kAtomThreads, 0, s>>>(p.nm, d.box, d.x1, part, d.flags + 15);
+    launch_pdl(k_scalev_ke, nb, kAtomThreads, 0, s, p, d.box, d.x1, d.mass, d.znum, part, nose, rqke, d.flags + 15);
+    if (scale) k_scalev_scale<<<nb, kAtomThreads, 0, s>>>(p.nm, d.box, d.x1, d.mass, d.znum);
 }
 
 // ------------------------------------------------------------ energy_calc --

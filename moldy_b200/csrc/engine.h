@@ -85,7 +85,8 @@ struct DeviceState {
                                   // [8] outer-row overflow, [9] its count,
                                   // [10] reverse half-row overflow, [11] its count,
                                   // [12] a link cell too full for the reverse-row masks,
-                                  // [13] a grid barrier of a fused run gave up waiting
+                                  // [13] a grid barrier of a fused run gave up waiting,
+                                  // [14], [15] tickets of the thermo and scalev sums (zero between launches)
     // per (cell rank r of the half stencil, round of 32 home atoms, atom j):
     // the home atoms of j's source cell whose half-list rows hold j (one bit
     // per home atom of the round), written by the half-list build
@@ -228,6 +229,7 @@ class Engine {
     int force_device(bool *rebuilt);     // queue force on the stream
     int fetch_force_out(moldy_force_out *out);
     int check_flags();
+    void finish_step(bool scalev, bool last, double *rec);
     int run_length(int left) const;
     int queue_run(int m, bool therm, double *rec, int rec0, bool last, bool &scalev, int *ntcs);
 
@@ -327,7 +329,9 @@ void launch_finalize_force(DeviceState &d, const Params &p, const double *part_e
                            int mode, cudaStream_t s);
 // therm: also take the update_therm_avs of the step that ended with the last
 // force evaluation (x1 and x2 unchanged since)
-int launch_drift(DeviceState &d, const Params &p, double *kin_partials, bool therm, cudaStream_t s);
+// scale: scale x1 for the scalev that ended the step before
+int launch_drift(DeviceState &d, const Params &p, double *kin_partials, bool therm, cudaStream_t s,
+                 bool scale = false);
 int launch_kinetic(DeviceState &d, const Params &p, double *partials, cudaStream_t s);
 // therm_nblk > 0: finish the drift kernel's deferred update_therm_avs first
 // rec_indexed: rec is the first thermo record and the box's rec_step says
@@ -355,12 +359,12 @@ void launch_md_init_x2(DeviceState &d, const Params &p, cudaStream_t s);
 // update_therm_avs with the thermo finalization in its last block; prep
 // when the call does not directly follow a force evaluation
 // rec: where the step's thermo record goes (kThermoRec doubles, device; may be null)
-int launch_therm(DeviceState &d, const Params &p, bool prep, double *rec, cudaStream_t s);
+int launch_therm(DeviceState &d, const Params &p, bool prep, double *rec, cudaStream_t s, bool mean = false);
 constexpr int kThermoRec = 11;
 constexpr int kRevRounds = 3;                  // rounds of 32 home atoms the reverse-row masks cover
 constexpr int kRevPlanes = 14 * kRevRounds;
 void launch_energy_calc(DeviceState &d, const Params &p, const Tables &t, cudaStream_t s);
-void launch_scalev(DeviceState &d, const Params &p, double nose, double rqke, cudaStream_t s);
+void launch_scalev(DeviceState &d, const Params &p, double nose, double rqke, bool mean, bool scale, cudaStream_t s);
 void launch_count_screened(const DeviceState &d, const Params &p, unsigned long long *out, cudaStream_t s);
 size_t adjoint_smem_bytes(int nlookup);
 void launch_table_adjoint(const DeviceState &d, const AdjointArgs &a, double *grads, double *scr,

@@ -1001,34 +1001,38 @@ k_forces_d(Params p, Tables t, const double4 *__restrict__ pos2, const BoxState 
 // Appends to atom a's row (entries kept in [cnt, cap), entry-major with
 // stride nm) the entries of one source row (n entries, entry k at
 // row[k * step]) whose FP32 distance is within keep2; own = bit 31 to set on
-// the kept entries.
+// the kept entries.  Every entry of a batch is evaluated and what is not kept
+// is not stored (predicates, no branches).
 template <bool FIX, int B>
 __device__ __forceinline__ int filter_row(const Params &p, const int32_t *__restrict__ row, size_t step, int n,
                                           int a, const double4 &pa, const int4 &qa, const double4 *__restrict__ pos,
                                           const int4 *__restrict__ posq, const float *bf, float keep2,
                                           int32_t own, int32_t *__restrict__ dst, int cap, int cnt) {
     const size_t stride = (size_t)p.nm;
+    int32_t *wr = dst + (size_t)cnt * stride + a;
     for (int k0 = 0; k0 < n; k0 += B) {
         int ee[B];
 #pragma unroll
-        for (int u = 0; u < B; ++u) ee[u] = (k0 + u < n) ? __ldg(&row[(size_t)(k0 + u) * step]) : -1;
+        for (int u = 0; u < B; ++u) {
+            ee[u] = k0 + u < n ? __ldg(row) : a;
+            row += step;
+        }
         double4 qq[FIX ? 1 : B];
         int4 qi[FIX ? B : 1];
 #pragma unroll
         for (int u = 0; u < B; ++u) {
-            const int j = ee[u] != -1 ? (ee[u] & kIdMask) : a;
-            if (FIX) qi[u] = __ldg(&posq[j]);
-            else qq[u] = ldg4(&pos[j]);
+            if (FIX) qi[u] = __ldg(&posq[ee[u] & kIdMask]);
+            else qq[u] = ldg4(&pos[ee[u] & kIdMask]);
         }
 #pragma unroll
         for (int u = 0; u < B; ++u) {
-            if (ee[u] == -1) continue;
             float rx, ry, rz;
             const float r2 = FIX ? fix_sep(bf, qa, qi[u], rx, ry, rz)
                                  : sep2_f32(bf, p.ivol, pa.x - qq[u].x, pa.y - qq[u].y, pa.z - qq[u].z);
-            if (!(r2 <= keep2)) continue;
-            if (cnt < cap) dst[(size_t)cnt * stride + a] = ee[u] | own;
-            ++cnt;
+            const bool keep = k0 + u < n && r2 <= keep2;
+            if (keep && cnt < cap) *wr = ee[u] | own;
+            wr += keep ? stride : 0;
+            cnt += keep ? 1 : 0;
         }
     }
     return cnt;

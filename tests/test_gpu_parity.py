@@ -610,3 +610,29 @@ def test_md_steps_graph_replay_matches_launches(gpu_lib, prec, ivol):
     assert len(ra) == len(rb) == 103
     for x, y in zip(ra, rb):
         assert x == y
+
+
+def test_scalev_scaling_by_the_next_drift_is_the_same(gpu_lib):
+    """Inside an md_steps call the drift after a scalev removes the mean and
+    scales x1; at the end of a call a kernel of its own does.  One call of 12
+    steps, and a call of two (the first scalev comes after the second step, and
+    both are one fused run in either) with ten of one step give the same state
+    bit for bit, with a light atom that scalev leaves alone."""
+    from moldy_b200 import MoldySystem, units
+    w = wl.make_workload(7, sigma=0.05, temperature=400.0, ivol=0, nbrupdate=5, seed=8)
+    w.atomic_mass = w.atomic_mass.copy()
+    w.atomic_mass[11] = 0.05
+    w.x1 = w.x1.copy()
+    w.x1[11] = 0.0
+    out = []
+    for calls in ([12], [2] + [1] * 10):
+        s = MoldySystem.from_workload(w)
+        s.md_init()
+        s.set_thermostat(3.0, 1.5 * units.BK * 800.0 * (w.nm - 3))
+        for steps in calls:
+            s.md_steps(steps)
+        out.append((s.get_state(), s.thermostat()))
+        s.close()
+    for k in ("x0", "x1", "x2", "b0", "b1"):
+        assert np.array_equal(out[0][0][k], out[1][0][k]), k
+    assert out[0][1] == out[1][1]
