@@ -49,7 +49,7 @@ namespace {
 constexpr int kTileWarps = 4;     // cells (warps) per block
 constexpr int kTileCap = 256;     // staged candidates per warp
 constexpr int kCgThreads = 512;   // control block
-constexpr int kPrepThreads = 256; // list check and binning block
+constexpr int kPrepThreads = 512; // list check and binning block
 
 struct BSys {
     int atom0, nm, cell0, ncell;
@@ -60,6 +60,8 @@ struct BSys {
     int pad;
     double b0[9], tg[9], vol;
     double rv2;                   // squared list radius
+    float rlo2, rhi2;             // FP32 squared distances below / above which the list test is decided
+    float clo2, chi2;             // the same from positions relative to a cell's centre (chi2 0: not used)
     double hs2;                   // squared half skin: rebuild once an atom moved farther
 };
 
@@ -84,16 +86,36 @@ __device__ __forceinline__ int stencil_off(int k, int nst) { return nst == 3 ? k
 
 __device__ __forceinline__ int wrapc(int c, int n) { return c < 0 ? c + n : (c >= n ? c - n : c); }
 
+// fixed-point record of a slot: x, y, z and the slot itself
+__device__ __forceinline__ int4 slot_record(const TileArgs &a, int slot) {
+    const double4 p = ldg4(&a.spos[slot]);
+    return make_int4(fix32(p.x), fix32(p.y), fix32(p.z), slot);
+}
+
+// (-2c, |c|^2) of the record's position c relative to the point cen
+__device__ __forceinline__ int4 rel_record(const float *bq, const int4 &q, const int4 &cen) {
+    const float dx = fix_to_float((int32_t)((uint32_t)q.x - (uint32_t)cen.x));
+    const float dy = fix_to_float((int32_t)((uint32_t)q.y - (uint32_t)cen.y));
+    const float dz = fix_to_float((int32_t)((uint32_t)q.z - (uint32_t)cen.z));
+    const float ux = fmaf(bq[6], dz, fmaf(bq[3], dy, bq[0] * dx));
+    const float uy = fmaf(bq[7], dz, fmaf(bq[4], dy, bq[1] * dx));
+    const float uz = fmaf(bq[8], dz, fmaf(bq[5], dy, bq[2] * dx));
+    return make_int4(__float_as_int(-2.0f * ux), __float_as_int(-2.0f * uy), __float_as_int(-2.0f * uz),
+                     __float_as_int(fmaf(uz, uz, fmaf(uy, uy, ux * ux))));
+}
+
 // Stages the candidates of cell c (the union of its stencil cells, in stencil
 // order) into the warp's tile; returns the count.  pre[0..ns] holds the prefix
 // of the stencil-cell sizes, cs[0..ns) their first sorted slot.
-template <bool FP>
-__device__ int stage_tile(const TileArgs &a, const BSys &S, int c, double4 *tp, double *tf, int *ti, int *pre,
-                          int *cs) {
+// rel: records (-2c, |c|^2) as float bits of each candidate's Cartesian position
+// c relative to the cell's centre cen, else slot_record's; ti holds the slots.
+__device__ int stage_tile(const TileArgs &a, const BSys &S, int c, int4 *tp, int *ti, int *pre, int *cs, bool rel,
+                          const float *bq, int4 &cen) {
     const int lane = threadIdx.x & 31;
     const int local = c - S.cell0;
     const int cx = local % S.nc[0], cy = (local / S.nc[0]) % S.nc[1], cz = local / (S.nc[0] * S.nc[1]);
     const int ns = S.nst[0] * S.nst[1] * S.nst[2];
+    cen = make_int4(fix32((cx + 0.5) / S.nc[0]), fix32((cy + 0.5) / S.nc[1]), fix32((cz + 0.5) / S.nc[2]), 0);
     int cnt = 0, start = 0;
     if (lane < ns) {
         int kx = lane % S.nst[0], ky = (lane / S.nst[0]) % S.nst[1], kz = lane / (S.nst[0] * S.nst[1]);
@@ -115,34 +137,41 @@ __device__ int stage_tile(const TileArgs &a, const BSys &S, int c, double4 *tp, 
     const int total = __shfl_sync(0xffffffffu, inc, 31);
     __syncwarp();
     const int nstage = total < a.cap ? total : a.cap;
-    for (int k = lane; k < nstage; k += 32) {
-        int q = 0;
-        while (pre[q + 1] <= k) ++q;
-        int slot = cs[q] + (k - pre[q]);
-        tp[k] = a.spos[slot];
-        if (FP) tf[k] = a.sfp[slot];
-        ti[k] = slot;
+    // lane by lane over the cells' slots: four loads in flight per lane
+    int q = 0;
+    for (int k0 = lane; k0 < nstage; k0 += 128) {
+        int slot[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int k = k0 + 32 * u;
+            slot[u] = -1;
+            if (k < nstage) {
+                while (pre[q + 1] <= k) ++q;      // k only grows
+                slot[u] = cs[q] + (k - pre[q]);
+            }
+        }
+        int4 r[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (slot[u] >= 0) r[u] = slot_record(a, slot[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (slot[u] >= 0) {
+                tp[k0 + 32 * u] = rel ? rel_record(bq, r[u], cen) : r[u];
+                ti[k0 + 32 * u] = slot[u];
+            }
     }
     __syncwarp();
     return total;
 }
 
-// candidate k of the staged tile, or from global memory past the tile's capacity
-template <bool FP>
-__device__ __forceinline__ void candidate(const TileArgs &a, int k, const double4 *tp, const double *tf,
-                                          const int *ti, const int *pre, const int *cs, double4 &p, double &fp,
-                                          int &slot) {
-    if (k < a.cap) {
-        p = tp[k];
-        fp = FP ? tf[k] : 0.0;
-        slot = ti[k];
-    } else {
-        int q = 0;
-        while (pre[q + 1] <= k) ++q;
-        slot = cs[q] + (k - pre[q]);
-        p = a.spos[slot];
-        fp = FP ? a.sfp[slot] : 0.0;
-    }
+// candidate k of the first cap staged records, or from global memory past them
+__device__ __forceinline__ int4 candidate(const TileArgs &a, int k, const int4 *tp, const int *pre, const int *cs,
+                                          int cap) {
+    if (k < cap) return tp[k];
+    int q = 0;
+    while (pre[q + 1] <= k) ++q;
+    return slot_record(a, cs[q] + (k - pre[q]));
 }
 
 __device__ __forceinline__ void pair_u(const double *b, double dx, double dy, double dz, double &ux, double &uy,
@@ -206,8 +235,8 @@ __device__ double block_max(double v, double *sh) {
 __device__ int prepare_system(BSys &S, const double *__restrict__ X, const double *__restrict__ mass,
                               double *__restrict__ Xb, int32_t *__restrict__ cell_of,
                               int32_t *__restrict__ cell_count, int32_t *__restrict__ cell_start,
-                              int32_t *__restrict__ cursor, int32_t *__restrict__ sorted,
-                              double4 *__restrict__ spos, unsigned long long *__restrict__ stats,
+                              int32_t *__restrict__ cursor, int32_t *__restrict__ unsorted,
+                              int32_t *__restrict__ sorted, double4 *__restrict__ spos, unsigned long long *__restrict__ stats,
                               int32_t *__restrict__ todo, int32_t *__restrict__ ntodo, bool all_spos) {
     __shared__ double sh[33];
     __shared__ int wsum[32];
@@ -284,20 +313,22 @@ __device__ int prepare_system(BSys &S, const double *__restrict__ X, const doubl
         }
         for (int i = tid; i < nm; i += nt) {
             const int a = a0 + i, c = cell_of[a];
-            sorted[cell_start[c] + atomicAdd(&cursor[c], 1)] = a;
+            unsorted[cell_start[c] + atomicAdd(&cursor[c], 1)] = a;
         }
         __syncthreads();
-        // ascending atom order inside each cell; the cells join the tile screen's work
-        for (int cl = tid; cl < S.ncell; cl += nt) {
-            const int c = S.cell0 + cl;
-            if (todo) todo[todo0 + cl] = c;
-            const int s0 = cell_start[c], s1 = cl + 1 < S.ncell ? cell_start[c + 1] : a0 + nm;
-            for (int i = s0 + 1; i < s1; ++i) {
-                const int v = sorted[i];
-                int j = i - 1;
-                while (j >= s0 && sorted[j] > v) { sorted[j + 1] = sorted[j]; --j; }
-                sorted[j + 1] = v;
-            }
+        // ascending atom order inside each cell: every atom counts the atoms of
+        // its cell that come before it (a thread per cell sorting in place, a
+        // chain of dependent loads, was most of the rebuild's time); the cells
+        // join the tile screen's work
+        if (todo)
+            for (int cl = tid; cl < S.ncell; cl += nt) todo[todo0 + cl] = S.cell0 + cl;
+        for (int hs = a0 + tid; hs < a0 + nm; hs += nt) {
+            const int v = unsorted[hs], c = cell_of[v];
+            const int s0 = cell_start[c], s1 = c + 1 < S.cell0 + S.ncell ? cell_start[c + 1] : a0 + nm;
+            int r = 0;
+#pragma unroll 4
+            for (int k = s0; k < s1; ++k) r += unsorted[k] < v ? 1 : 0;
+            sorted[s0 + r] = v;
         }
         __syncthreads();
     }
@@ -314,15 +345,16 @@ __device__ int prepare_system(BSys &S, const double *__restrict__ X, const doubl
 __global__ void __launch_bounds__(kPrepThreads)
 k_prepare(BSys *__restrict__ sys, const double *__restrict__ X, const double *__restrict__ mass,
           double *__restrict__ Xb, int32_t *__restrict__ cell_of, int32_t *__restrict__ cell_count,
-          int32_t *__restrict__ cell_start, int32_t *__restrict__ cursor, int32_t *__restrict__ sorted,
-          double4 *__restrict__ spos, unsigned long long *__restrict__ stats, int32_t *__restrict__ todo,
+          int32_t *__restrict__ cell_start, int32_t *__restrict__ cursor, int32_t *__restrict__ unsorted,
+          int32_t *__restrict__ sorted, double4 *__restrict__ spos, unsigned long long *__restrict__ stats,
+          int32_t *__restrict__ todo,
           int32_t *__restrict__ ntodo) {
     BSys &S = sys[blockIdx.x];
     if (!S.active) {
         if (threadIdx.x == 0) S.rebuild = 0;
         return;
     }
-    prepare_system(S, X, mass, Xb, cell_of, cell_count, cell_start, cursor, sorted, spos, stats, todo, ntodo,
+    prepare_system(S, X, mass, Xb, cell_of, cell_count, cell_start, cursor, unsorted, sorted, spos, stats, todo, ntodo,
                    true);
 }
 
@@ -330,15 +362,33 @@ k_prepare(BSys *__restrict__ sys, const double *__restrict__ X, const double *__
 // The tile screen finds, for every home atom of a cell of a rebuilt system,
 // the candidates inside the list radius and writes their cell-order slots
 // into the atom's compact row (entry-major, alist[e * ntot + slot]) in
-// candidate order.  LPH lanes
-// serve one home atom: they test LPH candidates at a time and place the hits
-// with one warp ballot, so no lane waits on another's pair arithmetic.
+// candidate order.  LPH lanes serve one home atom, each a run of consecutive
+// candidates (an odd number, so that the lanes' records fall into different
+// banks).  A lane collects its hits as bits of a word, three FMAs and two
+// shifts per candidate from records relative to the cell's centre; one scan of
+// the lanes' counts then places them.  The FP32 distance decides outside a band
+// around the list radius that bounds its error, the FP64 distance inside it:
+// the same pairs as an FP64 test of every candidate, which took 75
+// instructions each (and 86 with one ballot per candidate in FP32).  256
+// systems of 1024 atoms: 336 us as it was, 254 with ballots.  Grids of fewer than
+// three cells in a direction (a candidate's offset from the centre is then not
+// its image nearest the home atom) and candidates past the staging take the
+// ballot form.
 // The compact rows of the home atoms of cell c by one warp, with the warp's
-// tile (tp, ti: cap entries; pre, cs: 28); returns the longest row seen when
-// it exceeds pair_cap, else 0.
+// tile (tp, ti: cap entries; pre, cs: 28); returns the longest row seen when it
+// exceeds pair_cap, else 0.
+__device__ __noinline__ bool inside_list(const double4 *__restrict__ spos, const double *b, double rv2, int i, int j) {
+    const double4 p = spos[i], q = spos[j];
+    double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+    dx = dx - round(dx); dy = dy - round(dy); dz = dz - round(dz);
+    double ux, uy, uz;
+    pair_u(b, dx, dy, dz, ux, uy, uz);
+    return (ux * ux + uy * uy + uz * uz) < rv2;
+}
+
 template <int LPH>
-__device__ int screen_cell(const TileArgs &a, int c, int ntot, int pair_cap, int32_t *__restrict__ alist,
-                           int32_t *__restrict__ cnt_out, double4 *tp, int *ti, int *pre, int *cs) {
+__device__ __noinline__ int screen_cell(const TileArgs &a, int c, int ntot, int pair_cap, int32_t *__restrict__ alist,
+                           int32_t *__restrict__ cnt_out, int4 *tp, int *ti, int *pre, int *cs) {
     const int lane = threadIdx.x & 31;
     const int g = lane / LPH, gl = lane % LPH;
     const unsigned gmask = (LPH == 32 ? 0xffffffffu : ((1u << LPH) - 1u)) << (g * LPH);
@@ -347,31 +397,90 @@ __device__ int screen_cell(const TileArgs &a, int c, int ntot, int pair_cap, int
     const BSys &S = a.sys[a.cell_sys[c]];
     const int h0 = a.cell_start[c], h1 = a.cell_start[c + 1];
     if (h1 == h0) return 0;
-    double b[9];
+    float bq[9];                               // B0 per fixed-point unit
 #pragma unroll
-    for (int k = 0; k < 9; ++k) b[k] = S.b0[k];
-    const double rv2 = S.rv2;
-    const int total = stage_tile<false>(a, S, c, tp, nullptr, ti, pre, cs);
+    for (int k = 0; k < 9; ++k) bq[k] = (float)(S.b0[k] * kFixUnit);
+    const float rlo2 = S.rlo2, rhi2 = S.rhi2, chi2 = S.chi2, band = S.chi2 - S.clo2;
+    const bool rel = chi2 > 0.f;
+    int4 cen;
+    const int total = stage_tile(a, S, c, tp, ti, pre, cs, rel, bq, cen);
+    const int staged = total < a.cap ? total : a.cap;
+    // the home cell's place among the stencil cells
+    const int home = (S.nst[0] == 3 ? 1 : 0) + S.nst[0] * ((S.nst[1] == 3 ? 1 : 0) + S.nst[1] * (S.nst[2] == 3 ? 1 : 0));
     for (int hb = h0; hb < h1; hb += 32 / LPH) {
         const int hs = hb + g;
         const bool live = hs < h1;
-        const double4 ph = live ? a.spos[hs] : make_double4(0.0, 0.0, 0.0, 0.0);
-        int cnt = 0;
+        const int4 qh = slot_record(a, live ? hs : h0);
+        int cnt = 0, kk = 0;
+        if (rel) {
+            const int4 rh = rel_record(bq, qh, cen);
+            const float ax = -0.5f * __int_as_float(rh.x), ay = -0.5f * __int_as_float(rh.y),
+                        az = -0.5f * __int_as_float(rh.z);
+            const float thi = chi2 - __int_as_float(rh.w);
+            const int self = pre[home] + hs - h0;
+            while (kk < staged) {
+                const int left = staged - kk;
+                int chunk = ((left + LPH - 1) / LPH) | 1;
+                chunk = chunk < 31 ? chunk : 31;
+                const int kb = kk + gl * chunk;
+                unsigned m = 0u, mlo = 0u;     // bits of r^2 < chi2 and r^2 < clo2, first candidate highest
+#pragma unroll 4
+                for (int i = 0; i < chunk; ++i) {
+                    const int4 r = tp[kb + i < staged ? kb + i : 0];
+                    const float s = fmaf(az, __int_as_float(r.z),
+                                         fmaf(ay, __int_as_float(r.y),
+                                              fmaf(ax, __int_as_float(r.x), __int_as_float(r.w) - thi)));
+                    m = __funnelshift_l(__float_as_uint(s), m, 1);
+                    mlo = __funnelshift_l(__float_as_uint(s + band), mlo, 1);
+                }
+                int nk = staged - kb;
+                nk = live ? (nk < 0 ? 0 : (nk < chunk ? nk : chunk)) : 0;
+                const unsigned valid = (1u << nk) - 1u;              // nk <= 31
+                m = (__brev(m) >> (32 - chunk)) & valid;
+                mlo = __brev(mlo) >> (32 - chunk);
+                if (self >= kb && self < kb + chunk) m &= ~(1u << (self - kb));
+                unsigned rest = m & ~mlo;
+                while (rest) {                                        // rare
+                    const int i = __ffs(rest) - 1;
+                    rest &= rest - 1u;
+                    if (!inside_list(a.spos, S.b0, S.rv2, hs, ti[kb + i])) m &= ~(1u << i);
+                }
+                const int n = __popc(m);
+                int inc = n;
+#pragma unroll
+                for (int o = 1; o < LPH; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, inc, o, LPH);
+                    if (gl >= o) inc += y;
+                }
+                int e = cnt + inc - n;
+                cnt += __shfl_sync(0xffffffffu, inc, LPH - 1, LPH);
+                while (m) {
+                    const int i = __ffs(m) - 1;
+                    m &= m - 1u;
+                    if (e < pair_cap) alist[(size_t)e * ntot + hs] = ti[kb + i];
+                    ++e;
+                }
+                kk += LPH * chunk;
+            }
+            kk = staged;
+        }
         // every lane of the warp runs the same number of rounds (ballots are warp-wide)
-        for (int k0 = 0; k0 < total; k0 += LPH) {
+        for (int k0 = kk; k0 < total; k0 += LPH) {
             const int k = k0 + gl;
             bool hit = false;
             int slot = -1;
             if (live && k < total) {
-                double4 p; double fpk;
-                candidate<false>(a, k, tp, nullptr, ti, pre, cs, p, fpk, slot);
-                if (slot != hs) {
-                    double dx = ph.x - p.x, dy = ph.y - p.y, dz = ph.z - p.z;
-                    dx = dx - round(dx); dy = dy - round(dy); dz = dz - round(dz);
-                    double ux, uy, uz;
-                    pair_u(b, dx, dy, dz, ux, uy, uz);
-                    hit = (ux * ux + uy * uy + uz * uz) < rv2;
-                }
+                const int4 q = rel ? candidate(a, k, nullptr, pre, cs, 0) : candidate(a, k, tp, pre, cs, a.cap);
+                slot = q.w;
+                const float dx = fix_to_float((int32_t)((uint32_t)qh.x - (uint32_t)q.x));
+                const float dy = fix_to_float((int32_t)((uint32_t)qh.y - (uint32_t)q.y));
+                const float dz = fix_to_float((int32_t)((uint32_t)qh.z - (uint32_t)q.z));
+                const float ux = fmaf(bq[6], dz, fmaf(bq[3], dy, bq[0] * dx));
+                const float uy = fmaf(bq[7], dz, fmaf(bq[4], dy, bq[1] * dx));
+                const float uz = fmaf(bq[8], dz, fmaf(bq[5], dy, bq[2] * dx));
+                const float r2 = fmaf(uz, uz, fmaf(uy, uy, ux * ux));
+                hit = slot != hs && r2 <= rhi2;
+                if (hit && !(r2 < rlo2)) hit = inside_list(a.spos, S.b0, S.rv2, hs, slot);
             }
             const unsigned m = __ballot_sync(0xffffffffu, hit) & gmask;
             if (hit) {
@@ -393,7 +502,7 @@ template <int LPH>
 __global__ void __launch_bounds__(32 * kTileWarps)
 k_tile_screen(TileArgs a, int ntot, int pair_cap, int32_t *__restrict__ alist, int32_t *__restrict__ cnt_out,
               int32_t *__restrict__ flags, const int32_t *__restrict__ todo, const int32_t *__restrict__ ntodo) {
-    __shared__ double4 tpos[kTileWarps][kTileCap];
+    __shared__ int4 tpos[kTileWarps][kTileCap];
     __shared__ int tidx[kTileWarps][kTileCap];
     __shared__ int tpre[kTileWarps][28], tcs[kTileWarps][28];
     const int w = threadIdx.x >> 5;
@@ -610,7 +719,7 @@ struct EvalArgs {
     int32_t *queue;                  // [0] next system, [1] blocks done (both zero between launches)
     const double *X, *mass;
     double *Xb;
-    int32_t *cell_of, *cell_count, *cell_start, *cursor, *sorted;
+    int32_t *cell_of, *cell_count, *cell_start, *cursor, *unsorted, *sorted;
     double4 *spos;
     unsigned long long *stats;
     const int32_t *cell_sys;
@@ -664,14 +773,13 @@ k_batch_eval(EvalArgs a, Tables t) {
         if (!S.active) continue;
         // 1. list check, rebuild when due
         const int rebuilt = prepare_system(S, a.X, a.mass, a.Xb, a.cell_of, a.cell_count, a.cell_start, a.cursor,
-                                           a.sorted, a.spos, a.stats, nullptr, nullptr, false);
+                                           a.unsorted, a.sorted, a.spos, a.stats, nullptr, nullptr, false);
         if (rebuilt) {
             TileArgs ta;
             ta.sys = a.sys; ta.cell_sys = a.cell_sys; ta.cell_start = a.cell_start; ta.sorted = a.sorted;
             ta.spos = a.spos; ta.sfp = nullptr; ta.ncell = a.ncell; ta.cap = a.cap; ta.rc2 = a.rc2;
-            double4 *tp = reinterpret_cast<double4 *>(dsm) + (size_t)w * a.cap;
-            int *ti = reinterpret_cast<int *>(reinterpret_cast<double4 *>(dsm) + (size_t)kEvalWarps * a.cap) +
-                      (size_t)w * a.cap;
+            int4 *tp = reinterpret_cast<int4 *>(dsm) + (size_t)w * a.cap;
+            int *ti = reinterpret_cast<int *>(reinterpret_cast<int4 *>(dsm) + (size_t)kEvalWarps * a.cap) + (size_t)w * a.cap;
             for (int c = S.cell0 + w; c < S.cell0 + S.ncell; c += kEvalWarps)
                 overflow = max(overflow, screen_cell<LPH>(ta, c, a.ntot, a.pair_cap, a.alist, a.pcnt, tp, ti,
                                                           tpre[w], tcs[w]));
@@ -1341,7 +1449,7 @@ class BatchEngine {
     // device buffers
     BSys *sys = nullptr;
     int32_t *atom_sys = nullptr, *cell_sys = nullptr, *cell_of = nullptr, *cell_count = nullptr;
-    int32_t *cell_start = nullptr, *cursor = nullptr, *sorted = nullptr, *n_active = nullptr;
+    int32_t *cell_start = nullptr, *cursor = nullptr, *unsorted = nullptr, *sorted = nullptr, *n_active = nullptr;
     double *X = nullptr, *Xb = nullptr, *mass = nullptr, *f = nullptr, *rho = nullptr, *afrho = nullptr, *fp = nullptr;
     double *en_calc = nullptr, *en_force = nullptr, *vir = nullptr, *sfp = nullptr, *sysout = nullptr;
     double *cgv = nullptr;              // G, D, GS, XX, GG, DR, DGR (3*ntot each)
@@ -1414,7 +1522,7 @@ class BatchEngine {
     }
     int eval_prepare();
     size_t eval_smem() const {
-        return std::max((size_t)max_atoms * sizeof(int4), (size_t)kEvalWarps * (size_t)cap * (sizeof(double4) + sizeof(int)));
+        return std::max((size_t)max_atoms * sizeof(int4), (size_t)kEvalWarps * (size_t)cap * (sizeof(int4) + sizeof(int)));
     }
     bool persistent_applies() const {
         return persistent && mixed && !ecalc && all_heavy && eval_smem() + 8192 <= smem_optin;
@@ -1455,7 +1563,7 @@ BatchEngine::~BatchEngine() {
     cudaSetDevice(device);
     if (graph) cudaGraphExecDestroy(graph);
     drop_force_graph();
-    void *bufs[] = {sys, atom_sys, cell_sys, cell_of, cell_count, cell_start, cursor, sorted, n_active, X, Xb,
+    void *bufs[] = {sys, atom_sys, cell_sys, cell_of, cell_count, cell_start, cursor, unsorted, sorted, n_active, X, Xb,
                     mass, f, rho, afrho, fp, en_calc, en_force, vir, sfp, sysout, cgv, spos, cg, tab_r4, tab_e2,
                     tab_r4f, tab_e2f, tab_aux, stage, alist, pcnt, flags, stats, todo, ntodo, cg_order,
                     fm_fref, fm_sref, fm_gF, fm_gS, fm_loss, fm_mu, fm_nu, fm_grads, queue};
@@ -1499,6 +1607,7 @@ int BatchEngine::init(int n, const int32_t *na, double p, int dev) {
     BCHECK(balloc(&atom_sys, nt, "atom_sys"));
     BCHECK(balloc(&cell_of, nt, "cell_of"));
     BCHECK(balloc(&sorted, nt, "sorted"));
+    BCHECK(balloc(&unsorted, nt, "unsorted"));
     BCHECK(balloc(&n_active, 1, "n_active"));
     BCHECK(balloc(&X, 3 * nt, "X"));
     BCHECK(balloc(&Xb, 3 * nt, "build positions"));
@@ -1623,6 +1732,22 @@ int BatchEngine::layout() {
         const double rv = std::max(rcut, std::min(rcut + skin, 0.5 * wmin * (1.0 - 1e-9)));
         const double half = 0.5 * (rv - rcut);
         S.rv2 = rv * rv;
+        // the FP32 distance of a fixed-point difference against the FP64 one of
+        // the same positions: two coordinates rounded to 2^-33 box lengths (under
+        // 2^-31 |B0|_F in length) and fewer than 16 roundings of 2^-24, each of
+        // at most |B0|_F |B0^-1|_F r
+        double nb = 0.0, ni = 0.0;
+        for (int k = 0; k < 9; ++k) nb += b[k] * b[k];
+        for (int d = 0; d < 3; ++d) {
+            const double *p = b + 3 * ((d + 1) % 3), *q = b + 3 * ((d + 2) % 3);
+            const double cx = p[1] * q[2] - p[2] * q[1], cy = p[2] * q[0] - p[0] * q[2], cz = p[0] * q[1] - p[1] * q[0];
+            ni += (cx * cx + cy * cy + cz * cz) / (S.vol * S.vol);      // row d of the inverse
+        }
+        nb = std::sqrt(nb); ni = std::sqrt(ni);
+        const double band = 1.01 * (4.7e-10 * nb + 16.0 * 6.0e-8 * nb * ni * rv) + 4.0e-7 * rv;
+        const double lo = rv - band;
+        S.rlo2 = lo > 0.0 ? (float)(lo * lo) : -1.0f;
+        S.rhi2 = (float)((rv + band) * (rv + band));
         // a small margin keeps rounding in the displacement from hiding a crossing
         S.hs2 = half * half * (1.0 - 1e-6);
         for (int d = 0; d < 3; ++d) {
@@ -1631,6 +1756,16 @@ int BatchEngine::layout() {
             S.nc[d] = nc;
             S.nst[d] = nc >= 3 ? 3 : nc;
         }
+        // positions relative to a cell's centre, at most 1.5 cells off in each
+        // direction (reach): they carry under 8 ulp of the reach per component,
+        // the expanded square under 27 ulp of its square
+        double reach = 0.0;
+        for (int d = 0; d < 3; ++d)
+            reach += 1.5 / S.nc[d] * std::sqrt(b[3 * d] * b[3 * d] + b[3 * d + 1] * b[3 * d + 1] + b[3 * d + 2] * b[3 * d + 2]);
+        const double cband = band + 1.7e-6 * reach + 1.0e-6 * reach * reach / rv;
+        const bool rel = S.nc[0] >= 3 && S.nc[1] >= 3 && S.nc[2] >= 3 && cband < 0.1 * rv;
+        S.chi2 = rel ? (float)((rv + cband) * (rv + cband)) : 0.0f;
+        S.clo2 = rel ? (float)((rv - cband) * (rv - cband)) : 0.0f;
         S.atom0 = atom0[s];
         S.nm = natoms[s];
         S.cell0 = cell;
@@ -1685,9 +1820,9 @@ int BatchEngine::ready() {
 
 template <int LPH>
 static void launch_screen(const BatchEngine &E, const TileArgs &a, cudaStream_t s) {
-    // a persistent grid over the cells of the rebuilt systems (6 blocks of
-    // 37 KB shared memory fit one SM)
-    const int nb = std::max(1, std::min((E.ncell + kTileWarps - 1) / kTileWarps, 6 * E.nsm));
+    // a persistent grid over the cells of the rebuilt systems (8 blocks of
+    // 21 KB shared memory fit one SM)
+    const int nb = std::max(1, std::min((E.ncell + kTileWarps - 1) / kTileWarps, 8 * E.nsm));
     k_tile_screen<LPH><<<nb, 32 * kTileWarps, 0, s>>>(a, E.ntot, E.pair_cap, E.alist, E.pcnt, E.flags, E.todo,
                                                      E.ntodo);
 }
@@ -1727,7 +1862,7 @@ void BatchEngine::queue_evaluation(bool with_vir, bool use_mixed, bool ecalc, cu
     cudaStream_t s = stream;
     if (ecalc) en_calc_zero = false;
     if (ev) cudaEventRecord(ev[0], s);
-    k_prepare<<<nsys, kPrepThreads, 0, s>>>(sys, X, mass, Xb, cell_of, cell_count, cell_start, cursor, sorted, spos,
+    k_prepare<<<nsys, kPrepThreads, 0, s>>>(sys, X, mass, Xb, cell_of, cell_count, cell_start, cursor, unsorted, sorted, spos,
                                            stats, todo, ntodo);
     if (ev) cudaEventRecord(ev[1], s);
     TileArgs a;
@@ -1850,7 +1985,7 @@ int BatchEngine::queue_persistent(bool prepare) {
     EvalArgs a;
     a.sys = sys; a.order = cg_order; a.nsys = nsys; a.ntot = ntot; a.pair_cap = pair_cap; a.queue = queue;
     a.X = X; a.mass = mass; a.Xb = Xb; a.cell_of = cell_of; a.cell_count = cell_count; a.cell_start = cell_start;
-    a.cursor = cursor; a.sorted = sorted; a.spos = spos; a.stats = stats; a.cell_sys = cell_sys;
+    a.cursor = cursor; a.unsorted = unsorted; a.sorted = sorted; a.spos = spos; a.stats = stats; a.cell_sys = cell_sys;
     a.alist = alist; a.pcnt = pcnt; a.flags = flags; a.ncell = ncell; a.cap = cap; a.rc2 = rcut * rcut;
     a.f = f; a.rho = rho; a.afrho = afrho; a.fp = fp; a.en_force = en_force; a.sysout = sysout;
     eval_kernel(lph, lpa)<<<eval_grid, kEvalThreads, eval_smem(), stream>>>(a, tab);

@@ -386,3 +386,28 @@ def test_batch_persistent_evaluation(gpu_lib, oracle_mod):
     b.set_state(mass=m)
     assert not b.persistent_applies()
     b.close()
+
+
+@pytest.mark.parametrize("lanes", [4, 8, 16, 32])
+@pytest.mark.parametrize("skin", [0.0, 0.3])
+def test_tile_screen_forms_give_the_same_rows(gpu_lib, lanes, skin):
+    """Grids of two and of three to five cells per direction, strained: the
+    rows from cell-relative records (256 staged, all of them), from a mixture
+    (37 staged, no multiple of any lane count) and from the per-candidate form
+    alone (none staged) hold the same entries in the same order, so the forces
+    agree bit for bit."""
+    ws = mixed_systems([4, 5, 6, 7, 8, 4, 9], seed=6, sigma=0.15)
+    ref = None
+    for staged in (0, 37, 256):
+        with MoldyBatch.from_workloads(ws) as b:
+            b.set_skin(skin)
+            b.set_tiles(lanes, staged)
+            b.set_energy_calc(False)
+            out = b.force()
+            got = (b.row_entries(), b.forces(), out["pe"], out["tp"])
+        if ref is None:
+            ref = got
+        else:
+            assert got[0] == ref[0]
+            for x, y in zip(got[1:], ref[1:]):
+                assert np.array_equal(x, y)
