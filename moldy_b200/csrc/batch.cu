@@ -42,6 +42,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "pairs.cuh"
 
 namespace moldy {
 namespace {
@@ -532,11 +533,11 @@ __device__ __forceinline__ void frac_diff(const double4 &p, const double4 &q, do
 // (embed, src/potential_m.F90:148-169), and the atom's energy_calc energy
 // F + sum V_src/2 with the exact pair function at the FP64 distance
 // (src/dynamics_m.F90:412-483); one thread per atom in cell order, which
-// gathers B row entries before it evaluates them.  MIXED takes rho's
+// gathers B row entries before it evaluates them.  Mixed precision: rho's
 // separation B0 d, distance and table interpolation in FP32 from the FP64
 // difference and sums rho_i in FP64.  Entries are summed in row order at
 // every B.
-template <bool MIXED, int B, bool ECALC>
+template <int B, bool ECALC>
 __global__ void __launch_bounds__(256)
 k_cl_density(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__restrict__ alist,
              const int32_t *__restrict__ cnt, double *__restrict__ sfp, double *__restrict__ rho_out,
@@ -567,25 +568,15 @@ k_cl_density(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__rest
                 if (e0 + u >= n) continue;
                 double dx, dy, dz;
                 frac_diff(ph, pp[u], dx, dy, dz);
-                if (MIXED) {
-                    float ux, uy, uz;
-                    pair_uf(bf, (float)dx, (float)dy, (float)dz, ux, uy, uz);
-                    const float r2 = ux * ux + uy * uy + uz * uz;
-                    if (!(r2 < rc2f)) continue;
-                    rho += (double)lookup_phif(t, t.phi2f, r2 * rsqrt_ftz(r2));
-                    if (ECALC) {
-                        double vx, vy, vz;
-                        pair_u(b, dx, dy, dz, vx, vy, vz);
-                        ec += 0.5 * fetm_vee(t, sqrt(vx * vx + vy * vy + vz * vz));
-                    }
-                } else {
-                    double ux, uy, uz;
-                    pair_u(b, dx, dy, dz, ux, uy, uz);
-                    const double r2 = ux * ux + uy * uy + uz * uz;
-                    if (!(r2 < a.rc2)) continue;
-                    const double r = sqrt(r2);
-                    rho += lookup_phi(t, r);
-                    if (ECALC) ec += 0.5 * fetm_vee(t, r);
+                float ux, uy, uz;
+                pair_uf(bf, (float)dx, (float)dy, (float)dz, ux, uy, uz);
+                const float r2 = ux * ux + uy * uy + uz * uz;
+                if (!(r2 < rc2f)) continue;
+                rho += (double)lookup_phif(t, t.phi2f, r2 * rsqrt_ftz(r2));
+                if (ECALC) {
+                    double vx, vy, vz;
+                    pair_u(b, dx, dy, dz, vx, vy, vz);
+                    ec += 0.5 * fetm_vee(t, sqrt(vx * vx + vy * vy + vz * vz));
                 }
             }
         }
@@ -610,7 +601,7 @@ k_cl_density(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__rest
 // thread per atom, B row entries gathered at a time.  MIXED takes the
 // separation, the table interpolation and the pair force in FP32 and sums in
 // FP64.
-template <bool MIXED, int B, bool VIR>
+template <int B, bool VIR>
 __global__ void __launch_bounds__(256)
 k_cl_forces(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__restrict__ alist,
             const int32_t *__restrict__ cnt, const int32_t *__restrict__ slot_sys, const double *__restrict__ afrho,
@@ -644,27 +635,14 @@ k_cl_forces(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__restr
                 if (e0 + u >= n) continue;
                 double dx, dy, dz;
                 frac_diff(ph, pp[u], dx, dy, dz);
-                double fpair, vee;
-                if (MIXED) {
-                    float uxf, uyf, uzf;
-                    pair_uf(bf, (float)dx, (float)dy, (float)dz, uxf, uyf, uzf);
-                    const float r2 = uxf * uxf + uyf * uyf + uzf * uzf;
-                    if (!(r2 < rc2f)) continue;
-                    const float rr = rsqrt_ftz(r2), r = r2 * rr;
-                    const float4 q = lookup_r4f(t, r);
-                    fpair = (double)(-(q.y + q.w * ((float)fph + (float)fq[u])) * rr);
-                    vee = (double)q.x;
-                } else {
-                    double ux, uy, uz;
-                    pair_u(b, dx, dy, dz, ux, uy, uz);
-                    const double r2 = ux * ux + uy * uy + uz * uz;
-                    if (!(r2 < a.rc2)) continue;
-                    const double r = sqrt(r2);
-                    const double4 q = lookup_r4(t, r);     // V, V', phi, phi'
-                    const double rr = 1.0 / r;
-                    fpair = -q.y * rr - (q.w * fph + q.w * fq[u]) * rr;
-                    vee = q.x;
-                }
+                float uxf, uyf, uzf;
+                pair_uf(bf, (float)dx, (float)dy, (float)dz, uxf, uyf, uzf);
+                const float r2 = uxf * uxf + uyf * uyf + uzf * uzf;
+                if (!(r2 < rc2f)) continue;
+                const float rr = rsqrt_ftz(r2), r = r2 * rr;
+                const float4 q = lookup_r4f(t, r);
+                const double fpair = (double)(-(q.y + q.w * ((float)fph + (float)fq[u])) * rr);
+                const double vee = (double)q.x;
                 fx += dx * fpair; fy += dy * fpair; fz += dz * fpair;
                 ef += 0.5 * vee;
                 if (VIR && (ph.w + pp[u].w) > 0.1) {
@@ -674,6 +652,222 @@ k_cl_forces(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__restr
                 }
             }
         }
+        const int at = a.sorted[hs];
+        fout[3 * (size_t)at] = fx;
+        fout[3 * (size_t)at + 1] = fy;
+        fout[3 * (size_t)at + 2] = fz;
+        en_force[at] = afrho[at] + ef;
+        if (VIR) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) vir[6 * (size_t)at + k] = v[k];
+        }
+    }
+}
+
+// ------------------------------------------------- FP64 passes over lanes --
+// The FP64 density and force passes with L lanes of a warp per atom (lane g
+// takes the row entries g, g + L, ...), B entries gathered per lane at a time:
+// a row of some 24 entries, walked by one thread, was a chain of six gathers,
+// 26 us for 37 systems whatever their size.  NINT is evaluated only for pairs
+// across a face.  The choice of B changes no result.  The density pass writes
+// each atom's pairs inside the cut (14 of the 24 in the list) in row order, and
+// the force pass and the force-matching passes walk those.
+//
+// ORD (the quench, whose line searches follow every bit): each pair's terms
+// are those of the one-thread walk, and every lane adds them in row order,
+// passed along by shuffles, so energies and forces do not depend on L.
+// Else the root and its inverse come from one reciprocal square root, a table
+// interval is one load, and each lane sums its own entries; the lanes' sums
+// are combined in a fixed order.
+template <int L>
+__device__ __forceinline__ double lanes_sum(double v);
+
+// NINT per direction as frac_diff takes it
+__device__ __forceinline__ void frac_diff_near(const double4 &p, const double4 &q, double &dx, double &dy, double &dz) {
+    dx = p.x - q.x; dy = p.y - q.y; dz = p.z - q.z;
+    if (outside_half(dx, dy, dz)) { dx = dx - round(dx); dy = dy - round(dy); dz = dz - round(dz); }
+}
+
+template <bool ORD, int L, int B, bool ECALC>
+__global__ void __launch_bounds__(256, 3)
+k_cl_density_l(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__restrict__ alist,
+               const int32_t *__restrict__ cnt, double *__restrict__ sfp, double *__restrict__ rho_out,
+               double *__restrict__ afrho_out, double *__restrict__ fp_out, double *__restrict__ en_calc,
+               const int32_t *__restrict__ slot_sys, int32_t *__restrict__ ntodo, int32_t *__restrict__ clist,
+               int32_t *__restrict__ ccnt) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ntodo = 0;   // the tile screen before this pass has read it
+    const unsigned gmask = (L == 32 ? 0xffffffffu : ((1u << L) - 1u)) << ((threadIdx.x & 31) / L * L);
+    const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
+    const int g = threadIdx.x % L, per = gridDim.x * (256 / L);
+    const int rounds = (ntot + per - 1) / per;
+    for (int it = 0; it < rounds; ++it) {                  // the same for every lane: shuffles are warp-wide
+        const int at0 = it * per + blockIdx.x * (256 / L) + threadIdx.x / L;
+        const int hs = at0 < ntot ? at0 : ntot - 1;
+        const BSys &S = a.sys[slot_sys[hs]];
+        const bool live = at0 < ntot && S.active;
+        if (!__any_sync(0xffffffffu, live)) continue;
+        double b[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) b[k] = S.b0[k];
+        const double4 ph = ldg4(&a.spos[hs]);
+        int n = live ? cnt[hs] : 0;
+        n = n < pair_cap ? n : pair_cap;
+        const int nmax = __reduce_max_sync(0xffffffffu, n);
+        int kept = 0;
+        double rho = 0.0, ec = 0.0;
+        for (int e0 = 0; e0 < nmax; e0 += B * L) {
+            int jj[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                const int e = e0 + u * L + g;
+                jj[u] = e < n ? alist[(size_t)e * ntot + hs] : hs;
+            }
+            double4 pp[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) pp[u] = ldg4(&a.spos[jj[u]]);
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                double dx, dy, dz, ux, uy, uz, phi = 0.0, vee = 0.0;
+                frac_diff_near(ph, pp[u], dx, dy, dz);
+                pair_u(b, dx, dy, dz, ux, uy, uz);
+                const double r2 = ux * ux + uy * uy + uz * uz;
+                const bool hit = e0 + u * L + g < n && r2 < a.rc2;
+                // the pair joins the atom's row of pairs inside the cut, in row order
+                if (L == 1) {
+                    if (hit) clist[(size_t)kept++ * ntot + hs] = jj[u];
+                } else {
+                    const unsigned m = __ballot_sync(0xffffffffu, hit) & gmask;
+                    if (hit) clist[(size_t)(kept + __popc(m & below)) * ntot + hs] = jj[u];
+                    kept += __popc(m);
+                }
+                if (hit) {
+                    if (ORD) {
+                        const double r = sqrt(r2);
+                        phi = lookup_phi(t, r);
+                        if (ECALC) vee = fetm_vee(t, r);
+                    } else {
+                        double rr, dr;
+                        const double r = root_and_inverse(r2, rr);
+                        const double2 q = __ldg(&t.dp2[interval_d(t, r, dr)]);
+                        phi = fma(q.y, dr, q.x);
+                        if (ECALC) vee = fetm_vee(t, r);
+                    }
+                }
+                if (ORD && L > 1) {
+#pragma unroll
+                    for (int l = 0; l < L; ++l) {
+                        rho += __shfl_sync(0xffffffffu, phi, l, L);
+                        if (ECALC) ec += 0.5 * __shfl_sync(0xffffffffu, vee, l, L);
+                    }
+                } else {
+                    rho += phi;
+                    if (ECALC) ec += 0.5 * vee;
+                }
+            }
+        }
+        if (!ORD) {
+            rho = lanes_sum<L>(rho);
+            if (ECALC) ec = lanes_sum<L>(ec);
+        }
+        if (!live || g != 0) continue;
+        double f = 0.0, fd = 0.0;
+        if (rho > 1e-40) {
+            double2 e2 = lookup_e2(t, rho);
+            f = e2.x; fd = e2.y;
+        }
+        sfp[hs] = fd;
+        ccnt[hs] = kept;
+        const int at = a.sorted[hs];
+        rho_out[at] = rho;
+        afrho_out[at] = f;
+        fp_out[at] = fd;
+        if (ECALC) en_calc[at] = f + ec;
+    }
+}
+
+template <bool ORD, int L, int B, bool VIR>
+__global__ void __launch_bounds__(256, 2)
+k_cl_forces_l(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist, const int32_t *__restrict__ ccnt,
+              const int32_t *__restrict__ slot_sys, const double *__restrict__ afrho,
+              double *__restrict__ fout, double *__restrict__ en_force, double *__restrict__ vir) {
+    const int g = threadIdx.x % L, per = gridDim.x * (256 / L);
+    const int rounds = (ntot + per - 1) / per;
+    for (int it = 0; it < rounds; ++it) {
+        const int at0 = it * per + blockIdx.x * (256 / L) + threadIdx.x / L;
+        const int hs = at0 < ntot ? at0 : ntot - 1;
+        const BSys &S = a.sys[slot_sys[hs]];
+        const bool live = at0 < ntot && S.active;
+        if (!__any_sync(0xffffffffu, live)) continue;
+        double b[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) b[k] = S.b0[k];
+        const double4 ph = ldg4(&a.spos[hs]);
+        const double fph = a.sfp[hs];
+        const int n = live ? ccnt[hs] : 0;             // every entry inside the cut
+        const int nmax = __reduce_max_sync(0xffffffffu, n);
+        double fx = 0.0, fy = 0.0, fz = 0.0, ef = 0.0;
+        double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        for (int e0 = 0; e0 < nmax; e0 += B * L) {
+            int jj[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                const int e = e0 + u * L + g;
+                jj[u] = e < n ? clist[(size_t)e * ntot + hs] : hs;
+            }
+            double4 pp[B];
+            double fq[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) { pp[u] = ldg4(&a.spos[jj[u]]); fq[u] = __ldg(&a.sfp[jj[u]]); }
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                double dx, dy, dz, ux, uy, uz, fpair = 0.0, vee = 0.0;
+                frac_diff_near(ph, pp[u], dx, dy, dz);
+                pair_u(b, dx, dy, dz, ux, uy, uz);
+                const double r2 = ux * ux + uy * uy + uz * uz;
+                if (e0 + u * L + g < n) {
+                    if (ORD) {
+                        const double r = sqrt(r2);
+                        const double4 q = lookup_r4(t, r);     // V, V', phi, phi'
+                        const double rr = 1.0 / r;
+                        fpair = -q.y * rr - (q.w * fph + q.w * fq[u]) * rr;
+                        vee = q.x;
+                    } else {
+                        double rr, dr;
+                        const double r = root_and_inverse(r2, rr);
+                        const int idx = interval_d(t, r, dr);
+                        const double4 w = ldg4(&t.df4[idx]);
+                        const double2 qv = __ldg(&t.dv2[idx]);
+                        fpair = -fma(w.z, dr, w.x) * rr - (fma(w.w, dr, w.y) * (fph + fq[u])) * rr;
+                        vee = fma(qv.y, dr, qv.x);
+                    }
+                }
+                if (ORD && L > 1) {
+#pragma unroll
+                    for (int l = 0; l < L; ++l) {
+                        const double fl = __shfl_sync(0xffffffffu, fpair, l, L);
+                        fx += __shfl_sync(0xffffffffu, dx, l, L) * fl;
+                        fy += __shfl_sync(0xffffffffu, dy, l, L) * fl;
+                        fz += __shfl_sync(0xffffffffu, dz, l, L) * fl;
+                        ef += 0.5 * __shfl_sync(0xffffffffu, vee, l, L);
+                    }
+                } else {
+                    fx += dx * fpair; fy += dy * fpair; fz += dz * fpair;
+                    ef += 0.5 * vee;
+                    if (VIR && (ph.w + pp[u].w) > 0.1) {
+                        const double hf = 0.5 * fpair;
+                        v[0] += dx * dx * hf; v[1] += dy * dy * hf; v[2] += dz * dz * hf;
+                        v[3] += dx * dy * hf; v[4] += dx * dz * hf; v[5] += dy * dz * hf;
+                    }
+                }
+            }
+        }
+        if (!ORD) {
+            fx = lanes_sum<L>(fx); fy = lanes_sum<L>(fy); fz = lanes_sum<L>(fz); ef = lanes_sum<L>(ef);
+            if (VIR)
+#pragma unroll
+                for (int k = 0; k < 6; ++k) v[k] = lanes_sum<L>(v[k]);
+        }
+        if (!live || g != 0) continue;
         const int at = a.sorted[hs];
         fout[3 * (size_t)at] = fx;
         fout[3 * (size_t)at + 1] = fy;
@@ -986,11 +1180,13 @@ __device__ __forceinline__ double dmax(double a, double b) { return a > b ? a : 
 // from the forward pass (per atom), F' from its cell-order copy.
 
 // Loss and dL/dF, dL/dsigma of one evaluation; one block per system.  gF
-// goes to cell order (slot hs) for the pair passes.
+// goes to cell order (slot hs) for the pair passes, with F' beside it (w): one
+// 32-byte gather per neighbour.
 __global__ void __launch_bounds__(kCgThreads)
 k_fm_loss(const BSys *__restrict__ sys, const double *__restrict__ f, const double *__restrict__ fref,
           const double *__restrict__ sref, const double *__restrict__ sysout, const int32_t *__restrict__ sorted,
-          double wf, double ws, double *__restrict__ gF, double *__restrict__ gS, double *__restrict__ loss) {
+          double wf, double ws, const double *__restrict__ sfp, double4 *__restrict__ gF, double *__restrict__ gS,
+          double *__restrict__ loss) {
     __shared__ double sh[33];
     const BSys &S = sys[blockIdx.x];
     double lf = 0.0;
@@ -1000,9 +1196,7 @@ k_fm_loss(const BSys *__restrict__ sys, const double *__restrict__ f, const doub
         pair_u(S.b0, f[at], f[at + 1], f[at + 2], fx, fy, fz);
         const double dx = fx - fref[at], dy = fy - fref[at + 1], dz = fz - fref[at + 2];
         lf += dx * dx + dy * dy + dz * dz;
-        gF[3 * (size_t)hs] = 2.0 * wf * dx;
-        gF[3 * (size_t)hs + 1] = 2.0 * wf * dy;
-        gF[3 * (size_t)hs + 2] = 2.0 * wf * dz;
+        gF[hs] = make_double4(2.0 * wf * dx, 2.0 * wf * dy, 2.0 * wf * dz, sfp[hs]);
     }
     lf = block_sum(lf, sh);
     if (threadIdx.x == 0) {
@@ -1046,59 +1240,67 @@ __device__ __forceinline__ void fm_flush(const double *h, double *g, int nb) {
     }
 }
 
-// the pair geometry of slot hs and row entry j: u = B0 d, r; false beyond the cut
-__device__ __forceinline__ bool fm_pair(const BSys &S, const double4 &ph, const double4 &pj, double rc2,
-                                        double &ux, double &uy, double &uz, double &r) {
+// The pair of slot hs and row entry j (inside the cut): u = B0 d, r, 1/r, the
+// table interval q and the weight w1 of its upper node.
+__device__ __forceinline__ double fm_pair(const Tables &t, const double *b, const double4 &ph, const double4 &pj,
+                                          double &ux, double &uy, double &uz, double &rr, int &q, double &w1) {
     double dx, dy, dz;
-    frac_diff(ph, pj, dx, dy, dz);
-    pair_u(S.b0, dx, dy, dz, ux, uy, uz);
-    const double r2 = ux * ux + uy * uy + uz * uz;
-    if (!(r2 < rc2)) return false;
-    r = sqrt(r2);
-    return true;
+    frac_diff_near(ph, pj, dx, dy, dz);
+    pair_u(b, dx, dy, dz, ux, uy, uz);
+    const double r = root_and_inverse(ux * ux + uy * uy + uz * uz, rr);
+    q = interval_d(t, r, w1);
+    if (q > t.nr - 2) { q = t.nr - 2; w1 = 1.0; }
+    return r;
 }
 
-// lam per pair; mu_i; dL/d dvee and dL/d dphi
-__global__ void __launch_bounds__(256)
-k_fm_pairs_a(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__restrict__ alist,
-             const int32_t *__restrict__ cnt, const int32_t *__restrict__ slot_sys, const double *__restrict__ gF,
+constexpr int kFmGather = 2;      // row entries gathered before any is used
+
+// lam per pair; mu_i; dL/d dvee and dL/d dphi.  Bound by the latency of the
+// neighbours' gathers: rows hold the pairs inside the cut alone, two entries
+// are gathered at a time, and a neighbour is two 32-byte loads (position and
+// mass; dL/dF and F') and its interval one (256 systems of 1024 atoms: 225 us
+// with five 8-byte gathers and two nodes per listed entry).
+__global__ void __launch_bounds__(256, 2)
+k_fm_pairs_a(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
+             const int32_t *__restrict__ ccnt, const int32_t *__restrict__ slot_sys, const double4 *__restrict__ gF,
              const double *__restrict__ gS, double *__restrict__ mu, double *__restrict__ g_dvee,
              double *__restrict__ g_dphi, int nbr) {
     extern __shared__ double sh[];
     double *hdv = sh, *hdp = sh + nbr;
     for (int k = threadIdx.x; k < 2 * nbr; k += blockDim.x) sh[k] = 0.0;
     __syncthreads();
-    const double rmin = t.vp_rmin, range = t.vp_range, recipr = t.vp_reciprange, recipn = t.vp_recipnlkp,
-                 recips = t.vp_recipstep;
     for (int hs = blockIdx.x * blockDim.x + threadIdx.x; hs < ntot; hs += gridDim.x * blockDim.x) {
         const int s = slot_sys[hs];
         const BSys &S = a.sys[s];
-        const double4 ph = a.spos[hs];
-        const double fph = a.sfp[hs];
-        const double gx = gF[3 * (size_t)hs], gy = gF[3 * (size_t)hs + 1], gz = gF[3 * (size_t)hs + 2];
+        const double4 ph = ldg4(&a.spos[hs]), gh = ldg4(&gF[hs]);
         const double *G = gS + 9 * (size_t)s;
         const double ivol = 1.0 / S.vol;
-        int n = cnt[hs];
-        n = n < pair_cap ? n : pair_cap;
+        const int n = ccnt[hs];
         double m = 0.0;
-        for (int e = 0; e < n; ++e) {
-            const int j = alist[(size_t)e * ntot + hs];
-            const double4 pj = a.spos[j];
-            double ux, uy, uz, r;
-            if (!fm_pair(S, ph, pj, a.rc2, ux, uy, uz, r)) continue;
-            double w1;
-            const int q = fm_weights(r, rmin, range, recipr, recipn, recips, t.nlookup, w1);
-            const double dp = t.r4[q].w * (1.0 - w1) + t.r4[q + 1].w * w1;
-            double lam = (gx - gF[3 * (size_t)j]) * ux + (gy - gF[3 * (size_t)j + 1]) * uy +
-                         (gz - gF[3 * (size_t)j + 2]) * uz;
-            if (ph.w + pj.w > 0.1)
-                lam -= ivol * (ux * (G[0] * ux + G[3] * uy + G[6] * uz) + uy * (G[1] * ux + G[4] * uy + G[7] * uz) +
-                               uz * (G[2] * ux + G[5] * uy + G[8] * uz));
-            const double rr = 1.0 / r;
-            m -= lam * dp * rr;
-            if (hs < j) {
-                fm_hist(hdv, q, -lam * rr, w1);
-                fm_hist(hdp, q, -lam * (fph + a.sfp[j]) * rr, w1);
+        for (int e0 = 0; e0 < n; e0 += kFmGather) {
+            int jj[kFmGather];
+            double4 pp[kFmGather], gg[kFmGather];
+#pragma unroll
+            for (int u = 0; u < kFmGather; ++u) jj[u] = e0 + u < n ? clist[(size_t)(e0 + u) * ntot + hs] : hs;
+#pragma unroll
+            for (int u = 0; u < kFmGather; ++u) { pp[u] = ldg4(&a.spos[jj[u]]); gg[u] = ldg4(&gF[jj[u]]); }
+#pragma unroll
+            for (int u = 0; u < kFmGather; ++u) {
+                if (e0 + u >= n) continue;
+                double ux, uy, uz, rr, w1;
+                int q;
+                fm_pair(t, S.b0, ph, pp[u], ux, uy, uz, rr, q, w1);
+                const double4 w = ldg4(&t.df4[q]);
+                const double dp = fma(w.w, w1, w.y);
+                double lam = (gh.x - gg[u].x) * ux + (gh.y - gg[u].y) * uy + (gh.z - gg[u].z) * uz;
+                if (ph.w + pp[u].w > 0.1)
+                    lam -= ivol * (ux * (G[0] * ux + G[3] * uy + G[6] * uz) + uy * (G[1] * ux + G[4] * uy + G[7] * uz) +
+                                   uz * (G[2] * ux + G[5] * uy + G[8] * uz));
+                m -= lam * dp * rr;
+                if (hs < jj[u]) {
+                    fm_hist(hdv, q, -lam * rr, w1);
+                    fm_hist(hdp, q, -lam * (gh.w + gg[u].w) * rr, w1);
+                }
             }
         }
         mu[hs] = m;
@@ -1107,56 +1309,83 @@ k_fm_pairs_a(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__rest
     fm_flush(hdp, g_dphi, nbr);
 }
 
-// nu_i = mu_i De'(rho_i) and dL/d demb per atom
+// nu_i = mu_i De'(rho_i) and dL/d demb per atom.  The densities of a crystal
+// fall into a handful of the table's intervals, so the lanes of a warp that
+// share an interval are summed before one of them adds (256 systems of 1024
+// atoms: 40 us with an addition per atom, all to the same few addresses).
 __global__ void __launch_bounds__(256)
 k_fm_atoms(Tables t, int ntot, const int32_t *__restrict__ sorted, const double *__restrict__ rho,
            const double *__restrict__ mu, double *__restrict__ nu, double *__restrict__ g_demb) {
     extern __shared__ double sh[];
-    const int nb = t.nlookup + 1;
+    const int nb = t.nlookup + 1, lane = threadIdx.x & 31;
     for (int k = threadIdx.x; k < nb; k += blockDim.x) sh[k] = 0.0;
     __syncthreads();
-    for (int hs = blockIdx.x * blockDim.x + threadIdx.x; hs < ntot; hs += gridDim.x * blockDim.x) {
-        const double r = rho[sorted[hs]];
-        double v = 0.0;
+    for (int base = blockIdx.x * blockDim.x; base < ntot; base += gridDim.x * blockDim.x) {   // block-uniform
+        const int hs = base + threadIdx.x;
+        const double r = hs < ntot ? rho[sorted[hs]] : 0.0, m = hs < ntot ? mu[hs] : 0.0;
+        double v = 0.0, c0 = 0.0, c1 = 0.0;
+        int q = -1;
         if (r > 1e-40) {
             if (r >= t.e_rmax) {
-                atomicAdd(&sh[t.nlookup], mu[hs]);   // the last node alone, zero slope
+                q = t.nlookup;           // the last node alone, zero slope
+                c0 = m;
             } else {
                 double w1;
-                const int q = fm_weights(r, t.e_rmin, t.e_range, t.e_reciprange, t.e_recipnlkp, t.e_recipstep,
-                                         t.nlookup, w1);
-                v = mu[hs] * (t.e2[q + 1].y - t.e2[q].y) * t.e_recipstep;
-                fm_hist(sh, q, mu[hs], w1);
+                q = fm_weights(r, t.e_rmin, t.e_range, t.e_reciprange, t.e_recipnlkp, t.e_recipstep, t.nlookup, w1);
+                v = m * (t.e2[q + 1].y - t.e2[q].y) * t.e_recipstep;
+                c0 = m * (1.0 - w1);
+                c1 = m * w1;
             }
         }
-        nu[hs] = v;
+        if (hs < ntot) nu[hs] = v;
+        unsigned todo = __ballot_sync(0xffffffffu, q >= 0);
+        while (todo) {                   // warp-uniform: one interval per round
+            const int qq = __shfl_sync(0xffffffffu, q, __ffs(todo) - 1);
+            const bool mine = q == qq;
+            const double s0 = warp_sum(mine ? c0 : 0.0), s1 = warp_sum(mine ? c1 : 0.0);
+            if (lane == 0) {
+                atomicAdd(&sh[qq], s0);
+                if (qq < t.nlookup) atomicAdd(&sh[qq + 1], s1);
+            }
+            todo &= ~__ballot_sync(0xffffffffu, mine);
+        }
     }
     fm_flush(sh, g_demb, nb);
 }
 
 // dL/d phi = nu_i + nu_j per pair
-__global__ void __launch_bounds__(256)
-k_fm_pairs_c(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__restrict__ alist,
-             const int32_t *__restrict__ cnt, const int32_t *__restrict__ slot_sys, const double *__restrict__ nu,
+__global__ void __launch_bounds__(256, 3)
+k_fm_pairs_c(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
+             const int32_t *__restrict__ ccnt, const int32_t *__restrict__ slot_sys, const double *__restrict__ nu,
              double *__restrict__ g_phi, int nbr) {
     extern __shared__ double sh[];
     for (int k = threadIdx.x; k < nbr; k += blockDim.x) sh[k] = 0.0;
     __syncthreads();
     for (int hs = blockIdx.x * blockDim.x + threadIdx.x; hs < ntot; hs += gridDim.x * blockDim.x) {
         const BSys &S = a.sys[slot_sys[hs]];
-        const double4 ph = a.spos[hs];
+        const double4 ph = ldg4(&a.spos[hs]);
         const double nui = nu[hs];
-        int n = cnt[hs];
-        n = n < pair_cap ? n : pair_cap;
-        for (int e = 0; e < n; ++e) {
-            const int j = alist[(size_t)e * ntot + hs];
-            if (!(hs < j)) continue;
-            double ux, uy, uz, r;
-            if (!fm_pair(S, ph, a.spos[j], a.rc2, ux, uy, uz, r)) continue;
-            double w1;
-            const int q = fm_weights(r, t.vp_rmin, t.vp_range, t.vp_reciprange, t.vp_recipnlkp, t.vp_recipstep,
-                                     t.nlookup, w1);
-            fm_hist(sh, q, nui + nu[j], w1);
+        const int n = ccnt[hs];
+        for (int e0 = 0; e0 < n; e0 += kFmGather) {
+            int jj[kFmGather];
+            double4 pp[kFmGather];
+            double nj[kFmGather];
+#pragma unroll
+            for (int u = 0; u < kFmGather; ++u) jj[u] = e0 + u < n ? clist[(size_t)(e0 + u) * ntot + hs] : hs;
+#pragma unroll
+            for (int u = 0; u < kFmGather; ++u) {        // each pair once, from its lower slot
+                const int j = hs < jj[u] ? jj[u] : hs;
+                pp[u] = ldg4(&a.spos[j]);
+                nj[u] = nu[j];
+            }
+#pragma unroll
+            for (int u = 0; u < kFmGather; ++u) {
+                if (!(hs < jj[u])) continue;             // also the entries past the end (hs itself)
+                double ux, uy, uz, rr, w1;
+                int q;
+                fm_pair(t, S.b0, ph, pp[u], ux, uy, uz, rr, q, w1);
+                fm_hist(sh, q, nui + nj[u], w1);
+            }
         }
     }
     fm_flush(sh, g_phi, nbr);
@@ -1454,6 +1683,7 @@ class BatchEngine {
     double *en_calc = nullptr, *en_force = nullptr, *vir = nullptr, *sfp = nullptr, *sysout = nullptr;
     double *cgv = nullptr;              // G, D, GS, XX, GG, DR, DGR (3*ntot each)
     int32_t *alist = nullptr, *pcnt = nullptr, *flags = nullptr;
+    int32_t *clist = nullptr, *ccnt = nullptr;   // rows of the pairs inside the cut (FP64 passes)
     unsigned long long *stats = nullptr;   // system list builds, system evaluations
     int32_t *todo = nullptr, *ntodo = nullptr;   // cells of the systems rebuilt in this evaluation
     int32_t *cg_order = nullptr;                 // systems by descending size
@@ -1485,7 +1715,8 @@ class BatchEngine {
     int autotune(int nreps, double *times_ms, int32_t *chosen);
     // force matching: references (device), dL/dF in cell order, dL/dsigma,
     // per-system loss, mu, nu and the six table gradients; allocated on first use
-    double *fm_fref = nullptr, *fm_sref = nullptr, *fm_gF = nullptr, *fm_gS = nullptr, *fm_loss = nullptr;
+    double4 *fm_gF = nullptr;
+    double *fm_fref = nullptr, *fm_sref = nullptr, *fm_gS = nullptr, *fm_loss = nullptr;
     double *fm_mu = nullptr, *fm_nu = nullptr, *fm_grads = nullptr;
     int fm_nb = 0;
     bool fm_refs = false;
@@ -1565,7 +1796,7 @@ BatchEngine::~BatchEngine() {
     drop_force_graph();
     void *bufs[] = {sys, atom_sys, cell_sys, cell_of, cell_count, cell_start, cursor, unsorted, sorted, n_active, X, Xb,
                     mass, f, rho, afrho, fp, en_calc, en_force, vir, sfp, sysout, cgv, spos, cg, tab_r4, tab_e2,
-                    tab_r4f, tab_e2f, tab_aux, stage, alist, pcnt, flags, stats, todo, ntodo, cg_order,
+                    tab_r4f, tab_e2f, tab_aux, stage, alist, pcnt, clist, ccnt, flags, stats, todo, ntodo, cg_order,
                     fm_fref, fm_sref, fm_gF, fm_gS, fm_loss, fm_mu, fm_nu, fm_grads, queue};
     for (void *b : bufs)
         if (b) cudaFree(b);
@@ -1627,6 +1858,8 @@ int BatchEngine::init(int n, const int32_t *na, double p, int dev) {
     BCHECK(balloc(&stage, 3 * nt, "staging"));
     BCHECK(balloc(&alist, nt * (size_t)pair_cap, "compact list"));
     BCHECK(balloc(&pcnt, nt, "compact counts"));
+    BCHECK(balloc(&clist, nt * (size_t)pair_cap, "rows inside the cut"));
+    BCHECK(balloc(&ccnt, nt, "counts inside the cut"));
     BCHECK(balloc(&flags, 2, "flags"));
     BCUDA(cudaMemset(flags, 0, 2 * sizeof(int32_t)), "flags");
     BCHECK(balloc(&stats, 2, "list statistics"));
@@ -1827,34 +2060,52 @@ static void launch_screen(const BatchEngine &E, const TileArgs &a, cudaStream_t 
                                                      E.ntodo);
 }
 
-template <bool MIXED, int B>
-static void launch_passes(const BatchEngine &E, const TileArgs &a, bool with_vir, bool ecalc, cudaStream_t s,
-                          cudaEvent_t *ev) {
+template <int B>
+static void launch_passes_mixed(const BatchEngine &E, const TileArgs &a, bool with_vir, bool ecalc, cudaStream_t s,
+                                cudaEvent_t *ev) {
     const int nbs = grid_blocks(E.ntot, 256);
     // a system's slots are its atoms' index range, so atom_sys is the slot's system
     if (ecalc)
-        k_cl_density<MIXED, B, true><<<nbs, 256, 0, s>>>(a, E.tab, E.ntot, E.pair_cap, E.alist, E.pcnt, E.sfp,
-                                                         E.rho, E.afrho, E.fp, E.en_calc, E.atom_sys, E.ntodo);
+        k_cl_density<B, true><<<nbs, 256, 0, s>>>(a, E.tab, E.ntot, E.pair_cap, E.alist, E.pcnt, E.sfp, E.rho, E.afrho,
+                                                  E.fp, E.en_calc, E.atom_sys, E.ntodo);
     else
-        k_cl_density<MIXED, B, false><<<nbs, 256, 0, s>>>(a, E.tab, E.ntot, E.pair_cap, E.alist, E.pcnt, E.sfp,
-                                                          E.rho, E.afrho, E.fp, E.en_calc, E.atom_sys, E.ntodo);
+        k_cl_density<B, false><<<nbs, 256, 0, s>>>(a, E.tab, E.ntot, E.pair_cap, E.alist, E.pcnt, E.sfp, E.rho, E.afrho,
+                                                   E.fp, E.en_calc, E.atom_sys, E.ntodo);
     if (ev) cudaEventRecord(ev[3], s);
     if (with_vir)
-        k_cl_forces<MIXED, B, true><<<nbs, 256, 0, s>>>(a, E.tab, E.ntot, E.pair_cap, E.alist, E.pcnt, E.atom_sys,
-                                                        E.afrho, E.f, E.en_force, E.vir);
+        k_cl_forces<B, true><<<nbs, 256, 0, s>>>(a, E.tab, E.ntot, E.pair_cap, E.alist, E.pcnt, E.atom_sys, E.afrho, E.f,
+                                                 E.en_force, E.vir);
     else
-        k_cl_forces<MIXED, B, false><<<nbs, 256, 0, s>>>(a, E.tab, E.ntot, E.pair_cap, E.alist, E.pcnt, E.atom_sys,
-                                                         E.afrho, E.f, E.en_force, E.vir);
+        k_cl_forces<B, false><<<nbs, 256, 0, s>>>(a, E.tab, E.ntot, E.pair_cap, E.alist, E.pcnt, E.atom_sys, E.afrho,
+                                                  E.f, E.en_force, E.vir);
 }
 
-template <bool MIXED>
-static void launch_passes_b(const BatchEngine &E, const TileArgs &a, bool with_vir, bool ecalc, cudaStream_t s,
-                            cudaEvent_t *ev) {
-    switch (E.gather) {
-        case 1: launch_passes<MIXED, 1>(E, a, with_vir, ecalc, s, ev); break;
-        case 2: launch_passes<MIXED, 2>(E, a, with_vir, ecalc, s, ev); break;
-        default: launch_passes<MIXED, 4>(E, a, with_vir, ecalc, s, ev); break;
-    }
+// FP64: the quench (no virial) in row order, else lane sums
+template <int L, int LF, int B>
+static void launch_passes_fp64(const BatchEngine &E, const TileArgs &a, bool with_vir, bool ecalc, cudaStream_t s,
+                               cudaEvent_t *ev) {
+    const int nbs = grid_blocks((long long)E.ntot * L, 256), nbf = grid_blocks((long long)E.ntot * LF, 256);
+    auto den = with_vir ? (ecalc ? k_cl_density_l<false, L, B, true> : k_cl_density_l<false, L, B, false>)
+                        : (ecalc ? k_cl_density_l<true, L, B, true> : k_cl_density_l<true, L, B, false>);
+    den<<<nbs, 256, 0, s>>>(a, E.tab, E.ntot, E.pair_cap, E.alist, E.pcnt, E.sfp, E.rho, E.afrho, E.fp, E.en_calc,
+                            E.atom_sys, E.ntodo, E.clist, E.ccnt);
+    if (ev) cudaEventRecord(ev[3], s);
+    auto frc = with_vir ? k_cl_forces_l<false, LF, B, true> : k_cl_forces_l<true, LF, B, false>;
+    frc<<<nbf, 256, 0, s>>>(a, E.tab, E.ntot, E.clist, E.ccnt, E.atom_sys, E.afrho, E.f, E.en_force, E.vir);
+}
+
+template <int B>
+static void launch_passes_b(const BatchEngine &E, const TileArgs &a, bool use_mixed, bool with_vir, bool ecalc,
+                            cudaStream_t s, cudaEvent_t *ev) {
+    if (use_mixed) return launch_passes_mixed<B>(E, a, with_vir, ecalc, s, ev);
+    // the most lanes per atom that one resident wave holds (768 threads per SM
+    // in the density pass, 512 in the force pass)
+    const long long wave = (long long)E.nsm * 768, wavef = (long long)E.nsm * 512;
+    if (4LL * E.ntot <= wavef) return launch_passes_fp64<4, 4, B>(E, a, with_vir, ecalc, s, ev);
+    if (4LL * E.ntot <= wave) return launch_passes_fp64<4, 2, B>(E, a, with_vir, ecalc, s, ev);
+    if (2LL * E.ntot <= wavef) return launch_passes_fp64<2, 2, B>(E, a, with_vir, ecalc, s, ev);
+    if (2LL * E.ntot <= wave) return launch_passes_fp64<2, 1, B>(E, a, with_vir, ecalc, s, ev);
+    launch_passes_fp64<1, 1, B>(E, a, with_vir, ecalc, s, ev);
 }
 
 // list check (and rebuild) and the tile passes for the systems marked active
@@ -1875,10 +2126,11 @@ void BatchEngine::queue_evaluation(bool with_vir, bool use_mixed, bool ecalc, cu
         default: launch_screen<8>(*this, a, s); break;
     }
     if (ev) cudaEventRecord(ev[2], s);
-    if (use_mixed)
-        launch_passes_b<true>(*this, a, with_vir, ecalc, s, ev);
-    else
-        launch_passes_b<false>(*this, a, with_vir, ecalc, s, ev);
+    switch (gather) {
+        case 1: launch_passes_b<1>(*this, a, use_mixed, with_vir, ecalc, s, ev); break;
+        case 2: launch_passes_b<2>(*this, a, use_mixed, with_vir, ecalc, s, ev); break;
+        default: launch_passes_b<4>(*this, a, use_mixed, with_vir, ecalc, s, ev); break;
+    }
     if (ev) cudaEventRecord(ev[4], s);
     launches += 4;
 }
@@ -1894,7 +2146,10 @@ int BatchEngine::take_overflow() {
     int need = h[1] + 8;
     if (alist) cudaFree(alist);
     alist = nullptr;
+    if (clist) cudaFree(clist);
+    clist = nullptr;
     if (balloc(&alist, (size_t)ntot * (size_t)need, "compact list") != MOLDY_OK) return -1;
+    if (balloc(&clist, (size_t)ntot * (size_t)need, "rows inside the cut") != MOLDY_OK) return -1;
     pair_cap = need;
     if (graph) { cudaGraphExecDestroy(graph); graph = nullptr; }
     drop_force_graph();
@@ -2143,7 +2398,7 @@ int BatchEngine::set_references(const double *fref_xyz, const double *sref) {
     if (!fm_fref) {
         BCHECK(balloc(&fm_fref, 3 * nt, "reference forces"));
         BCHECK(balloc(&fm_sref, 9 * (size_t)nsys, "reference stresses"));
-        BCHECK(balloc(&fm_gF, 3 * nt, "dL/dF"));
+        BCHECK(balloc(&fm_gF, nt, "dL/dF"));
         BCHECK(balloc(&fm_gS, 9 * (size_t)nsys, "dL/dsigma"));
         BCHECK(balloc(&fm_loss, nsys, "loss"));
         BCHECK(balloc(&fm_mu, nt, "mu"));
@@ -2184,7 +2439,8 @@ int BatchEngine::force_matching(double wf, double ws, double *loss, double *grad
         if (attempt >= 2) return set_last_error(MOLDY_ERR_CAPACITY, "compact list keeps overflowing");
     }
     cudaStream_t s = stream;
-    k_fm_loss<<<nsys, kCgThreads, 0, s>>>(sys, f, fm_fref, fm_sref, sysout, sorted, wf, ws, fm_gF, fm_gS, fm_loss);
+    k_fm_loss<<<nsys, kCgThreads, 0, s>>>(sys, f, fm_fref, fm_sref, sysout, sorted, wf, ws, sfp, fm_gF, fm_gS,
+                                       fm_loss);
     BCUDA(cudaMemsetAsync(fm_grads, 0, 6 * (size_t)nb * sizeof(double), s), "table gradients");
     TileArgs a;
     a.sys = sys; a.cell_sys = cell_sys; a.cell_start = cell_start; a.sorted = sorted;
@@ -2198,10 +2454,11 @@ int BatchEngine::force_matching(double wf, double ws, double *loss, double *grad
     const int g = std::min(grid_blocks(ntot, 256), 2 * nsm);
     // vee and emb get no gradient: the loss holds no energy
     double *gdv = fm_grads + nb, *gp = fm_grads + 2 * nb, *gdp = fm_grads + 3 * nb, *gde = fm_grads + 5 * nb;
-    k_fm_pairs_a<<<g, 256, smem_r, s>>>(a, tab, ntot, pair_cap, alist, pcnt, atom_sys, fm_gF, fm_gS, fm_mu, gdv, gdp,
+    k_fm_pairs_a<<<g, 256, smem_r, s>>>(a, tab, ntot, clist, ccnt, atom_sys, fm_gF, fm_gS, fm_mu, gdv, gdp,
                                        nbr);
     k_fm_atoms<<<g, 256, smem_e, s>>>(tab, ntot, sorted, rho, fm_mu, fm_nu, gde);
-    k_fm_pairs_c<<<g, 256, smem_r / 2, s>>>(a, tab, ntot, pair_cap, alist, pcnt, atom_sys, fm_nu, gp, nbr);
+    const int gc = std::min(grid_blocks(ntot, 256), 3 * nsm);   // half the shared memory
+    k_fm_pairs_c<<<gc, 256, smem_r / 2, s>>>(a, tab, ntot, clist, ccnt, atom_sys, fm_nu, gp, nbr);
     launches += 4;
     BCUDA(cudaGetLastError(), "force matching launch");
     if (loss) BCUDA(cudaMemcpyAsync(loss, fm_loss, (size_t)nsys * sizeof(double), cudaMemcpyDeviceToHost, s), "loss");

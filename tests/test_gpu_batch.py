@@ -411,3 +411,25 @@ def test_tile_screen_forms_give_the_same_rows(gpu_lib, lanes, skin):
             assert got[0] == ref[0]
             for x, y in zip(got[1:], ref[1:]):
                 assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("nsys,n,gather", [(3, 5, 4), (37, 8, 2), (9, 14, 1), (31, 14, 4)])
+def test_fp64_lanes_follow_the_oracle_and_the_quench_walk(gpu_lib, oracle_mod, nsys, n, gather):
+    """The FP64 passes take four lanes per atom, two, or one as the batch grows
+    (750, 37,888, 49,392 and 170,128 atoms: 4 and 4, 2 and 2 or 1, 2 and 1, 1
+    and 1 in the density and the force pass): one system against the oracle,
+    every system against the row-order walk that the quench takes (its first
+    function value and the forces it leaves)."""
+    ws = mixed_systems([n] * (nsys - 1) + [n + 1 if n < 14 else n], seed=9)
+    with MoldyBatch.from_workloads(ws) as b:
+        b.set_gather(gather)
+        out = b.force()
+        f = b.forces()
+        w = ws[-1]
+        o, en = oracle_eval(oracle_mod, w)
+        assert rel_norm_err(b.split(f)[-1], o.forces()) <= 1e-10
+        assert abs(out["pe_calc"][-1] - en.sum()) <= 1e-10 * abs(en.sum())
+        assert rel_norm_err(out["tp"][-1], o.force_out()["tp"]) <= 1e-10
+        q = b.quench(maxfn=1)
+        assert np.max(np.abs(q["pe"] - out["pe_calc"]) / np.abs(q["pe"])) <= 1e-13
+        assert rel_norm_err(b.forces(), f) <= 1e-12
