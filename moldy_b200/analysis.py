@@ -65,11 +65,9 @@ def rneighbour(hist, natoms, binsperangstrom=50) -> np.ndarray:
         for jsp in range(isp, ns):
             irdf = hist[:, isp, jsp] + (hist[:, jsp, isp] if isp != jsp else 0)
             lim = 4 * min(int(natoms[isp]), int(natoms[jsp]))
-            icount = 0
-            for ibin in range(1, maxbin + 1):
-                if icount < lim:
-                    icount += int(irdf[ibin])
-                    rneighbour_ = float(np.float32(ibin) / np.float32(binsperangstrom))
+            if lim > 0 and maxbin >= 1:
+                ibin = 1 + min(int(np.searchsorted(np.cumsum(irdf[1:]), lim)), maxbin - 1)
+                rneighbour_ = float(np.float32(ibin) / np.float32(binsperangstrom))
             rn[isp, jsp] = rn[jsp, isp] = rneighbour_
     return rn
 
@@ -81,9 +79,9 @@ def ackland_jones(system, rn, mode="list", species=None, with_chi=True) -> dict:
     rn = np.ascontiguousarray(np.atleast_2d(rn), dtype=np.float64)
     sp, ns = _species(system, species, rn.shape[0])
     L = _lib.load()
-    aj = np.zeros(system.nm, dtype=np.int32)
-    nn = np.zeros(system.nm, dtype=np.int32)
-    chi = np.zeros(8 * system.nm, dtype=np.int32) if with_chi else None
+    aj = np.empty(system.nm, dtype=np.int32)
+    nn = np.empty(system.nm, dtype=np.int32)
+    chi = np.empty(8 * system.nm, dtype=np.int32) if with_chi else None
     check(L.moldy_gpu_ackland_jones(system._h, MODES[mode], None if sp is None else sp.ctypes.data_as(_lib.I), ns,
                                     rn.ctypes.data_as(_lib.D), aj.ctypes.data_as(_lib.I),
                                     nn.ctypes.data_as(_lib.I), None if chi is None else chi.ctypes.data_as(_lib.I)))

@@ -92,7 +92,7 @@ class MoldyBatch:
         return a
 
     def get_state(self) -> np.ndarray:
-        c = [np.zeros(self.ntot) for _ in range(3)]
+        c = [np.empty(self.ntot) for _ in range(3)]
         check(self._L.moldy_gpu_batch_get_state(self._h, *[_dp(a) for a in c]))
         return np.stack(c, axis=1)
 
@@ -115,9 +115,9 @@ class MoldyBatch:
         check(self._L.moldy_gpu_batch_force(self._h, _dp(out)))
 
     def forces(self) -> np.ndarray:
-        c = [np.zeros(self.ntot) for _ in range(3)]
-        check(self._L.moldy_gpu_batch_get_forces(self._h, *[_dp(a) for a in c]))
-        return np.stack(c, axis=1)
+        out = np.empty((self.ntot, 3))
+        self.forces_xyz_into(out)
+        return out
 
     def forces_into(self, fx, fy, fz):
         """Fractional forces into three preallocated contiguous float64 arrays."""

@@ -140,6 +140,54 @@ Profiler::~Profiler() {
         (E).prof.launches[(id)] += (nk);    \
     } while (0)
 
+// ---------------------------------------------------------- staged copies --
+CopyStage::~CopyStage() {
+    if (head) cudaFreeHost(head);
+    for (int k = 0; k < 2; ++k)
+        if (ev[k]) cudaEventDestroy(ev[k]);
+}
+
+cudaError_t CopyStage::open(size_t head_bytes) {
+    if (piece) return cudaSuccess;
+    const size_t hb = (head_bytes + 255) & ~(size_t)255;
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < 2 && e == cudaSuccess; ++k)
+        if (!ev[k]) e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&head, hb + 2 * kStageBytes);
+    if (e == cudaSuccess) piece = head + hb;
+    return e;
+}
+
+// Device to host.  Pageable memory is filled through two pinned pieces: the
+// copy of one runs while the host empties the other (1.3 MB in 120 us instead
+// of 270 us); complete on return.  Pinned destinations, and 64 KB or less,
+// which the driver stages as fast, are one queued copy: the caller waits for
+// the stream.
+cudaError_t CopyStage::out(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+    cudaPointerAttributes at;
+    const bool pinned = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+    if (!pinned) cudaGetLastError();
+    if (pinned || !piece || bytes <= 65536) {
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
+    }
+    const size_t n = (bytes + kStageBytes - 1) / kStageBytes;
+    for (size_t k = 0; k <= n; ++k) {
+        if (k < n) {
+            const size_t o = k * kStageBytes, len = bytes - o < kStageBytes ? bytes - o : kStageBytes;
+            cudaError_t e = cudaMemcpyAsync(piece + (k & 1) * kStageBytes, (const char *)src + o, len, cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaEventRecord(ev[k & 1], s);
+            if (e != cudaSuccess) return e;
+        }
+        if (k > 0) {
+            const size_t q = k - 1, o = q * kStageBytes, len = bytes - o < kStageBytes ? bytes - o : kStageBytes;
+            cudaError_t e = cudaEventSynchronize(ev[q & 1]);
+            if (e != cudaSuccess) return e;
+            std::memcpy((char *)dst + o, piece + (q & 1) * kStageBytes, len);
+        }
+    }
+    return cudaSuccess;
+}
+
 // ------------------------------------------------------------------ Engine --
 Engine::Engine(const moldy_params &p) {
     prm.rnear = p.rnear;
@@ -171,11 +219,10 @@ Engine::~Engine() {
                     d.znum, d.en_atom, d.ic, d.cell_start, d.cell_atoms, d.cell_pos, d.cell_count,
                     d.ic_new, d.arr_count, d.arr_start, d.arr_list, d.work, d.new_count,
                     d.new_start, d.cell_atoms2, d.nlist, d.numn, d.posq, d.posq2, d.pos2, d.alist,
-                    d.pair_cnt, d.olist, d.out_cnt, d.rlist, d.numr, d.xout, d.xhalf, d.mlist, d.mid_cnt, d.xbuild, d.tab_r4, d.tab_e2,
-                    d.tab_r4f, d.tab_e2f, d.tab_aux, d.partials, d.run_scratch, d.flags, d.revmask, d.box, d.scan_tmp, d.adj, d.rdf};
+                    d.pair_cnt, d.olist, d.out_cnt, d.rlist, d.numr, d.xout, d.xhalf, d.mlist, d.mid_cnt, d.xbuild,
+                    d.partials, d.run_scratch, d.flags, d.revmask, d.box, d.scan_tmp, d.adj, d.rdf};
     for (void *b : bufs)
         if (b) cudaFree(b);
-    if (host_box_) cudaFreeHost(host_box_);
     if (host_rec_) cudaFreeHost(host_rec_);
     if (d.thermo_rec) cudaFree(d.thermo_rec);
     if (stream_) cudaStreamDestroy(stream_);
@@ -286,93 +333,77 @@ int Engine::check_ready() {
     return MOLDY_OK;
 }
 
+DeviceTables::~DeviceTables() {
+    if (dev) cudaFree(dev);
+}
+
 // Device copies of the host tables (lookup_m layout): double4 r nodes up to
 // the first node from which vee, dvee, phi and dphi are all zero, double2 rho
 // nodes, FP32 copies of both, and the Tables descriptor.  rcull is the radius
 // at and beyond which every pair contributes exactly zero (exact mode: the
 // largest knot), times 1 + 1e-12; 1e150 when the tables never reach zero.
-int upload_device_tables(const HostTables &h, double4 **r4d, float4 **r4fd, double2 **e2d, float2 **e2fd,
-                         void **auxd,
-                         Tables &t, double *rcull_out) {
+// All of them lie in one block that is kept while it is large enough (a fit
+// sets new knots for every gradient; freeing and allocating five buffers took
+// half of that call) and filled by one copy in stream order.
+int upload_device_tables(const HostTables &h, DeviceTables &dt, cudaStream_t s, Tables &t, double *rcull_out) {
     int n = h.nlookup;
     int cut = n + 1;
     for (int i = n; i >= 0; --i) {
         if (h.vee[i] != 0.0 || h.dvee[i] != 0.0 || h.phi[i] != 0.0 || h.dphi[i] != 0.0) break;
         cut = i;
     }
-    int nr = (cut <= n - 1) ? cut + 2 : n + 1;
-    std::vector<double4> r4(nr);
+    const int nr = (cut <= n - 1) ? cut + 2 : n + 1;
+    // sections, each a multiple of 32 bytes long: the 256-bit loads stay aligned
+    const size_t nrs = (size_t)nr, pad = (nrs + 3) & ~(size_t)3;
+    const size_t o_df4 = nrs * sizeof(double4), o_r4f = o_df4 + nrs * sizeof(double4),
+                 o_phi2 = o_r4f + 2 * nrs * sizeof(float4), o_dv2 = o_phi2 + pad * sizeof(double2),
+                 o_dp2 = o_dv2 + pad * sizeof(double2), o_phi2f = o_dp2 + pad * sizeof(double2),
+                 o_e2 = o_phi2f + pad * sizeof(float2), bytes = o_e2 + ((size_t)n + 1) * sizeof(double2);
+    CUDA_CHECK(cudaStreamSynchronize(s), "tables");    // nothing queued reads the block any more
+    if (dt.cap < bytes) {
+        if (dt.dev) cudaFree(dt.dev);
+        dt.dev = nullptr;
+        dt.cap = 0;
+        CHECK(dev_alloc(&dt.dev, bytes, "tables"));
+        dt.host.resize(bytes + 32);
+        dt.cap = bytes;
+    }
+    unsigned char *hb = dt.host.data() + (-reinterpret_cast<uintptr_t>(dt.host.data()) & 31);   // 32-byte sections
+    double4 *r4 = reinterpret_cast<double4 *>(hb), *df4 = reinterpret_cast<double4 *>(hb + o_df4);
+    float4 *r4f = reinterpret_cast<float4 *>(hb + o_r4f);
+    double2 *phi2 = reinterpret_cast<double2 *>(hb + o_phi2), *dv2 = reinterpret_cast<double2 *>(hb + o_dv2),
+            *dp2 = reinterpret_cast<double2 *>(hb + o_dp2), *e2 = reinterpret_cast<double2 *>(hb + o_e2);
+    float2 *phi2f = reinterpret_cast<float2 *>(hb + o_phi2f);
     // FP32 nodes in pairs (node k, node k+1 - node k) so that one 32-byte load
     // brings an interval and its interpolation is one fused multiply-add per
     // value (the difference is the FP32 subtraction the device would do); the
-    // density table keeps (phi_k, phi_k+1 - phi_k) side by side
-    std::vector<float4> r4f(2 * (size_t)nr, make_float4(0.f, 0.f, 0.f, 0.f));
-    std::vector<double2> phi2(nr, make_double2(0.0, 0.0));
-    std::vector<float2> phi2f(nr, make_float2(0.f, 0.f));
+    // density table keeps (phi_k, phi_k+1 - phi_k) side by side; FP64 intervals
+    // as (node, step): (V', phi'), (V), (phi).  The last stored node has no
+    // step, so it is what every distance beyond it takes.
     for (int i = 0; i < nr; ++i) {
+        const int j = i + 1 < nr ? i + 1 : i;
         r4[i] = make_double4(h.vee[i], h.dvee[i], h.phi[i], h.dphi[i]);
-        const float4 q = make_float4((float)h.vee[i], (float)h.dvee[i], (float)h.phi[i], (float)h.dphi[i]);
-        r4f[2 * (size_t)i] = q;
-        phi2[i].x = h.phi[i];
-        phi2f[i].x = (float)h.phi[i];
-        if (i > 0) phi2[i - 1].y = h.phi[i];
-    }
-    for (int i = 0; i + 1 < nr; ++i) {
-        const float4 a = r4f[2 * (size_t)i], b = r4f[2 * (size_t)i + 2];
+        df4[i] = make_double4(h.dvee[i], h.dphi[i], h.dvee[j] - h.dvee[i], h.dphi[j] - h.dphi[i]);
+        dv2[i] = make_double2(h.vee[i], h.vee[j] - h.vee[i]);
+        dp2[i] = make_double2(h.phi[i], h.phi[j] - h.phi[i]);
+        phi2[i] = make_double2(h.phi[i], j > i ? h.phi[j] : 0.0);
+        const float4 a = make_float4((float)h.vee[i], (float)h.dvee[i], (float)h.phi[i], (float)h.dphi[i]);
+        const float4 b = make_float4((float)h.vee[j], (float)h.dvee[j], (float)h.phi[j], (float)h.dphi[j]);
+        r4f[2 * (size_t)i] = a;
         r4f[2 * (size_t)i + 1] = make_float4(b.x - a.x, b.y - a.y, b.z - a.z, b.w - a.w);
-        phi2f[i].y = phi2f[i + 1].x - phi2f[i].x;
+        phi2f[i] = make_float2(a.z, b.z - a.z);
     }
-    // FP64 intervals as (node, step): (V', phi') and (V), (phi); the last stored
-    // node has no step, so it is what every distance beyond it takes
-    std::vector<double4> df4(nr);
-    std::vector<double2> dv2(nr), dp2(nr);
-    for (int i = 0; i < nr; ++i) {
-        const double4 a = r4[i], b = r4[i + 1 < nr ? i + 1 : i];
-        df4[i] = make_double4(a.y, a.w, b.y - a.y, b.w - a.w);
-        dv2[i] = make_double2(a.x, b.x - a.x);
-        dp2[i] = make_double2(a.z, b.z - a.z);
-    }
-    std::vector<double2> e2(n + 1);
-    std::vector<float2> e2f(n + 1);
-    for (int i = 0; i <= n; ++i) {
-        e2[i] = make_double2(h.emb[i], h.demb[i]);
-        e2f[i] = make_float2((float)h.emb[i], (float)h.demb[i]);
-    }
-    void *old[] = {*r4d, *e2d, *r4fd, *e2fd, *auxd};
-    for (void *b : old)
-        if (b) cudaFree(b);
-    *r4d = nullptr; *e2d = nullptr; *r4fd = nullptr; *e2fd = nullptr; *auxd = nullptr;
-    CHECK(dev_alloc(r4d, nr, "tables"));
-    CHECK(dev_alloc(r4fd, 2 * (size_t)nr, "tables"));
-    // df4 (nr double4), phi2, dv2, dp2 (nr double2 each), then phi2f (nr float2), one copy
-    const size_t aux_bytes = (size_t)nr * (sizeof(double4) + 3 * sizeof(double2) + sizeof(float2));
-    std::vector<unsigned char> aux_h(aux_bytes);
-    size_t off = 0;
-    size_t at[5];
-    const void *parts[5] = {df4.data(), phi2.data(), dv2.data(), dp2.data(), phi2f.data()};
-    const size_t sizes[5] = {sizeof(double4), sizeof(double2), sizeof(double2), sizeof(double2), sizeof(float2)};
-    for (int k = 0; k < 5; ++k) {
-        at[k] = off;
-        std::memcpy(aux_h.data() + off, parts[k], nr * sizes[k]);
-        off += nr * sizes[k];
-    }
-    unsigned char *aux = nullptr;
-    CHECK(dev_alloc(&aux, aux_bytes, "tables"));
-    *auxd = aux;
-    CHECK(dev_alloc(e2d, n + 1, "tables"));
-    CHECK(dev_alloc(e2fd, n + 1, "tables"));
-    CUDA_CHECK(cudaMemcpy(*r4d, r4.data(), nr * sizeof(double4), cudaMemcpyHostToDevice), "tables");
-    CUDA_CHECK(cudaMemcpy(*r4fd, r4f.data(), 2 * (size_t)nr * sizeof(float4), cudaMemcpyHostToDevice), "tables");
-    CUDA_CHECK(cudaMemcpy(aux, aux_h.data(), aux_bytes, cudaMemcpyHostToDevice), "tables");
-    CUDA_CHECK(cudaMemcpy(*e2d, e2.data(), (n + 1) * sizeof(double2), cudaMemcpyHostToDevice), "tables");
-    CUDA_CHECK(cudaMemcpy(*e2fd, e2f.data(), (n + 1) * sizeof(float2), cudaMemcpyHostToDevice), "tables");
-
-    t.r4 = *r4d; t.e2 = *e2d; t.r4f = *r4fd; t.e2f = *e2fd;
-    t.df4 = reinterpret_cast<const double4 *>(aux + at[0]);
-    t.phi2 = reinterpret_cast<const double2 *>(aux + at[1]);
-    t.dv2 = reinterpret_cast<const double2 *>(aux + at[2]);
-    t.dp2 = reinterpret_cast<const double2 *>(aux + at[3]);
-    t.phi2f = reinterpret_cast<const float2 *>(aux + at[4]);
+    for (int i = 0; i <= n; ++i) e2[i] = make_double2(h.emb[i], h.demb[i]);
+    CUDA_CHECK(cudaMemcpyAsync(dt.dev, hb, bytes, cudaMemcpyHostToDevice, s), "tables");
+    CUDA_CHECK(cudaStreamSynchronize(s), "tables");
+    t.r4 = reinterpret_cast<const double4 *>(dt.dev);
+    t.df4 = reinterpret_cast<const double4 *>(dt.dev + o_df4);
+    t.r4f = reinterpret_cast<const float4 *>(dt.dev + o_r4f);
+    t.phi2 = reinterpret_cast<const double2 *>(dt.dev + o_phi2);
+    t.dv2 = reinterpret_cast<const double2 *>(dt.dev + o_dv2);
+    t.dp2 = reinterpret_cast<const double2 *>(dt.dev + o_dp2);
+    t.phi2f = reinterpret_cast<const float2 *>(dt.dev + o_phi2f);
+    t.e2 = reinterpret_cast<const double2 *>(dt.dev + o_e2);
     t.nlookup = n;
     t.nr = nr;
     t.idx_cut = cut;
@@ -418,7 +449,7 @@ int set_last_error(int code, const std::string &msg) { return fail(code, msg); }
 
 int Engine::upload_tables() {
     double rc = 0.0;
-    CHECK(upload_device_tables(ht, &d.tab_r4, &d.tab_r4f, &d.tab_e2, &d.tab_e2f, &d.tab_aux, tab, &rc));
+    CHECK(upload_device_tables(ht, tabs, stream_, tab, &rc));
     rcut = rc < 1e150 ? rc : prm.rnear;
     set_list_radii();
     potential_set_ = true;
@@ -511,22 +542,29 @@ int Engine::set_state(const double *x0, const double *y0, const double *z0, cons
     return MOLDY_OK;
 }
 
+int Engine::open_stage() {
+    CUDA_CHECK(stage.open(sizeof(BoxState)), "pinned staging");
+    host_box_ = reinterpret_cast<BoxState *>(stage.head);
+    return MOLDY_OK;
+}
+
 int Engine::get_state(double *x0, double *y0, double *z0, double *x1, double *y1, double *z1,
                       double *x2, double *y2, double *z2, double *b0, double *b1, double *b2,
                       double *tgid) {
     size_t nm = (size_t)prm.nm, nb = nm * sizeof(double);
     cudaStream_t s = stream_;
+    CHECK(open_stage());
     if (x0 || y0 || z0) {
         double *tmp = d.en_atom;
         k_unpack_pos<<<(prm.nm + 255) / 256, 256, 0, s>>>(prm.nm, d.pos, tmp);
-        if (x0) CUDA_CHECK(cudaMemcpyAsync(x0, tmp, nb, cudaMemcpyDeviceToHost, s), "get x0");
-        if (y0) CUDA_CHECK(cudaMemcpyAsync(y0, tmp + nm, nb, cudaMemcpyDeviceToHost, s), "get y0");
-        if (z0) CUDA_CHECK(cudaMemcpyAsync(z0, tmp + 2 * nm, nb, cudaMemcpyDeviceToHost, s), "get z0");
+        if (x0) CUDA_CHECK(stage.out(x0, tmp, nb, s), "get x0");
+        if (y0) CUDA_CHECK(stage.out(y0, tmp + nm, nb, s), "get y0");
+        if (z0) CUDA_CHECK(stage.out(z0, tmp + 2 * nm, nb, s), "get z0");
     }
     double *v1[3] = {x1, y1, z1}, *v2[3] = {x2, y2, z2};
     for (int k = 0; k < 3; ++k) {
-        if (v1[k]) CUDA_CHECK(cudaMemcpyAsync(v1[k], d.x1 + k * nm, nb, cudaMemcpyDeviceToHost, s), "get x1");
-        if (v2[k]) CUDA_CHECK(cudaMemcpyAsync(v2[k], d.x2 + k * nm, nb, cudaMemcpyDeviceToHost, s), "get x2");
+        if (v1[k]) CUDA_CHECK(stage.out(v1[k], d.x1 + k * nm, nb, s), "get x1");
+        if (v2[k]) CUDA_CHECK(stage.out(v2[k], d.x2 + k * nm, nb, s), "get x2");
     }
     if (b0) CUDA_CHECK(cudaMemcpyAsync(b0, d.box->b0, 9 * sizeof(double), cudaMemcpyDeviceToHost, s), "get b0");
     if (b1) CUDA_CHECK(cudaMemcpyAsync(b1, d.box->b1, 9 * sizeof(double), cudaMemcpyDeviceToHost, s), "get b1");
@@ -539,17 +577,19 @@ int Engine::get_state(double *x0, double *y0, double *z0, double *x1, double *y1
 int Engine::get_array3(const double *dev, double *a, double *b, double *c) {
     size_t nm = (size_t)prm.nm, nb = nm * sizeof(double);
     double *o[3] = {a, b, c};
+    CHECK(open_stage());
     for (int k = 0; k < 3; ++k)
-        if (o[k]) CUDA_CHECK(cudaMemcpyAsync(o[k], dev + k * nm, nb, cudaMemcpyDeviceToHost, stream_), "get array");
+        if (o[k]) CUDA_CHECK(stage.out(o[k], dev + k * nm, nb, stream_), "get array");
     CUDA_CHECK(cudaStreamSynchronize(stream_), "get array");
     return MOLDY_OK;
 }
 
 int Engine::get_density(double *rho, double *afrho, double *dafrho) {
     size_t nb = (size_t)prm.nm * sizeof(double);
-    if (rho) CUDA_CHECK(cudaMemcpyAsync(rho, d.rho, nb, cudaMemcpyDeviceToHost, stream_), "get rho");
-    if (afrho) CUDA_CHECK(cudaMemcpyAsync(afrho, d.afrho, nb, cudaMemcpyDeviceToHost, stream_), "get afrho");
-    if (dafrho) CUDA_CHECK(cudaMemcpyAsync(dafrho, d.dafrho, nb, cudaMemcpyDeviceToHost, stream_), "get dafrho");
+    CHECK(open_stage());
+    if (rho) CUDA_CHECK(stage.out(rho, d.rho, nb, stream_), "get rho");
+    if (afrho) CUDA_CHECK(stage.out(afrho, d.afrho, nb, stream_), "get afrho");
+    if (dafrho) CUDA_CHECK(stage.out(dafrho, d.dafrho, nb, stream_), "get dafrho");
     CUDA_CHECK(cudaStreamSynchronize(stream_), "get density");
     return MOLDY_OK;
 }
@@ -721,10 +761,7 @@ int Engine::force_device(bool *rebuilt) {
 }
 
 int Engine::fetch_force_out(moldy_force_out *out) {
-    if (!host_box_) {
-        CUDA_CHECK(cudaMallocHost((void **)&host_box_, sizeof(BoxState) * 4), "pinned staging");
-        host_box_cap_ = 4;
-    }
+    CHECK(open_stage());
     CUDA_CHECK(cudaMemcpyAsync(host_box_, d.box, sizeof(BoxState), cudaMemcpyDeviceToHost, stream_), "box");
     CHECK(check_flags());
     CUDA_CHECK(cudaGetLastError(), "force");
@@ -825,10 +862,7 @@ int Engine::velocityverlet(moldy_force_out *out) {
 int Engine::update_therm_avs(double *s123) {
     CHECK(check_ready());
     LAUNCH(*this, K_THERM, 2, stream_, launch_therm(d, prm, true, nullptr, stream_));   // prep, sums
-    if (!host_box_) {
-        CUDA_CHECK(cudaMallocHost((void **)&host_box_, sizeof(BoxState) * 4), "pinned staging");
-        host_box_cap_ = 4;
-    }
+    CHECK(open_stage());
     CUDA_CHECK(cudaMemcpyAsync(host_box_, d.box, sizeof(BoxState), cudaMemcpyDeviceToHost, stream_), "box");
     CHECK(check_flags());
     if (s123) { s123[0] = host_box_[0].s1; s123[1] = host_box_[0].s2; s123[2] = host_box_[0].s3; }

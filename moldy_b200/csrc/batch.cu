@@ -1690,13 +1690,12 @@ class BatchEngine {
     int pair_cap = 48;                  // compact-row entries per atom
     double4 *spos = nullptr;
     CgState *cg = nullptr;
-    double4 *tab_r4 = nullptr;
-    double2 *tab_e2 = nullptr;
-    float4 *tab_r4f = nullptr;
-    float2 *tab_e2f = nullptr;
-    void *tab_aux = nullptr;
+    DeviceTables tabs;
+    CopyStage copies;
+    int32_t *host_flags = nullptr;      // there too: overflow flags, results of one evaluation
+    double *host_out = nullptr;
     double *stage = nullptr;            // host-to-device staging (3*ntot)
-    int *host_active = nullptr;         // pinned
+    int *host_active = nullptr;         // in the pinned head of copies
     cudaGraphExec_t graph = nullptr;
     int graph_lph = -1, graph_cap = -1, graph_maxfn = -1, graph_criterion = -1, graph_gather = -1;
     double graph_fmax = -1.0;
@@ -1795,12 +1794,11 @@ BatchEngine::~BatchEngine() {
     if (graph) cudaGraphExecDestroy(graph);
     drop_force_graph();
     void *bufs[] = {sys, atom_sys, cell_sys, cell_of, cell_count, cell_start, cursor, unsorted, sorted, n_active, X, Xb,
-                    mass, f, rho, afrho, fp, en_calc, en_force, vir, sfp, sysout, cgv, spos, cg, tab_r4, tab_e2,
-                    tab_r4f, tab_e2f, tab_aux, stage, alist, pcnt, clist, ccnt, flags, stats, todo, ntodo, cg_order,
+                    mass, f, rho, afrho, fp, en_calc, en_force, vir, sfp, sysout, cgv, spos, cg, stage, alist, pcnt, clist, ccnt, flags, stats, todo, ntodo, cg_order,
                     fm_fref, fm_sref, fm_gF, fm_gS, fm_loss, fm_mu, fm_nu, fm_grads, queue};
     for (void *b : bufs)
         if (b) cudaFree(b);
-    if (host_active) cudaFreeHost(host_active);
+
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -1868,7 +1866,10 @@ int BatchEngine::init(int n, const int32_t *na, double p, int dev) {
     BCUDA(cudaMemset(queue, 0, 2 * sizeof(int32_t)), "system queue");
     BCUDA(cudaMemset(ntodo, 0, sizeof(int32_t)), "screen work count");
     BCUDA(cudaMemset(stats, 0, 2 * sizeof(unsigned long long)), "list statistics");
-    BCUDA(cudaMallocHost((void **)&host_active, sizeof(int)), "pinned");
+    BCUDA(copies.open(16 + 13 * (size_t)n * sizeof(double)), "pinned");
+    host_active = reinterpret_cast<int *>(copies.head);
+    host_flags = reinterpret_cast<int32_t *>(copies.head + 8);
+    host_out = reinterpret_cast<double *>(copies.head + 16);
     std::vector<int32_t> as(nt);
     for (int s = 0; s < n; ++s)
         for (int i = 0; i < na[s]; ++i) as[atom0[s] + i] = s;
@@ -1890,15 +1891,19 @@ int BatchEngine::set_fetm(int nv, const double *av, const double *rv, int np, co
     int rc = build_fetm_tables(ht, nv, av, rv, np, ap, rp, 1, nlookup);
     if (rc != MOLDY_OK) return set_last_error(rc, "FETRANSMETAL set-up failed");
     double rcull = 0.0;
-    BCHECK(upload_device_tables(ht, &tab_r4, &tab_r4f, &tab_e2, &tab_e2f, &tab_aux, tab, &rcull));
-    drop_force_graph();   // the graph holds the table descriptor and the cut
+    BCHECK(upload_device_tables(ht, tabs, stream, tab, &rcull));
+    drop_force_graph();   // the graphs hold the table descriptor and the cut
+    if (graph) { cudaGraphExecDestroy(graph); graph = nullptr; }
     // every pair beyond the table cut and the pair function's knots contributes zero
     double r = rcull < 1e150 ? rcull : 0.0;
     for (int i = 0; i < nv; ++i) r = std::max(r, rv[i] * (1.0 + 1e-12));
     if (!(r > 0.0) || r > 1e100) return set_last_error(MOLDY_ERR_UNSUPPORTED, "tables without a finite cut");
+    // the lists depend on the positions, the boxes, the skin and this radius
+    // alone: new functions with the same cut leave them as they are
+    const bool same_cut = potential_set && r == rcut;
     rcut = r;
     potential_set = true;
-    if (boxes_set) return layout();
+    if (boxes_set && !same_cut) return layout();
     return MOLDY_OK;
 }
 
@@ -2139,10 +2144,11 @@ void BatchEngine::queue_evaluation(bool with_vir, bool use_mixed, bool ecalc, cu
 // list stale (the caller evaluates again) and returns the largest row seen,
 // or 0
 int BatchEngine::take_overflow() {
-    int32_t h[2] = {0, 0};
-    if (cudaMemcpy(h, flags, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
+    if (cudaMemcpyAsync(host_flags, flags, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, stream) != cudaSuccess) return -1;
+    if (cudaStreamSynchronize(stream) != cudaSuccess) return -1;
+    const int32_t h[2] = {host_flags[0], host_flags[1]};
     if (!h[0]) return 0;
-    cudaMemset(flags, 0, sizeof(h));
+    if (cudaMemsetAsync(flags, 0, sizeof(h), stream) != cudaSuccess) return -1;
     int need = h[1] + 8;
     if (alist) cudaFree(alist);
     alist = nullptr;
@@ -2280,15 +2286,18 @@ int BatchEngine::force(double *out13) {
     BCHECK(ready());
     for (int attempt = 0;; ++attempt) {
         BCHECK(evaluate_once(true));
-        BCUDA(cudaStreamSynchronize(stream), "batch force");
+        // the results and the overflow flags come back behind the launches: one wait
+        if (out13)
+            BCUDA(cudaMemcpyAsync(host_out, sysout, 13 * (size_t)nsys * sizeof(double), cudaMemcpyDeviceToHost, stream),
+                  "results");
         BCUDA(cudaGetLastError(), "batch force");
         int ov = take_overflow();
+        BCUDA(cudaGetLastError(), "batch force");
         if (ov < 0) return set_last_error(MOLDY_ERR_CUDA, "compact list re-allocation failed");
         if (ov == 0) break;
         if (attempt >= 2) return set_last_error(MOLDY_ERR_CAPACITY, "compact list keeps overflowing");
     }
-    if (out13)
-        BCUDA(cudaMemcpy(out13, sysout, 13 * (size_t)nsys * sizeof(double), cudaMemcpyDeviceToHost), "results");
+    if (out13) std::memcpy(out13, host_out, 13 * (size_t)nsys * sizeof(double));
     return MOLDY_OK;
 }
 
@@ -2432,7 +2441,6 @@ int BatchEngine::force_matching(double wf, double ws, double *loss, double *grad
         queue_evaluation(true, false, false);
         k_sys_reduce<<<nsys, kCgThreads, 0, stream>>>(sys, en_calc, en_force, vir, f, 1, sysout);
         launches += 2;
-        BCUDA(cudaStreamSynchronize(stream), "force matching");
         int ov = take_overflow();
         if (ov < 0) return set_last_error(MOLDY_ERR_CUDA, "compact list re-allocation failed");
         if (ov == 0) break;
@@ -2498,10 +2506,9 @@ int BatchEngine::get_array(const double *dev, int stride, double *a, double *b, 
         double *outs[3] = {a, b, c};
         for (int k = 0; k < 3; ++k)
             if (outs[k])
-                BCUDA(cudaMemcpyAsync(outs[k], stage + k * nt, nt * sizeof(double), cudaMemcpyDeviceToHost, stream),
-                      "copy back");
+                BCUDA(copies.out(outs[k], stage + k * nt, nt * sizeof(double), stream), "copy back");
     } else if (a) {
-        BCUDA(cudaMemcpyAsync(a, dev, nt * sizeof(double), cudaMemcpyDeviceToHost, stream), "copy back");
+        BCUDA(copies.out(a, dev, nt * sizeof(double), stream), "copy back");
     }
     BCUDA(cudaStreamSynchronize(stream), "copy back");
     return MOLDY_OK;
@@ -2517,7 +2524,7 @@ int BatchEngine::copy_xyz(double *dev, const double *src, double *dst) {
         pos_set = true;
         state_set = pos_set && boxes_set;
     }
-    if (dst) BCUDA(cudaMemcpyAsync(dst, dev, bytes, cudaMemcpyDeviceToHost, stream), "copy back");
+    if (dst) BCUDA(copies.out(dst, dev, bytes, stream), "copy back");
     BCUDA(cudaStreamSynchronize(stream), "interleaved copy");
     return MOLDY_OK;
 }

@@ -57,7 +57,6 @@ struct Tables {
     const double4 *r4;      // per node (vee, dvee, phi, dphi), nodes 0..nr-1
     const double2 *e2;      // per node (emb, demb), nodes 0..nlookup
     const float4 *r4f;      // FP32 copy of r4 for the mixed path, node pairs: [2k] = node k, [2k+1] = node k+1
-    const float2 *e2f;
     const double2 *phi2;    // per node k (phi_k, phi_k+1): one load per density lookup
     const double4 *df4;     // per interval (dvee, dphi, their steps to the next node); the last has step zero
     const double2 *dv2, *dp2;   // per interval (vee, step) and (phi, step)

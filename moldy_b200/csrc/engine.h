@@ -67,12 +67,6 @@ struct DeviceState {
     // xbuild holds the positions at build time
     int32_t *mlist = nullptr, *mid_cnt = nullptr;
     int4 *xbuild = nullptr;                // fixed-point (posq) snapshot
-    // tables
-    double4 *tab_r4 = nullptr;
-    double2 *tab_e2 = nullptr;
-    float4 *tab_r4f = nullptr;
-    float2 *tab_e2f = nullptr;
-    void *tab_aux = nullptr;               // phi2 / phi2f node-pair tables
     // per-step thermo records of an md_steps call (kThermoRec doubles each), grown on demand
     double *thermo_rec = nullptr;
     int thermo_cap = 0;
@@ -124,6 +118,25 @@ struct HostTables {
     double av[8] = {0}, rv[8] = {0}, ap[8] = {0}, rp[8] = {0};
     double bier_cut1 = 0, bier_cut2 = 0, sc[4] = {0, 0, 0, 0};
     double phi_cut1 = 0, phi_cut2 = 0, bier_a = 0, bier_zed = 0;
+};
+
+// The device block of the tables, kept while it is large enough.
+struct DeviceTables {
+    unsigned char *dev = nullptr;
+    size_t cap = 0;
+    std::vector<unsigned char> host;
+    ~DeviceTables();
+};
+
+// One pinned allocation per engine, made on first use: a head for small
+// results and two pieces for copies into pageable memory.
+constexpr size_t kStageBytes = 256 << 10;
+struct CopyStage {
+    unsigned char *head = nullptr, *piece = nullptr;
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    cudaError_t open(size_t head_bytes);
+    cudaError_t out(void *dst, const void *src, size_t bytes, cudaStream_t s);
+    ~CopyStage();
 };
 
 // Kernel families timed by the optional per-kernel CUDA-event profiler.
@@ -222,6 +235,9 @@ class Engine {
     Params prm;
     HostTables ht;
     Tables tab;
+    DeviceTables tabs;
+    CopyStage stage;
+    int open_stage();
 
   private:
     int check_ready();
@@ -259,8 +275,7 @@ class Engine {
     void clear_mid_dirty() { mid_dirty_ = false; }
   private:
     double *part_embed_ = nullptr, *part_force_ = nullptr;   // slices of d.partials
-    BoxState *host_box_ = nullptr;                            // pinned staging
-    int host_box_cap_ = 0;
+    BoxState *host_box_ = nullptr;                            // the head of the pinned stage
     double *host_rec_ = nullptr;                              // pinned thermo records
     int host_rec_cap_ = 0;
 };
@@ -369,9 +384,7 @@ void launch_count_screened(const DeviceState &d, const Params &p, unsigned long 
 size_t adjoint_smem_bytes(int nlookup);
 void launch_table_adjoint(const DeviceState &d, const AdjointArgs &a, double *grads, double *scr,
                           const double *gF, cudaStream_t s);
-int upload_device_tables(const HostTables &h, double4 **r4d, float4 **r4fd, double2 **e2d, float2 **e2fd,
-                         void **auxd,
-                         Tables &t, double *rcull_out);
+int upload_device_tables(const HostTables &h, DeviceTables &dt, cudaStream_t s, Tables &t, double *rcull_out);
 int build_fetm_tables(HostTables &ht, int nv, const double *av, const double *rv, int np,
                       const double *ap, const double *rp, int uselookup, int nlookup);
 int set_last_error(int code, const std::string &msg);

@@ -600,11 +600,10 @@ int Engine::ackland_jones(int mode, const int32_t *species, int nspec, const dou
     prof.launches[K_RDF] += 1;
     int32_t flag = 0;
     RCUDA(cudaMemcpyAsync(&flag, a.flags, sizeof(int32_t), cudaMemcpyDeviceToHost, s), "analysis flag");
-    RCUDA(cudaMemcpyAsync(aj, o, nm * sizeof(int32_t), cudaMemcpyDeviceToHost, s), "classes");
-    RCUDA(cudaMemcpyAsync(nn, o + nm, nm * sizeof(int32_t), cudaMemcpyDeviceToHost, s), "coordination");
-    if (chi)
-        RCUDA(cudaMemcpyAsync(chi, o + 2 * (size_t)nm, 8 * (size_t)nm * sizeof(int32_t), cudaMemcpyDeviceToHost, s),
-              "angle counts");
+    RCHECK(open_stage());
+    RCUDA(stage.out(aj, o, nm * sizeof(int32_t), s), "classes");
+    RCUDA(stage.out(nn, o + nm, nm * sizeof(int32_t), s), "coordination");
+    if (chi) RCUDA(stage.out(chi, o + 2 * (size_t)nm, 8 * (size_t)nm * sizeof(int32_t), s), "angle counts");
     RCUDA(cudaStreamSynchronize(s), "ackland_jones");
     RCUDA(cudaGetLastError(), "ackland_jones");
     if (flag)

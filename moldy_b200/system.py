@@ -25,11 +25,16 @@ Every call goes through ``libmoldy_gpu.so``; errors come back as
 from __future__ import annotations
 
 import ctypes
+import struct
 
 import numpy as np
 
 from . import _lib
 from ._lib import check
+
+_THERMO_KEYS = [f[0] for f in _lib.Thermo._fields_]
+_THERMO_REC = struct.Struct("11d2i")       # _lib.Thermo
+assert _THERMO_REC.size == ctypes.sizeof(_lib.Thermo)
 
 
 def _f64(a):
@@ -168,7 +173,7 @@ class MoldySystem:
 
     def get_state(self) -> dict:
         n = self.nm
-        cols = [np.zeros(n) for _ in range(9)]
+        cols = [np.empty(n) for _ in range(9)]
         mats = [np.zeros(9) for _ in range(4)]
         check(self._L.moldy_gpu_get_state(self._h, *[_dp(c) for c in cols],
                                           *[_dp(m) for m in mats]))
@@ -183,7 +188,7 @@ class MoldySystem:
         return _mat_from_f(m)
 
     def forces(self) -> np.ndarray:
-        f = [np.zeros(self.nm) for _ in range(3)]
+        f = [np.empty(self.nm) for _ in range(3)]
         check(self._L.moldy_gpu_get_forces(self._h, *[_dp(a) for a in f]))
         return np.stack(f, axis=1)
 
@@ -305,8 +310,9 @@ class MoldySystem:
             return None
         arr = (_lib.Thermo * max(int(nsteps), 1))()
         check(self._L.moldy_gpu_md_steps(self._h, int(nsteps), arr))
-        keys = [f[0] for f in _lib.Thermo._fields_]
-        return [{k: getattr(arr[i], k) for k in keys} for i in range(int(nsteps))]
+        # the records as native tuples: an attribute read of a ctypes field costs
+        # 0.2 us, a fifth of 100 fused steps of a small system
+        return [dict(zip(_THERMO_KEYS, rec)) for rec in _THERMO_REC.iter_unpack(memoryview(arr).cast("B"))][:int(nsteps)]
 
     def set_thermostat(self, nose: float, rqke: float):
         """simparam%nose and simparam%rqke of scalev; nose = 0 switches it off."""

@@ -433,3 +433,39 @@ def test_fp64_lanes_follow_the_oracle_and_the_quench_walk(gpu_lib, oracle_mod, n
         q = b.quench(maxfn=1)
         assert np.max(np.abs(q["pe"] - out["pe_calc"]) / np.abs(q["pe"])) <= 1e-13
         assert rel_norm_err(b.forces(), f) <= 1e-12
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_new_functions_on_kept_lists_and_tables(gpu_lib, prec):
+    """A potential set on an engine that holds lists, table buffers and captured
+    graphs of an earlier one: same cut, shorter cut, longer cut, larger and
+    smaller tables, each followed by an evaluation and a quench, against an
+    engine that saw nothing else.  Same pairs and terms, sums in FP64 of some 60
+    terms in another order at most: 1e-12 (mixed: 1e-6 for the FP32 terms)."""
+    from dataclasses import replace
+
+    from moldy_b200.potentials import FE_FE
+
+    def cut(scale):
+        return replace(FE_FE, rv=tuple(scale * np.asarray(FE_FE.rv)), rp=tuple(scale * np.asarray(FE_FE.rp)))
+
+    soft = replace(FE_FE, av=tuple(1.01 * np.asarray(FE_FE.av)))
+    ws = mixed_systems([4, 5, 4], seed=12)
+    tol = 1e-12 if prec == "fp64" else 1e-6
+    with MoldyBatch.from_workloads(ws) as b:
+        b.set_precision(prec)
+        b.force()
+        b.quench(maxfn=2)
+        for pot, nl in [(soft, 5000), (cut(0.97), 5000), (cut(1.03), 9000), (FE_FE, 2000), (FE_FE, 5000)]:
+            x = np.concatenate([w.x0 for w in ws])
+            with MoldyBatch.from_workloads(ws) as ref:
+                ref.set_precision(prec)
+                for e in (ref, b):
+                    e.set_up_fetm(pot, nlookup=nl)
+                    e.set_positions(x)
+                o, r = b.force(), ref.force()
+                assert np.max(np.abs(o["pe"] - r["pe"]) / np.abs(r["pe"])) <= tol
+                assert rel_norm_err(b.forces(), ref.forces()) <= tol
+                q, p = b.quench(maxfn=2), ref.quench(maxfn=2)
+                assert np.max(np.abs(q["pe"] - p["pe"]) / np.abs(p["pe"])) <= 1e-12
+                assert rel_norm_err(b.get_state(), ref.get_state()) <= 1e-12
