@@ -32,6 +32,7 @@ namespace moldy {
 namespace {
 
 constexpr int kRdfThreads = 256;
+constexpr int kRowThreads = 256;      // of the kernels that walk half-list rows
 constexpr int kNearCap = 32;          // neighbours inside the Ackland-Jones cutoff per atom
 constexpr int kMaxSpecies = 8;
 constexpr int kSmemHistBytes = 48 * 1024;
@@ -108,59 +109,52 @@ __device__ void init_block(const HistArgs &a, unsigned int *sh, unsigned int *sc
     __syncthreads();
 }
 
-// mode 0: the half-list rows (src/analysis_m.F90:580-608).  The lanes of a
-// warp walk their rows in step; lanes whose pairs fall in the same bin are
-// grouped with __match_any_sync and one of them adds the group's count, since
-// the pairs of neighbouring atoms crowd into the same few shell bins.
+// mode 0: the half-list rows (src/analysis_m.F90:580-608).  kRowLanes lanes
+// share the row of an atom, so that a row is read in whole sectors and the
+// gathers of kHistBatch entries per lane are under way together: what bounds
+// the walk is their latency.  The lanes add to the shared histogram one by
+// one; one lane per row, which grouped the lanes of equal bins first
+// (__match_any_sync), took 123 us for 128,000 atoms, this 62 us (two entries
+// under way: 75 us).  FP32 roots with a guard in place of the FP64 ones, and
+// image corrections behind a branch, were slower (83 us).
+constexpr int kRowLanes = 8, kHistBatch = 4, kNearBatch = 2;
+
 template <bool SMEM>
-__global__ void __launch_bounds__(kRdfThreads)
+__global__ void __launch_bounds__(kRowThreads, 4)
 k_rdf_list(HistArgs a, const int32_t *__restrict__ nlist, const int32_t *__restrict__ numn) {
     extern __shared__ unsigned int sh[];
     __shared__ double b[9];
     __shared__ unsigned int sclose, snat[kMaxSpecies];
     init_block<SMEM>(a, sh, &sclose, b, snat);
-    const int lane = threadIdx.x & 31;
+    const int l = threadIdx.x & (kRowLanes - 1), groups = blockDim.x / kRowLanes;
     unsigned int close = 0;
-    // block-uniform loop: every lane takes part in every __match_any_sync
-    for (int base = blockIdx.x * blockDim.x; base < a.nm; base += gridDim.x * blockDim.x) {
-        const int i = base + threadIdx.x;
-        const bool live = i < a.nm && a.znum[i] != 0;
-        const int si = live ? species_of(a.spec, i) : 0;
-        if (live) atomicAdd(&snat[si], 1u);
-        const double4 pi = live ? a.pos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
-        const int n = live ? numn[i] : 0;
-        const int nmax = __reduce_max_sync(0xffffffffu, n);
-        // four row entries gathered before they are evaluated
-        for (int k0 = 0; k0 < nmax; k0 += 4) {
-            int jj[4];
-            double4 pp[4];
-            int zz[4];
+    for (int i = blockIdx.x * groups + threadIdx.x / kRowLanes; i < a.nm; i += gridDim.x * groups) {
+        if (a.znum[i] == 0) continue;
+        const int si = species_of(a.spec, i);
+        if (l == 0) atomicAdd(&snat[si], 1u);
+        const double4 pi = a.pos[i];
+        const int n = numn[i];
+        const int32_t *row = nlist + (size_t)i * a.nnbrs;
+        for (int k0 = l; k0 < n; k0 += kRowLanes * kHistBatch) {
+            int jj[kHistBatch], zz[kHistBatch];
+            double4 pp[kHistBatch];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) jj[u] = k0 + u < n ? nlist[(size_t)i * a.nnbrs + k0 + u] : -1;
+            for (int u = 0; u < kHistBatch; ++u) jj[u] = k0 + u * kRowLanes < n ? row[k0 + u * kRowLanes] : -1;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int j = jj[u] >= 0 ? jj[u] : 0;
+            for (int u = 0; u < kHistBatch; ++u) {
+                const int j = jj[u] >= 0 ? jj[u] : i;
                 pp[u] = a.pos[j];
                 zz[u] = a.znum[j];
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (k0 + u >= nmax) break;                 // warp-uniform
-                int key = -1;
-                if (jj[u] >= 0 && zz[u] != 0) {
-                    const double rsq = pair_sep2(b, a.ivol, pi, pp[u]);
-                    if (!(rsq > a.rsqmax)) {
-                        const double r = __dsqrt_rn(rsq);
-                        const int ibin = (int)__dmul_rn(r, (double)a.bpa);
-                        if (r <= 2.0) close += 1;
-                        if (ibin <= a.maxbin) key = (ibin * a.nspec + si) * a.nspec + species_of(a.spec, jj[u]);
-                    }
-                }
-                const unsigned int m = __match_any_sync(0xffffffffu, key);
-                if (key >= 0 && lane == __ffs(m) - 1) {
-                    if (SMEM) atomicAdd(&sh[key], (unsigned int)__popc(m));
-                    else atomicAdd(&a.hist[key], (unsigned long long)__popc(m));
-                }
+            for (int u = 0; u < kHistBatch; ++u) {
+                if (jj[u] < 0 || zz[u] == 0) continue;
+                const double rsq = pair_sep2(b, a.ivol, pi, pp[u]);
+                if (rsq > a.rsqmax) continue;
+                const double r = __dsqrt_rn(rsq);
+                const int ibin = (int)__dmul_rn(r, (double)a.bpa);
+                if (r <= 2.0) close += 1;
+                if (ibin <= a.maxbin) hist_add<SMEM>(a, sh, ibin, si, species_of(a.spec, jj[u]));
             }
         }
     }
@@ -260,23 +254,53 @@ __device__ __forceinline__ void near_add(const AjArgs &a, int i, int j) {
     else atomicExch(&a.flags[0], 1);
 }
 
-// mode 0: the full list of analysis_m.F90:562-578 from the half-list rows
-__global__ void __launch_bounds__(kRdfThreads)
+// mode 0: the full list of analysis_m.F90:562-578 from the half-list rows,
+// walked as in k_rdf_list; the lanes of a row take its slots with one atomic
+// (128,000 atoms: 111 us with one lane per row and an atomic per entry, 77 us).
+__global__ void __launch_bounds__(kRowThreads, 5)
 k_aj_near_list(AjArgs a, const int32_t *__restrict__ nlist, const int32_t *__restrict__ numn) {
     __shared__ double b[9];
     if (threadIdx.x < 9) b[threadIdx.x] = a.box->b0[threadIdx.x];
     __syncthreads();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nm; i += gridDim.x * blockDim.x) {
-        const double4 pi = a.pos[i];
-        const int si = species_of(a.spec, i);
-        const int n = numn[i];
-        for (int k = 0; k < n; ++k) {
-            const int j = nlist[(size_t)i * a.nnbrs + k];
-            const int sj = species_of(a.spec, j);
-            // the same rsq from either end: the image rule and the rounding are symmetric
-            const double rsq = pair_sep2(b, a.ivol, pi, a.pos[j]);
-            if (!(rsq > a.thr[si * a.nspec + sj])) near_add(a, i, j);
-            if (!(rsq > a.thr[sj * a.nspec + si])) near_add(a, j, i);
+    const int lane = threadIdx.x & 31, l = lane & (kRowLanes - 1), groups = blockDim.x / kRowLanes;
+    const unsigned int mine = ((1u << kRowLanes) - 1u) << (lane - l);
+    // block-uniform loops: every lane takes part in every ballot
+    for (int base = blockIdx.x * groups; base < a.nm; base += gridDim.x * groups) {
+        const int i = base + threadIdx.x / kRowLanes;
+        const bool live = i < a.nm;
+        const double4 pi = live ? a.pos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
+        const int si = live ? species_of(a.spec, i) : 0;
+        const int n = live ? numn[i] : 0;
+        const int nmax = __reduce_max_sync(0xffffffffu, n);
+        const int32_t *row = nlist + (size_t)i * a.nnbrs;
+        for (int k0 = 0; k0 < nmax; k0 += kRowLanes * kNearBatch) {
+            int jj[kNearBatch];
+            double4 pp[kNearBatch];
+#pragma unroll
+            for (int u = 0; u < kNearBatch; ++u) jj[u] = k0 + u * kRowLanes + l < n ? row[k0 + u * kRowLanes + l] : -1;
+#pragma unroll
+            for (int u = 0; u < kNearBatch; ++u) pp[u] = a.pos[jj[u] >= 0 ? jj[u] : 0];
+#pragma unroll
+            for (int u = 0; u < kNearBatch; ++u) {
+                bool own = false;
+                if (jj[u] >= 0) {
+                    const int j = jj[u], sj = species_of(a.spec, j);
+                    // the same rsq from either end: the image rule and the rounding are symmetric
+                    const double rsq = pair_sep2(b, a.ivol, pi, pp[u]);
+                    own = !(rsq > a.thr[si * a.nspec + sj]);
+                    if (!(rsq > a.thr[sj * a.nspec + si])) near_add(a, j, i);
+                }
+                const unsigned int m = __ballot_sync(0xffffffffu, own) & mine;
+                const int first = m ? __ffs(m) - 1 : lane;
+                int slot = 0;
+                if (own && lane == first) slot = atomicAdd(&a.ncount[i], __popc(m));
+                slot = __shfl_sync(0xffffffffu, slot, first);
+                if (own) {
+                    const int k = slot + __popc(m & ((1u << lane) - 1u));
+                    if (k < kNearCap) a.near[(size_t)i * kNearCap + k] = jj[u];
+                    else atomicExch(&a.flags[0], 1);
+                }
+            }
         }
     }
 }
@@ -335,38 +359,127 @@ __device__ int aj_assign(const int *chi, int nn) {
     return (double)fccscore < (double)hcpscore ? 2 : 3;
 }
 
-__global__ void __launch_bounds__(kRdfThreads)
+// one bond angle as the routine computes it
+__device__ __noinline__ int chi_exact(const double *b, int ivol, const double4 &pi, const double4 &pj,
+                                      const double4 &pk) {
+    const double rsqj = pair_sep2(b, ivol, pi, pj), rsqk = pair_sep2(b, ivol, pi, pk);
+    const double rsq = pair_sep2(b, ivol, pk, pj);
+    return chi_bin(__ddiv_rn(__ddiv_rn(__dsub_rn(__dadd_rn(rsqj, rsqk), rsq), 2.0),
+                             __dsqrt_rn(__dmul_rn(rsqj, rsqk))));
+}
+
+// Bond angles and classes, one thread per atom.  The routine's cosine takes an
+// FP64 separation, two divisions and a square root per neighbour pair (91
+// pairs per bcc atom), which bounded the kernel: 162 us for 128,000 atoms, this
+// one 62 us.  The count only asks between which of nine bounds the cosine
+// lies, and all but some 0.2 % of the pairs are far from every bound: their
+// cosine is the FP32 product of unit vectors, and a table of kCosCells equal
+// cells of [-1, 1] gives the counter to raise, eight 8-bit counters in a pair
+// of words (the bound at 1 ends the last cell).  A cell that comes within
+// kCosGuard of a bound sends the pair to the routine's arithmetic, and so does
+// every pair with a neighbour for which the product is not known to be that
+// close.
+//
+// The guard: a unit vector is an FP64 separation rounded to FP32 (2^-24 per
+// component) times a reciprocal root good to 2 ulp of a norm that has three
+// roundings, so each is within 6 * 2^-24 and the product of two, with its own
+// three roundings, within 16 * 2^-24 = 1e-6 of the cosine; the cell index adds
+// one rounding of a number below 2^12, 2^-13 of a cell.  The routine's own
+// value differs from the cosine by its rounding, below 1e-9 for separations
+// between 0.1 and 100 A.  The three separations close a triangle only where
+// no image correction can differ: components below a quarter of the box.
+constexpr int kCosCells = 4096;
+constexpr float kCosGuard = 4e-6f;
+constexpr int kClassThreads = 256;
+
+// Cell k lies past the bounds whose cells end below it; the cells that a bound's
+// guard interval touches are the exact ones.
+__device__ __forceinline__ void cos_table(uint2 *tab) {
+    constexpr float bound[8] = {-0.945f, -0.915f, -0.755f, -0.705f, -0.195f, 0.195f, 0.245f, 0.795f};
+    for (int k = threadIdx.x; k < kCosCells; k += blockDim.x) {
+        int past = 0;
+        bool exact = k == kCosCells - 1;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int first = (int)(((double)bound[j] - (double)kCosGuard + 1.0) * (0.5 * kCosCells)),
+                      last = (int)(((double)bound[j] + (double)kCosGuard + 1.0) * (0.5 * kCosCells));
+            past += k > last;
+            exact |= k >= first && k <= last;
+        }
+        const int c = past < 4 ? past : past - 1;        // the fifth interval is the unused band
+        uint2 v = make_uint2(past < 4 ? 1u << (8 * c) : 0u, past > 4 ? 1u << (8 * (c - 4)) : 0u);
+        if (exact) v.y = 0xffffffffu;
+        tab[k] = v;
+    }
+}
+
+__global__ void __launch_bounds__(kClassThreads, 4)
 k_aj_classify(AjArgs a, int32_t *__restrict__ aj, int32_t *__restrict__ nnout, int32_t *__restrict__ chiout) {
     __shared__ double b[9];
+    __shared__ uint2 tab[kCosCells];
     if (threadIdx.x < 9) b[threadIdx.x] = a.box->b0[threadIdx.x];
+    cos_table(tab);
     __syncthreads();
+    bool tame = true;                                    // box entries for which the rounding stays below the guard
+    for (int k = 0; k < 9; ++k) tame &= fabs(b[k]) <= 1e5;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nm; i += gridDim.x * blockDim.x) {
         int n = a.ncount[i];
         n = n < kNearCap ? n : kNearCap;
-        int chi[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         const int32_t *nb = a.near + (size_t)i * kNearCap;
         const double4 pi = a.pos[i];
-        // rsq from the centre, as the routine computes it (x0(i) - x0(j))
-        double nr[kNearCap];
-        for (int p = 0; p < n; ++p) nr[p] = pair_sep2(b, a.ivol, pi, a.pos[nb[p]]);
+        float ux[kNearCap], uy[kNearCap], uz[kNearCap];
+        for (int p0 = 0; p0 < n; p0 += 4) {               // four gathers under way together
+            const int4 j4 = reinterpret_cast<const int4 *>(nb)[p0 / 4];
+            const int jj[4] = {j4.x, j4.y, j4.z, j4.w};
+            double4 pj[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) pj[u] = a.pos[p0 + u < n ? jj[u] : i];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                double dx = pi.x - pj[u].x, dy = pi.y - pj[u].y, dz = pi.z - pj[u].z;
+                bool ok = tame && fabs(dx) <= 2.0 && fabs(dy) <= 2.0 && fabs(dz) <= 2.0;
+                min_image(a.ivol, dx, dy, dz);
+                ok = ok && fabs(dx) < 0.249 && fabs(dy) < 0.249 && fabs(dz) < 0.249;
+                const float x = (float)(b[0] * dx + b[3] * dy + b[6] * dz), y = (float)(b[1] * dx + b[4] * dy + b[7] * dz),
+                            z = (float)(b[2] * dx + b[5] * dy + b[8] * dz);
+                const float rr = x * x + y * y + z * z;
+                ok = ok && rr >= 0.01f && rr <= 1e4f;
+                const float inv = ok ? rsqrtf(rr) : __int_as_float(0x7fffffff);   // NaN: the last, exact cell
+                ux[p0 + u] = x * inv;                     // kNearCap is a multiple of 4
+                uy[p0 + u] = y * inv;
+                uz[p0 + u] = z * inv;
+            }
+        }
+        int chi[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         for (int p = 0; p < n; ++p) {
-            const int j = nb[p];
-            const double rsqj = nr[p];
-            const double4 pj = a.pos[j];
+            const float x = ux[p], y = uy[p], z = uz[p];
+            unsigned int lo = 0u, hi = 0u;               // at most 31 pairs: no carry between the counters
             for (int q = p + 1; q < n; ++q) {
-                const int k = nb[q];
-                const double rsqk = nr[q];
-                const double rsq = pair_sep2(b, a.ivol, a.pos[k], pj);
-                const double ct = __ddiv_rn(__ddiv_rn(__dsub_rn(__dadd_rn(rsqj, rsqk), rsq), 2.0),
-                                            __dsqrt_rn(__dmul_rn(rsqj, rsqk)));
-                const int c = chi_bin(ct);
-                if (c >= 0) chi[c] += 1;
+                const float ct = x * ux[q] + y * uy[q] + z * uz[q];
+                const float cell = fminf((ct + 1.0f) * (0.5f * kCosCells), (float)(kCosCells - 1));   // NaN: the last
+                const uint2 v = tab[(int)fmaxf(cell, 0.0f)];
+                if (v.y != 0xffffffffu) {
+                    lo += v.x;
+                    hi += v.y;
+                } else {
+                    const int c = chi_exact(b, a.ivol, pi, a.pos[nb[p]], a.pos[nb[q]]);
+                    if (c >= 4) hi += 1u << (8 * (c - 4));
+                    else if (c >= 0) lo += 1u << (8 * c);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                chi[c] += (int)((lo >> (8 * c)) & 255u);
+                chi[4 + c] += (int)((hi >> (8 * c)) & 255u);
             }
         }
         aj[i] = aj_assign(chi, n);
         nnout[i] = n;
-        if (chiout)
-            for (int c = 0; c < 8; ++c) chiout[8 * (size_t)i + c] = chi[c];
+        if (chiout) {
+            int4 *o = reinterpret_cast<int4 *>(chiout + 8 * (size_t)i);
+            o[0] = make_int4(chi[0], chi[1], chi[2], chi[3]);
+            o[1] = make_int4(chi[4], chi[5], chi[6], chi[7]);
+        }
     }
 }
 
@@ -469,6 +582,12 @@ int check_species(const int32_t *species, int nm, int nspec) {
     return MOLDY_OK;
 }
 
+// blocks of the row kernels: `per_sm` per SM, no more than there are rows
+int row_blocks(int nm, int per_sm) {
+    const int per = kRowThreads / kRowLanes;
+    return std::max(1, std::min((nm + per - 1) / per, per_sm * 148));
+}
+
 int host_box(const DeviceState &d, cudaStream_t s, double *b0) {
     BoxState hb;
     RCUDA(cudaMemcpyAsync(&hb, d.box, sizeof(BoxState), cudaMemcpyDeviceToHost, s), "box");
@@ -521,8 +640,8 @@ int Engine::rdf(int mode, int maxbin, int bpa, const int32_t *species, int nspec
     const bool use_smem = smem <= (size_t)kSmemHistBytes;
     const int nb = std::max(1, std::min((nm + kRdfThreads - 1) / kRdfThreads, 4 * 148));
     if (mode == 0) {
-        if (use_smem) k_rdf_list<true><<<nb, kRdfThreads, smem, s>>>(a, d.nlist, d.numn);
-        else k_rdf_list<false><<<nb, kRdfThreads, 0, s>>>(a, d.nlist, d.numn);
+        if (use_smem) k_rdf_list<true><<<row_blocks(nm, 4), kRowThreads, smem, s>>>(a, d.nlist, d.numn);
+        else k_rdf_list<false><<<row_blocks(nm, 4), kRowThreads, 0, s>>>(a, d.nlist, d.numn);
         prof.launches[K_RDF] += 1;
     } else {
         RCHECK(grid_fill(g, nm, d.pos, cell_of, count, cursor, s));
@@ -589,21 +708,23 @@ int Engine::ackland_jones(int mode, const int32_t *species, int nspec, const dou
     a.nm = nm; a.ivol = prm.ivol; a.nspec = nspec; a.nnbrs = prm.nnbrs;
     const int blocks = std::max(1, std::min((nm + kRdfThreads - 1) / kRdfThreads, 8 * 148));
     if (mode == 0) {
-        k_aj_near_list<<<blocks, kRdfThreads, 0, s>>>(a, d.nlist, d.numn);
+        k_aj_near_list<<<row_blocks(nm, 40), kRowThreads, 0, s>>>(a, d.nlist, d.numn);
         prof.launches[K_RDF] += 1;
     } else {
         RCHECK(grid_fill(g, nm, d.pos, cell_of, count, cursor, s));
         k_aj_near_all<<<blocks, kRdfThreads, 0, s>>>(a, g);
         prof.launches[K_RDF] += 4;
     }
-    k_aj_classify<<<blocks, kRdfThreads, 0, s>>>(a, o, o + nm, chi ? o + 2 * (size_t)nm : nullptr);
+    int32_t *ochi = o, *oaj = o + 8 * (size_t)nm, *onn = oaj + nm;   // the counts first: 16-byte stores
+    const int cb = std::max(1, std::min((nm + kClassThreads - 1) / kClassThreads, 4 * 148));
+    k_aj_classify<<<cb, kClassThreads, 0, s>>>(a, oaj, onn, chi ? ochi : nullptr);
     prof.launches[K_RDF] += 1;
     int32_t flag = 0;
     RCUDA(cudaMemcpyAsync(&flag, a.flags, sizeof(int32_t), cudaMemcpyDeviceToHost, s), "analysis flag");
     RCHECK(open_stage());
-    RCUDA(stage.out(aj, o, nm * sizeof(int32_t), s), "classes");
-    RCUDA(stage.out(nn, o + nm, nm * sizeof(int32_t), s), "coordination");
-    if (chi) RCUDA(stage.out(chi, o + 2 * (size_t)nm, 8 * (size_t)nm * sizeof(int32_t), s), "angle counts");
+    RCUDA(stage.out(aj, oaj, nm * sizeof(int32_t), s), "classes");
+    RCUDA(stage.out(nn, onn, nm * sizeof(int32_t), s), "coordination");
+    if (chi) RCUDA(stage.out(chi, ochi, 8 * (size_t)nm * sizeof(int32_t), s), "angle counts");
     RCUDA(cudaStreamSynchronize(s), "ackland_jones");
     RCUDA(cudaGetLastError(), "ackland_jones");
     if (flag)

@@ -134,3 +134,28 @@ def test_gpu_rdf_rejects_bad_input(gpu_lib):
     with pytest.raises(MoldyError):
         analysis.rdf(s, 100, 50, "list", species=np.zeros(w.nm), nspec=9)
     s.close()
+
+
+@pytest.mark.parametrize("n,sigma,ivol,shift,bins", [(3, 0.0, 1, 0.0, 300), (3, 0.2, 2, 0.0, 300), (4, 0.0, 5, 0.0, 20000),
+                                                     (5, 0.3, 1, 3.0, 20000), (7, 0.02, 3, 0.0, 300),
+                                                     (16, 0.25, 1, 0.0, 300)])
+def test_gpu_row_and_angle_paths_match_oracle(oracle_mod, gpu_lib, n, sigma, ivol, shift, bins):
+    """Where the angle count leaves the FP32 cosines or might have to: boxes so
+    small that neighbours lie beyond a quarter of them, no images in one
+    direction or in any, positions outside the box, pairs brought to 0.02 A, a
+    perfect lattice (whole shells in one bin) and 700,000 pairs of a hot one;
+    histograms in shared memory and beyond it.  Integers: identical."""
+    w = wl.make_workload(n, sigma=sigma, temperature=0.0, ivol=ivol, seed=21)
+    if sigma == 0.3:
+        w.x0 = w.x0.copy()
+        w.x0[7] = w.x0[30] + 0.02 / np.linalg.norm(w.b0[:, 0]) * np.array([1.0, 0.0, 0.0])
+    w.x0 = w.x0 + shift
+    o, g = same_state(oracle_mod, w, steps=0)
+    bpa = 50 if bins == 300 else 4000
+    ho, hg = o.rdf(bins, bpa, mode=0), analysis.rdf(g, bins, bpa, "list")
+    assert np.array_equal(ho["hist"], hg["hist"]) and ho["nclose"] == hg["nclose"]
+    rn = np.array([[2.4]])
+    ro, rg = o.ackland_jones(rn, mode=0), analysis.ackland_jones(g, rn, "list")
+    for k in ("nn", "chi", "aj"):
+        assert np.array_equal(ro[k], rg[k]), k
+    g.close()
