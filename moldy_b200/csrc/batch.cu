@@ -206,6 +206,38 @@ __device__ double block_sum(double v, double *sh) {
     return sh[32];
 }
 
+// K block sums at once (the last one a maximum with MAX), each with the
+// additions of block_sum in its order: two barriers and one shuffle tree deep
+// instead of K times three barriers and two trees.  sh: K * 33.
+template <int K, bool MAX>
+__device__ void block_sums(double (&v)[K], double *sh) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const double y = __shfl_down_sync(0xffffffffu, v[k], o);
+            v[k] = MAX && k == K - 1 ? fmax(v[k], y) : v[k] + y;
+        }
+    }
+    __syncthreads();
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < K; ++k) sh[33 * k + w] = v[k];
+    __syncthreads();
+    for (int k = w; k < K; k += nw) {
+        double x = lane < nw ? sh[33 * k + lane] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) {
+            const double y = __shfl_down_sync(0xffffffffu, x, o);
+            x = MAX && k == K - 1 ? fmax(x, y) : x + y;
+        }
+        if (lane == 0) sh[33 * k + 32] = x;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = sh[33 * k + 32];
+}
+
 __device__ double block_max(double v, double *sh) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
@@ -232,8 +264,9 @@ __device__ double block_max(double v, double *sh) {
 // block size up to 1024); todo, when given, receives the rebuilt cells for
 // the tile screen.  Every atom's cell-order copy goes to spos when all_spos,
 // else only a rebuilt system's (the tile screen reads it).  Returns whether
-// the system was rebuilt (the same in every thread).
-__device__ int prepare_system(BSys &S, const double *__restrict__ X, const double *__restrict__ mass,
+// the system was rebuilt (the same in every thread).  X may have been written
+// earlier in the same kernel (no read-only loads).
+__device__ int prepare_system(BSys &S, const double *X, const double *__restrict__ mass,
                               double *__restrict__ Xb, int32_t *__restrict__ cell_of,
                               int32_t *__restrict__ cell_count, int32_t *__restrict__ cell_start,
                               int32_t *__restrict__ cursor, int32_t *__restrict__ unsorted,
@@ -1396,6 +1429,16 @@ struct CgVecs {
     double *X, *G, *D, *GS, *XX, *GG, *DR, *DGR;
 };
 
+// what the list check of a system that asks for a function value needs
+struct PrepArgs {
+    const double *mass;
+    double *Xb;
+    int32_t *cell_of, *cell_count, *cell_start, *cursor, *unsorted, *sorted;
+    double4 *spos;
+    unsigned long long *stats;
+    int32_t *todo, *ntodo;
+};
+
 // One block per system, the largest systems first (order).  On entry after
 // an evaluation it finishes derivs
 // (pe = sum of energy_calc energies, g = -tg f, f = pe + press vol) and runs
@@ -1403,11 +1446,20 @@ struct CgVecs {
 // marks the system active) or returns (the system is done).  Scalars are
 // computed identically by every thread; vector sums use fixed-order block
 // reductions.  The statement labels follow src/quench_m.F90:323-551.
+//
+// What bounds it is the chain of passes over vectors in L2, each with its
+// barriers: after an evaluation, derivs; then every sum that the decisions may
+// ask for in one pass; then the copies, the new direction, g* and dginit in one
+// (elementwise, so the copies and the direction wait as flags until the pass
+// that first needs them); then the new x.  Four passes and three reductions
+// where one pass per statement took nine and eight; each sum keeps its order,
+// so every value is bit for bit what it was.  192 systems, 142,000 atoms:
+// 42 us, now @@ us.
 __global__ void __launch_bounds__(kCgThreads)
 k_cg(BSys *__restrict__ sys, CgState *__restrict__ cg, CgVecs v, const double *__restrict__ fvec,
      const double *__restrict__ en_calc, double press, int maxfn, int criterion, double fmax_tol,
-     int *__restrict__ n_active, const int32_t *__restrict__ order) {
-    __shared__ double sh[33];
+     int *__restrict__ n_active, const int32_t *__restrict__ order, PrepArgs p) {
+    __shared__ double sh[7 * 33];
     const int sid = order[blockIdx.x];
     BSys &S = sys[sid];
     CgState st = cg[sid];
@@ -1419,8 +1471,12 @@ k_cg(BSys *__restrict__ sys, CgState *__restrict__ cg, CgVecs v, const double *_
     double *X = v.X + base, *G = v.G + base, *D = v.D + base, *GS = v.GS + base;
     double *XX = v.XX + base, *GG = v.GG + base, *DR = v.DR + base, *DGR = v.DGR + base;
     const double dfn = 0.1, acc = 5.0e-7 * (double)S.nm;
-    double c = 0.0, dtest, gamma, toplin, xold;
+    double c = 0.0, dtest, gamma = 0.0, toplin, xold;
+    double dg = 0.0, gg = 0.0, gsg = 0.0, gdgr = 0.0, gdr = 0.0;   // g.d, g.g, g.g*, g.dgr, g.dr at the new point
     int guard = 0;
+    bool keep = false;       // (xx, gg) <- (x, g) due
+    bool back = false;       // g <- gg due
+    int turn = 0;            // direction due: 1 with gamma, 2 restart
 
     if (st.label == 0) {
         st.xnew = 0.0; st.dgstep = 0.0; st.itcrs = 0; st.maxfnk = 0; st.fmin = 0.0; st.dginit = 0.0;
@@ -1445,8 +1501,33 @@ k_cg(BSys *__restrict__ sys, CgState *__restrict__ cg, CgVecs v, const double *_
             pair_u(S.b0, fx, fy, fz, rx, ry, rz);
             fm = fmax(fm, sqrt(rx * rx + ry * ry + rz * rz));
         }
-        st.pe = block_sum(pe, sh);
-        st.last_fmax = block_max(fm, sh);
+        __syncthreads();
+        // (g.d only counts from the second evaluation on; g.dgr and g.dr only
+        // for the three-term direction, and only if (x, g) becomes (xx, gg))
+        double q[7] = {0.0, 0.0, 0.0, 0.0, 0.0, pe, fm};
+        if (st.itcrs < nref) {
+            #pragma unroll 4
+            for (int i = tid; i < n; i += nt) {
+                const double g = G[i];
+                q[0] += D[i] * g;
+                q[1] += g * g;
+                q[2] += GS[i] * g;
+                q[3] += g * DGR[i];
+                q[4] += g * DR[i];
+            }
+        } else {
+            #pragma unroll 4
+            for (int i = tid; i < n; i += nt) {
+                const double g = G[i];
+                q[0] += D[i] * g;
+                q[1] += g * g;
+                q[2] += GS[i] * g;
+            }
+        }
+        block_sums<7, true>(q, sh);
+        dg = q[0]; gg = q[1]; gsg = q[2]; gdgr = q[3]; gdr = q[4];
+        st.pe = q[5];
+        st.last_fmax = q[6];
         st.f = st.pe + press * S.vol;
     }
     goto L190_AFTER;
@@ -1460,22 +1541,50 @@ L30:
     if (++guard > 100000) { st.iflag = 4; goto DONE; }
     if (st.maxfnk >= st.maxfnc) goto L50;
     st.f = st.fmin;
-    #pragma unroll 4
-    for (int i = tid; i < n; i += nt) { X[i] = XX[i]; G[i] = GG[i]; }
-    __syncthreads();
+    back = true;
 L50:
     if (st.iflag > 0) goto DONE;
-    if (st.itcrs <= nref) goto L70;
-    #pragma unroll 4
-    for (int i = tid; i < n; i += nt) D[i] = -G[i];
-    __syncthreads();
-L70:
     st.iterc = st.iterc + 1;
     {
-        double s = 0.0;
-        #pragma unroll 4
-        for (int i = tid; i < n; i += nt) { GS[i] = G[i]; s += D[i] * G[i]; }
-        st.dginit = block_sum(s, sh);
+        // 0 as it stands, 1 three terms, 2 restart, 3 steepest descent (a due
+        // direction is never followed by 3)
+        const int dir = st.itcrs > nref ? 3 : turn;
+        const double *gsrc = back ? GG : G;               // g is gg wherever a direction is due
+        double q[1] = {0.0};
+        for (int i0 = tid; i0 < n; i0 += 4 * nt) {        // loads of four elements first: the stores may alias
+            double g[4], x[4], d[4], e[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * nt;
+                const bool in = i < n;
+                g[u] = in ? gsrc[i] : 0.0;
+                x[u] = in && keep ? X[i] : 0.0;
+                d[u] = in && dir != 3 ? D[i] : 0.0;
+                e[u] = in && dir == 1 ? DR[i] : (in && dir == 2 ? GS[i] : 0.0);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * nt;
+                if (i >= n) break;
+                if (keep) { XX[i] = x[u]; GG[i] = g[u]; }
+                if (back) G[i] = g[u];
+                double dn = d[u];
+                if (dir == 1) dn = -g[u] + st.beta * d[u] + gamma * e[u];
+                if (dir == 2) {
+                    DR[i] = d[u];
+                    DGR[i] = g[u] - e[u];
+                    dn = -g[u] + st.beta * d[u];
+                }
+                if (dir == 3) dn = -g[u];
+                if (dir != 0) D[i] = dn;
+                GS[i] = g[u];
+                q[0] += dn * g[u];
+            }
+        }
+        keep = back = false;
+        turn = 0;
+        block_sums<1, false>(q, sh);
+        st.dginit = q[0];
     }
     if (st.dginit >= 0.0) goto L320;
     st.xmin = 0.0;
@@ -1491,13 +1600,30 @@ L170:
     if (++guard > 100000) { st.iflag = 4; goto DONE; }
     c = st.xnew - st.xmin;
     {
-        double s = 0.0;
-        #pragma unroll 4
-        for (int i = tid; i < n; i += nt) {
-            X[i] = XX[i] + c * D[i];
-            s += fabs(X[i] - XX[i]);
+        double q[1] = {0.0};
+        for (int i0 = tid; i0 < n; i0 += 4 * nt) {
+            double xx[4], d[4], g[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * nt;
+                const bool in = i < n;
+                xx[u] = in ? (keep ? X[i] : XX[i]) : 0.0;
+                d[u] = in ? D[i] : 0.0;
+                g[u] = in && keep ? G[i] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * nt;
+                if (i >= n) break;
+                if (keep) { XX[i] = xx[u]; GG[i] = g[u]; }
+                const double x = xx[u] + c * d[u];
+                X[i] = x;
+                q[0] += fabs(x - xx[u]);
+            }
         }
-        dtest = block_sum(s, sh);
+        keep = false;
+        block_sums<1, false>(q, sh);
+        dtest = q[0];
     }
     if (dtest <= 0.0) st.clt = 0.7;
     if (dtest <= 0.0) goto L300;
@@ -1507,23 +1633,13 @@ L170:
 
 L190_AFTER:
     if (st.maxfnc <= 1) goto L210;
-    {
-        double s = 0.0;
-        #pragma unroll 4
-        for (int i = tid; i < n; i += nt) s += D[i] * G[i];
-        st.gnew = block_sum(s, sh);
-    }
+    st.gnew = dg;
     if (st.f < st.fmin) goto L210;
     if (st.f > st.fmin) goto L250;
     if (fabs(st.gnew) > fabs(st.gmin)) goto L250;
 L210:
     st.maxfnk = st.maxfnc;
-    {
-        double s = 0.0;
-        #pragma unroll 4
-        for (int i = tid; i < n; i += nt) s += G[i] * G[i];
-        st.gsumsq = block_sum(s, sh);
-    }
+    st.gsumsq = gg;
     if (criterion == 1 ? !(st.last_fmax <= fmax_tol) : (st.gsumsq > acc)) goto L250;
     goto DONE;
 L250:
@@ -1532,18 +1648,11 @@ L250:
     goto L30;
 L270:
     if (st.maxfnk < st.maxfnc) goto L300;
-    #pragma unroll 4
-    for (int i = tid; i < n; i += nt) { XX[i] = X[i]; GG[i] = G[i]; }
-    __syncthreads();
+    keep = true;
     if (st.maxfnc <= 1) goto L10;
     st.gm = st.gnew;
     if (st.gm <= st.dginit) goto L310;
-    {
-        double s = 0.0;
-        #pragma unroll 4
-        for (int i = tid; i < n; i += nt) s += GS[i] * G[i];
-        st.ggstar = block_sum(s, sh);
-    }
+    st.ggstar = gsg;
     st.beta = (st.gsumsq - st.ggstar) / (st.gm - st.dginit);
 L300:
     if (fabs(st.gm) > st.clt * fabs(st.dginit)) goto L310;
@@ -1586,30 +1695,26 @@ L380:
 L390:
     if (st.itcrs >= nref) goto L420;
     if (fabs(st.ggstar) >= 0.2 * st.gsumsq) goto L420;
-    {
-        double s1 = 0.0, s2 = 0.0;
+    if (keep) {                        // gg is g
+        gamma = gdgr;
+        c = gdr;
+    } else {
+        double q[2] = {0.0, 0.0};
         #pragma unroll 4
-        for (int i = tid; i < n; i += nt) { s1 += GG[i] * DGR[i]; s2 += GG[i] * DR[i]; }
-        gamma = block_sum(s1, sh);
-        c = block_sum(s2, sh);
+        for (int i = tid; i < n; i += nt) { q[0] += GG[i] * DGR[i]; q[1] += GG[i] * DR[i]; }
+        block_sums<2, false>(q, sh);
+        gamma = q[0];
+        c = q[1];
     }
     gamma = gamma / st.gamden;
     if (fabs(st.beta * st.gm + gamma * c) >= 0.2 * st.gsumsq) goto L420;
-    #pragma unroll 4
-    for (int i = tid; i < n; i += nt) D[i] = -GG[i] + st.beta * D[i] + gamma * DR[i];
-    __syncthreads();
+    turn = 1;
     st.itcrs = st.itcrs + 1;
     goto L30;
 L420:
     st.itcrs = 2;
     st.gamden = st.gm - st.dginit;
-    #pragma unroll 4
-    for (int i = tid; i < n; i += nt) {
-        DR[i] = D[i];
-        DGR[i] = GG[i] - GS[i];
-        D[i] = -GG[i] + st.beta * D[i];
-    }
-    __syncthreads();
+    turn = 2;
     goto L30;
 
 CALLF:
@@ -1620,13 +1725,23 @@ CALLF:
         S.active = 1;
         atomicAdd(n_active, 1);
     }
+    __syncthreads();
+    // the list check of the evaluation that follows (a launch of its own read
+    // the positions back, 14 us a round)
+    prepare_system(S, v.X, p.mass, p.Xb, p.cell_of, p.cell_count, p.cell_start, p.cursor, p.unsorted, p.sorted, p.spos,
+                   p.stats, p.todo, p.ntodo, true);
     return;
 DONE:
+    if (back) {
+        #pragma unroll 4
+        for (int i = tid; i < n; i += nt) { X[i] = XX[i]; G[i] = GG[i]; }
+    }
     __syncthreads();
     if (tid == 0) {
         st.done = 1;
         cg[sid] = st;
         S.active = 0;
+        S.rebuild = 0;
     }
 }
 
@@ -1727,7 +1842,7 @@ class BatchEngine {
     // the quench needs and a plain force evaluation only when asked
     // ev (5 events, may be null): recorded before k_prepare, the tile screen,
     // the density pass and the force pass, and after the force pass
-    void queue_evaluation(bool with_vir, bool use_mixed, bool ecalc, cudaEvent_t *ev = nullptr);
+    void queue_evaluation(bool with_vir, bool use_mixed, bool ecalc, cudaEvent_t *ev = nullptr, bool prepare = true);
     int kernel_times(int rebuild, double *ms4);
     bool ecalc = true;                  // moldy_gpu_batch_force computes energy_calc's energies
     int ready();
@@ -2114,12 +2229,13 @@ static void launch_passes_b(const BatchEngine &E, const TileArgs &a, bool use_mi
 }
 
 // list check (and rebuild) and the tile passes for the systems marked active
-void BatchEngine::queue_evaluation(bool with_vir, bool use_mixed, bool ecalc, cudaEvent_t *ev) {
+void BatchEngine::queue_evaluation(bool with_vir, bool use_mixed, bool ecalc, cudaEvent_t *ev, bool prepare) {
     cudaStream_t s = stream;
     if (ecalc) en_calc_zero = false;
     if (ev) cudaEventRecord(ev[0], s);
-    k_prepare<<<nsys, kPrepThreads, 0, s>>>(sys, X, mass, Xb, cell_of, cell_count, cell_start, cursor, unsorted, sorted, spos,
-                                           stats, todo, ntodo);
+    if (prepare)
+        k_prepare<<<nsys, kPrepThreads, 0, s>>>(sys, X, mass, Xb, cell_of, cell_count, cell_start, cursor, unsorted, sorted,
+                                               spos, stats, todo, ntodo);
     if (ev) cudaEventRecord(ev[1], s);
     TileArgs a;
     a.sys = sys; a.cell_sys = cell_sys; a.cell_start = cell_start; a.sorted = sorted;
@@ -2137,7 +2253,7 @@ void BatchEngine::queue_evaluation(bool with_vir, bool use_mixed, bool ecalc, cu
         default: launch_passes_b<4>(*this, a, use_mixed, with_vir, ecalc, s, ev); break;
     }
     if (ev) cudaEventRecord(ev[4], s);
-    launches += 4;
+    launches += prepare ? 4 : 3;
 }
 
 // compact-row overflow of the last evaluations: grows the rows, marks every
@@ -2541,8 +2657,8 @@ int BatchEngine::quench(int maxfn, int criterion, double fmax, double *out8) {
     BCUDA(cudaMemsetAsync(cg, 0, nsys * sizeof(CgState), s), "CG state");
     BCUDA(cudaMemsetAsync(n_active, 0, sizeof(int), s), "counter");
     // first pass: every system asks for its first function value
-    k_cg<<<nsys, kCgThreads, 0, s>>>(sys, cg, v, f, en_calc, press, maxfn, criterion, fmax, n_active,
-                                         cg_order);
+    const PrepArgs pa{mass, Xb, cell_of, cell_count, cell_start, cursor, unsorted, sorted, spos, stats, todo, ntodo};
+    k_cg<<<nsys, kCgThreads, 0, s>>>(sys, cg, v, f, en_calc, press, maxfn, criterion, fmax, n_active, cg_order, pa);
     launches += 1;
     BCUDA(cudaGetLastError(), "quench start");
     // one round: evaluate the active systems, then advance every state machine
@@ -2553,10 +2669,10 @@ int BatchEngine::quench(int maxfn, int criterion, double fmax, double *out8) {
         BCUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "capture");
         // FP64 passes: the line search compares energies that differ in the
         // seventh digit, below the rounding of FP32 distances
-        queue_evaluation(false, false, true);
+        queue_evaluation(false, false, true, nullptr, false);
         cudaMemsetAsync(n_active, 0, sizeof(int), s);
-        k_cg<<<nsys, kCgThreads, 0, s>>>(sys, cg, v, f, en_calc, press, maxfn, criterion, fmax, n_active,
-                                         cg_order);
+        k_cg<<<nsys, kCgThreads, 0, s>>>(sys, cg, v, f, en_calc, press, maxfn, criterion, fmax, n_active, cg_order,
+                                         pa);
         cudaError_t e = cudaStreamEndCapture(s, &g);
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -2572,14 +2688,14 @@ int BatchEngine::quench(int maxfn, int criterion, double fmax, double *out8) {
         }
         graph_lph = lph; graph_cap = cap; graph_maxfn = maxfn; graph_criterion = criterion; graph_fmax = fmax;
         graph_gather = gather;
-        launches -= 4;   // captured, not run; counted per replay below
+        launches -= 3;   // captured, not run; counted per replay below
     }
     // VA14CD evaluates at most maxfn times; a few rounds more let every
     // system reach its return
     const int rounds = maxfn + 8;
     for (int r = 0; r < rounds; ++r) {
         BCUDA(cudaGraphLaunch(graph, s), "graph launch");
-        launches += 5;
+        launches += 4;
         if ((r & 7) == 7 || r == rounds - 1) {
             BCUDA(cudaMemcpyAsync(host_active, n_active, sizeof(int), cudaMemcpyDeviceToHost, s), "counter");
             BCUDA(cudaStreamSynchronize(s), "quench");
