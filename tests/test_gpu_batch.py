@@ -469,3 +469,19 @@ def test_new_functions_on_kept_lists_and_tables(gpu_lib, prec):
                 q, p = b.quench(maxfn=2), ref.quench(maxfn=2)
                 assert np.max(np.abs(q["pe"] - p["pe"]) / np.abs(p["pe"])) <= 1e-12
                 assert rel_norm_err(b.get_state(), ref.get_state()) <= 1e-12
+
+
+def test_one_lane_rows_longer_than_the_buffer(gpu_lib):
+    """Cells compressed by a fifth, 40 or so pairs inside the cut per atom:
+    the one-lane density pass of the quench evaluates its kept pairs in several
+    pieces.  Against the passes of a force evaluation; 170,128 atoms."""
+    rng = np.random.default_rng(4)
+    w = wl.make_workload(14, sigma=0.08, temperature=0.0, ivol=1, seed=3, strain=-0.2 * np.eye(3))
+    w2 = wl.make_workload(14, sigma=0.12, temperature=0.0, ivol=1, seed=5,
+                          strain=-0.2 * np.eye(3) + wl.random_symmetric_strain(rng, 0.02))
+    with MoldyBatch.from_workloads([w, w2] * 15 + [w]) as b:
+        out = b.force()
+        f = b.forces()
+        q = b.quench(maxfn=1)
+        assert np.max(np.abs(q["pe"] - out["pe_calc"]) / np.abs(q["pe"])) <= 1e-13
+        assert rel_norm_err(b.forces(), f) <= 1e-12
