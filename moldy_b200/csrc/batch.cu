@@ -955,7 +955,15 @@ k_cl_forces_l(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
 //      two passes is a shared-memory load;
 //   3. runs the density pass (rho, F, F') and the force pass with LPA lanes
 //      per atom: lane g takes the row entries g, g + LPA, ...; the lanes'
-//      FP64 sums are combined by shuffles in a fixed order;
+//      FP64 sums are combined by shuffles in a fixed order.  One block of 24
+//      warps per SM has few warps to hide latency with, so every row entry is
+//      loaded one batch ahead (across atoms), the gathers and table reads of a
+//      batch are under way together without branches between them, and the
+//      density pass writes the pairs inside the cut (14 of 24 entries) to rows
+//      of their own, which the force pass walks.  1024 systems, 2.1 million
+//      atoms: 1025 us with 16 warps, a branch per pair and the list rows in
+//      both passes, 780 us without those, 698 us with 24 warps (32 with two
+//      entries a batch 722, 16 with six 852);
 //   4. reduces the system's energy, largest force and virial in a fixed
 //      order (the results of k_sys_reduce).
 // Separations come from the 32-bit fixed-point difference (the integer
@@ -963,14 +971,14 @@ k_cl_forces_l(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
 // terms run in FP32, and every sum accumulates in FP64.  Pairs enter the
 // virial without the mass filter: the path runs only when every atom is
 // heavier than 0.05, so every pair passes m_i + m_j > 0.1.
-constexpr int kEvalThreads = 512;
+constexpr int kEvalThreads = 768;
 constexpr int kEvalWarps = kEvalThreads / 32;
 constexpr int kEvalGather = 4;       // row entries a lane loads before it uses any
 
 struct EvalArgs {
     BSys *sys;
     const int32_t *order;            // systems by descending size
-    int nsys, ntot, pair_cap;
+    int nsys, ntot, pair_cap, screen_warps;   // screen_warps: warps whose tiles fit
     int32_t *queue;                  // [0] next system, [1] blocks done (both zero between launches)
     const double *X, *mass;
     double *Xb;
@@ -978,7 +986,7 @@ struct EvalArgs {
     double4 *spos;
     unsigned long long *stats;
     const int32_t *cell_sys;
-    int32_t *alist, *pcnt, *flags;
+    int32_t *alist, *pcnt, *flags, *clist, *ccnt;
     int ncell, cap;
     double rc2;
     double *f, *rho, *afrho, *fp, *en_force, *sysout;
@@ -1004,6 +1012,20 @@ __device__ __forceinline__ float rec_sep(const float *bq, const int4 &qi, const 
     return fmaf(uz, uz, fmaf(uy, uy, ux * ux));
 }
 
+// node interval and offset of r; the last stored node has no step (the tail)
+__device__ __forceinline__ int interval_f(const Tables &t, float r, float &dr) {
+    const float x = fmaf(r, t.recipstep_f, t.xoff_f);
+    float fl;
+    const int idx = floor_small(fmaxf(x, 0.f), fl);
+    dr = x - fl;
+    return idx < t.nr - 1 ? idx : t.nr - 1;
+}
+
+// entry e of atom i's row, whatever stands there where e or i is past the end
+__device__ __forceinline__ int row_entry(const int32_t *rows, int e, int pair_cap, int ntot, int a0, int i, int nm) {
+    return e < pair_cap && i < nm ? rows[(size_t)e * ntot + a0 + i] : 0;
+}
+
 template <int LPH, int LPA>
 __global__ void __launch_bounds__(kEvalThreads, 1)
 k_batch_eval(EvalArgs a, Tables t) {
@@ -1016,6 +1038,7 @@ k_batch_eval(EvalArgs a, Tables t) {
     const float rc2f = (float)a.rc2;
     constexpr int kAtomsPerRound = kEvalThreads / LPA;
     const int g = tid % LPA;
+    const unsigned gmask = ((1u << LPA) - 1u) << ((tid & 31) / LPA * LPA), below = (1u << (tid & 31)) - 1u;
     int overflow = 0;
     for (;;) {
         if (tid == 0) s_next = atomicAdd(&a.queue[0], 1);
@@ -1034,8 +1057,8 @@ k_batch_eval(EvalArgs a, Tables t) {
             ta.sys = a.sys; ta.cell_sys = a.cell_sys; ta.cell_start = a.cell_start; ta.sorted = a.sorted;
             ta.spos = a.spos; ta.sfp = nullptr; ta.ncell = a.ncell; ta.cap = a.cap; ta.rc2 = a.rc2;
             int4 *tp = reinterpret_cast<int4 *>(dsm) + (size_t)w * a.cap;
-            int *ti = reinterpret_cast<int *>(reinterpret_cast<int4 *>(dsm) + (size_t)kEvalWarps * a.cap) + (size_t)w * a.cap;
-            for (int c = S.cell0 + w; c < S.cell0 + S.ncell; c += kEvalWarps)
+            int *ti = reinterpret_cast<int *>(reinterpret_cast<int4 *>(dsm) + (size_t)a.screen_warps * a.cap) + (size_t)w * a.cap;
+            for (int c = S.cell0 + w; w < a.screen_warps && c < S.cell0 + S.ncell; c += a.screen_warps)
                 overflow = max(overflow, screen_cell<LPH>(ta, c, a.ntot, a.pair_cap, a.alist, a.pcnt, tp, ti,
                                                           tpre[w], tcs[w]));
             __syncthreads();                   // rows written; the tiles' memory is reused below
@@ -1052,30 +1075,57 @@ k_batch_eval(EvalArgs a, Tables t) {
             rec[i] = make_int4(fix32(a.X[at]), fix32(a.X[at + 1]), fix32(a.X[at + 2]), 0);
         }
         __syncthreads();
-        // 3a. density, F and F'
+        // 3a. density, F and F'; the pairs inside the cut go to the atom's
+        // compact row, which the force pass walks
+        int jn[kEvalGather];                   // row entries of the next batch, loaded one batch ahead
+        int nn = tid / LPA < nm ? a.pcnt[a0 + tid / LPA] : 0;
+#pragma unroll
+        for (int u = 0; u < kEvalGather; ++u) jn[u] = row_entry(a.alist, u * LPA + g, a.pair_cap, a.ntot, a0, tid / LPA, nm);
         for (int i0 = 0; i0 < nm; i0 += kAtomsPerRound) {
-            const int i = i0 + tid / LPA;
+            const int i = i0 + tid / LPA, inext = i + kAtomsPerRound;
             const bool live = i < nm;
-            const int hs = a0 + (live ? i : 0);
-            const int4 qi = rec[live ? i : 0];
-            int n = live ? a.pcnt[hs] : 0;
-            n = n < a.pair_cap ? n : a.pair_cap;
+            const int hs = a0 + (live ? i : 0), self = live ? i : 0;
+            const int4 qi = rec[self];
+            const int n = nn < a.pair_cap ? nn : a.pair_cap;
+            const int nmax = __reduce_max_sync(0xffffffffu, n);
+            nn = inext < nm ? a.pcnt[a0 + inext] : 0;
+            const int at = a.sorted[hs];
+            int kept = 0;
             double rho = 0.0;
-            for (int e0 = g; e0 < n; e0 += kEvalGather * LPA) {
+            for (int e0 = 0; e0 < nmax; e0 += kEvalGather * LPA) {
                 int jj[kEvalGather];
+                bool in[kEvalGather];
+                const int ef = e0 + kEvalGather * LPA;
 #pragma unroll
                 for (int u = 0; u < kEvalGather; ++u) {
-                    const int e = e0 + u * LPA;
-                    jj[u] = e < n ? a.alist[(size_t)e * a.ntot + hs] - a0 : -1;
+                    in[u] = e0 + u * LPA + g < n;
+                    jj[u] = in[u] ? jn[u] - a0 : self;
+                    jn[u] = ef < nmax ? row_entry(a.alist, ef + u * LPA + g, a.pair_cap, a.ntot, a0, i, nm)
+                                      : row_entry(a.alist, u * LPA + g, a.pair_cap, a.ntot, a0, inext, nm);
                 }
+                float r[kEvalGather];
 #pragma unroll
                 for (int u = 0; u < kEvalGather; ++u) {
-                    if (jj[u] < 0) continue;
-                    const int4 qj = rec[jj[u]];
                     float dx, dy, dz;
-                    const float r2 = rec_sep(bq, qi, qj, dx, dy, dz);
-                    if (r2 < rc2f) rho += (double)lookup_phif(t, t.phi2f, r2 * rsqrt_ftz(r2));
+                    const float r2 = rec_sep(bq, qi, rec[jj[u]], dx, dy, dz);
+                    in[u] = in[u] && r2 < rc2f;
+                    r[u] = r2 * rsqrt_ftz(r2);
                 }
+#pragma unroll
+                for (int u = 0; u < kEvalGather; ++u) {
+                    float dr;
+                    const float2 q = t.phi2f[interval_f(t, r[u], dr)];
+                    const float ph = fmaf(q.y, dr, q.x);
+                    if (in[u]) rho += (double)ph;
+                    const unsigned m = __ballot_sync(0xffffffffu, in[u]) & gmask;
+                    if (in[u]) a.clist[(size_t)(kept + __popc(m & below)) * a.ntot + hs] = jj[u];
+                    kept += __popc(m);
+                }
+            }
+            if (nmax == 0) {
+#pragma unroll
+                for (int u = 0; u < kEvalGather; ++u)
+                    jn[u] = row_entry(a.alist, u * LPA + g, a.pair_cap, a.ntot, a0, inext, nm);
             }
             rho = lanes_sum<LPA>(rho);
             if (live && g == 0) {
@@ -1085,7 +1135,7 @@ k_batch_eval(EvalArgs a, Tables t) {
                     fe = e2.x; fd = e2.y;
                 }
                 rec[i].w = __float_as_int((float)fd);
-                const int at = a.sorted[hs];
+                a.ccnt[hs] = kept;
                 a.rho[at] = rho;
                 a.afrho[at] = fe;
                 a.fp[at] = fd;
@@ -1094,41 +1144,60 @@ k_batch_eval(EvalArgs a, Tables t) {
         __syncthreads();
         // 3b. forces, force-routine energy, virial moments
         double sef = 0.0, sfm = 0.0, sv[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        nn = tid / LPA < nm ? a.ccnt[a0 + tid / LPA] : 0;
+#pragma unroll
+        for (int u = 0; u < kEvalGather; ++u) jn[u] = row_entry(a.clist, u * LPA + g, a.pair_cap, a.ntot, a0, tid / LPA, nm);
         for (int i0 = 0; i0 < nm; i0 += kAtomsPerRound) {
-            const int i = i0 + tid / LPA;
+            const int i = i0 + tid / LPA, inext = i + kAtomsPerRound;
             const bool live = i < nm;
-            const int hs = a0 + (live ? i : 0);
-            const int4 qi = rec[live ? i : 0];
+            const int hs = a0 + (live ? i : 0), self = live ? i : 0;
+            const int4 qi = rec[self];
             const float fpi = __int_as_float(qi.w);
-            int n = live ? a.pcnt[hs] : 0;
-            n = n < a.pair_cap ? n : a.pair_cap;
+            const int n = nn, nmax = __reduce_max_sync(0xffffffffu, n);
+            nn = inext < nm ? a.ccnt[a0 + inext] : 0;
+            const int at = a.sorted[hs];
+            const double emb = a.afrho[at];
             double fx = 0.0, fy = 0.0, fz = 0.0, ef = 0.0, v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-            for (int e0 = g; e0 < n; e0 += kEvalGather * LPA) {
+            for (int e0 = 0; e0 < nmax; e0 += kEvalGather * LPA) {
                 int jj[kEvalGather];
+                const int enext = e0 + kEvalGather * LPA;
 #pragma unroll
                 for (int u = 0; u < kEvalGather; ++u) {
-                    const int e = e0 + u * LPA;
-                    jj[u] = e < n ? a.alist[(size_t)e * a.ntot + hs] - a0 : -1;
+                    jj[u] = e0 + u * LPA + g < n ? jn[u] : self;
+                    jn[u] = enext < nmax ? row_entry(a.clist, enext + u * LPA + g, a.pair_cap, a.ntot, a0, i, nm)
+                                         : row_entry(a.clist, u * LPA + g, a.pair_cap, a.ntot, a0, inext, nm);
                 }
+                float dx[kEvalGather], dy[kEvalGather], dz[kEvalGather], fp[kEvalGather], vee[kEvalGather];
 #pragma unroll
                 for (int u = 0; u < kEvalGather; ++u) {
-                    if (jj[u] < 0) continue;
                     const int4 qj = rec[jj[u]];
-                    float dx, dy, dz;
-                    const float r2 = rec_sep(bq, qi, qj, dx, dy, dz);
-                    if (!(r2 < rc2f)) continue;
-                    const float rr = rsqrt_ftz(r2), r = r2 * rr;
-                    const float4 q = lookup_r4f(t, r);
-                    const float fpair = -(q.y + q.w * (fpi + __int_as_float(qj.w))) * rr;
-                    fx += (double)(dx * fpair);
-                    fy += (double)(dy * fpair);
-                    fz += (double)(dz * fpair);
-                    ef += (double)q.x;
-                    const float hf = 0.5f * fpair;
-                    const float hx = dx * hf, hy = dy * hf;
-                    v[0] += (double)(dx * hx); v[1] += (double)(dy * hy); v[2] += (double)(dz * (dz * hf));
-                    v[3] += (double)(dy * hx); v[4] += (double)(dz * hx); v[5] += (double)(dz * hy);
+                    float r2 = rec_sep(bq, qi, qj, dx[u], dy[u], dz[u]);
+                    // an entry past the end is the atom itself: d = 0 and a finite fp add zero
+                    r2 = e0 + u * LPA + g < n ? r2 : 1.0f;
+                    const float rr = rsqrt_ftz(r2);
+                    float dr;
+                    const int idx = interval_f(t, r2 * rr, dr);
+                    float4 lo, st;
+                    ldg8f(&t.r4f[2 * idx], lo, st);
+                    vee[u] = fmaf(st.x, dr, lo.x);
+                    fp[u] = -(fmaf(st.y, dr, lo.y) + fmaf(st.w, dr, lo.w) * (fpi + __int_as_float(qj.w))) * rr;
                 }
+#pragma unroll
+                for (int u = 0; u < kEvalGather; ++u) {
+                    if (e0 + u * LPA + g < n) ef += (double)vee[u];
+                    fx += (double)(dx[u] * fp[u]);
+                    fy += (double)(dy[u] * fp[u]);
+                    fz += (double)(dz[u] * fp[u]);
+                    const float hf = 0.5f * fp[u];
+                    const float hx = dx[u] * hf, hy = dy[u] * hf;
+                    v[0] += (double)(dx[u] * hx); v[1] += (double)(dy[u] * hy); v[2] += (double)(dz[u] * (dz[u] * hf));
+                    v[3] += (double)(dy[u] * hx); v[4] += (double)(dz[u] * hx); v[5] += (double)(dz[u] * hy);
+                }
+            }
+            if (nmax == 0) {
+#pragma unroll
+                for (int u = 0; u < kEvalGather; ++u)
+                    jn[u] = row_entry(a.clist, u * LPA + g, a.pair_cap, a.ntot, a0, inext, nm);
             }
             fx = lanes_sum<LPA>(fx); fy = lanes_sum<LPA>(fy); fz = lanes_sum<LPA>(fz);
             ef = lanes_sum<LPA>(ef);
@@ -1137,11 +1206,10 @@ k_batch_eval(EvalArgs a, Tables t) {
             if (live && g == 0) {
                 // fixed-point units to box lengths (exact scalings)
                 fx *= kFixUnit; fy *= kFixUnit; fz *= kFixUnit;
-                const int at = a.sorted[hs];
                 a.f[3 * (size_t)at] = fx;
                 a.f[3 * (size_t)at + 1] = fy;
                 a.f[3 * (size_t)at + 2] = fz;
-                const double eat = a.afrho[at] + 0.5 * ef;
+                const double eat = emb + 0.5 * ef;
                 a.en_force[at] = eat;
                 sef += eat;
 #pragma unroll
@@ -1896,7 +1964,7 @@ class BatchEngine {
     }
     int eval_prepare();
     size_t eval_smem() const {
-        return std::max((size_t)max_atoms * sizeof(int4), (size_t)kEvalWarps * (size_t)cap * (sizeof(int4) + sizeof(int)));
+        return std::max((size_t)max_atoms * sizeof(int4), 16 * (size_t)cap * (sizeof(int4) + sizeof(int)));
     }
     bool persistent_applies() const {
         return persistent && mixed && !ecalc && all_heavy && eval_smem() + 8192 <= smem_optin;
@@ -2390,9 +2458,10 @@ int BatchEngine::queue_persistent(bool prepare) {
     if (prepare) BCHECK(eval_prepare());
     EvalArgs a;
     a.sys = sys; a.order = cg_order; a.nsys = nsys; a.ntot = ntot; a.pair_cap = pair_cap; a.queue = queue;
+    a.screen_warps = std::min((size_t)kEvalWarps, eval_smem() / (std::max(cap, 1) * (sizeof(int4) + sizeof(int))));
     a.X = X; a.mass = mass; a.Xb = Xb; a.cell_of = cell_of; a.cell_count = cell_count; a.cell_start = cell_start;
     a.cursor = cursor; a.unsorted = unsorted; a.sorted = sorted; a.spos = spos; a.stats = stats; a.cell_sys = cell_sys;
-    a.alist = alist; a.pcnt = pcnt; a.flags = flags; a.ncell = ncell; a.cap = cap; a.rc2 = rcut * rcut;
+    a.alist = alist; a.pcnt = pcnt; a.flags = flags; a.clist = clist; a.ccnt = ccnt; a.ncell = ncell; a.cap = cap; a.rc2 = rcut * rcut;
     a.f = f; a.rho = rho; a.afrho = afrho; a.fp = fp; a.en_force = en_force; a.sysout = sysout;
     eval_kernel(lph, lpa)<<<eval_grid, kEvalThreads, eval_smem(), stream>>>(a, tab);
     ++launches;

@@ -485,3 +485,27 @@ def test_one_lane_rows_longer_than_the_buffer(gpu_lib):
         q = b.quench(maxfn=1)
         assert np.max(np.abs(q["pe"] - out["pe_calc"]) / np.abs(q["pe"])) <= 1e-13
         assert rel_norm_err(b.forces(), f) <= 1e-12
+
+
+@pytest.mark.parametrize("lpa", [1, 2, 4])
+@pytest.mark.parametrize("sizes", [[4], [5, 4, 8], [4, 9, 5]])
+def test_persistent_rows_inside_the_cut(gpu_lib, lpa, sizes):
+    """Atom counts that are no multiple of an atom round, lanes without an
+    atom, rows of no pairs (a cell stretched until every atom is alone) beside
+    ordinary ones: the persistent evaluation against the FP64 passes.  FP32
+    pair terms: 2e-6 of the largest force and of the energies (the virial, a
+    small difference of large terms, has its own bound in the test above)."""
+    ws = mixed_systems(sizes, seed=31)
+    far = wl.make_workload(4, sigma=0.05, temperature=0.0, ivol=1, seed=2, strain=0.9 * np.eye(3))
+    ws = ws + [far] + ws[:1]
+    with MoldyBatch.from_workloads(ws) as b:
+        b.set_energy_calc(False)
+        ref, fr = b.force(), b.forces()
+        b.set_precision("mixed")
+        b.set_atom_lanes(lpa)
+        assert b.persistent_applies()
+        for _ in range(2):                                   # lists built, lists kept
+            out, f = b.force(), b.forces()
+            assert np.max(np.abs(f - fr)) <= 2e-6 * np.max(np.abs(fr))
+            assert np.max(np.abs(out["pe"] - ref["pe"])) <= 2e-6 * np.max(np.abs(ref["pe"]))
+        assert not np.any(b.split(f)[len(sizes)])
