@@ -323,7 +323,8 @@ k_therm(Params p, BoxState *__restrict__ box, const double *__restrict__ x1,
 // evaluation that left them); mean: for a scalev that follows
 int launch_therm(DeviceState &d, const Params &p, bool prep, double *rec, cudaStream_t s, bool mean) {
     if (prep) k_therm_prep<<<1, 1, 0, s>>>(p, d.box);
-    int nblocks = stream_blocks(p.nm);
+    // with the mean, scalev's grouping of the atoms (launch_scalev)
+    int nblocks = mean ? grid_blocks(p.nm, kAtomThreads) : stream_blocks(p.nm);
     launch_pdl(mean ? k_therm<true> : k_therm<false>, nblocks, kAtomThreads, 0, s, p, d.box, d.x1, d.x2, d.mass, d.znum,
                d.partials, rec, d.flags + 14);
     return nblocks;
@@ -407,7 +408,11 @@ k_scalev_scale(int nm, const BoxState *__restrict__ box, double *__restrict__ x1
 // mean: the mean is not in the box yet; scale: scale x1 now (else the next
 // drift does)
 void launch_scalev(DeviceState &d, const Params &p, double nose, double rqke, bool mean, bool scale, cudaStream_t s) {
-    const int nb = stream_blocks(p.nm);
+    // Mean and energy are summed over up to 1,184 blocks, as they were as passes
+    // of their own: the scaling factor multiplies every velocity, so another
+    // order of these sums (592 blocks, 1 us a step less at 1,024,000 atoms) would
+    // move every trajectory of a thermostatted run by its last bits.
+    const int nb = grid_blocks(p.nm, kAtomThreads);
     double *part = d.partials + (size_t)kMaxBlocks * kPartials;
     if (mean) k_scalev_mean<<<nb, kAtomThreads, 0, s>>>(p.nm, d.box, d.x1, part, d.flags + 15);
     launch_pdl(k_scalev_ke, nb, kAtomThreads, 0, s, p, d.box, d.x1, d.mass, d.znum, part, nose, rqke, d.flags + 15);
