@@ -210,7 +210,8 @@ const char *moldy_gpu_kernel_name(int32_t kernel);
 /* The screening-density pass and the force pass are compiled in
  * MOLDY_TUNE_VARIANTS variants each: how many list entries a thread gathers
  * before using them, with or without L2 prefetches of the next atom's data,
- * and two or three resident blocks per SM (registers per thread).
+ * and the resident threads per SM.  Which one a new handle runs follows from
+ * the precision and the number of atoms; setting or tuning them overrides it.
  * moldy_gpu_autotune times every variant on the current configuration with
  * nreps force evaluations (positions, velocities, the rebuild counter and the
  * neighbour list are left unchanged) and keeps the fastest of each pass.

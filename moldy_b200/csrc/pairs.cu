@@ -35,6 +35,11 @@
 // the minimum image) and keeps rho, F, F', the forces, the energy, the virial
 // and every other sum in FP64: each pair's FP32 terms are converted once and
 // accumulated in FP64.
+//
+// These two kernels run the exact functions in FP64 and mixed precision below
+// kStAtoms atoms; k_screen_d / k_forces_d (FP64 tables) and k_screen_st /
+// k_forces_st (mixed precision, large systems, tables in shared memory) are the
+// same passes without branches in their inner loops.
 #include <type_traits>
 
 #include "engine.h"
@@ -86,7 +91,7 @@ __device__ __forceinline__ void prefetch_l2(const void *ptr) {
 // Keeps pair (a, j) iff its distance is inside the table range, sums rho_a,
 // embeds.  FP64: the exact distance decides.  Mixed: the FP32 distance decides
 // outside the band [rin, rscreen] around the cut, the FP64 one inside it.
-template <bool MIXED, bool EXACT, int B, bool PF, int MINB>
+template <bool MIXED, int B, bool PF, int MINB>
 __global__ void __launch_bounds__(256, MINB)
 k_screen_density(Params p, Tables t, const double4 *__restrict__ pos, const int4 *__restrict__ posq,
                  double4 *__restrict__ pos2, int4 *__restrict__ posq2, const BoxState *__restrict__ box,
@@ -170,7 +175,7 @@ k_screen_density(Params p, Tables t, const double4 *__restrict__ pos, const int4
                     double r2 = rx * rx + ry * ry + rz * rz;
                     if (!(r2 <= t.rcull2)) continue;
                     double r = sqrt(r2);
-                    rho_a += EXACT ? fetm_phi(t, r) : lookup_phi(t, r);
+                    rho_a += fetm_phi(t, r);
                     if (cnt < p.pair_cap) alist[(size_t)cnt * stride + a] = ee[u];
                     ++cnt;
                 }
@@ -183,7 +188,7 @@ k_screen_density(Params p, Tables t, const double4 *__restrict__ pos, const int4
         // embed (src/potential_m.F90:148-169): rho <= 1e-40 keeps the old values
         double fd;
         if (rho_a > 1e-40) {
-            double2 e = EXACT ? embed_funcs(t, rho_a) : lookup_e2(t, rho_a);
+            double2 e = MIXED ? lookup_e2(t, rho_a) : embed_funcs(t, rho_a);
             afrho[a] = e.x;
             dafrho[a] = e.y;
             fd = e.y;
@@ -278,7 +283,7 @@ __device__ __forceinline__ void second_half(const Params &p, const double *stg, 
 // up to FP64 rounding of the per-atom terms, and it needs no per-pair
 // conversion to FP64 in the mixed pass.  The pair energy is summed from the
 // copy in the owner's row.
-template <bool MIXED, bool EXACT, int B, bool PF, bool STRESS, int MINB>
+template <bool MIXED, int B, bool PF, bool STRESS, int MINB>
 __global__ void __launch_bounds__(256, MINB)
 k_forces(Params p, Tables t, const double4 *__restrict__ pos2, const int4 *__restrict__ posq2,
          const BoxState *__restrict__ box,
@@ -407,7 +412,7 @@ k_forces(Params p, Tables t, const double4 *__restrict__ pos2, const int4 *__res
                     const double rz = b[2] * dx + b[5] * dy + b[8] * dz;
                     const double r = sqrt(rx * rx + ry * ry + rz * rz);
                     const double rr = 1.0 / r;
-                    const double4 tv = EXACT ? pair_funcs(t, r) : lookup_r4(t, r);    // vee, dvee, phi, dphi
+                    const double4 tv = pair_funcs(t, r);    // vee, dvee, phi, dphi
                     const double fp = -tv.y * rr - (tv.w * pa.w + tv.w * q.w) * rr;
                     const double gxp = dx * fp, gyp = dy * fp, gzp = dz * fp;
                     fxa += gxp; fya += gyp; fza += gzp;
@@ -1154,8 +1159,13 @@ void launch_mid_build(DeviceState &d, const Params &p, double rmid, double rout,
 // The mixed passes of at least kStAtoms atoms in lookup mode keep their tables
 // in shared memory (ST: one block per SM); smaller systems, whose atoms would
 // fill few such blocks, tables above kStNodes nodes and the FP64 passes read
-// them through L1 with blocks of 256.
-constexpr int kStAtoms = 100000;
+// them through L1 with blocks of 256.  One block per SM fills late: NPT steps
+// of L1 forms / screening in shared memory / both (us): 101,306 atoms 59.1 /
+// 59.0 / 59.0, 250,000 100 / 96 / 101, 524,288 169 / 160 / 166, 810,448 - / 225 /
+// 230, 913,066 - / 242 / 239, 1,024,000 276 / 260 / 254, 2,000,000 499 / 459 /
+// 444.
+constexpr int kStAtoms = 100000;         // screening-density pass
+constexpr int kStForceAtoms = 850000;    // force pass
 constexpr int kStNodes = 6000;           // 24 bytes per node: 144 KB beside 48 bytes per thread
 
 constexpr size_t force_smem(int nodes, int nt) {
@@ -1173,12 +1183,12 @@ static int sd_variant(DeviceState &d, const Params &p, const Tables &t, bool mix
 #define SD_ARGS p, t, d.pos, d.posq, d.pos2, d.posq2, d.box, d.mlist, d.mid_cnt, d.alist, d.pair_cnt, \
                 d.rho, d.afrho, d.dafrho, partials, d.flags, store_rho
     int nb = grid_blocks(p.nm, 256);
-    if (t.exact) LAUNCH_WAVE((k_screen_density<false, true, B, PF, MINB>), nb, s, SD_ARGS);
+    if (t.exact) LAUNCH_WAVE((k_screen_density<false, B, PF, MINB>), nb, s, SD_ARGS);
     else if (mixed && st_applies(p, t))
         LAUNCH_WAVE_SMEM((k_screen_st<B, PF, 256 * MINB>), 256 * MINB, (size_t)t.nr * sizeof(float2),
                          kStNodes * sizeof(float2), nb, s, p, t, d.pos, d.posq, d.posq2, d.box, d.mlist, d.mid_cnt,
                          d.alist, d.pair_cnt, d.rho, d.afrho, d.dafrho, partials, d.flags, store_rho);
-    else if (mixed) LAUNCH_WAVE((k_screen_density<true, false, B, PF, MINB>), nb, s, SD_ARGS);
+    else if (mixed) LAUNCH_WAVE((k_screen_density<true, B, PF, MINB>), nb, s, SD_ARGS);
     else LAUNCH_WAVE((k_screen_d<B, PF, MINB>), nb, s, p, t, d.pos, d.pos2, d.box, d.mlist, d.mid_cnt, d.alist,
                      d.pair_cnt, d.rho, d.afrho, d.dafrho, partials, d.flags, store_rho);
 #undef SD_ARGS
@@ -1206,17 +1216,17 @@ int launch_screen_density(DeviceState &d, const Params &p, const Tables &t, bool
 }
 
 template <int B, bool PF, bool STRESS, int MINB>
-static int forces_variant(DeviceState &d, const Params &p, const Tables &t, bool mixed, int mode, double *partials,
-                          cudaStream_t s) {
+static int forces_variant(DeviceState &d, const Params &p, const Tables &t, bool mixed, bool st, int mode,
+                          double *partials, cudaStream_t s) {
 #define FORCE_ARGS p, t, d.pos2, d.posq2, d.box, d.alist, d.pair_cnt, d.mass, d.znum, d.del2, d.f, d.x1, d.x2, \
                    d.stress, partials, mode
     int nb = grid_blocks(p.nm, 256);
-    if (t.exact) LAUNCH_WAVE((k_forces<false, true, B, PF, STRESS, MINB>), nb, s, FORCE_ARGS);
-    else if (mixed && !STRESS && st_applies(p, t))
+    if (t.exact) LAUNCH_WAVE((k_forces<false, B, PF, STRESS, MINB>), nb, s, FORCE_ARGS);
+    else if (mixed && !STRESS && st)
         LAUNCH_WAVE_SMEM((k_forces_st<B, PF, 256 * MINB>), 256 * MINB,
                          force_smem(t.nr, 256 * MINB), force_smem(kStNodes, 256 * MINB), nb, s, p, t, d.posq2, d.box, d.alist, d.pair_cnt,
                          d.mass, d.znum, d.del2, d.f, d.x1, d.x2, partials, mode);
-    else if (mixed) LAUNCH_WAVE((k_forces<true, false, B, PF, STRESS, MINB>), nb, s, FORCE_ARGS);
+    else if (mixed) LAUNCH_WAVE((k_forces<true, B, PF, STRESS, MINB>), nb, s, FORCE_ARGS);
     else LAUNCH_WAVE((k_forces_d<B, PF, STRESS, MINB>), nb, s, p, t, d.pos2, d.box, d.alist, d.pair_cnt, d.mass,
                      d.znum, d.del2, d.f, d.x1, d.x2, d.stress, partials, mode);
 #undef FORCE_ARGS
@@ -1226,17 +1236,20 @@ static int forces_variant(DeviceState &d, const Params &p, const Tables &t, bool
 int launch_forces(DeviceState &d, const Params &p, const Tables &t, bool mixed, int mode,
                   int variant, double *partials, cudaStream_t s) {
     mixed = mixed && mixed_applies(p);
+    // by default the shared-memory form from kStForceAtoms atoms on, with a
+    // variant asked for wherever it applies
+    const bool st = mixed && st_applies(p, t) && (variant >= 0 || p.nm >= kStForceAtoms);
     if (variant < 0) variant = t.exact ? 1 : (mixed ? 7 : 3);
-    if (p.atomstress) return forces_variant<2, false, true, 2>(d, p, t, mixed, mode, partials, s);
+    if (p.atomstress) return forces_variant<2, false, true, 2>(d, p, t, mixed, st, mode, partials, s);
     switch (variant) {
-    case 0: return forces_variant<2, true, false, 4>(d, p, t, mixed, mode, partials, s);
-    case 1: return forces_variant<4, true, false, 4>(d, p, t, mixed, mode, partials, s);
-    case 2: return forces_variant<2, true, false, 2>(d, p, t, mixed, mode, partials, s);
-    case 3: return forces_variant<4, true, false, 2>(d, p, t, mixed, mode, partials, s);
-    case 4: return forces_variant<2, false, false, 3>(d, p, t, mixed, mode, partials, s);
-    case 5: return forces_variant<4, false, false, 3>(d, p, t, mixed, mode, partials, s);
-    case 6: return forces_variant<2, true, false, 3>(d, p, t, mixed, mode, partials, s);
-    default: return forces_variant<4, true, false, 3>(d, p, t, mixed, mode, partials, s);
+    case 0: return forces_variant<2, true, false, 4>(d, p, t, mixed, st, mode, partials, s);
+    case 1: return forces_variant<4, true, false, 4>(d, p, t, mixed, st, mode, partials, s);
+    case 2: return forces_variant<2, true, false, 2>(d, p, t, mixed, st, mode, partials, s);
+    case 3: return forces_variant<4, true, false, 2>(d, p, t, mixed, st, mode, partials, s);
+    case 4: return forces_variant<2, false, false, 3>(d, p, t, mixed, st, mode, partials, s);
+    case 5: return forces_variant<4, false, false, 3>(d, p, t, mixed, st, mode, partials, s);
+    case 6: return forces_variant<2, true, false, 3>(d, p, t, mixed, st, mode, partials, s);
+    default: return forces_variant<4, true, false, 3>(d, p, t, mixed, st, mode, partials, s);
     }
 }
 
