@@ -553,7 +553,7 @@ int Engine::get_state(double *x0, double *y0, double *z0, double *x1, double *y1
                       double *tgid) {
     size_t nm = (size_t)prm.nm, nb = nm * sizeof(double);
     cudaStream_t s = stream_;
-    CHECK(open_stage());
+    (void)open_stage();   // without it the copies go the driver's way
     if (x0 || y0 || z0) {
         double *tmp = d.en_atom;
         k_unpack_pos<<<(prm.nm + 255) / 256, 256, 0, s>>>(prm.nm, d.pos, tmp);
@@ -577,7 +577,7 @@ int Engine::get_state(double *x0, double *y0, double *z0, double *x1, double *y1
 int Engine::get_array3(const double *dev, double *a, double *b, double *c) {
     size_t nm = (size_t)prm.nm, nb = nm * sizeof(double);
     double *o[3] = {a, b, c};
-    CHECK(open_stage());
+    (void)open_stage();   // without it the copies go the driver's way
     for (int k = 0; k < 3; ++k)
         if (o[k]) CUDA_CHECK(stage.out(o[k], dev + k * nm, nb, stream_), "get array");
     CUDA_CHECK(cudaStreamSynchronize(stream_), "get array");
@@ -586,7 +586,7 @@ int Engine::get_array3(const double *dev, double *a, double *b, double *c) {
 
 int Engine::get_density(double *rho, double *afrho, double *dafrho) {
     size_t nb = (size_t)prm.nm * sizeof(double);
-    CHECK(open_stage());
+    (void)open_stage();   // without it the copies go the driver's way
     if (rho) CUDA_CHECK(stage.out(rho, d.rho, nb, stream_), "get rho");
     if (afrho) CUDA_CHECK(stage.out(afrho, d.afrho, nb, stream_), "get afrho");
     if (dafrho) CUDA_CHECK(stage.out(dafrho, d.dafrho, nb, stream_), "get dafrho");

@@ -182,13 +182,6 @@ __device__ __forceinline__ void pair_u(const double *b, double dx, double dy, do
     uz = b[2] * dx + b[5] * dy + b[8] * dz;
 }
 
-template <int LPH>
-__device__ __forceinline__ double group_sum(double v) {
-#pragma unroll
-    for (int o = LPH / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // ------------------------------------------------------ block reductions --
 // fixed-order sum over the block, returned to every thread
 __device__ double block_sum(double v, double *sh) {
@@ -960,7 +953,7 @@ k_cl_forces_l(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
 //      loaded one batch ahead (across atoms), the gathers and table reads of a
 //      batch are under way together without branches between them, and the
 //      density pass writes the pairs inside the cut (14 of 24 entries) to rows
-//      of their own, which the force pass walks.  1024 systems, 2.1 million
+//      of their own, which the force pass walks.  1024 systems, 2.85 million
 //      atoms: 1025 us with 16 warps, a branch per pair and the list rows in
 //      both passes, 780 us without those, 698 us with 24 warps (32 with two
 //      entries a batch 722, 16 with six 852);
@@ -1549,7 +1542,7 @@ struct PrepArgs {
 // (elementwise, so the copies and the direction wait as flags until the pass
 // that first needs them); then the new x.  Four passes and three reductions
 // where one pass per statement took nine and eight; each sum keeps its order,
-// so every value is bit for bit what it was.  192 systems, 142,000 atoms:
+// so every value is bit for bit what it was.  192 systems, 161,000 atoms:
 // 36 us a round, now 34 with the list check of the next evaluation, which
 // took 14 us as a launch of its own.
 __global__ void __launch_bounds__(kCgThreads)

@@ -721,7 +721,7 @@ int Engine::ackland_jones(int mode, const int32_t *species, int nspec, const dou
     prof.launches[K_RDF] += 1;
     int32_t flag = 0;
     RCUDA(cudaMemcpyAsync(&flag, a.flags, sizeof(int32_t), cudaMemcpyDeviceToHost, s), "analysis flag");
-    RCHECK(open_stage());
+    (void)open_stage();
     RCUDA(stage.out(aj, oaj, nm * sizeof(int32_t), s), "classes");
     RCUDA(stage.out(nn, onn, nm * sizeof(int32_t), s), "coordination");
     if (chi) RCUDA(stage.out(chi, ochi, 8 * (size_t)nm * sizeof(int32_t), s), "angle counts");

@@ -944,6 +944,11 @@ static void run_shape(int nm, int &lanes, int &threads, int &blocks) {
 // every atom has a thread of its own, and in mixed precision, whose pair terms
 // are shorter, up to two atoms per thread.
 bool run_applies(const Params &p, const Tables &t, bool mixed) {
+    // the whole grid has to be resident: a partition of the device takes the launches
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < kRunBlocks)
+        return false;
     return p.nm <= (mixed ? 2 : 1) * kRunBlocks * kRunThreads && !t.exact && !p.atomstress && (p.ivol == 0 || p.ivol == 1 || p.ivol == 4) &&
            run_smem(t, mixed) <= 200 * 1024;
 }
