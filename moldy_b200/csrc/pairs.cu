@@ -50,13 +50,12 @@ namespace moldy {
 // One wave of resident blocks for the kernel (nt threads, smem
 // bytes of dynamic shared memory): every block then runs the same number of
 // grid-stride iterations (to within one), and no partly filled last wave
-// idles the SMs.  Computed once per instantiation.
+// idles the SMs.  Computed once per instantiation: it sizes grids, nothing else.
 template <typename K>
 static int one_wave(K kernel, int nt = 256, size_t smem = 0) {
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (smem > 0) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, nt, smem) != cudaSuccess) {
         cudaGetLastError();
         per_sm = 0;
@@ -73,13 +72,19 @@ static int one_wave(K kernel, int nt = 256, size_t smem = 0) {
     } while (0)
 
 // NT threads per block and SMEM bytes of tables, at most MAXS (512 threads and
-// more fill an SM's registers: one block per SM whatever the tables take)
-#define LAUNCH_WAVE_SMEM(KERNEL, NT, SMEM, MAXS, NB, S, ...) \
-    do {                                                     \
-        static const int wave_ = one_wave(KERNEL, NT, MAXS); \
-        NB = (p.nm + NT - 1) / NT;                           \
-        NB = NB < wave_ ? NB : wave_;                        \
-        launch_pdl(KERNEL, NB, NT, SMEM, S, __VA_ARGS__);    \
+// more fill an SM's registers: one block per SM whatever the tables take).
+// The limit above 48 KB belongs to the kernel in the current device's context,
+// so it is raised at every launch (under 1 us, and a replayed step makes none);
+// a failure stays the last error, as that of the launch after it would.
+#define LAUNCH_WAVE_SMEM(KERNEL, NT, SMEM, MAXS, NB, S, ...)                                              \
+    do {                                                                                                  \
+        if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(MAXS)) ==     \
+            cudaSuccess) {                                                                                \
+            static const int wave_ = one_wave(KERNEL, NT, MAXS);                                          \
+            NB = (p.nm + NT - 1) / NT;                                                                    \
+            NB = NB < wave_ ? NB : wave_;                                                                 \
+            launch_pdl(KERNEL, NB, NT, SMEM, S, __VA_ARGS__);                                             \
+        }                                                                                                 \
     } while (0)
 
 // L2 prefetch of one address (no register result; the address is always
