@@ -13,8 +13,9 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libmoldy_gpu.so")
-SOURCES = ["api.cu", "cells.cu", "nlist.cu", "eam.cu", "pairs.cu", "run.cu", "noalloc.cu", "adjoint.cu", "batch.cu", "rdf.cu", "tables.cpp"]
-HEADERS = ["common.cuh", "engine.h", "box.cuh", "pairs.cuh"]
+SOURCES = ["api.cu", "cells.cu", "nlist.cu", "eam.cu", "pairs.cu", "run.cu", "noalloc.cu", "adjoint.cu", "batch.cu", "rdf.cu", "copystage.cpp",
+           "tables.cpp"]
+HEADERS = ["common.cuh", "engine.h", "box.cuh", "pairs.cuh", "copystage.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

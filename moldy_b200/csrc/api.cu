@@ -114,11 +114,11 @@ void Profiler::harvest() {
     for (auto &p : pending) {
         float ms = 0.f;
         if (cudaEventElapsedTime(&ms, p.a, p.b) == cudaSuccess) total_ms[p.id] += ms;
+        else cudaGetLastError();   // its own error, and no other: a failed launch is reported by the caller
         pool.push_back(p.a);
         pool.push_back(p.b);
     }
     pending.clear();
-    cudaGetLastError();
 }
 
 void Profiler::reset() {
@@ -139,54 +139,6 @@ Profiler::~Profiler() {
         (E).prof.end((id), (s));            \
         (E).prof.launches[(id)] += (nk);    \
     } while (0)
-
-// ---------------------------------------------------------- staged copies --
-CopyStage::~CopyStage() {
-    if (head) cudaFreeHost(head);
-    for (int k = 0; k < 2; ++k)
-        if (ev[k]) cudaEventDestroy(ev[k]);
-}
-
-cudaError_t CopyStage::open(size_t head_bytes) {
-    if (piece) return cudaSuccess;
-    const size_t hb = (head_bytes + 255) & ~(size_t)255;
-    cudaError_t e = cudaSuccess;
-    for (int k = 0; k < 2 && e == cudaSuccess; ++k)
-        if (!ev[k]) e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&head, hb + 2 * kStageBytes);
-    if (e == cudaSuccess) piece = head + hb;
-    return e;
-}
-
-// Device to host.  Pageable memory is filled through two pinned pieces: the
-// copy of one runs while the host empties the other (1.3 MB in 120 us instead
-// of 270 us); complete on return.  Pinned destinations, and 64 KB or less,
-// which the driver stages as fast, are one queued copy: the caller waits for
-// the stream.
-cudaError_t CopyStage::out(void *dst, const void *src, size_t bytes, cudaStream_t s) {
-    cudaPointerAttributes at;
-    const bool pinned = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
-    if (!pinned) cudaGetLastError();
-    if (pinned || !piece || bytes <= 65536) {
-        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
-    }
-    const size_t n = (bytes + kStageBytes - 1) / kStageBytes;
-    for (size_t k = 0; k <= n; ++k) {
-        if (k < n) {
-            const size_t o = k * kStageBytes, len = bytes - o < kStageBytes ? bytes - o : kStageBytes;
-            cudaError_t e = cudaMemcpyAsync(piece + (k & 1) * kStageBytes, (const char *)src + o, len, cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess) e = cudaEventRecord(ev[k & 1], s);
-            if (e != cudaSuccess) return e;
-        }
-        if (k > 0) {
-            const size_t q = k - 1, o = q * kStageBytes, len = bytes - o < kStageBytes ? bytes - o : kStageBytes;
-            cudaError_t e = cudaEventSynchronize(ev[q & 1]);
-            if (e != cudaSuccess) return e;
-            std::memcpy((char *)dst + o, piece + (q & 1) * kStageBytes, len);
-        }
-    }
-    return cudaSuccess;
-}
 
 // ------------------------------------------------------------------ Engine --
 Engine::Engine(const moldy_params &p) {
@@ -539,6 +491,7 @@ int Engine::set_state(const double *x0, const double *y0, const double *z0, cons
     if (x0 && zn && mass && del2 && b0) state_set_ = true;
     if (x0 || y0 || z0 || b0 || mass) forces_current_ = false;
     CUDA_CHECK(cudaStreamSynchronize(s), "set_state");
+    CUDA_CHECK(cudaGetLastError(), "set_state");
     return MOLDY_OK;
 }
 
@@ -753,6 +706,7 @@ static int queue_force(Engine &E, int mode, int &ntc, int ntcm, bool &cells_read
            nbf = launch_forces(d, p, E.tab, mixed, mode == 1 ? 1 : 0, E.variant[K_PAIR], pf, s));
     LAUNCH(E, K_FINALIZE, 1, s, launch_finalize_force(d, p, pe, nbe, pf, nbf, pk, E.kin_blocks, mode, s));
     if (rebuilt) *rebuilt = rb;
+    CUDA_CHECK(cudaGetLastError(), "force launches");
     return MOLDY_OK;
 }
 
@@ -761,6 +715,7 @@ int Engine::force_device(bool *rebuilt) {
 }
 
 int Engine::fetch_force_out(moldy_force_out *out) {
+    CUDA_CHECK(cudaGetLastError(), "force");
     CHECK(open_stage());
     CUDA_CHECK(cudaMemcpyAsync(host_box_, d.box, sizeof(BoxState), cudaMemcpyDeviceToHost, stream_), "box");
     CHECK(check_flags());
@@ -862,6 +817,7 @@ int Engine::velocityverlet(moldy_force_out *out) {
 int Engine::update_therm_avs(double *s123) {
     CHECK(check_ready());
     LAUNCH(*this, K_THERM, 2, stream_, launch_therm(d, prm, true, nullptr, stream_));   // prep, sums
+    CUDA_CHECK(cudaGetLastError(), "update_therm_avs");
     CHECK(open_stage());
     CUDA_CHECK(cudaMemcpyAsync(host_box_, d.box, sizeof(BoxState), cudaMemcpyDeviceToHost, stream_), "box");
     CHECK(check_flags());
@@ -1322,7 +1278,8 @@ struct moldy_gpu {
 #define GUARD(h)                                                                   \
     do {                                                                           \
         if (!(h) || !(h)->e) return fail(MOLDY_ERR_INVALID, "null handle");        \
-        cudaSetDevice((h)->e->device());                                          \
+        cudaSetDevice((h)->e->device());                                           \
+        cudaGetLastError(); /* an error that another caller left is not this call's */ \
     } while (0)
 
 #define TRY(expr)                                                                  \

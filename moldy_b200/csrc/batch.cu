@@ -2829,7 +2829,8 @@ struct moldy_batch {
 #define BGUARD(h)                                                                      \
     do {                                                                               \
         if (!(h) || !(h)->e) return moldy::set_last_error(MOLDY_ERR_INVALID, "null handle"); \
-        cudaSetDevice((h)->e->device);                                                \
+        cudaSetDevice((h)->e->device);                                                 \
+        cudaGetLastError(); /* an error that another caller left is not this call's */ \
     } while (0)
 #define BTRY(expr)                                                                     \
     try {                                                                              \

@@ -10,6 +10,7 @@
 
 #include "../../include/moldy_gpu.h"
 #include "common.cuh"
+#include "copystage.h"
 
 namespace moldy {
 
@@ -126,17 +127,6 @@ struct DeviceTables {
     size_t cap = 0;
     std::vector<unsigned char> host;
     ~DeviceTables();
-};
-
-// One pinned allocation per engine, made on first use: a head for small
-// results and two pieces for copies into pageable memory.
-constexpr size_t kStageBytes = 256 << 10;
-struct CopyStage {
-    unsigned char *head = nullptr, *piece = nullptr;
-    cudaEvent_t ev[2] = {nullptr, nullptr};
-    cudaError_t open(size_t head_bytes);
-    cudaError_t out(void *dst, const void *src, size_t bytes, cudaStream_t s);
-    ~CopyStage();
 };
 
 // Kernel families timed by the optional per-kernel CUDA-event profiler.
