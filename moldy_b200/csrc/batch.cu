@@ -87,9 +87,21 @@ __device__ __forceinline__ int stencil_off(int k, int nst) { return nst == 3 ? k
 
 __device__ __forceinline__ int wrapc(int c, int n) { return c < 0 ? c + n : (c >= n ? c - n : c); }
 
+// One 32-byte load of spos that sees what this launch has stored: the
+// persistent evaluation writes a rebuilt system's slots and screens them in the
+// same launch, so a read-only load (ldg4) would be undefined here.
+__device__ __forceinline__ double4 load_slot(const double4 *p) {
+    double4 v;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+
 // fixed-point record of a slot: x, y, z and the slot itself
 __device__ __forceinline__ int4 slot_record(const TileArgs &a, int slot) {
-    const double4 p = ldg4(&a.spos[slot]);
+    const double4 p = load_slot(&a.spos[slot]);
     return make_int4(fix32(p.x), fix32(p.y), fix32(p.z), slot);
 }
 
@@ -404,8 +416,8 @@ k_prepare(BSys *__restrict__ sys, const double *__restrict__ X, const double *__
 // The compact rows of the home atoms of cell c by one warp, with the warp's
 // tile (tp, ti: cap entries; pre, cs: 28); returns the longest row seen when it
 // exceeds pair_cap, else 0.
-__device__ __noinline__ bool inside_list(const double4 *__restrict__ spos, const double *b, double rv2, int i, int j) {
-    const double4 p = spos[i], q = spos[j];
+__device__ __noinline__ bool inside_list(const double4 *spos, const double *b, double rv2, int i, int j) {
+    const double4 p = load_slot(&spos[i]), q = load_slot(&spos[j]);
     double dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
     dx = dx - round(dx); dy = dy - round(dy); dz = dz - round(dz);
     double ux, uy, uz;
