@@ -1889,6 +1889,8 @@ class BatchEngine {
     HostTables ht;
     Tables tab;
     double rcut = 0.0;
+    double list_cut = 0.0;              // the cut that the lists and grids on the device cover (0: none)
+    bool layout_due = true;             // the last layout did not complete
     double skin = 0.3;                  // list radius rcut + skin (less where a box is too narrow)
     bool potential_set = false, state_set = false, boxes_set = false, pos_set = false;
     cudaStream_t stream = nullptr;
@@ -2116,11 +2118,10 @@ int BatchEngine::set_fetm(int nv, const double *av, const double *rv, int np, co
     for (int i = 0; i < nv; ++i) r = std::max(r, rv[i] * (1.0 + 1e-12));
     if (!(r > 0.0) || r > 1e100) return set_last_error(MOLDY_ERR_UNSUPPORTED, "tables without a finite cut");
     // the lists depend on the positions, the boxes, the skin and this radius
-    // alone: new functions with the same cut leave them as they are
-    const bool same_cut = potential_set && r == rcut;
+    // alone: new functions with the cut of a completed layout leave them as they are
     rcut = r;
     potential_set = true;
-    if (boxes_set && !same_cut) return layout();
+    if (boxes_set && (layout_due || rcut != list_cut)) return layout();
     return MOLDY_OK;
 }
 
@@ -2139,8 +2140,9 @@ int BatchEngine::set_state(const double *x0, const double *y0, const double *z0,
         all_heavy = *std::min_element(m, m + nt) > 0.05;
     }
     if (b0) {
+        std::vector<BSys> next = hsys;   // takes hsys's place once every box is regular
         for (int s = 0; s < nsys; ++s) {
-            BSys &S = hsys[s];
+            BSys &S = next[s];
             const double *b = b0 + 9 * (size_t)s;
             for (int k = 0; k < 9; ++k) S.b0[k] = b[k];
             double vol = b[0] * (b[4] * b[8] - b[7] * b[5]) + b[1] * (b[5] * b[6] - b[3] * b[8]) +
@@ -2154,6 +2156,7 @@ int BatchEngine::set_state(const double *x0, const double *y0, const double *z0,
                     S.tg[i + 3 * j] = t;
                 }
         }
+        hsys.swap(next);
         boxes_set = true;
         BCHECK(layout());
     }
@@ -2169,6 +2172,7 @@ int BatchEngine::set_state(const double *x0, const double *y0, const double *z0,
 // unique minimum image), and cells at least rv wide perpendicular to each
 // face.  Every list is marked stale.
 int BatchEngine::layout() {
+    layout_due = true;
     int cell = 0;
     std::vector<int32_t> csys;
     for (int s = 0; s < nsys; ++s) {
@@ -2236,6 +2240,7 @@ int BatchEngine::layout() {
         for (void *bp : bufs)
             if (bp) cudaFree(bp);
         cell_sys = cell_count = cell_start = cursor = todo = nullptr;
+        list_cut = 0.0;
         ncell = cell;
         BCHECK(balloc(&todo, ncell, "screen work"));
         BCHECK(balloc(&cell_sys, ncell, "cell_sys"));
@@ -2257,6 +2262,8 @@ int BatchEngine::layout() {
           "cell_sys");
     BCUDA(cudaMemcpyAsync(sys, hsys.data(), nsys * sizeof(BSys), cudaMemcpyHostToDevice, stream), "systems");
     BCUDA(cudaStreamSynchronize(stream), "layout");
+    list_cut = rcut;
+    layout_due = false;
     return MOLDY_OK;
 }
 
@@ -2270,6 +2277,10 @@ int BatchEngine::set_skin(double sk) {
 int BatchEngine::ready() {
     if (!potential_set) return set_last_error(MOLDY_ERR_ORDER, "the potential is not set");
     if (!state_set) return set_last_error(MOLDY_ERR_ORDER, "positions and boxes are not set");
+    // a longer cut whose layout was refused: the lists would miss pairs
+    if (!(list_cut >= rcut))
+        return set_last_error(MOLDY_ERR_ORDER, "the lists do not cover the potential's cut: the last boxes or the last "
+                                               "potential were refused");
     return MOLDY_OK;
 }
 
