@@ -331,13 +331,16 @@ int upload_device_tables(const HostTables &h, DeviceTables &dt, cudaStream_t s, 
     // value (the difference is the FP32 subtraction the device would do); the
     // density table keeps (phi_k, phi_k+1 - phi_k) side by side; FP64 intervals
     // as (node, step): (V', phi'), (V), (phi).  The last stored node has no
-    // step, so it is what every distance beyond it takes.
+    // step, so it is what every distance beyond it takes; neither has a node
+    // that is not finite (V at r = 0), which the whole interval above it takes
+    // (inf w + b dr, not inf + (b - inf) dr).
+    auto step = [](double lo, double hi) { return std::isfinite(lo) ? hi - lo : 0.0; };
     for (int i = 0; i < nr; ++i) {
         const int j = i + 1 < nr ? i + 1 : i;
         r4[i] = make_double4(h.vee[i], h.dvee[i], h.phi[i], h.dphi[i]);
-        df4[i] = make_double4(h.dvee[i], h.dphi[i], h.dvee[j] - h.dvee[i], h.dphi[j] - h.dphi[i]);
-        dv2[i] = make_double2(h.vee[i], h.vee[j] - h.vee[i]);
-        dp2[i] = make_double2(h.phi[i], h.phi[j] - h.phi[i]);
+        df4[i] = make_double4(h.dvee[i], h.dphi[i], step(h.dvee[i], h.dvee[j]), step(h.dphi[i], h.dphi[j]));
+        dv2[i] = make_double2(h.vee[i], step(h.vee[i], h.vee[j]));
+        dp2[i] = make_double2(h.phi[i], step(h.phi[i], h.phi[j]));
         phi2[i] = make_double2(h.phi[i], j > i ? h.phi[j] : 0.0);
         const float4 a = make_float4((float)h.vee[i], (float)h.dvee[i], (float)h.phi[i], (float)h.dphi[i]);
         const float4 b = make_float4((float)h.vee[j], (float)h.dvee[j], (float)h.phi[j], (float)h.dphi[j]);

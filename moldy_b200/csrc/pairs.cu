@@ -856,8 +856,8 @@ k_screen_d(Params p, Tables t, const double4 *__restrict__ pos, double4 *__restr
                 const double rz = b[2] * dx + b[5] * dy + b[8] * dz;
                 const double r2 = rx * rx + ry * ry + rz * rz;
                 const bool in = k0 + u < n && r2 <= t.rcull2;
-                double rr, dr;
-                const double r = root_and_inverse(in ? r2 : 1.0, rr);
+                double dr;
+                const double r = root(in ? r2 : 1.0);
                 const double2 q = __ldg(&t.dp2[interval_d(t, r, dr)]);
                 if (in) {
                     rho_a += fma(q.y, dr, q.x);

@@ -108,13 +108,24 @@ static __device__ float keep_radius2(const double *sb, double r) {
 // r = sqrt(r2) and 1/r of a positive r2 from one reciprocal square root: the
 // product r2 y is corrected by half its residual times y and then 1/r by its
 // own residual (one Newton step each), which leaves both within an ulp, in 6
-// operations where a square root and a division took two full routines.
+// operations where a square root and a division took two full routines.  Two
+// atoms at one point: r = 0, the table's first node, and 1/r is not a number
+// (the pair has no direction).  The high word tells, without the FP64 units.
 __device__ __forceinline__ double root_and_inverse(double r2, double &rr) {
     const double y = rsqrt(r2);
     double r = r2 * y;
     r = fma(fma(-r, r, r2), 0.5 * y, r);
     rr = fma(fma(-r, y, 1.0), y, y);
-    return r;
+    return __double2hiint(r2) == 0 ? 0.0 : r;
+}
+
+// r alone; of 0 it gives that of the smallest normal number, 1.5e-154 (one
+// integer maximum)
+__device__ __forceinline__ double root(double r2) {
+    r2 = __hiloint2double(max(__double2hiint(r2), 0x00100000), __double2loint(r2));
+    const double y = rsqrt(r2);
+    const double r = r2 * y;
+    return fma(fma(-r, r, r2), 0.5 * y, r);
 }
 
 // Interval of r in the stored nodes and the offset in it; beyond the last
