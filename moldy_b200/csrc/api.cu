@@ -593,6 +593,11 @@ int Engine::check_flags() {
     CUDA_CHECK(cudaMemcpyAsync(&st, &d.box->status, sizeof(st), cudaMemcpyDeviceToHost, stream_), "flags");
     CUDA_CHECK(cudaStreamSynchronize(stream_), "synchronize");
     prof.harvest();
+    if (f[7]) {
+        cudaMemsetAsync(d.flags, 0, sizeof(f), stream_);
+        cells_ready_ = list_ready_ = false;   // such atoms lie in cells that are not theirs
+        return fail(MOLDY_ERR_INVALID, "the position of an atom is not a finite number");
+    }
     if (f[0]) {
         cudaMemsetAsync(d.flags, 0, sizeof(f), stream_);
         char msg[200];

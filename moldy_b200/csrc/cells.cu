@@ -15,14 +15,24 @@
 
 namespace moldy {
 
+// The link cell of a position.  One that is not finite (a run that blew up) has
+// none: flag 7 is set and the atom takes the cell `lost` (any but one and the
+// same for all atoms, which the serial chain passes would be at for hours).
+__device__ __forceinline__ int link_cell(const double4 &p, int nlcx, int nlcy, int nlcz, int lost,
+                                         int32_t *__restrict__ flags) {
+    const int ix = cell_coord(p.x, nlcx), iy = cell_coord(p.y, nlcy), iz = cell_coord(p.z, nlcz);
+    if ((unsigned)ix < (unsigned)nlcx && (unsigned)iy < (unsigned)nlcy && (unsigned)iz < (unsigned)nlcz)
+        return ix + nlcx * iy + nlcx * nlcy * iz;
+    atomicExch(&flags[7], 1);
+    return lost;
+}
+
 __global__ void k_assign_cells(const double4 *__restrict__ pos, int nm, int nlcx, int nlcy,
                                int nlcz, int32_t *__restrict__ ic_out,
-                               int32_t *__restrict__ count) {
+                               int32_t *__restrict__ count, int32_t *__restrict__ flags) {
     int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= nm) return;
-    double4 p = pos[a];
-    int ix = cell_coord(p.x, nlcx), iy = cell_coord(p.y, nlcy), iz = cell_coord(p.z, nlcz);
-    int c = ix + nlcx * iy + nlcx * nlcy * iz;
+    const int c = link_cell(pos[a], nlcx, nlcy, nlcz, a % (nlcx * nlcy * nlcz), flags);
     ic_out[a] = c;
     if (count) atomicAdd(&count[c], 1);
 }
@@ -206,7 +216,7 @@ void launch_linkup(DeviceState &d, const Params &p, cudaStream_t s) {
     int nb = (p.nm + kAtomThreads - 1) / kAtomThreads;
     int nbc = (int)(((long long)p.ncell * 32 + kAtomThreads - 1) / kAtomThreads);   // a warp per cell
     cudaMemsetAsync(d.cell_count, 0, sizeof(int32_t) * p.ncell, s);
-    k_assign_cells<<<nb, kAtomThreads, 0, s>>>(d.pos, p.nm, p.nlcx, p.nlcy, p.nlcz, d.ic, d.cell_count);
+    k_assign_cells<<<nb, kAtomThreads, 0, s>>>(d.pos, p.nm, p.nlcx, p.nlcy, p.nlcz, d.ic, d.cell_count, d.flags);
     launch_exclusive_scan(d.cell_count, d.cell_start, p.ncell, s, d.scan_tmp);
     cudaMemsetAsync(d.new_count, 0, sizeof(int32_t) * p.ncell, s);
     k_fill_cells<<<nb, kAtomThreads, 0, s>>>(d.ic, p.nm, d.cell_start, d.new_count, d.cell_atoms);
@@ -216,14 +226,13 @@ void launch_linkup(DeviceState &d, const Params &p, cudaStream_t s) {
 // ------------------------------------------------------------------ relink --
 __global__ void k_relink_assign(const double4 *__restrict__ pos, int nm, int nlcx, int nlcy,
                                 int nlcz, const int32_t *__restrict__ ic,
-                                int32_t *__restrict__ ic_new, int32_t *__restrict__ arr_count) {
+                                int32_t *__restrict__ ic_new, int32_t *__restrict__ arr_count,
+                                int32_t *__restrict__ flags) {
     int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= nm) return;
-    double4 p = pos[a];
-    int ix = cell_coord(p.x, nlcx), iy = cell_coord(p.y, nlcy), iz = cell_coord(p.z, nlcz);
-    int c = ix + nlcx * iy + nlcx * nlcy * iz;
+    const int old = ic[a], c = link_cell(pos[a], nlcx, nlcy, nlcz, old, flags);
     ic_new[a] = c;
-    if (c != ic[a]) atomicAdd(&arr_count[c], 1);
+    if (c != old) atomicAdd(&arr_count[c], 1);
 }
 
 __global__ void k_relink_arrivals(int nm, const int32_t *__restrict__ ic,
@@ -413,7 +422,7 @@ void launch_relink(DeviceState &d, const Params &p, cudaStream_t s) {
     int nb = (p.nm + kAtomThreads - 1) / kAtomThreads;
     cudaMemsetAsync(d.arr_count, 0, sizeof(int32_t) * p.ncell, s);
     k_relink_assign<<<nb, kAtomThreads, 0, s>>>(d.pos, p.nm, p.nlcx, p.nlcy, p.nlcz, d.ic, d.ic_new,
-                                                d.arr_count);
+                                                d.arr_count, d.flags);
     launch_exclusive_scan(d.arr_count, d.arr_start, p.ncell, s, d.scan_tmp);
     cudaMemsetAsync(d.new_count, 0, sizeof(int32_t) * p.ncell, s);
     k_relink_arrivals<<<nb, kAtomThreads, 0, s>>>(p.nm, d.ic, d.ic_new, d.arr_start, d.new_count,

@@ -107,7 +107,8 @@ __device__ __forceinline__ double realsep_exact(const double *b, double dx, doub
     return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), __dmul_rn(rz, rz)));
 }
 
-// link-cell coordinate of a fractional position (src/linkcell_m.F90:150-152)
+// link-cell coordinate of a fractional position (src/linkcell_m.F90:150-152);
+// outside [0, nlc) when the position is not finite
 __device__ __forceinline__ int cell_coord(double x, int nlc) {
     const double hmeps = 0.4999999999;
     return (int)__dmul_rn(__dadd_rn(__dsub_rn(x, round(x)), hmeps), (double)nlc);

@@ -77,6 +77,7 @@ struct DeviceState {
     int32_t *flags = nullptr;     // [0] neighbour overflow, [1] relink inconsistency,
                                   // [2] overflow atom, [3] active-list overflow, [4] its count,
                                   // [5] intermediate-row overflow, [6] its count,
+                                  // [7] a position that is not finite (link cells),
                                   // [8] outer-row overflow, [9] its count,
                                   // [10] reverse half-row overflow, [11] its count,
                                   // [12] a link cell too full for the reverse-row masks,

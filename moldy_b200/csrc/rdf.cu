@@ -79,7 +79,7 @@ __device__ __forceinline__ void bin_pair(const HistArgs &a, const double *b, uns
     const double r = __dsqrt_rn(rsq);
     const int ibin = (int)__dmul_rn(r, (double)a.bpa);
     if (r <= 2.0) close += 1;                      // the routine's "too close" warning
-    if (ibin > a.maxbin) return;
+    if ((unsigned)ibin > (unsigned)a.maxbin) return;   // also a distance that is not a number
     hist_add<SMEM>(a, sh, ibin, si, species_of(a.spec, j));
 }
 
@@ -154,7 +154,7 @@ k_rdf_list(HistArgs a, const int32_t *__restrict__ nlist, const int32_t *__restr
                 const double r = __dsqrt_rn(rsq);
                 const int ibin = (int)__dmul_rn(r, (double)a.bpa);
                 if (r <= 2.0) close += 1;
-                if (ibin <= a.maxbin) hist_add<SMEM>(a, sh, ibin, si, species_of(a.spec, jj[u]));
+                if ((unsigned)ibin <= (unsigned)a.maxbin) hist_add<SMEM>(a, sh, ibin, si, species_of(a.spec, jj[u]));
             }
         }
     }
