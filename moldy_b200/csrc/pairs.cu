@@ -743,7 +743,9 @@ k_forces_st(Params p, Tables t, const int4 *__restrict__ posq2, const BoxState *
 #pragma unroll
                     for (int w = 0; w < 2; ++w) {
                         const bool live = e0 + u + w < ne;
-                        const float s = live ? r2[w] : 1.0f;
+                        // an entry past the end is the atom itself: d = 0 and the last node's fp, which is
+                        // finite whatever the table holds further in, add zero
+                        const float s = live ? r2[w] : 1.0e30f;
                         rr[w] = rsqrt_ftz(s);
                         float dr;
                         const int idx = interval(t, s * rr[w], dr);
@@ -754,7 +756,6 @@ k_forces_st(Params p, Tables t, const int4 *__restrict__ posq2, const BoxState *
                             const float2 qv = sv[idx];
                             pe += (double)fmaf(qv.y, dr, qv.x);
                         }
-                        // an entry past the end is the atom itself: d = 0 and a finite fp add zero
                     }
 #pragma unroll
                     for (int w = 0; w < 2; ++w) {
@@ -955,12 +956,13 @@ k_forces_d(Params p, Tables t, const double4 *__restrict__ pos2, const BoxState 
                 const double rz = b[2] * dx + b[5] * dy + b[8] * dz;
                 const double r2 = rx * rx + ry * ry + rz * rz;
                 double rr, dr;
-                const double r = root_and_inverse(live ? r2 : 1.0, rr);
+                const double r = root_and_inverse(r2, rr);
                 const int idx = interval_d(t, r, dr);
                 const double4 w = ldg4(&t.df4[idx]);
                 const double dvee = fma(w.z, dr, w.x), dphi = fma(w.w, dr, w.y);
-                const double fp = -dvee * rr - (dphi * pa.w + dphi * q.w) * rr;
-                const double gx = dx * fp, gy = dy * fp, gz = dz * fp;   // zero past the end (d = 0)
+                // an entry past the end is the atom itself (d = 0), whatever the table holds at r = 0
+                const double fp = live ? -dvee * rr - (dphi * pa.w + dphi * q.w) * rr : 0.0;
+                const double gx = dx * fp, gy = dy * fp, gz = dz * fp;
                 fxa += gx; fya += gy; fza += gz;
                 if (live && (ee[u] & kOwnBit)) {   // the owner's copy carries the pair energy
                     const double2 qv = __ldg(&t.dv2[idx]);
