@@ -1905,6 +1905,7 @@ class BatchEngine {
     int32_t *clist = nullptr, *ccnt = nullptr;   // rows of the pairs inside the cut (FP64 passes)
     unsigned long long *stats = nullptr;   // system list builds, system evaluations
     int32_t *todo = nullptr, *ntodo = nullptr;   // cells of the systems rebuilt in this evaluation
+    bool quench_open = false;           // a quench that did not end may have left work in todo
     int32_t *cg_order = nullptr;                 // systems by descending size
     int pair_cap = 48;                  // compact-row entries per atom
     double4 *spos = nullptr;
@@ -2281,6 +2282,13 @@ int BatchEngine::ready() {
     if (!(list_cut >= rcut))
         return set_last_error(MOLDY_ERR_ORDER, "the lists do not cover the potential's cut: the last boxes or the last "
                                                "potential were refused");
+    if (quench_open) {
+        // todo holds every cell once: the cells of systems that k_cg binned and
+        // no screen took are dropped, and every list is built anew
+        BCUDA(cudaMemsetAsync(ntodo, 0, sizeof(int32_t), stream), "screen work count");
+        k_set_active<<<(nsys + 255) / 256, 256, 0, stream>>>(nsys, sys, 1, 1);
+        quench_open = false;
+    }
     return MOLDY_OK;
 }
 
@@ -2772,6 +2780,7 @@ int BatchEngine::quench(int maxfn, int criterion, double fmax, double *out8) {
     BCUDA(cudaMemsetAsync(n_active, 0, sizeof(int), s), "counter");
     // first pass: every system asks for its first function value
     const PrepArgs pa{mass, Xb, cell_of, cell_count, cell_start, cursor, unsorted, sorted, spos, stats, todo, ntodo};
+    quench_open = true;   // until every system is done
     k_cg<<<nsys, kCgThreads, 0, s>>>(sys, cg, v, f, en_calc, press, maxfn, criterion, fmax, n_active, cg_order, pa);
     launches += 1;
     BCUDA(cudaGetLastError(), "quench start");
@@ -2833,6 +2842,7 @@ int BatchEngine::quench(int maxfn, int criterion, double fmax, double *out8) {
     // leave every system active for later force calls
     k_set_active<<<(nsys + 255) / 256, 256, 0, s>>>(nsys, sys, 1, 0);
     BCUDA(cudaStreamSynchronize(s), "quench");
+    quench_open = unfinished > 0;
     int ov = take_overflow();
     if (ov != 0)
         return set_last_error(MOLDY_ERR_CAPACITY, "an atom had " + std::to_string(ov) +
