@@ -813,6 +813,15 @@ int Engine::ensure_active_capacity(int min_pair, int min_mid, int min_out) {
 int Engine::velocityverlet(moldy_force_out *out) {
     CHECK(check_ready());
     bool rb = false;
+    if (runs_apply() && run_length(1) > 0) {   // the sums of md_steps' step
+        CHECK(ensure_active_capacity(0));
+        CHECK(queue_run(1, false, nullptr, 0, true, false));
+        ntc_ = ntc_ + 1 == ntcm_ ? 0 : ntc_ + 1;
+        CHECK(fetch_force_out(out));
+        if (out) out->rebuilt = 0;
+        forces_current_ = true;
+        return MOLDY_OK;
+    }
     LAUNCH(*this, K_DRIFT, 1, stream_,
                kin_blocks = launch_drift(d, prm, d.partials + 2 * (size_t)kMaxBlocks * kPartials, false, stream_));
     CHECK(queue_force(*this, 1, ntc_, ntcm_, cells_ready_, list_ready_, &rb, stream_));
@@ -824,7 +833,8 @@ int Engine::velocityverlet(moldy_force_out *out) {
 
 int Engine::update_therm_avs(double *s123) {
     CHECK(check_ready());
-    LAUNCH(*this, K_THERM, 2, stream_, launch_therm(d, prm, true, nullptr, stream_));   // prep, sums
+    if (runs_apply()) CHECK(queue_run_therm(nullptr, 0));
+    else LAUNCH(*this, K_THERM, 2, stream_, launch_therm(d, prm, true, nullptr, stream_));   // prep, sums
     CUDA_CHECK(cudaGetLastError(), "update_therm_avs");
     CHECK(open_stage());
     CUDA_CHECK(cudaMemcpyAsync(host_box_, d.box, sizeof(BoxState), cudaMemcpyDeviceToHost, stream_), "box");
@@ -864,9 +874,16 @@ int Engine::run_length(int left) const {
     return m;
 }
 
-// Queues a fused run of m steps and advances the host-side state; the pieces
-// are launched one by one while profiling (the same results bit for bit).
-int Engine::queue_run(int m, bool therm, double *rec, int rec0, bool last, bool &scalev, int *ntcs) {
+// Whether this engine's ordinary steps are taken by runs.  Then all of them
+// are, a single step and velocityverlet's too, and so are all sums of
+// update_therm_avs: how steps are split into calls changes no bit.
+bool Engine::runs_apply() const { return run_applies(prm, tab, precision_ == MOLDY_PREC_MIXED); }
+
+// Queues a fused run of m steps; therm: the step before awaits its
+// update_therm_avs; last: the run's last step stores rho and the forces; tail:
+// update_therm_avs of the run's last step, too.  The pieces are launched one by
+// one while profiling (the same results bit for bit).
+int Engine::queue_run(int m, bool therm, double *rec, int rec0, bool last, bool tail) {
     const bool mixed = precision_ == MOLDY_PREC_MIXED;
     cudaStream_t s = stream_;
     int rc = 0;
@@ -882,10 +899,28 @@ int Engine::queue_run(int m, bool therm, double *rec, int rec0, bool last, bool 
             pieces(K_PAIR, 2 * q + 2, 2 * q + 2);
         }
         pieces(K_FINALIZE, 2 * m + 1, 2 * m + 1);
+        if (tail) pieces(K_THERM, 2 * m + 2, 2 * m + 2);
     } else {
-        pieces(K_PAIR, 0, 2 * m + 1);
+        pieces(K_PAIR, 0, 2 * m + 1 + (tail ? 1 : 0));
     }
     if (rc) return cuda_fail((cudaError_t)rc, "fused run of steps");
+    therm_blocks = 0;
+    therm_rec = nullptr;
+    skip_rho = false;
+    return MOLDY_OK;
+}
+
+// update_therm_avs as a run's last piece takes it, by itself
+int Engine::queue_run_therm(double *rec, int k) {
+    int rc = 0;
+    LAUNCH(*this, K_THERM, 1, stream_,
+           rc = launch_run(d, prm, tab, precision_ == MOLDY_PREC_MIXED, rmid, rcut, rout, 0, 2, 2, 0, rec, k, 0, stream_));
+    return rc ? cuda_fail((cudaError_t)rc, "update_therm_avs") : MOLDY_OK;
+}
+
+// Host-side state of m steps of a run; whether scalev ends the last one
+bool Engine::advance_run(int m, int *ntcs) {
+    bool scalev = false;
     for (int q = 0; q < m; ++q) {
         ntc_ = ntc_ + 1;
         if (ntc_ == ntcm_) ntc_ = 0;
@@ -897,10 +932,7 @@ int Engine::queue_run(int m, bool therm, double *rec, int rec0, bool last, bool 
             scalev = nose_ > 0.0;
         }
     }
-    therm_blocks = 0;
-    therm_rec = nullptr;
-    skip_rho = false;
-    return MOLDY_OK;
+    return scalev;
 }
 
 // update_therm_avs of a step whose sums the next drift does not take, and the
@@ -947,23 +979,22 @@ int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
     cudaGraphExec_t step_graph = nullptr;
     bool graph_failed = prof.on || nsteps < 8, rec_synced = false;
     long long per_replay[K_COUNT] = {};
-    const bool mixed = precision_ == MOLDY_PREC_MIXED;
+    const bool runs = runs_apply();
     for (int k = 0; k < nsteps; ++k) {
         bool rb = false;
         // consecutive steps of a small system that need no half-list build, up
         // to and including one that is followed by a relink or scalev: one launch
-        const int run = !scale_pending && run_applies(prm, tab, mixed) ? run_length(nsteps - k) : 0;
-        if (run >= 2) {
+        const int run = runs ? run_length(nsteps - k) : 0;
+        if (run > 0) {
             CHECK(ensure_active_capacity(0));
-            bool scalev = false;
-            CHECK(queue_run(run, therm_pending, thermo ? d.thermo_rec : nullptr, k - 1, k + run == nsteps, scalev,
-                            &ntcs[k]));
-            for (int q = 0; q < run; ++q) rbs[k + q] = 0;
+            const int first = k;
             k += run - 1;
-            rec_synced = false;
-            therm_pending = !(scalev || k == nsteps - 1);
-            if (!therm_pending) finish_step(scalev, k == nsteps - 1, thermo ? d.thermo_rec + (size_t)kThermoRec * k : nullptr);
-            scale_pending = scalev && k < nsteps - 1;
+            const bool scalev = advance_run(run, &ntcs[first]);
+            // the next run takes this one's last update_therm_avs
+            const bool next = !scalev && k < nsteps - 1 && run_length(nsteps - 1 - k) > 0;
+            CHECK(queue_run(run, therm_pending, thermo ? d.thermo_rec : nullptr, first - 1, k == nsteps - 1, !next));
+            therm_pending = next;
+            if (scalev) LAUNCH(*this, K_SCALEV, 3, stream_, launch_scalev(d, prm, nose_, rqke_, true, true, stream_));
             if (ntc_ == 0) LAUNCH(*this, K_RELINK, 6, stream_, launch_relink(d, prm, stream_));
             continue;
         }
@@ -1063,9 +1094,16 @@ int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
         CHECK(queue_force(*this, 1, ntc_, ntcm_, cells_ready_, list_ready_, &rb, stream_));
         ntcs[k] = ntc_;
         rbs[k] = rb ? 1 : 0;
-        therm_pending = !(scalev || k == nsteps - 1);
-        if (!therm_pending) finish_step(scalev, k == nsteps - 1, thermo ? d.thermo_rec + (size_t)kThermoRec * k : nullptr);
-        scale_pending = scalev && k < nsteps - 1;
+        if (runs) {
+            therm_pending = !scalev && k < nsteps - 1 && run_length(nsteps - 1 - k) > 0;
+            if (!therm_pending) CHECK(queue_run_therm(thermo ? d.thermo_rec : nullptr, k));
+            if (scalev) LAUNCH(*this, K_SCALEV, 3, stream_, launch_scalev(d, prm, nose_, rqke_, true, true, stream_));
+        } else {
+            therm_pending = !(scalev || k == nsteps - 1);
+            if (!therm_pending)
+                finish_step(scalev, k == nsteps - 1, thermo ? d.thermo_rec + (size_t)kThermoRec * k : nullptr);
+            scale_pending = scalev && k < nsteps - 1;
+        }
         if (ntc_ == 0) LAUNCH(*this, K_RELINK, 6, stream_, launch_relink(d, prm, stream_));
     }
     if (step_graph) cudaGraphExecDestroy(step_graph);

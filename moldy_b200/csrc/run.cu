@@ -14,6 +14,9 @@
 //   B  (F' of step s published)          forces, the second half-kick, and the
 //      first half-kick and drift of step s + 1
 //
+// and, where the step after the run is not another run's, a last piece with the
+// update_therm_avs of the run's last step.
+//
 // L lanes of a warp share one atom's rows, so that a row of 14 to 20 entries
 // is one or two rounds of independent gathers instead of a serial walk; rows
 // are written in the order one lane would write them (a ballot places each
@@ -27,8 +30,13 @@
 //
 // Sums over an atom's pairs are grouped by lane and partial sums by block, in
 // a fixed order, so a run gives the same bits every time.  A run may be cut
-// into launches of single pieces (h0..h1): per-launch profiling does that, and
-// the results are the same bit for bit.
+// into launches of single pieces (h0..h1), as per-launch profiling does, and
+// steps may be cut into runs in any way: the results are the same bit for bit.
+// So every sum has one grouping (the atoms of a block, lane 0 of each group),
+// the box advances by the same code inside a run and at its end, and the last
+// piece takes its sums as piece A of the next run would.  The steps between
+// that launch the passes one by one (half-list builds) are the same steps
+// however a run is cut, and their update_therm_avs is taken here, too.
 #include <type_traits>
 
 #include "box.cuh"
@@ -65,7 +73,8 @@ struct RunArgs {
     int rec0;                                 // index of the record of the step before the run
     double rmid, rcut, rout;
     int m;                                    // steps of the run
-    int h0, h1;                               // pieces of this launch (0: first drift, 2s+1: A, 2s+2: B, 2m+1: box)
+    int h0, h1;                               // pieces of this launch (0: first drift, 2s+1: A, 2s+2: B, 2m+1: box,
+                                              // 2m+2: update_therm_avs of the last step)
     int therm;                                // the step before the run awaits its update_therm_avs
     int store;                                // 1: the run's last step also stores rho and the forces
 };
@@ -206,10 +215,9 @@ __device__ __forceinline__ double cof_at(const double *b, int i, int j) {
     return b[i1 + 3 * j1] * b[i2 + 3 * j2] - b[i2 + 3 * j1] * b[i1 + 3 * j2];
 }
 
-// The box half-kick that ends a step and the box quantities of its
-// update_therm_avs (finalize_box and therm_prep, one matrix element per
-// lane), by one warp.
-__device__ void warp_finalize(const Params &p, RunShared &s, int lane) {
+// The box half-kick that ends a step (finalize_box), one matrix element per
+// lane, by one warp.
+__device__ __forceinline__ void warp_half_kick(const Params &p, RunShared &s, int lane) {
     BoxState &B = s.box;
     const int e = lane < 9 ? lane : 0, i = e % 3, j = e / 3;
     const double *D = s.sum + kColF + 1, *M = s.sum + kColK;
@@ -230,32 +238,50 @@ __device__ void warp_finalize(const Params &p, RunShared &s, int lane) {
         if (lane < 9) { B.b2[e] = b2; B.b1[e] = b1; }
         __syncwarp();
     }
-    if (p.ivol != 1) {
-        double tg = 0.0, td = 0.0;
+}
+
+// The box quantities of a step's update_therm_avs (therm_prep), likewise.
+__device__ __forceinline__ void warp_therm_prep(const Params &p, RunShared &s, int lane) {
+    BoxState &B = s.box;
+    const int e = lane < 9 ? lane : 0, i = e % 3, j = e / 3;
+    double tg = 0.0, td = 0.0;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            tg += B.b0[k + 3 * i] * B.b0[k + 3 * j];
-            td = td + B.b1[k + 3 * i] * B.b0[k + 3 * j] + B.b0[k + 3 * i] * B.b1[k + 3 * j];
-        }
-        if (lane < 9) { s.tmp[e] = tg; s.tmp[9 + e] = td; }
-        __syncwarp();
-        double det = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) det += s.tmp[k] * cof_at(s.tmp, k, 0);
-        const double inv = cof_at(s.tmp, j, i) / det;
-        if (lane < 9) s.tmp[18 + e] = inv;
-        if (lane == 0 && fabs(det) == 0.0) B.status = MOLDY_ERR_SINGULAR_BOX;
-        __syncwarp();
-        double g = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) g += s.tmp[18 + i + 3 * k] * s.tmp[9 + k + 3 * j];
-        const double vol = mat_volume(B.b0);
-        if (lane < 9) {
-            B.th_tgid[e] = g;
-            B.th_cof[3 * i + j] = cof_at(B.b0, i, j) / vol;
-        }
-        __syncwarp();
+    for (int k = 0; k < 3; ++k) {
+        tg += B.b0[k + 3 * i] * B.b0[k + 3 * j];
+        td = td + B.b1[k + 3 * i] * B.b0[k + 3 * j] + B.b0[k + 3 * i] * B.b1[k + 3 * j];
     }
+    if (p.ivol == 1) td = 0.0;                        // the box does not move
+    if (lane < 9) { s.tmp[e] = tg; s.tmp[9 + e] = td; }
+    __syncwarp();
+    double det = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) det += s.tmp[k] * cof_at(s.tmp, k, 0);
+    const double inv = cof_at(s.tmp, j, i) / det;
+    if (lane < 9) s.tmp[18 + e] = inv;
+    if (lane == 0 && fabs(det) == 0.0) B.status = MOLDY_ERR_SINGULAR_BOX;
+    __syncwarp();
+    double g = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) g += s.tmp[18 + i + 3 * k] * s.tmp[9 + k + 3 * j];
+    const double vol = mat_volume(B.b0);
+    if (lane < 9) {
+        B.th_tgid[e] = g;
+        B.th_cof[3 * i + j] = cof_at(B.b0, i, j) / vol;
+    }
+    __syncwarp();
+}
+
+// A step's thermo record (therm_store) from its box b0, b1, the three sums of
+// update_therm_avs and its energy, by one thread
+__device__ __noinline__ void step_record(const Params &p, const double *b0, const double *b1, const double *s3, double pe,
+                                         double *r) {
+    const double bk = 1.3806504e-23 / 1.602176487e-19;
+    const double ke = s3[2] / (p.deltat * p.deltat) / 2.0, vol = mat_volume(b0);
+    double boxke = 0.0;
+    for (int k = 0; k < 9; ++k) boxke = boxke + (b1[k] * b1[k]) / p.bdel2;
+    const double te = ke + pe, hh = te + p.press * vol;
+    r[0] = ke; r[1] = pe; r[2] = te; r[3] = hh; r[4] = hh + boxke; r[5] = vol;
+    r[6] = s3[0]; r[7] = s3[1]; r[8] = s3[2]; r[9] = ke / (1.5 * bk * (double)p.nm); r[10] = boxke;
 }
 
 // The box half of velocityverlet's first part, and the list decision of
@@ -475,34 +501,38 @@ k_run(Params p, Tables t, RunArgs a) {
     Tab tab;
     double2 *se;
     const int ne_emb = t.nlookup + 1 < kRunEmb ? t.nlookup + 1 : kRunEmb;
+    const bool pairs = a.h0 <= 2 * a.m;           // a piece of this launch reads the tables
     if constexpr (MIXED) {
         float4 *r4 = reinterpret_cast<float4 *>(dsm);
         float2 *ph = reinterpret_cast<float2 *>(r4 + 2 * (size_t)t.nr);
         se = reinterpret_cast<double2 *>(ph + ((t.nr + 1) & ~1));
-        for (int k = tid; k < 2 * t.nr; k += blockDim.x) r4[k] = __ldg(&t.r4f[k]);
-        for (int k = tid; k < t.nr; k += blockDim.x) ph[k] = __ldg(&t.phi2f[k]);
+        for (int k = tid; pairs && k < 2 * t.nr; k += blockDim.x) r4[k] = __ldg(&t.r4f[k]);
+        for (int k = tid; pairs && k < t.nr; k += blockDim.x) ph[k] = __ldg(&t.phi2f[k]);
         tab.r4 = r4; tab.phi = ph;
     } else {
         double4 *r4 = reinterpret_cast<double4 *>(dsm);
         double2 *ph = reinterpret_cast<double2 *>(r4 + t.nr);
         se = ph + t.nr;
-        for (int k = tid; k < t.nr; k += blockDim.x) { r4[k] = t.r4[k]; ph[k] = __ldg(&t.phi2[k]); }
+        for (int k = tid; pairs && k < t.nr; k += blockDim.x) { r4[k] = t.r4[k]; ph[k] = __ldg(&t.phi2[k]); }
         tab.r4 = r4; tab.phi = ph;
     }
-    for (int k = tid; k < ne_emb; k += blockDim.x) se[k] = __ldg(&t.e2[k]);
+    for (int k = tid; pairs && k < ne_emb; k += blockDim.x) se[k] = __ldg(&t.e2[k]);
     box_load(s.box, a.box);
     if (tid == 0) s.fail = 0;
     __syncthreads();
 
     unsigned epoch = 0;
     for (int h = a.h0; h <= a.h1; ++h) {
-        if (h == 0) {
-            // ---- first half-kick and drift of the run's first step (k_drift)
+        if (h == 0 && a.m > 0) {
+            // ---- first half-kick and drift of the run's first step (k_drift),
+            // with the sums in piece B's grouping
             double k6[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
             float d2 = 0.f, bs[9];
 #pragma unroll
             for (int k = 0; k < 9; ++k) bs[k] = (float)(s.box.b0[k] * kFixUnit);
-            for (int i = blockIdx.x * blockDim.x + tid; i < nm; i += gridDim.x * blockDim.x) {
+            for (int it = 0; it < rounds; ++it) {
+                const int i = first + it * per_round;
+                if (i >= nm || g != 0) continue;
                 const double ex = a.x1[i], ey = a.x1[nm + i], ez = a.x1[2 * nm + i];
                 const double wx = a.x2[i], wy = a.x2[nm + i], wz = a.x2[2 * nm + i];
                 double4 q = a.pos[i];
@@ -519,9 +549,9 @@ k_run(Params p, Tables t, RunArgs a) {
             continue;
         }
         if (h == 2 * a.m + 1) {
-            // ---- the box at the end of the run, by block 0
+            // ---- the box at the end of the run; by every block where the last piece follows
             const int pb = (a.m - 1) & 1;
-            if (blockIdx.x == 0) {
+            if (blockIdx.x == 0 || a.h1 > h) {
                 for (int c = warp; c < kColT; c += nw)
                     if (c != kColMax) {
                         const double x = reduce_col(a, pb, c);
@@ -529,17 +559,54 @@ k_run(Params p, Tables t, RunArgs a) {
                     }
                 __syncthreads();
                 if (tid == 0) {
-                    // finalize_box takes embedding energy, pairs; pair energy, virial; kinetic moments
+                    // finalize_box takes embedding energy, pairs; pair energy, virial; kinetic moments;
+                    // the half-kick is that of the steps before
                     double sr[15];
                     sr[0] = s.sum[kColE]; sr[1] = s.sum[kColE + 1];
                     for (int k = 0; k < 7; ++k) sr[2 + k] = s.sum[kColF + k];
                     for (int k = 0; k < 6; ++k) sr[9 + k] = s.sum[kColK + k];
                     if (s.box.mid_rebuild) s.box.outdisp2 = dbits(s.sum[kColOut]);
                     if (s.box.out_rebuild) s.box.halfdisp2 = dbits(s.sum[kColHalf]);
-                    finalize_box(p, s.box, sr, 1);
+                    finalize_box(p, s.box, sr, 0);
                 }
+                __syncwarp();
+                if (warp == 0) warp_half_kick(p, s, lane);
             }
             if (!end_piece(a, s, epoch, 0u, false, 0)) return;
+            continue;
+        }
+        if (h == 2 * a.m + 2) {
+            // ---- update_therm_avs of the run's last step, in piece A's grouping
+            if (warp == 0) {
+                warp_therm_prep(p, s, lane);
+                if (lane < 9) s.box.tgid[lane] = s.box.th_tgid[lane];
+            }
+            __syncthreads();
+            double vt[3] = {0.0, 0.0, 0.0};
+            for (int it = 0; it < rounds; ++it) {
+                const int i = first + it * per_round;
+                if (i >= nm || g != 0 || a.znum[i] == 0) continue;
+                therm_terms(vt, s.box.th_tgid, s.box.b0, s.box.th_cof, a.mass[i], a.x1[i], a.x1[nm + i],
+                            a.x1[2 * nm + i], a.x2[i], a.x2[nm + i], a.x2[2 * nm + i]);
+            }
+            warp_columns<3>(s, kA_T, vt);
+            if (!end_piece(a, s, epoch, 0x1cu, true, 0)) return;
+            if (blockIdx.x == 0 && warp == 0) {
+                double s3[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) s3[k] = reduce_col(a, 0, kColT + k);
+                if (lane == 0) {
+                    BoxState &B = s.box;
+                    double r[kThermoRec], tg[9], tgdot[9], tginv[9], tgid[9], vol;
+                    step_record(p, B.b0, B.b1, s3, B.pe, r);
+                    if (a.rec)
+                        for (int k = 0; k < kThermoRec; ++k) a.rec[(size_t)kThermoRec * (size_t)(a.rec0 + a.m) + k] = r[k];
+                    B.ke = r[0]; B.te = r[2]; B.h = r[3]; B.th = r[4]; B.vol = r[5]; B.s1 = r[6]; B.s2 = r[7];
+                    B.s3 = r[8]; B.temp = r[9]; B.boxke = r[10];
+                    therm_box(p, B.b0, B.b1, tg, tgdot, tginv, tgid, vol);
+                    for (int k = 0; k < 9; ++k) { B.tg[k] = tg[k]; B.tgdot[k] = tgdot[k]; B.tginv[k] = tginv[k]; }
+                }
+            }
             continue;
         }
         const int step = (h - 1) >> 1, buf = step & 1, pbuf = buf ^ 1;
@@ -569,8 +636,10 @@ k_run(Params p, Tables t, RunArgs a) {
                             if (s.box.mid_rebuild) s.box.outdisp2 = dbits(s.sum[kColOut]);
                             if (s.box.out_rebuild) s.box.halfdisp2 = dbits(s.sum[kColHalf]);
                         }
-                        warp_finalize(p, s, lane);
+                        warp_half_kick(p, s, lane);
                     }
+                    // of a fixed box they are the same at every step
+                    if (p.ivol == 1 ? step == 0 || h == a.h0 : fin || a.therm) warp_therm_prep(p, s, lane);
                     if (lane < 9) {
                         s.box.rec_b0[lane] = s.box.b0[lane];
                         s.box.rec_b1[lane] = s.box.b1[lane];
@@ -726,14 +795,7 @@ k_run(Params p, Tables t, RunArgs a) {
             // the energy of that step: of this run, or as the launches before it left it
             const double pe = fin ? reduce_col(a, pbuf, kColE) + reduce_col(a, pbuf, kColF) : s.box.pe;
             if (lane == 0) {
-                const double bk = 1.3806504e-23 / 1.602176487e-19;
-                const double ke = s3[2] / (p.deltat * p.deltat) / 2.0, vol = mat_volume(s.box.rec_b0);
-                double boxke = 0.0;
-                for (int k = 0; k < 9; ++k) boxke = boxke + (s.box.rec_b1[k] * s.box.rec_b1[k]) / p.bdel2;
-                const double te = ke + pe, hh = te + p.press * vol;
-                double *r = a.rec + (size_t)kThermoRec * (size_t)(a.rec0 + step);
-                r[0] = ke; r[1] = pe; r[2] = te; r[3] = hh; r[4] = hh + boxke; r[5] = vol;
-                r[6] = s3[0]; r[7] = s3[1]; r[8] = s3[2]; r[9] = ke / (1.5 * bk * (double)nm); r[10] = boxke;
+                step_record(p, s.box.rec_b0, s.box.rec_b1, s3, pe, a.rec + (size_t)kThermoRec * (size_t)(a.rec0 + step));
             }
             __syncwarp();
         }
@@ -900,6 +962,7 @@ k_run(Params p, Tables t, RunArgs a) {
             return;
     }
     // the box for the launches that follow: every block has read it before the last barrier
+    __syncthreads();
     if (blockIdx.x == 0) box_store(a.box, s.box);
 }
 
@@ -954,7 +1017,7 @@ bool run_applies(const Params &p, const Tables &t, bool mixed) {
 }
 
 size_t run_scratch_bytes() { return 2 * (size_t)kCols * kRunBlocks * sizeof(double) +
-           (size_t)(2 * kRunMaxSteps + 2) * kBarStride * sizeof(unsigned long long); }
+           (size_t)(2 * kRunMaxSteps + 3) * kBarStride * sizeof(unsigned long long); }
 
 int launch_run(DeviceState &d, const Params &p, const Tables &t, bool mixed, double rmid, double rcut, double rout,
                int m, int h0, int h1, int therm, double *rec, int rec0, int store, cudaStream_t s) {
