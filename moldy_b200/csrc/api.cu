@@ -833,7 +833,7 @@ int Engine::velocityverlet(moldy_force_out *out) {
 
 int Engine::update_therm_avs(double *s123) {
     CHECK(check_ready());
-    if (runs_apply()) CHECK(queue_run_therm(nullptr, 0));
+    if (runs_apply()) queue_run_therm(nullptr, 0);
     else LAUNCH(*this, K_THERM, 2, stream_, launch_therm(d, prm, true, nullptr, stream_));   // prep, sums
     CUDA_CHECK(cudaGetLastError(), "update_therm_avs");
     CHECK(open_stage());
@@ -881,7 +881,7 @@ bool Engine::runs_apply() const { return run_applies(prm, tab, precision_ == MOL
 
 // Queues a fused run of m steps; therm: the step before awaits its
 // update_therm_avs; last: the run's last step stores rho and the forces; tail:
-// update_therm_avs of the run's last step, too.  The pieces are launched one by
+// update_therm_avs of the run's last step as well.  The pieces are launched one by
 // one while profiling (the same results bit for bit).
 int Engine::queue_run(int m, bool therm, double *rec, int rec0, bool last, bool tail) {
     const bool mixed = precision_ == MOLDY_PREC_MIXED;
@@ -899,23 +899,20 @@ int Engine::queue_run(int m, bool therm, double *rec, int rec0, bool last, bool 
             pieces(K_PAIR, 2 * q + 2, 2 * q + 2);
         }
         pieces(K_FINALIZE, 2 * m + 1, 2 * m + 1);
-        if (tail) pieces(K_THERM, 2 * m + 2, 2 * m + 2);
     } else {
-        pieces(K_PAIR, 0, 2 * m + 1 + (tail ? 1 : 0));
+        pieces(K_PAIR, 0, 2 * m + 1);
     }
     if (rc) return cuda_fail((cudaError_t)rc, "fused run of steps");
+    if (tail) queue_run_therm(rec, rec0 + m);
     therm_blocks = 0;
     therm_rec = nullptr;
     skip_rho = false;
     return MOLDY_OK;
 }
 
-// update_therm_avs as a run's last piece takes it, by itself
-int Engine::queue_run_therm(double *rec, int k) {
-    int rc = 0;
-    LAUNCH(*this, K_THERM, 1, stream_,
-           rc = launch_run(d, prm, tab, precision_ == MOLDY_PREC_MIXED, rmid, rcut, rout, 0, 2, 2, 0, rec, k, 0, stream_));
-    return rc ? cuda_fail((cudaError_t)rc, "update_therm_avs") : MOLDY_OK;
+// update_therm_avs with the runs' sums; k: the index of the step's record
+void Engine::queue_run_therm(double *rec, int k) {
+    LAUNCH(*this, K_THERM, 1, stream_, launch_run_therm(d, prm, rec, k, stream_));
 }
 
 // Host-side state of m steps of a run; whether scalev ends the last one
@@ -1096,7 +1093,7 @@ int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
         rbs[k] = rb ? 1 : 0;
         if (runs) {
             therm_pending = !scalev && k < nsteps - 1 && run_length(nsteps - 1 - k) > 0;
-            if (!therm_pending) CHECK(queue_run_therm(thermo ? d.thermo_rec : nullptr, k));
+            if (!therm_pending) queue_run_therm(thermo ? d.thermo_rec : nullptr, k);
             if (scalev) LAUNCH(*this, K_SCALEV, 3, stream_, launch_scalev(d, prm, nose_, rqke_, true, true, stream_));
         } else {
             therm_pending = !(scalev || k == nsteps - 1);

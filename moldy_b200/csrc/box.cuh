@@ -14,6 +14,22 @@ __device__ __forceinline__ void kin_moment(double (&v)[6], double m, double ux, 
     v[3] += m * ux * uy; v[4] += m * ux * uz; v[5] += m * uy * uz;
 }
 
+// True in every thread of the block that finishes last of the grid, once the
+// partials of all blocks are visible to it; the ticket is left at zero for the
+// next launch.
+__device__ __forceinline__ bool last_block(int32_t *ticket) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+        if (last) *ticket = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last != 0;
+}
+
 // ---------------------------------------------------------- thermo sums ----
 // update_therm_avs (src/dynamics_m.F90:649-734): tg, tgdot (ivol != 1),
 // tgid = tg^-1 tgdot, vol, and per-atom s1 = sum |F|^2, s2 = sum |F|^4,
@@ -62,7 +78,7 @@ static __device__ void therm_prep(const Params &p, const double *b, const double
 // The box algebra of k_finalize_force, by one thread on the block's shared
 // copy of the box: sr holds the 15 reduced sums (embedding energy, pair
 // count; pair energy, virial moments; kinetic moments).
-static __device__ void finalize_box(const Params &p, BoxState &B, const double *sr, int mode) {
+static __device__ void finalize_box(const Params &p, BoxState &B, const double *sr, int mode, bool prep = true) {
     const double *se = sr, *sf = sr + 2, *sk = sr + 9;
     // the box algebra runs on register copies and is stored once at the end
     double b0[9], b1[9], b2[9], tp[9], tk[9], tc[9], tg[9], tgdot[9], fb[9];
@@ -122,7 +138,7 @@ static __device__ void finalize_box(const Params &p, BoxState &B, const double *
     }
 #pragma unroll
     for (int k = 0; k < 9; ++k) { B.b1[k] = b1[k]; B.b2[k] = b2[k]; }
-    therm_prep(p, b0, b1, B);       // for the update_therm_avs that follows
+    if (prep) therm_prep(p, b0, b1, B);       // for the update_therm_avs that follows
 }
 
 // update_therm_avs (src/dynamics_m.F90:649-734), one atom's terms: s1 += |F|^2,

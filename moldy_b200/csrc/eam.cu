@@ -93,22 +93,6 @@ __global__ void k_therm_prep(Params p, BoxState *__restrict__ box) {
     therm_prep(p, b0, b1, *box);
 }
 
-// True in every thread of the block that finishes last of the grid, once the
-// partials of all blocks are visible to it; the ticket is left at zero for the
-// next launch.
-__device__ __forceinline__ bool last_block(int32_t *ticket) {
-    __shared__ int last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
-        if (last) *ticket = 0;
-    }
-    __syncthreads();
-    if (last) __threadfence();
-    return last != 0;
-}
-
 // ------------------------------------------------ intermediate-list check --
 // therm_nblk > 0: first finish the update_therm_avs that the drift kernel
 // took for the step that has just ended (its block partials), before the box

@@ -240,7 +240,7 @@ class Engine {
     int run_length(int left) const;
     bool runs_apply() const;
     int queue_run(int m, bool therm, double *rec, int rec0, bool last, bool tail);
-    int queue_run_therm(double *rec, int k);
+    void queue_run_therm(double *rec, int k);
     bool advance_run(int m, int *ntcs);
 
     cudaStream_t stream_ = nullptr;
@@ -352,15 +352,16 @@ void launch_mid_decide(DeviceState &d, const Params &p, double rmid, double rcut
                        int rec_indexed = 0);
 // runs of steps in one launch (run.cu): whether they apply, their device
 // scratch, and the pieces h0..h1 (0: first drift, 2s+1 and 2s+2: the two
-// pieces of step s, 2m+1: the final box, 2m+2: update_therm_avs of the last
-// step) of a run of m steps; therm: the step before awaits its
-// update_therm_avs; rec, rec0: thermo records and the index of that step's
-// (m = 0, piece 2: of the step itself); store: the last step stores rho and the forces.  Returns the
+// pieces of step s, 2m+1: the final box) of a run of m steps; therm: the step
+// before awaits its update_therm_avs; rec, rec0: thermo records and the index
+// of that step's; store: the last step stores rho and the forces.  Returns the
 // CUDA status of the launch.
 bool run_applies(const Params &p, const Tables &t, bool mixed);
 size_t run_scratch_bytes();
 int launch_run(DeviceState &d, const Params &p, const Tables &t, bool mixed, double rmid, double rcut, double rout,
                int m, int h0, int h1, int therm, double *rec, int rec0, int store, cudaStream_t s);
+// update_therm_avs with the sums of a run, of the step whose record has index k
+void launch_run_therm(DeviceState &d, const Params &p, double *rec, int k, cudaStream_t s);
 void launch_set_rec_step(DeviceState &d, int step, cudaStream_t s);
 // the outer list from the half list when k_mid_decide asked for it, then the
 // intermediate list from the outer list when it asked for that

@@ -14,8 +14,8 @@
 //   B  (F' of step s published)          forces, the second half-kick, and the
 //      first half-kick and drift of step s + 1
 //
-// and, where the step after the run is not another run's, a last piece with the
-// update_therm_avs of the run's last step.
+// The update_therm_avs of the run's last step is piece A's of the run that
+// follows at once, else a launch of its own (k_run_therm).
 //
 // L lanes of a warp share one atom's rows, so that a row of 14 to 20 entries
 // is one or two rounds of independent gathers instead of a serial walk; rows
@@ -33,10 +33,10 @@
 // into launches of single pieces (h0..h1), as per-launch profiling does, and
 // steps may be cut into runs in any way: the results are the same bit for bit.
 // So every sum has one grouping (the atoms of a block, lane 0 of each group),
-// the box advances by the same code inside a run and at its end, and the last
-// piece takes its sums as piece A of the next run would.  The steps between
-// that launch the passes one by one (half-list builds) are the same steps
-// however a run is cut, and their update_therm_avs is taken here, too.
+// the box advances by the same code inside a run and at its end, and
+// k_run_therm takes its sums as piece A does.  The steps between that launch
+// the passes one by one (half-list builds) are the same steps however a run is
+// cut, and their update_therm_avs is taken here, too.
 #include <type_traits>
 
 #include "box.cuh"
@@ -73,8 +73,7 @@ struct RunArgs {
     int rec0;                                 // index of the record of the step before the run
     double rmid, rcut, rout;
     int m;                                    // steps of the run
-    int h0, h1;                               // pieces of this launch (0: first drift, 2s+1: A, 2s+2: B, 2m+1: box,
-                                              // 2m+2: update_therm_avs of the last step)
+    int h0, h1;                               // pieces of this launch (0: first drift, 2s+1: A, 2s+2: B, 2m+1: box)
     int therm;                                // the step before the run awaits its update_therm_avs
     int store;                                // 1: the run's last step also stores rho and the forces
 };
@@ -185,6 +184,18 @@ __device__ __forceinline__ bool end_piece(const RunArgs &a, RunShared &s, unsign
     return s.fail == 0;
 }
 
+// finalize_box at the end of a run, by one thread (out of line: its registers
+// do not count against the pieces)
+__device__ __noinline__ void end_box(const Params &p, RunShared &s) {
+    double sr[15];
+    sr[0] = s.sum[kColE]; sr[1] = s.sum[kColE + 1];
+    for (int k = 0; k < 7; ++k) sr[2 + k] = s.sum[kColF + k];
+    for (int k = 0; k < 6; ++k) sr[9 + k] = s.sum[kColK + k];
+    if (s.box.mid_rebuild) s.box.outdisp2 = (unsigned long long)__double_as_longlong(s.sum[kColOut]);
+    if (s.box.out_rebuild) s.box.halfdisp2 = (unsigned long long)__double_as_longlong(s.sum[kColHalf]);
+    finalize_box(p, s.box, sr, 0, false);
+}
+
 // Column col of buffer buf over the blocks, by one warp: the same bits in every block
 __device__ __forceinline__ double reduce_col(const RunArgs &a, int buf, int col) {
     const double *c = column(a, buf, col);
@@ -241,7 +252,7 @@ __device__ __forceinline__ void warp_half_kick(const Params &p, RunShared &s, in
 }
 
 // The box quantities of a step's update_therm_avs (therm_prep), likewise.
-__device__ __forceinline__ void warp_therm_prep(const Params &p, RunShared &s, int lane) {
+__device__ __noinline__ void warp_therm_prep(const Params &p, RunShared &s, int lane) {
     BoxState &B = s.box;
     const int e = lane < 9 ? lane : 0, i = e % 3, j = e / 3;
     double tg = 0.0, td = 0.0;
@@ -273,7 +284,7 @@ __device__ __forceinline__ void warp_therm_prep(const Params &p, RunShared &s, i
 
 // A step's thermo record (therm_store) from its box b0, b1, the three sums of
 // update_therm_avs and its energy, by one thread
-__device__ __noinline__ void step_record(const Params &p, const double *b0, const double *b1, const double *s3, double pe,
+__device__ __forceinline__ void step_record(const Params &p, const double *b0, const double *b1, const double *s3, double pe,
                                          double *r) {
     const double bk = 1.3806504e-23 / 1.602176487e-19;
     const double ke = s3[2] / (p.deltat * p.deltat) / 2.0, vol = mat_volume(b0);
@@ -501,29 +512,28 @@ k_run(Params p, Tables t, RunArgs a) {
     Tab tab;
     double2 *se;
     const int ne_emb = t.nlookup + 1 < kRunEmb ? t.nlookup + 1 : kRunEmb;
-    const bool pairs = a.h0 <= 2 * a.m;           // a piece of this launch reads the tables
     if constexpr (MIXED) {
         float4 *r4 = reinterpret_cast<float4 *>(dsm);
         float2 *ph = reinterpret_cast<float2 *>(r4 + 2 * (size_t)t.nr);
         se = reinterpret_cast<double2 *>(ph + ((t.nr + 1) & ~1));
-        for (int k = tid; pairs && k < 2 * t.nr; k += blockDim.x) r4[k] = __ldg(&t.r4f[k]);
-        for (int k = tid; pairs && k < t.nr; k += blockDim.x) ph[k] = __ldg(&t.phi2f[k]);
+        for (int k = tid; k < 2 * t.nr; k += blockDim.x) r4[k] = __ldg(&t.r4f[k]);
+        for (int k = tid; k < t.nr; k += blockDim.x) ph[k] = __ldg(&t.phi2f[k]);
         tab.r4 = r4; tab.phi = ph;
     } else {
         double4 *r4 = reinterpret_cast<double4 *>(dsm);
         double2 *ph = reinterpret_cast<double2 *>(r4 + t.nr);
         se = ph + t.nr;
-        for (int k = tid; pairs && k < t.nr; k += blockDim.x) { r4[k] = t.r4[k]; ph[k] = __ldg(&t.phi2[k]); }
+        for (int k = tid; k < t.nr; k += blockDim.x) { r4[k] = t.r4[k]; ph[k] = __ldg(&t.phi2[k]); }
         tab.r4 = r4; tab.phi = ph;
     }
-    for (int k = tid; pairs && k < ne_emb; k += blockDim.x) se[k] = __ldg(&t.e2[k]);
+    for (int k = tid; k < ne_emb; k += blockDim.x) se[k] = __ldg(&t.e2[k]);
     box_load(s.box, a.box);
     if (tid == 0) s.fail = 0;
     __syncthreads();
 
     unsigned epoch = 0;
     for (int h = a.h0; h <= a.h1; ++h) {
-        if (h == 0 && a.m > 0) {
+        if (h == 0) {
             // ---- first half-kick and drift of the run's first step (k_drift),
             // with the sums in piece B's grouping
             double k6[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -549,9 +559,9 @@ k_run(Params p, Tables t, RunArgs a) {
             continue;
         }
         if (h == 2 * a.m + 1) {
-            // ---- the box at the end of the run; by every block where the last piece follows
+            // ---- the box at the end of the run, by block 0
             const int pb = (a.m - 1) & 1;
-            if (blockIdx.x == 0 || a.h1 > h) {
+            if (blockIdx.x == 0) {
                 for (int c = warp; c < kColT; c += nw)
                     if (c != kColMax) {
                         const double x = reduce_col(a, pb, c);
@@ -560,53 +570,14 @@ k_run(Params p, Tables t, RunArgs a) {
                 __syncthreads();
                 if (tid == 0) {
                     // finalize_box takes embedding energy, pairs; pair energy, virial; kinetic moments;
-                    // the half-kick is that of the steps before
-                    double sr[15];
-                    sr[0] = s.sum[kColE]; sr[1] = s.sum[kColE + 1];
-                    for (int k = 0; k < 7; ++k) sr[2 + k] = s.sum[kColF + k];
-                    for (int k = 0; k < 6; ++k) sr[9 + k] = s.sum[kColK + k];
-                    if (s.box.mid_rebuild) s.box.outdisp2 = dbits(s.sum[kColOut]);
-                    if (s.box.out_rebuild) s.box.halfdisp2 = dbits(s.sum[kColHalf]);
-                    finalize_box(p, s.box, sr, 0);
+                    // the half-kick is that of the steps before, and what update_therm_avs
+                    // needs is formed where it is taken
+                    end_box(p, s);
                 }
                 __syncwarp();
                 if (warp == 0) warp_half_kick(p, s, lane);
             }
             if (!end_piece(a, s, epoch, 0u, false, 0)) return;
-            continue;
-        }
-        if (h == 2 * a.m + 2) {
-            // ---- update_therm_avs of the run's last step, in piece A's grouping
-            if (warp == 0) {
-                warp_therm_prep(p, s, lane);
-                if (lane < 9) s.box.tgid[lane] = s.box.th_tgid[lane];
-            }
-            __syncthreads();
-            double vt[3] = {0.0, 0.0, 0.0};
-            for (int it = 0; it < rounds; ++it) {
-                const int i = first + it * per_round;
-                if (i >= nm || g != 0 || a.znum[i] == 0) continue;
-                therm_terms(vt, s.box.th_tgid, s.box.b0, s.box.th_cof, a.mass[i], a.x1[i], a.x1[nm + i],
-                            a.x1[2 * nm + i], a.x2[i], a.x2[nm + i], a.x2[2 * nm + i]);
-            }
-            warp_columns<3>(s, kA_T, vt);
-            if (!end_piece(a, s, epoch, 0x1cu, true, 0)) return;
-            if (blockIdx.x == 0 && warp == 0) {
-                double s3[3];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) s3[k] = reduce_col(a, 0, kColT + k);
-                if (lane == 0) {
-                    BoxState &B = s.box;
-                    double r[kThermoRec], tg[9], tgdot[9], tginv[9], tgid[9], vol;
-                    step_record(p, B.b0, B.b1, s3, B.pe, r);
-                    if (a.rec)
-                        for (int k = 0; k < kThermoRec; ++k) a.rec[(size_t)kThermoRec * (size_t)(a.rec0 + a.m) + k] = r[k];
-                    B.ke = r[0]; B.te = r[2]; B.h = r[3]; B.th = r[4]; B.vol = r[5]; B.s1 = r[6]; B.s2 = r[7];
-                    B.s3 = r[8]; B.temp = r[9]; B.boxke = r[10];
-                    therm_box(p, B.b0, B.b1, tg, tgdot, tginv, tgid, vol);
-                    for (int k = 0; k < 9; ++k) { B.tg[k] = tg[k]; B.tgdot[k] = tgdot[k]; B.tginv[k] = tginv[k]; }
-                }
-            }
             continue;
         }
         const int step = (h - 1) >> 1, buf = step & 1, pbuf = buf ^ 1;
@@ -962,8 +933,54 @@ k_run(Params p, Tables t, RunArgs a) {
             return;
     }
     // the box for the launches that follow: every block has read it before the last barrier
-    __syncthreads();
     if (blockIdx.x == 0) box_store(a.box, s.box);
+}
+
+// update_therm_avs of a step, with piece A's grouping of the atoms (the run's
+// blocks, lane 0 of every group of `lanes`); the last block to finish sums the
+// blocks and stores what follows (therm_store).  rec may be null.
+__global__ void __launch_bounds__(kRunThreads)
+k_run_therm(Params p, RunArgs a, int lanes, int32_t *__restrict__ ticket) {
+    __shared__ RunShared s;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    const int g = tid & (lanes - 1), per_block = blockDim.x / lanes, per_round = gridDim.x * per_block;
+    box_load(s.box, a.box);
+    __syncthreads();
+    if (warp == 0) warp_therm_prep(p, s, lane);
+    __syncthreads();
+    double vt[3] = {0.0, 0.0, 0.0};
+    for (int i = blockIdx.x * per_block + tid / lanes; i < p.nm; i += per_round) {
+        if (g != 0 || a.znum[i] == 0) continue;
+        therm_terms(vt, s.box.th_tgid, s.box.b0, s.box.th_cof, a.mass[i], a.x1[i], a.x1[p.nm + i], a.x1[2 * p.nm + i],
+                    a.x2[i], a.x2[p.nm + i], a.x2[2 * p.nm + i]);
+    }
+    warp_columns<3>(s, kA_T, vt);
+    __syncthreads();
+    if (tid < 3) {                                    // end_piece's order
+        double x = s.warp[0][kA_T + tid];
+        for (int q = 1; q < nw; ++q) x = x + s.warp[q][kA_T + tid];
+        column(a, 0, kColT + tid)[blockIdx.x] = x;
+    }
+    if (!last_block(ticket)) return;
+    if (warp != 0) return;
+    double s3[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) s3[k] = reduce_col(a, 0, kColT + k);
+    if (lane != 0) return;
+    BoxState &B = *a.box;
+    double r[kThermoRec], tg[9], tgdot[9], tginv[9], tgid[9], vol;
+    step_record(p, s.box.b0, s.box.b1, s3, s.box.pe, r);
+    if (a.rec)
+        for (int k = 0; k < kThermoRec; ++k) a.rec[(size_t)kThermoRec * (size_t)a.rec0 + k] = r[k];
+    B.ke = r[0]; B.te = r[2]; B.h = r[3]; B.th = r[4]; B.vol = r[5]; B.s1 = r[6]; B.s2 = r[7]; B.s3 = r[8];
+    B.temp = r[9]; B.boxke = r[10];
+    therm_box(p, s.box.b0, s.box.b1, tg, tgdot, tginv, tgid, vol);
+    for (int k = 0; k < 9; ++k) {
+        B.tg[k] = tg[k]; B.tgdot[k] = tgdot[k]; B.tginv[k] = tginv[k];
+        B.tgid[k] = s.box.th_tgid[k];
+        B.th_tgid[k] = s.box.th_tgid[k]; B.th_cof[k] = s.box.th_cof[k];
+    }
+    if (s.box.status) B.status = s.box.status;
 }
 
 using RunKernel = void (*)(Params, Tables, RunArgs);
@@ -1017,13 +1034,10 @@ bool run_applies(const Params &p, const Tables &t, bool mixed) {
 }
 
 size_t run_scratch_bytes() { return 2 * (size_t)kCols * kRunBlocks * sizeof(double) +
-           (size_t)(2 * kRunMaxSteps + 3) * kBarStride * sizeof(unsigned long long); }
+           (size_t)(2 * kRunMaxSteps + 2) * kBarStride * sizeof(unsigned long long); }
 
-int launch_run(DeviceState &d, const Params &p, const Tables &t, bool mixed, double rmid, double rcut, double rout,
-               int m, int h0, int h1, int therm, double *rec, int rec0, int store, cudaStream_t s) {
-    int lanes, threads, blocks;
-    run_shape(p.nm, lanes, threads, blocks);
-    RunArgs a;
+static RunArgs run_args(DeviceState &d, double *rec, int rec0) {
+    RunArgs a = {};
     a.pos = d.pos; a.pos2 = d.pos2; a.posq = d.posq; a.posq2 = d.posq2; a.box = d.box;
     a.nlist = d.nlist; a.numn = d.numn; a.rlist = d.rlist; a.numr = d.numr;
     a.olist = d.olist; a.out_cnt = d.out_cnt; a.mlist = d.mlist; a.mid_cnt = d.mid_cnt;
@@ -1031,7 +1045,16 @@ int launch_run(DeviceState &d, const Params &p, const Tables &t, bool mixed, dou
     a.mass = d.mass; a.del2 = d.del2; a.znum = d.znum; a.x1 = d.x1; a.x2 = d.x2; a.f = d.f;
     a.rho = d.rho; a.afrho = d.afrho; a.dafrho = d.dafrho;
     a.part = d.run_scratch; a.bar = reinterpret_cast<unsigned long long *>(d.run_scratch + 2 * (size_t)kCols * kRunBlocks);
-    a.flags = d.flags; a.rec = rec; a.rec0 = rec0; a.rmid = rmid; a.rcut = rcut; a.rout = rout;
+    a.flags = d.flags; a.rec = rec; a.rec0 = rec0;
+    return a;
+}
+
+int launch_run(DeviceState &d, const Params &p, const Tables &t, bool mixed, double rmid, double rcut, double rout,
+               int m, int h0, int h1, int therm, double *rec, int rec0, int store, cudaStream_t s) {
+    int lanes, threads, blocks;
+    run_shape(p.nm, lanes, threads, blocks);
+    RunArgs a = run_args(d, rec, rec0);
+    a.rmid = rmid; a.rcut = rcut; a.rout = rout;
     a.m = m; a.h0 = h0; a.h1 = h1; a.therm = therm; a.store = store;
     RunKernel k = mixed ? run_kernel<true>(lanes) : run_kernel<false>(lanes);
     const size_t smem = run_smem(t, mixed);
@@ -1043,6 +1066,12 @@ int launch_run(DeviceState &d, const Params &p, const Tables &t, bool mixed, dou
     void *args[] = {&pp, &tt, &a};
     return (int)cudaLaunchCooperativeKernel((const void *)k, dim3((unsigned)blocks), dim3((unsigned)threads), args, smem,
                                             s);
+}
+
+void launch_run_therm(DeviceState &d, const Params &p, double *rec, int k, cudaStream_t s) {
+    int lanes, threads, blocks;
+    run_shape(p.nm, lanes, threads, blocks);
+    k_run_therm<<<blocks, threads, 0, s>>>(p, run_args(d, rec, k), lanes, d.flags + 14);
 }
 
 }  // namespace moldy
