@@ -334,7 +334,10 @@ int upload_device_tables(const HostTables &h, DeviceTables &dt, cudaStream_t s, 
     // step, so it is what every distance beyond it takes; neither has a node
     // that is not finite (V at r = 0), which the whole interval above it takes
     // (inf w + b dr, not inf + (b - inf) dr).
-    auto step = [](double lo, double hi) { return std::isfinite(lo) ? hi - lo : 0.0; };
+    double all = 0.0;                                 // stays zero while every node is finite
+    for (int i = 0; i < nr; ++i) all += 0.0 * h.vee[i] + 0.0 * h.dvee[i] + 0.0 * h.phi[i] + 0.0 * h.dphi[i];
+    const bool finite = all == 0.0;
+    auto step = [finite](double lo, double hi) { return finite || std::isfinite(lo) ? hi - lo : 0.0; };
     for (int i = 0; i < nr; ++i) {
         const int j = i + 1 < nr ? i + 1 : i;
         r4[i] = make_double4(h.vee[i], h.dvee[i], h.phi[i], h.dphi[i]);

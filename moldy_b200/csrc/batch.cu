@@ -702,6 +702,20 @@ k_cl_forces(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__restr
     }
 }
 
+// The rows that the FP64 force pass and the force-matching passes walk: those
+// of the pairs inside the cut that the density pass left, or, where the device
+// had no memory for them, the list rows, whose pairs beyond the cut are left out.
+// ALL in the kernels that walk them: list rows.
+struct Rows {
+    const int32_t *ids, *cnt;
+    int cap;
+    template <bool ALL>
+    __device__ __forceinline__ int length(int hs) const {
+        const int n = cnt[hs];
+        return ALL && n > cap ? cap : n;
+    }
+};
+
 // ------------------------------------------------- FP64 passes over lanes --
 // The FP64 density and force passes with L lanes of a warp per atom (lane g
 // takes the row entries g, g + L, ...), B entries gathered per lane at a time:
@@ -709,7 +723,7 @@ k_cl_forces(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__restr
 // 26 us for 37 systems whatever their size.  NINT is evaluated only for pairs
 // across a face.  The choice of B changes no result.  The density pass writes
 // each atom's pairs inside the cut (14 of the 24 in the list) in row order, and
-// the force pass and the force-matching passes walk those.
+// the force pass and the force-matching passes walk those (Rows).
 //
 // ORD (the quench, whose line searches follow every bit): each pair's terms
 // are those of the one-thread walk, and every lane adds them in row order,
@@ -745,7 +759,9 @@ k_cl_density_l(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__re
                const int32_t *__restrict__ cnt, double *__restrict__ sfp, double *__restrict__ rho_out,
                double *__restrict__ afrho_out, double *__restrict__ fp_out, double *__restrict__ en_calc,
                const int32_t *__restrict__ slot_sys, int32_t *__restrict__ ntodo, int32_t *__restrict__ clist,
-               int32_t *__restrict__ ccnt) {
+               int cstride, int32_t *__restrict__ ccnt) {
+    // without rows of their own (Rows), clist is ccnt and cstride 0: the stores go
+    // to the atom's own count, which no pass then reads
     if (blockIdx.x == 0 && threadIdx.x == 0) *ntodo = 0;   // the tile screen before this pass has read it
     const unsigned gmask = (L == 32 ? 0xffffffffu : ((1u << L) - 1u)) << ((threadIdx.x & 31) / L * L);
     const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
@@ -796,13 +812,13 @@ k_cl_density_l(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__re
                 // the pair joins the atom's row of pairs inside the cut, in row order
                 if (L == 1) {
                     if (hit) {
-                        clist[(size_t)kept++ * ntot + hs] = jj[u];
+                        clist[(size_t)kept++ * cstride + hs] = jj[u];
                         if (kBack) back[held++][threadIdx.x] = r2;
                     }
                     if (kBack) continue;
                 } else {
                     const unsigned m = __ballot_sync(0xffffffffu, hit) & gmask;
-                    if (hit) clist[(size_t)(kept + __popc(m & below)) * ntot + hs] = jj[u];
+                    if (hit) clist[(size_t)(kept + __popc(m & below)) * cstride + hs] = jj[u];
                     kept += __popc(m);
                 }
                 if (hit) {
@@ -851,9 +867,9 @@ k_cl_density_l(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__re
     }
 }
 
-template <bool ORD, int L, int B, bool VIR>
+template <bool ORD, int L, int B, bool VIR, bool ALL>
 __global__ void __launch_bounds__(256, 2)
-k_cl_forces_l(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist, const int32_t *__restrict__ ccnt,
+k_cl_forces_l(TileArgs a, Tables t, int ntot, Rows rows,
               const int32_t *__restrict__ slot_sys, const double *__restrict__ afrho,
               double *__restrict__ fout, double *__restrict__ en_force, double *__restrict__ vir) {
     const int g = threadIdx.x % L, per = gridDim.x * (256 / L);
@@ -869,7 +885,7 @@ k_cl_forces_l(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
         for (int k = 0; k < 9; ++k) b[k] = S.b0[k];
         const double4 ph = ldg4(&a.spos[hs]);
         const double fph = a.sfp[hs];
-        const int n = live ? ccnt[hs] : 0;             // every entry inside the cut
+        const int n = live ? rows.length<ALL>(hs) : 0;
         const int nmax = __reduce_max_sync(0xffffffffu, n);
         double fx = 0.0, fy = 0.0, fz = 0.0, ef = 0.0;
         double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -878,7 +894,7 @@ k_cl_forces_l(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
 #pragma unroll
             for (int u = 0; u < B; ++u) {
                 const int e = e0 + u * L + g;
-                jj[u] = e < n ? clist[(size_t)e * ntot + hs] : hs;
+                jj[u] = e < n ? rows.ids[(size_t)e * ntot + hs] : hs;
             }
             double4 pp[B];
             double fq[B];
@@ -890,7 +906,7 @@ k_cl_forces_l(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
                 frac_diff_near(ph, pp[u], dx, dy, dz);
                 pair_u(b, dx, dy, dz, ux, uy, uz);
                 const double r2 = ux * ux + uy * uy + uz * uz;
-                if (e0 + u * L + g < n) {
+                if (e0 + u * L + g < n && (!ALL || r2 < a.rc2)) {
                     if (ORD) {
                         const double r = sqrt(r2);
                         const double4 q = lookup_r4(t, r);     // V, V', phi, phi'
@@ -1377,14 +1393,14 @@ __device__ __forceinline__ void fm_flush(const double *h, double *g, int nb) {
 // The pair of slot hs and row entry j (inside the cut): u = B0 d, r, 1/r, the
 // table interval q and the weight w1 of its upper node.
 __device__ __forceinline__ double fm_pair(const Tables &t, const double *b, const double4 &ph, const double4 &pj,
-                                          double &ux, double &uy, double &uz, double &rr, int &q, double &w1) {
+                                          double &ux, double &uy, double &uz, double &rr, int &q, double &w1) {   // r^2
     double dx, dy, dz;
     frac_diff_near(ph, pj, dx, dy, dz);
     pair_u(b, dx, dy, dz, ux, uy, uz);
-    const double r = root_and_inverse(ux * ux + uy * uy + uz * uz, rr);
+    const double r2 = ux * ux + uy * uy + uz * uz, r = root_and_inverse(r2, rr);
     q = interval_d(t, r, w1);
     if (q > t.nr - 2) { q = t.nr - 2; w1 = 1.0; }
-    return r;
+    return r2;
 }
 
 constexpr int kFmGather = 2;      // row entries gathered before any is used
@@ -1394,9 +1410,9 @@ constexpr int kFmGather = 2;      // row entries gathered before any is used
 // are gathered at a time, and a neighbour is two 32-byte loads (position and
 // mass; dL/dF and F') and its interval one (256 systems of 1024 atoms: 225 us
 // with five 8-byte gathers and two nodes per listed entry).
+template <bool ALL>
 __global__ void __launch_bounds__(256, 2)
-k_fm_pairs_a(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
-             const int32_t *__restrict__ ccnt, const int32_t *__restrict__ slot_sys, const double4 *__restrict__ gF,
+k_fm_pairs_a(TileArgs a, Tables t, int ntot, Rows rows, const int32_t *__restrict__ slot_sys, const double4 *__restrict__ gF,
              const double *__restrict__ gS, double *__restrict__ mu, double *__restrict__ g_dvee,
              double *__restrict__ g_dphi, int nbr) {
     extern __shared__ double sh[];
@@ -1409,13 +1425,13 @@ k_fm_pairs_a(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
         const double4 ph = ldg4(&a.spos[hs]), gh = ldg4(&gF[hs]);
         const double *G = gS + 9 * (size_t)s;
         const double ivol = 1.0 / S.vol;
-        const int n = ccnt[hs];
+        const int n = rows.length<ALL>(hs);
         double m = 0.0;
         for (int e0 = 0; e0 < n; e0 += kFmGather) {
             int jj[kFmGather];
             double4 pp[kFmGather], gg[kFmGather];
 #pragma unroll
-            for (int u = 0; u < kFmGather; ++u) jj[u] = e0 + u < n ? clist[(size_t)(e0 + u) * ntot + hs] : hs;
+            for (int u = 0; u < kFmGather; ++u) jj[u] = e0 + u < n ? rows.ids[(size_t)(e0 + u) * ntot + hs] : hs;
 #pragma unroll
             for (int u = 0; u < kFmGather; ++u) { pp[u] = ldg4(&a.spos[jj[u]]); gg[u] = ldg4(&gF[jj[u]]); }
 #pragma unroll
@@ -1423,7 +1439,8 @@ k_fm_pairs_a(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
                 if (e0 + u >= n) continue;
                 double ux, uy, uz, rr, w1;
                 int q;
-                fm_pair(t, S.b0, ph, pp[u], ux, uy, uz, rr, q, w1);
+                const double r2 = fm_pair(t, S.b0, ph, pp[u], ux, uy, uz, rr, q, w1);
+                if (ALL && !(r2 < a.rc2)) continue;
                 const double4 w = ldg4(&t.df4[q]);
                 const double dp = fma(w.w, w1, w.y);
                 double lam = (gh.x - gg[u].x) * ux + (gh.y - gg[u].y) * uy + (gh.z - gg[u].z) * uz;
@@ -1488,9 +1505,9 @@ k_fm_atoms(Tables t, int ntot, const int32_t *__restrict__ sorted, const double 
 }
 
 // dL/d phi = nu_i + nu_j per pair
+template <bool ALL>
 __global__ void __launch_bounds__(256, 3)
-k_fm_pairs_c(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
-             const int32_t *__restrict__ ccnt, const int32_t *__restrict__ slot_sys, const double *__restrict__ nu,
+k_fm_pairs_c(TileArgs a, Tables t, int ntot, Rows rows, const int32_t *__restrict__ slot_sys, const double *__restrict__ nu,
              double *__restrict__ g_phi, int nbr) {
     extern __shared__ double sh[];
     for (int k = threadIdx.x; k < nbr; k += blockDim.x) sh[k] = 0.0;
@@ -1499,13 +1516,13 @@ k_fm_pairs_c(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
         const BSys &S = a.sys[slot_sys[hs]];
         const double4 ph = ldg4(&a.spos[hs]);
         const double nui = nu[hs];
-        const int n = ccnt[hs];
+        const int n = rows.length<ALL>(hs);
         for (int e0 = 0; e0 < n; e0 += kFmGather) {
             int jj[kFmGather];
             double4 pp[kFmGather];
             double nj[kFmGather];
 #pragma unroll
-            for (int u = 0; u < kFmGather; ++u) jj[u] = e0 + u < n ? clist[(size_t)(e0 + u) * ntot + hs] : hs;
+            for (int u = 0; u < kFmGather; ++u) jj[u] = e0 + u < n ? rows.ids[(size_t)(e0 + u) * ntot + hs] : hs;
 #pragma unroll
             for (int u = 0; u < kFmGather; ++u) {        // each pair once, from its lower slot
                 const int j = hs < jj[u] ? jj[u] : hs;
@@ -1517,7 +1534,8 @@ k_fm_pairs_c(TileArgs a, Tables t, int ntot, const int32_t *__restrict__ clist,
                 if (!(hs < jj[u])) continue;             // also the entries past the end (hs itself)
                 double ux, uy, uz, rr, w1;
                 int q;
-                fm_pair(t, S.b0, ph, pp[u], ux, uy, uz, rr, q, w1);
+                const double r2 = fm_pair(t, S.b0, ph, pp[u], ux, uy, uz, rr, q, w1);
+                if (ALL && !(r2 < a.rc2)) continue;
                 fm_hist(sh, q, nui + nj[u], w1);
             }
         }
@@ -1902,7 +1920,15 @@ class BatchEngine {
     double *en_calc = nullptr, *en_force = nullptr, *vir = nullptr, *sfp = nullptr, *sysout = nullptr;
     double *cgv = nullptr;              // G, D, GS, XX, GG, DR, DGR (3*ntot each)
     int32_t *alist = nullptr, *pcnt = nullptr, *flags = nullptr;
-    int32_t *clist = nullptr, *ccnt = nullptr;   // rows of the pairs inside the cut (FP64 passes)
+    // rows of the pairs inside the cut, written by every FP64 or persistent
+    // evaluation for itself (slots; in the persistent one indices within the
+    // system).  The last buffer to be made and the first to be given back: every
+    // evaluation can do without them
+    int32_t *clist = nullptr, *ccnt = nullptr;
+    bool rows_refused = false;          // the device had no memory for them
+    bool inside_rows();
+    template <typename T> int alloc(T **p, size_t n, const char *what);
+    Rows rows() const { return clist ? Rows{clist, ccnt, pair_cap} : Rows{alist, pcnt, pair_cap}; }
     unsigned long long *stats = nullptr;   // system list builds, system evaluations
     int32_t *todo = nullptr, *ntodo = nullptr;   // cells of the systems rebuilt in this evaluation
     bool quench_open = false;           // a quench that did not end may have left work in todo
@@ -2009,6 +2035,23 @@ static int balloc(T **p, size_t n, const char *what) {
     return MOLDY_OK;
 }
 
+// A buffer asked for after the batch was made: the rows of the pairs inside the
+// cut make room for it
+template <typename T>
+int BatchEngine::alloc(T **p, size_t n, const char *what) {
+    int rc = balloc(p, n, what);
+    if (rc != MOLDY_OK && clist) {
+        cudaStreamSynchronize(stream);
+        cudaFree(clist);
+        clist = nullptr;
+        rows_refused = true;
+        if (graph) { cudaGraphExecDestroy(graph); graph = nullptr; }
+        drop_force_graph();
+        rc = balloc(p, n, what);
+    }
+    return rc;
+}
+
 BatchEngine::~BatchEngine() {
     cudaSetDevice(device);
     if (graph) cudaGraphExecDestroy(graph);
@@ -2076,7 +2119,6 @@ int BatchEngine::init(int n, const int32_t *na, double p, int dev) {
     BCHECK(balloc(&stage, 3 * nt, "staging"));
     BCHECK(balloc(&alist, nt * (size_t)pair_cap, "compact list"));
     BCHECK(balloc(&pcnt, nt, "compact counts"));
-    BCHECK(balloc(&clist, nt * (size_t)pair_cap, "rows inside the cut"));
     BCHECK(balloc(&ccnt, nt, "counts inside the cut"));
     BCHECK(balloc(&flags, 2, "flags"));
     BCUDA(cudaMemset(flags, 0, 2 * sizeof(int32_t)), "flags");
@@ -2102,6 +2144,7 @@ int BatchEngine::init(int n, const int32_t *na, double p, int dev) {
     std::vector<double> m(nt, 55.845);
     BCUDA(cudaMemcpy(mass, m.data(), nt * sizeof(double), cudaMemcpyHostToDevice), "mass");
     hsys.assign(n, BSys());
+    (void)inside_rows();
     return MOLDY_OK;
 }
 
@@ -2243,11 +2286,11 @@ int BatchEngine::layout() {
         cell_sys = cell_count = cell_start = cursor = todo = nullptr;
         list_cut = 0.0;
         ncell = cell;
-        BCHECK(balloc(&todo, ncell, "screen work"));
-        BCHECK(balloc(&cell_sys, ncell, "cell_sys"));
-        BCHECK(balloc(&cell_count, ncell, "cell_count"));
-        BCHECK(balloc(&cell_start, ncell + 1, "cell_start"));
-        BCHECK(balloc(&cursor, ncell, "cursor"));
+        BCHECK(alloc(&todo, ncell, "screen work"));
+        BCHECK(alloc(&cell_sys, ncell, "cell_sys"));
+        BCHECK(alloc(&cell_count, ncell, "cell_count"));
+        BCHECK(alloc(&cell_start, ncell + 1, "cell_start"));
+        BCHECK(alloc(&cursor, ncell, "cursor"));
         if (graph) { cudaGraphExecDestroy(graph); graph = nullptr; }
         drop_force_graph();
     }
@@ -2329,10 +2372,11 @@ static void launch_passes_fp64(const BatchEngine &E, const TileArgs &a, bool wit
     auto den = with_vir ? (ecalc ? k_cl_density_l<false, L, B, true> : k_cl_density_l<false, L, B, false>)
                         : (ecalc ? k_cl_density_l<true, L, B, true> : k_cl_density_l<true, L, B, false>);
     den<<<nbs, 256, 0, s>>>(a, E.tab, E.ntot, E.pair_cap, E.alist, E.pcnt, E.sfp, E.rho, E.afrho, E.fp, E.en_calc,
-                            E.atom_sys, E.ntodo, E.clist, E.ccnt);
+                            E.atom_sys, E.ntodo, E.clist ? E.clist : E.ccnt, E.clist ? E.ntot : 0, E.ccnt);
     if (ev) cudaEventRecord(ev[3], s);
-    auto frc = with_vir ? k_cl_forces_l<false, LF, B, true> : k_cl_forces_l<true, LF, B, false>;
-    frc<<<nbf, 256, 0, s>>>(a, E.tab, E.ntot, E.clist, E.ccnt, E.atom_sys, E.afrho, E.f, E.en_force, E.vir);
+    auto frc = E.clist ? (with_vir ? k_cl_forces_l<false, LF, B, true, false> : k_cl_forces_l<true, LF, B, false, false>)
+                       : (with_vir ? k_cl_forces_l<false, LF, B, true, true> : k_cl_forces_l<true, LF, B, false, true>);
+    frc<<<nbf, 256, 0, s>>>(a, E.tab, E.ntot, E.rows(), E.atom_sys, E.afrho, E.f, E.en_force, E.vir);
 }
 
 template <int B>
@@ -2391,14 +2435,30 @@ int BatchEngine::take_overflow() {
     alist = nullptr;
     if (clist) cudaFree(clist);
     clist = nullptr;
+    rows_refused = false;               // asked for again by the next evaluation
     if (balloc(&alist, (size_t)ntot * (size_t)need, "compact list") != MOLDY_OK) return -1;
-    if (balloc(&clist, (size_t)ntot * (size_t)need, "rows inside the cut") != MOLDY_OK) return -1;
     pair_cap = need;
     if (graph) { cudaGraphExecDestroy(graph); graph = nullptr; }
     drop_force_graph();
     k_set_active<<<(nsys + 255) / 256, 256, 0, stream>>>(nsys, sys, 1, 1);
     if (cudaStreamSynchronize(stream) != cudaSuccess) return -1;
     return h[1];
+}
+
+// The rows of the pairs inside the cut, as long as the list rows (192 bytes an
+// atom of 808): the evaluations that write them do without where the device
+// has no memory for them, the FP64 passes by walking the list rows, the
+// persistent launch by leaving the batch to the per-pass form.  False in that
+// case.
+bool BatchEngine::inside_rows() {
+    if (clist || rows_refused) return clist != nullptr;
+    if (balloc(&clist, (size_t)ntot * (size_t)pair_cap, "rows inside the cut") != MOLDY_OK) {
+        clist = nullptr;
+        rows_refused = true;
+    }
+    if (graph) { cudaGraphExecDestroy(graph); graph = nullptr; }
+    drop_force_graph();
+    return clist != nullptr;
 }
 
 // The launches of one force evaluation of every system: the persistent
@@ -2411,7 +2471,8 @@ int BatchEngine::evaluate_once(bool with_reduce) {
         en_calc_zero = true;
     }
     if (ecalc) en_calc_zero = false;
-    if (persistent_applies()) {
+    const bool in_rows = (!mixed || persistent_applies()) && inside_rows();
+    if (in_rows && persistent_applies()) {
         if (!fgraph || fg_lph != lph || fg_lpa != lpa || fg_cap != cap) {
             drop_force_graph();
             BCHECK(eval_prepare());
@@ -2496,7 +2557,7 @@ int BatchEngine::queue_persistent(bool prepare) {
 // ms2[1] with every list rebuilt (binning and compact rows in the same launch)
 int BatchEngine::eval_times(double *ms2) {
     BCHECK(ready());
-    if (!persistent_applies())
+    if (!persistent_applies() || !inside_rows())
         return set_last_error(MOLDY_ERR_UNSUPPORTED, "the persistent evaluation does not apply (FP64, energy_calc, "
                                                      "an atom of mass <= 0.05, or a system too large)");
     cudaEvent_t e0, e1;
@@ -2579,6 +2640,7 @@ int BatchEngine::autotune(int nreps, double *times_ms, int32_t *chosen) {
     evaluate(true);   // rows sized before timing
     BCUDA(cudaStreamSynchronize(stream), "autotune");
     if (take_overflow() < 0) return set_last_error(MOLDY_ERR_CUDA, "compact list re-allocation failed");
+    if (!mixed) inside_rows();
     int bl = 0;
     for (int k = 0; k < 4; ++k) {
         lph = lanes[k];
@@ -2596,7 +2658,7 @@ int BatchEngine::autotune(int nreps, double *times_ms, int32_t *chosen) {
     gather = gathers[bg];
     // lanes per atom of the persistent evaluation (lists current)
     double tp[3] = {0.0, 0.0, 0.0};
-    const bool pers = persistent_applies();
+    const bool pers = persistent_applies() && inside_rows();
     if (pers) {
         const int lanes_a[3] = {1, 2, 4};
         int bp = 0;
@@ -2643,13 +2705,13 @@ int BatchEngine::set_references(const double *fref_xyz, const double *sref) {
     if (!fref_xyz || !sref) return set_last_error(MOLDY_ERR_INVALID, "null reference array");
     const size_t nt = (size_t)ntot;
     if (!fm_fref) {
-        BCHECK(balloc(&fm_fref, 3 * nt, "reference forces"));
-        BCHECK(balloc(&fm_sref, 9 * (size_t)nsys, "reference stresses"));
-        BCHECK(balloc(&fm_gF, nt, "dL/dF"));
-        BCHECK(balloc(&fm_gS, 9 * (size_t)nsys, "dL/dsigma"));
-        BCHECK(balloc(&fm_loss, nsys, "loss"));
-        BCHECK(balloc(&fm_mu, nt, "mu"));
-        BCHECK(balloc(&fm_nu, nt, "nu"));
+        BCHECK(alloc(&fm_fref, 3 * nt, "reference forces"));
+        BCHECK(alloc(&fm_sref, 9 * (size_t)nsys, "reference stresses"));
+        BCHECK(alloc(&fm_gF, nt, "dL/dF"));
+        BCHECK(alloc(&fm_gS, 9 * (size_t)nsys, "dL/dsigma"));
+        BCHECK(alloc(&fm_loss, nsys, "loss"));
+        BCHECK(alloc(&fm_mu, nt, "mu"));
+        BCHECK(alloc(&fm_nu, nt, "nu"));
     }
     BCUDA(cudaMemcpyAsync(fm_fref, fref_xyz, 3 * nt * sizeof(double), cudaMemcpyHostToDevice, stream), "references");
     BCUDA(cudaMemcpyAsync(fm_sref, sref, 9 * (size_t)nsys * sizeof(double), cudaMemcpyHostToDevice, stream),
@@ -2670,11 +2732,12 @@ int BatchEngine::force_matching(double wf, double ws, double *loss, double *grad
     if (fm_nb != nb) {
         if (fm_grads) cudaFree(fm_grads);
         fm_grads = nullptr;
-        BCHECK(balloc(&fm_grads, 6 * (size_t)nb, "table gradients"));
+        BCHECK(alloc(&fm_grads, 6 * (size_t)nb, "table gradients"));
         fm_nb = nb;
     }
     // the forward in FP64, energy_calc not needed
     for (int attempt = 0;; ++attempt) {
+        inside_rows();
         k_set_active<<<(nsys + 255) / 256, 256, 0, stream>>>(nsys, sys, 1, 0);
         queue_evaluation(true, false, false);
         k_sys_reduce<<<nsys, kCgThreads, 0, stream>>>(sys, en_calc, en_force, vir, f, 1, sysout);
@@ -2692,19 +2755,21 @@ int BatchEngine::force_matching(double wf, double ws, double *loss, double *grad
     a.sys = sys; a.cell_sys = cell_sys; a.cell_start = cell_start; a.sorted = sorted;
     a.spos = spos; a.sfp = sfp; a.ncell = ncell; a.cap = cap; a.rc2 = rcut * rcut;
     const size_t smem_r = 2 * (size_t)nbr * sizeof(double), smem_e = (size_t)nb * sizeof(double);
-    BCUDA(cudaFuncSetAttribute(k_fm_pairs_a, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_r), "smem");
+    auto pairs_a = clist ? k_fm_pairs_a<false> : k_fm_pairs_a<true>;
+    auto pairs_c = clist ? k_fm_pairs_c<false> : k_fm_pairs_c<true>;
+    BCUDA(cudaFuncSetAttribute(pairs_a, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_r), "smem");
     BCUDA(cudaFuncSetAttribute(k_fm_atoms, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_e), "smem");
-    BCUDA(cudaFuncSetAttribute(k_fm_pairs_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem_r / 2)),
+    BCUDA(cudaFuncSetAttribute(pairs_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem_r / 2)),
           "smem");
     // histogram kernels: two blocks per SM, so each flush serves many atoms
     const int g = std::min(grid_blocks(ntot, 256), 2 * nsm);
     // vee and emb get no gradient: the loss holds no energy
     double *gdv = fm_grads + nb, *gp = fm_grads + 2 * nb, *gdp = fm_grads + 3 * nb, *gde = fm_grads + 5 * nb;
-    k_fm_pairs_a<<<g, 256, smem_r, s>>>(a, tab, ntot, clist, ccnt, atom_sys, fm_gF, fm_gS, fm_mu, gdv, gdp,
+    pairs_a<<<g, 256, smem_r, s>>>(a, tab, ntot, rows(), atom_sys, fm_gF, fm_gS, fm_mu, gdv, gdp,
                                        nbr);
     k_fm_atoms<<<g, 256, smem_e, s>>>(tab, ntot, sorted, rho, fm_mu, fm_nu, gde);
     const int gc = std::min(grid_blocks(ntot, 256), 3 * nsm);   // half the shared memory
-    k_fm_pairs_c<<<gc, 256, smem_r / 2, s>>>(a, tab, ntot, clist, ccnt, atom_sys, fm_nu, gp, nbr);
+    pairs_c<<<gc, 256, smem_r / 2, s>>>(a, tab, ntot, rows(), atom_sys, fm_nu, gp, nbr);
     launches += 4;
     BCUDA(cudaGetLastError(), "force matching launch");
     if (loss) BCUDA(cudaMemcpyAsync(loss, fm_loss, (size_t)nsys * sizeof(double), cudaMemcpyDeviceToHost, s), "loss");
@@ -2720,6 +2785,7 @@ int BatchEngine::force_matching(double wf, double ws, double *loss, double *grad
 // list first.  The per-system reduction is not included.
 int BatchEngine::kernel_times(int rebuild, double *ms4) {
     BCHECK(ready());
+    if (!mixed) inside_rows();
     cudaEvent_t ev[5];
     for (auto &e : ev) BCUDA(cudaEventCreate(&e), "event");
     k_set_active<<<(nsys + 255) / 256, 256, 0, stream>>>(nsys, sys, 1, rebuild ? 1 : 0);
@@ -2769,6 +2835,7 @@ int BatchEngine::copy_xyz(double *dev, const double *src, double *dst) {
 
 int BatchEngine::quench(int maxfn, int criterion, double fmax, double *out8) {
     BCHECK(ready());
+    inside_rows();
     if (maxfn < 1) return set_last_error(MOLDY_ERR_INVALID, "maxfn < 1");
     cudaStream_t s = stream;
     size_t nt3 = 3 * (size_t)ntot;
