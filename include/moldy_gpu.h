@@ -234,6 +234,10 @@ int moldy_gpu_set_outer_skin(moldy_gpu *h, double skin);
 int moldy_gpu_get_outer_builds(moldy_gpu *h, int32_t *builds);
 int moldy_gpu_autotune(moldy_gpu *h, int32_t nreps, double *times_ms, int32_t *chosen);
 int moldy_gpu_set_variants(moldy_gpu *h, int32_t screen, int32_t density, int32_t forces);
+/* How long a grid barrier of a run of steps waits for the other blocks before
+ * the call ends with MOLDY_ERR_CUDA (default 2^20 polls, about half a second,
+ * and 10 s from then on; at most 60).  The state is lost then: set it anew. */
+int moldy_gpu_set_run_wait(moldy_gpu *h, int64_t polls, double seconds);
 /* out3[0]: directed interacting pairs (inside the table range) of the last
  * force evaluation, twice the contributing half-list pairs; out3[1]: how many
  * times the intermediate list (half-list pairs within the table cut + skin)

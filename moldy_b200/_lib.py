@@ -99,6 +99,7 @@ SIGNATURES = {
     "moldy_gpu_kernel_stats": [H, ctypes.c_int32, D, ctypes.POINTER(ctypes.c_int64)],
     "moldy_gpu_kernel_name": [ctypes.c_int32],
     "moldy_gpu_autotune": [H, ctypes.c_int32, D, I],
+    "moldy_gpu_set_run_wait": [H, ctypes.c_int64, ctypes.c_double],
     "moldy_gpu_set_variants": [H, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32],
     "moldy_gpu_get_list_stats": [H, D],
     "moldy_gpu_set_iron_carbon_fe": [H, ctypes.c_int32],

@@ -596,6 +596,12 @@ int Engine::check_flags() {
     CUDA_CHECK(cudaMemcpyAsync(&st, &d.box->status, sizeof(st), cudaMemcpyDeviceToHost, stream_), "flags");
     CUDA_CHECK(cudaStreamSynchronize(stream_), "synchronize");
     prof.harvest();
+    if (f[13]) {
+        cudaMemsetAsync(d.flags, 0, sizeof(f), stream_);
+        list_ready_ = false;                  // rows may be of different steps
+        mid_dirty_ = true;
+        return fail(MOLDY_ERR_CUDA, "a grid barrier of a fused run of steps gave up waiting; the state is not usable");
+    }
     if (f[7]) {
         cudaMemsetAsync(d.flags, 0, sizeof(f), stream_);
         cells_ready_ = list_ready_ = false;   // such atoms lie in cells that are not theirs
@@ -612,10 +618,6 @@ int Engine::check_flags() {
     if (f[1]) {
         cudaMemsetAsync(d.flags, 0, sizeof(f), stream_);
         return fail(MOLDY_ERR_CAPACITY, "link-cell relink produced inconsistent cell counts");
-    }
-    if (f[13]) {
-        cudaMemsetAsync(d.flags, 0, sizeof(f), stream_);
-        return fail(MOLDY_ERR_CUDA, "a grid barrier of a fused run of steps gave up waiting; the state is not usable");
     }
     if (f[10]) {
         cudaMemsetAsync(d.flags, 0, sizeof(f), stream_);
@@ -893,7 +895,7 @@ int Engine::queue_run(int m, bool therm, double *rec, int rec0, bool last, bool 
     auto pieces = [&](int id, int h0, int h1) {
         LAUNCH(*this, id, 1, s,
                if (!rc) rc = launch_run(d, prm, tab, mixed, rmid, rcut, rout, m, h0, h1, therm ? 1 : 0, rec, rec0,
-                                        last ? 1 : 0, s));
+                                        last ? 1 : 0, run_wait_, s));
     };
     if (prof.on) {
         pieces(K_DRIFT, 0, 0);
@@ -916,6 +918,11 @@ int Engine::queue_run(int m, bool therm, double *rec, int rec0, bool last, bool 
 // update_therm_avs with the runs' sums; k: the index of the step's record
 void Engine::queue_run_therm(double *rec, int k) {
     LAUNCH(*this, K_THERM, 1, stream_, launch_run_therm(d, prm, rec, k, stream_));
+}
+
+void Engine::set_run_wait(unsigned polls, double seconds) {
+    run_wait_.polls = polls;
+    run_wait_.ns = (unsigned long long)(seconds * 1e9);
 }
 
 // Host-side state of m steps of a run; whether scalev ends the last one
@@ -1592,6 +1599,14 @@ int moldy_gpu_set_variants(moldy_gpu *h, int32_t screen, int32_t density, int32_
     h->e->variant[moldy::K_SCREEN] = screen;
     h->e->variant[moldy::K_DENSITY] = density;
     h->e->variant[moldy::K_PAIR] = forces;
+    return MOLDY_OK;
+}
+
+int moldy_gpu_set_run_wait(moldy_gpu *h, int64_t polls, double seconds) {
+    GUARD(h);
+    if (polls < 0 || polls > 0x7fffffff || !(seconds >= 0.0 && seconds <= 60.0))
+        return fail(MOLDY_ERR_INVALID, "polls or seconds out of range");
+    h->e->set_run_wait((unsigned)polls, seconds);
     return MOLDY_OK;
 }
 

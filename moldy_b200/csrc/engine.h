@@ -156,6 +156,13 @@ struct Profiler {
     ~Profiler();
 };
 
+// How long a grid barrier of a run waits: so many polls (a poll takes some
+// 0.5 us), then so many nanoseconds more.
+struct RunWait {
+    unsigned polls = 1u << 20;
+    unsigned long long ns = 10000000000ull;
+};
+
 class Engine {
   public:
     explicit Engine(const moldy_params &p);
@@ -230,6 +237,8 @@ class Engine {
     CopyStage stage;
     int open_stage();
 
+    void set_run_wait(unsigned polls, double seconds);
+
   private:
     int check_ready();
     int upload_tables();
@@ -237,6 +246,7 @@ class Engine {
     int fetch_force_out(moldy_force_out *out);
     int check_flags();
     void finish_step(bool scalev, bool last, double *rec);
+    RunWait run_wait_;
     int run_length(int left) const;
     bool runs_apply() const;
     int queue_run(int m, bool therm, double *rec, int rec0, bool last, bool tail);
@@ -359,7 +369,7 @@ void launch_mid_decide(DeviceState &d, const Params &p, double rmid, double rcut
 bool run_applies(const Params &p, const Tables &t, bool mixed);
 size_t run_scratch_bytes();
 int launch_run(DeviceState &d, const Params &p, const Tables &t, bool mixed, double rmid, double rcut, double rout,
-               int m, int h0, int h1, int therm, double *rec, int rec0, int store, cudaStream_t s);
+               int m, int h0, int h1, int therm, double *rec, int rec0, int store, RunWait wait, cudaStream_t s);
 // update_therm_avs with the sums of a run, of the step whose record has index k
 void launch_run_therm(DeviceState &d, const Params &p, double *rec, int k, cudaStream_t s);
 void launch_set_rec_step(DeviceState &d, int step, cudaStream_t s);

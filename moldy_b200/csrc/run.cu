@@ -53,7 +53,6 @@ constexpr int kRunEmb = 256;                  // emb nodes kept in shared memory
 // columns of a block's partial sums
 constexpr int kColF = 0, kColK = 7, kColE = 13, kColMax = 15, kColOut = 16, kColHalf = 17, kColT = 18, kCols = 21;
 constexpr int kBarStride = 4;                 // 32 bytes between barrier words
-constexpr unsigned kSpinLimit = 1u << 21;     // polls before a barrier gives up (about a second)
 
 struct RunArgs {
     double4 *pos, *pos2;
@@ -76,6 +75,7 @@ struct RunArgs {
     int h0, h1;                               // pieces of this launch (0: first drift, 2s+1: A, 2s+2: B, 2m+1: box)
     int therm;                                // the step before the run awaits its update_therm_avs
     int store;                                // 1: the run's last step also stores rho and the forces
+    RunWait wait;                             // how long a barrier waits for the other blocks
 };
 
 // What the threads of a block share beside the tables
@@ -93,6 +93,12 @@ struct RunShared {
 __device__ __forceinline__ unsigned long long load_relaxed(const unsigned long long *p) {
     unsigned long long v;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long v;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(v));
     return v;
 }
 
@@ -135,8 +141,11 @@ constexpr int kA_E = 0, kA_T = 2, kA_Out = 5, kA_Half = 6, kB_F = 0, kB_K = 7, k
 // block polls both with one load.  No atomic returns a value, so the first
 // poll leaves right after the arrival.  (A word per block polled by every
 // block was slower: 143 x 143 polls of ten lines, 15.5 against 13.3 us per
-// step at 2,000 atoms.)  False when the others did not arrive within the limit
-// (flag 13 is then set and the kernel ends).
+// step at 2,000 atoms.)  A cooperative launch's blocks are all resident, so the
+// others arrive within microseconds unless the device stands still; a barrier
+// gives up after that many polls and, from then on, that much time (a device
+// that is only slow, or stopped by a debugger, is waited for).  False in that
+// case: flag 13 is set and the kernel ends.
 __device__ __forceinline__ bool end_piece(const RunArgs &a, RunShared &s, unsigned &epoch, unsigned mask, bool piece_a,
                                           int buf) {
     __syncthreads();
@@ -167,13 +176,21 @@ __device__ __forceinline__ bool end_piece(const RunArgs &a, RunShared &s, unsign
             }
             red_add_release(w + 1, 1u);
             unsigned long long v = load_relaxed(a.bar + (size_t)(epoch - 1) * kBarStride);
-            for (unsigned it = 0; (unsigned)(v >> 32) != gridDim.x;
-                 v = load_relaxed(a.bar + (size_t)(epoch - 1) * kBarStride))
-                if (++it > kSpinLimit) {
+            unsigned it = 0;
+            for (unsigned long long t0 = 0ull; (unsigned)(v >> 32) != gridDim.x;
+                 v = load_relaxed(a.bar + (size_t)(epoch - 1) * kBarStride)) {
+                if (it < a.wait.polls) {
+                    ++it;
+                    continue;
+                }
+                const unsigned long long now = global_ns();
+                if (t0 == 0ull) t0 = now;
+                if (now - t0 >= a.wait.ns) {
                     s.fail = 1;
                     atomicExch(&a.flags[13], 1);
                     break;
                 }
+            }
             __threadfence();
             s.disp2 = __uint_as_float((unsigned)v);
         }
@@ -528,8 +545,9 @@ k_run(Params p, Tables t, RunArgs a) {
     }
     for (int k = tid; k < ne_emb; k += blockDim.x) se[k] = __ldg(&t.e2[k]);
     box_load(s.box, a.box);
-    if (tid == 0) s.fail = 0;
+    if (tid == 0) s.fail = a.flags[13];       // an earlier run of the call gave up: so does this one
     __syncthreads();
+    if (s.fail) return;
 
     unsigned epoch = 0;
     for (int h = a.h0; h <= a.h1; ++h) {
@@ -1050,10 +1068,11 @@ static RunArgs run_args(DeviceState &d, double *rec, int rec0) {
 }
 
 int launch_run(DeviceState &d, const Params &p, const Tables &t, bool mixed, double rmid, double rcut, double rout,
-               int m, int h0, int h1, int therm, double *rec, int rec0, int store, cudaStream_t s) {
+               int m, int h0, int h1, int therm, double *rec, int rec0, int store, RunWait wait, cudaStream_t s) {
     int lanes, threads, blocks;
     run_shape(p.nm, lanes, threads, blocks);
     RunArgs a = run_args(d, rec, rec0);
+    a.wait = wait;
     a.rmid = rmid; a.rcut = rcut; a.rout = rout;
     a.m = m; a.h0 = h0; a.h1 = h1; a.therm = therm; a.store = store;
     RunKernel k = mixed ? run_kernel<true>(lanes) : run_kernel<false>(lanes);

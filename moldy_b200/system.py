@@ -407,6 +407,10 @@ class MoldySystem:
         check(self._L.moldy_gpu_get_outer_builds(self._h, ctypes.byref(n)))
         return int(n.value)
 
+    def set_run_wait(self, polls: int = 1 << 20, seconds: float = 10.0):
+        """How long a grid barrier of a run of steps waits before the call fails."""
+        check(self._L.moldy_gpu_set_run_wait(self._h, int(polls), float(seconds)))
+
     def set_variants(self, screen: int, density: int, forces: int):
         check(self._L.moldy_gpu_set_variants(self._h, int(screen), int(density), int(forces)))
 
