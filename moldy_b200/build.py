@@ -15,7 +15,7 @@ OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libmoldy_gpu.so")
 SOURCES = ["api.cu", "cells.cu", "nlist.cu", "eam.cu", "pairs.cu", "run.cu", "noalloc.cu", "adjoint.cu", "batch.cu", "rdf.cu", "copystage.cpp",
            "tables.cpp"]
-HEADERS = ["common.cuh", "engine.h", "box.cuh", "pairs.cuh", "copystage.h"]
+HEADERS = ["common.cuh", "engine.h", "box.cuh", "pairs.cuh", "copystage.h", "rules.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -36,14 +36,17 @@
 // and every other sum in FP64: each pair's FP32 terms are converted once and
 // accumulated in FP64.
 //
-// These two kernels run the exact functions in FP64 and mixed precision below
-// kStAtoms atoms; k_screen_d / k_forces_d (FP64 tables) and k_screen_st /
-// k_forces_st (mixed precision, large systems, tables in shared memory) are the
-// same passes without branches in their inner loops.
+// These two kernels run the exact functions in FP64, and mixed precision where
+// the tables stay outside shared memory (rules.h: small systems, the force pass
+// up to medium ones, long tables) or with per-atom stresses; k_screen_d /
+// k_forces_d (FP64 tables) and k_screen_st / k_forces_st (mixed precision, large
+// systems, tables in shared memory) are the same passes without branches in
+// their inner loops.
 #include <type_traits>
 
 #include "engine.h"
 #include "pairs.cuh"
+#include "rules.h"
 
 namespace moldy {
 
@@ -1162,26 +1165,9 @@ void launch_mid_build(DeviceState &d, const Params &p, double rmid, double rout,
 // L2 prefetches of the next atom's rows and per-atom data; bit 2 asks for 768
 // resident threads per SM instead of 512 (variants 0 and 1: 1024), fewer
 // registers each and more warps to hide the gather latency.
-//
-// The mixed passes of at least kStAtoms atoms in lookup mode keep their tables
-// in shared memory (ST: one block per SM); smaller systems, whose atoms would
-// fill few such blocks, tables above kStNodes nodes and the FP64 passes read
-// them through L1 with blocks of 256.  One block per SM fills late: NPT steps
-// of L1 forms / screening in shared memory / both (us): 101,306 atoms 59.1 /
-// 59.0 / 59.0, 250,000 100 / 96 / 101, 524,288 169 / 160 / 166, 810,448 - / 225 /
-// 230, 913,066 - / 242 / 239, 1,024,000 276 / 260 / 254, 2,000,000 499 / 459 /
-// 444.
-constexpr int kStAtoms = 100000;         // screening-density pass
-constexpr int kStForceAtoms = 850000;    // force pass
-constexpr int kStNodes = 6000;           // 24 bytes per node: 144 KB beside 48 bytes per thread
 
 constexpr size_t force_smem(int nodes, int nt) {
     return (size_t)nodes * sizeof(float4) + (size_t)((nodes + 1) & ~1) * sizeof(float2) + (size_t)nt * 6 * sizeof(double);
-}
-
-static bool st_applies(const Params &p, const Tables &t) {
-    const long long cap = p.mid_cap > p.pair_cap ? p.mid_cap : p.pair_cap;
-    return p.nm >= kStAtoms && t.nr <= kStNodes && p.nm * (cap + 16) < (1LL << 32);   // 32-bit row offsets
 }
 
 template <int B, bool PF, int MINB>
@@ -1191,7 +1177,7 @@ static int sd_variant(DeviceState &d, const Params &p, const Tables &t, bool mix
                 d.rho, d.afrho, d.dafrho, partials, d.flags, store_rho
     int nb = grid_blocks(p.nm, 256);
     if (t.exact) LAUNCH_WAVE((k_screen_density<false, B, PF, MINB>), nb, s, SD_ARGS);
-    else if (mixed && st_applies(p, t))
+    else if (mixed && screen_in_smem(p.nm, t.nr, p.mid_cap, p.pair_cap))
         LAUNCH_WAVE_SMEM((k_screen_st<B, PF, 256 * MINB>), 256 * MINB, (size_t)t.nr * sizeof(float2),
                          kStNodes * sizeof(float2), nb, s, p, t, d.pos, d.posq, d.posq2, d.box, d.mlist, d.mid_cnt,
                          d.alist, d.pair_cnt, d.rho, d.afrho, d.dafrho, partials, d.flags, store_rho);
@@ -1209,7 +1195,7 @@ static inline bool mixed_applies(const Params &p) { return p.ivol == 0 || p.ivol
 int launch_screen_density(DeviceState &d, const Params &p, const Tables &t, bool mixed, int variant,
                           double *partials, cudaStream_t s, bool store_rho) {
     mixed = mixed && mixed_applies(p);
-    if (variant < 0) variant = t.exact ? 1 : (mixed ? (st_applies(p, t) ? 6 : 7) : 6);
+    if (variant < 0) variant = t.exact ? 1 : (mixed ? (screen_in_smem(p.nm, t.nr, p.mid_cap, p.pair_cap) ? 6 : 7) : 6);
     switch (variant) {
     case 0: return sd_variant<4, true, 4>(d, p, t, mixed, partials, store_rho ? 1 : 0, s);
     case 1: return sd_variant<8, true, 4>(d, p, t, mixed, partials, store_rho ? 1 : 0, s);
@@ -1243,9 +1229,7 @@ static int forces_variant(DeviceState &d, const Params &p, const Tables &t, bool
 int launch_forces(DeviceState &d, const Params &p, const Tables &t, bool mixed, int mode,
                   int variant, double *partials, cudaStream_t s) {
     mixed = mixed && mixed_applies(p);
-    // by default the shared-memory form from kStForceAtoms atoms on, with a
-    // variant asked for wherever it applies
-    const bool st = mixed && st_applies(p, t) && (variant >= 0 || p.nm >= kStForceAtoms);
+    const bool st = mixed && forces_in_smem(p.nm, t.nr, p.mid_cap, p.pair_cap);
     if (variant < 0) variant = t.exact ? 1 : (mixed ? 7 : 3);
     if (p.atomstress) return forces_variant<2, false, true, 2>(d, p, t, mixed, st, mode, partials, s);
     switch (variant) {

@@ -44,3 +44,20 @@ def test_hard_core_reaches_nothing(gpu_lib, prec, n):
     assert np.isfinite(a[2]).all() and np.isfinite(a[0])
     for p, q in zip(a, b):
         assert np.array_equal(p, q)
+
+
+def test_every_variant_of_the_large_passes_gives_the_same_forces(gpu_lib):
+    """877,952 atoms: both mixed passes with their tables in shared memory."""
+    w = wl.make_workload(76, sigma=0.08, temperature=300.0, ivol=0, seed=5)
+    g = MoldySystem.from_workload(w, precision="mixed")
+    g.force()
+    f, rho = g.forces(), g.density()["rho"]
+    for v in range(8):
+        g.set_variants(v, 0, v)
+        g.force()
+        assert np.array_equal(g.forces(), f) and np.array_equal(g.density()["rho"], rho), v
+    g.close()
+    g = MoldySystem.from_workload(w, precision="fp64")
+    g.force()
+    assert np.sqrt(np.mean(((g.forces() - f) @ w.b0.T) ** 2)) < 1e-5
+    g.close()
