@@ -636,9 +636,8 @@ k_cl_density(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__rest
 // its force-routine energy F + sum V/2, and with VIR the symmetric per-atom
 // moment S = sum d d^T fp / 2 over pairs with m_i + m_j > 0.1 (stored xx, yy,
 // zz, xy, xz, yz), from which the virial sum (B0 d) d^T fp / 2 is B0 S; one
-// thread per atom, B row entries gathered at a time.  MIXED takes the
-// separation, the table interpolation and the pair force in FP32 and sums in
-// FP64.
+// thread per atom, B row entries gathered at a time.  Mixed precision: the
+// separation, the table interpolation and the pair force in FP32, sums in FP64.
 template <int B, bool VIR>
 __global__ void __launch_bounds__(256)
 k_cl_forces(TileArgs a, Tables t, int ntot, int pair_cap, const int32_t *__restrict__ alist,

@@ -351,25 +351,16 @@ __device__ __forceinline__ double fetm_dphi(const Tables &t, double r) {
     return s;
 }
 
-// (vee, dvee, phi, dphi) at r through the table or the exact functions
+// (vee, dvee, phi, dphi) at r by the exact functions
 __device__ __forceinline__ double4 pair_funcs(const Tables &t, double r) {
-    if (t.exact) return make_double4(fetm_vee(t, r), fetm_dvee(t, r), fetm_phi(t, r), fetm_dphi(t, r));
-    return lookup_r4(t, r);
+    return make_double4(fetm_vee(t, r), fetm_dvee(t, r), fetm_phi(t, r), fetm_dphi(t, r));
 }
 
-__device__ __forceinline__ double density_func(const Tables &t, double r) {
-    if (t.exact) return fetm_phi(t, r);
-    return lookup_phi(t, r);
-}
-
-// (F(rho), F'(rho)): src/fetransmetal.F90:375-404 or the emb tables
-__device__ __forceinline__ double2 embed_funcs(const Tables &t, double rho) {
-    if (t.exact) {
-        double f = -(1.0 * sqrt(rho > 0.0 ? rho : 0.0));
-        double d = rho > 0.0 ? -(0.5 / sqrt(rho)) : 0.0;
-        return make_double2(f, d);
-    }
-    return lookup_e2(t, rho);
+// (F(rho), F'(rho)): src/fetransmetal.F90:375-404
+__device__ __forceinline__ double2 embed_funcs(double rho) {
+    double f = -(1.0 * sqrt(rho > 0.0 ? rho : 0.0));
+    double d = rho > 0.0 ? -(0.5 / sqrt(rho)) : 0.0;
+    return make_double2(f, d);
 }
 
 // ----------------------------------------------------------- box algebra --

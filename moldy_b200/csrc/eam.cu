@@ -394,7 +394,7 @@ k_scalev_scale(int nm, const BoxState *__restrict__ box, double *__restrict__ x1
 void launch_scalev(DeviceState &d, const Params &p, double nose, double rqke, bool mean, bool scale, cudaStream_t s) {
     // Mean and energy are summed over up to 1,184 blocks, as they were as passes
     // of their own: the scaling factor multiplies every velocity, so another
-    // order of these sums (592 blocks, 1 us a step less at 1,024,000 atoms) would
+    // order of these sums (592 blocks, 7 us a step less at 1,024,000 atoms) would
     // move every trajectory of a thermostatted run by its last bits.
     const int nb = grid_blocks(p.nm, kAtomThreads);
     double *part = d.partials + (size_t)kMaxBlocks * kPartials;

@@ -196,7 +196,7 @@ k_screen_density(Params p, Tables t, const double4 *__restrict__ pos, const int4
         // embed (src/potential_m.F90:148-169): rho <= 1e-40 keeps the old values
         double fd;
         if (rho_a > 1e-40) {
-            double2 e = MIXED ? lookup_e2(t, rho_a) : embed_funcs(t, rho_a);
+            double2 e = MIXED ? lookup_e2(t, rho_a) : embed_funcs(rho_a);
             afrho[a] = e.x;
             dafrho[a] = e.y;
             fd = e.y;
@@ -805,7 +805,8 @@ k_forces_st(Params p, Tables t, const int4 *__restrict__ posq2, const BoxState *
 // NINT is evaluated only for pairs across a face, the root and its inverse
 // come from one reciprocal square root, an interval is one 32-byte load of
 // what the pair needs (V on the owner's copy alone), and entries that do not
-// count are predicated off.  432,000 atoms: see the variants' rule below.
+// count are predicated off.  2,000,000 atoms: screening 423 -> 266 us, forces
+// 497 -> 294 (the default variants of either time).
 template <int B, bool PF, int MINB>
 __global__ void __launch_bounds__(256, MINB)
 k_screen_d(Params p, Tables t, const double4 *__restrict__ pos, double4 *__restrict__ pos2,
@@ -1195,6 +1196,10 @@ static inline bool mixed_applies(const Params &p) { return p.ivol == 0 || p.ivol
 int launch_screen_density(DeviceState &d, const Params &p, const Tables &t, bool mixed, int variant,
                           double *partials, cudaStream_t s, bool store_rho) {
     mixed = mixed && mixed_applies(p);
+    // us per launch, every variant (0..7), on a new handle's default lists.  FP64:
+    // 16,000 atoms 20.4 22.0 16.9 17.0 17.0 20.7 16.9 20.8, 54,000 23 29 19 19 19
+    // 26 19 25, 250,000 53 66 48 49 44 60 44 62, 432,000 79 95 76 76 66 91 66 93,
+    // 1,024,000 162 202 162 158 140 197 136 202: 6.
     if (variant < 0) variant = t.exact ? 1 : (mixed ? (screen_in_smem(p.nm, t.nr, p.mid_cap, p.pair_cap) ? 6 : 7) : 6);
     switch (variant) {
     case 0: return sd_variant<4, true, 4>(d, p, t, mixed, partials, store_rho ? 1 : 0, s);
@@ -1230,6 +1235,9 @@ int launch_forces(DeviceState &d, const Params &p, const Tables &t, bool mixed, 
                   int variant, double *partials, cudaStream_t s) {
     mixed = mixed && mixed_applies(p);
     const bool st = mixed && forces_in_smem(p.nm, t.nr, p.mid_cap, p.pair_cap);
+    // as above; FP64: 16,000 atoms 25.1 25.0 19.0 18.9 24.0 22.4 24.0 23.0, 54,000
+    // 31 32 21 21 26 27 27 27, 250,000 70 78 52 50 65 66 66 68, 432,000 103 114 75
+    // 74 89 98 91 100, 1,024,000 222 251 162 155 202 217 200 218: 3.
     if (variant < 0) variant = t.exact ? 1 : (mixed ? 7 : 3);
     if (p.atomstress) return forces_variant<2, false, true, 2>(d, p, t, mixed, st, mode, partials, s);
     switch (variant) {

@@ -381,9 +381,11 @@ __device__ __noinline__ int chi_exact(const double *b, int ivol, const double4 &
 // close.
 //
 // The guard: a unit vector is an FP64 separation rounded to FP32 (2^-24 per
-// component) times a reciprocal root good to 2 ulp of a norm that has three
-// roundings, so each is within 6 * 2^-24 and the product of two, with its own
-// three roundings, within 16 * 2^-24 = 1e-6 of the cosine; the cell index adds
+// component) times a reciprocal root good to 2 ulp (4 * 2^-24) of a squared norm
+// of such components (2 * 2^-24, halved) with three roundings (halved), and the
+// product's rounding, so each is within 8.5 * 2^-24 and the product of two, with
+// its own three roundings, within 20 * 2^-24 = 1.2e-6 of the cosine, a third of
+// the guard; the cell index adds
 // one rounding of a number below 2^12, 2^-13 of a cell.  The routine's own
 // value differs from the cosine by its rounding, below 1e-9 for separations
 // between 0.1 and 100 A.  The three separations close a triangle only where

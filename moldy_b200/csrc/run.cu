@@ -1037,10 +1037,13 @@ static void run_shape(int nm, int &lanes, int &threads, int &blocks) {
 // A run keeps one block of at most 512 threads per SM (its box algebra, list
 // builds and both pair pieces share the registers), the launched passes up to
 // 1024.  Against those passes (us per step, NPT, launched / run): mixed 54,000
-// atoms 45.7 / 31.0, 78,608 51.4 / 52.9, 128,000 69.6 / 54.9, 170,368 74.1 /
-// 76.2; FP64 54,000 51.7 / 42.7, 101,306 68.4 / 78.4.  So runs are taken while
-// every atom has a thread of its own, and in mixed precision, whose pair terms
-// are shorter, up to two atoms per thread.
+// atoms 46.2 / 32.8, 71,874 48.4 / 36.1, 78,608 52.6 / 53.9, 85,750 54.9 / 54.7,
+// 93,312 55.1 / 55.1, 109,744 54.9 / 55.8, 128,000 68.7 / 56.2, 148,176 70.9 /
+// 57.6, 159,014 74.1 / 76.2; FP64 54,000 53.6 / 44.2, 71,874 55.4 / 48.8, 78,608
+// 69.0 / 78.2, 101,306 72.2 / 79.8.  So runs are taken while every atom has a
+// thread of its own, and in mixed precision, whose pair terms are shorter, up to
+// two atoms per thread: just past one the second round is half empty and the
+// two forms are equal to 2 %, so the rule has no gap there.
 bool run_applies(const Params &p, const Tables &t, bool mixed) {
     // the whole grid has to be resident: a partition of the device takes the launches
     int dev = 0, sms = 0;
