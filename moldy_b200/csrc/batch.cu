@@ -1390,15 +1390,21 @@ __device__ __forceinline__ void fm_flush(const double *h, double *g, int nb) {
 }
 
 // The pair of slot hs and row entry j (inside the cut): u = B0 d, r, 1/r, the
-// table interval q and the weight w1 of its upper node.
+// table interval q and the weight w1 of its upper node; returns r^2.  The
+// gradient has nbr nodes, all up to the cut: past the last stored node (a knot
+// of the pair function whose amplitude is zero) the functions are zero, their
+// derivatives by the nodes are not.
 __device__ __forceinline__ double fm_pair(const Tables &t, const double *b, const double4 &ph, const double4 &pj,
-                                          double &ux, double &uy, double &uz, double &rr, int &q, double &w1) {   // r^2
+                                          int nbr, double &ux, double &uy, double &uz, double &rr, int &q, double &w1) {
     double dx, dy, dz;
     frac_diff_near(ph, pj, dx, dy, dz);
     pair_u(b, dx, dy, dz, ux, uy, uz);
     const double r2 = ux * ux + uy * uy + uz * uz, r = root_and_inverse(r2, rr);
-    q = interval_d(t, r, w1);
-    if (q > t.nr - 2) { q = t.nr - 2; w1 = 1.0; }
+    const double x = fma(r, t.vp_recipstep, t.vp_xoff);        // interval_d, over nbr nodes
+    const double lo = __dadd_rd(fmin(fmax(x, 0.0), (double)(nbr - 1)), 4503599627370496.0);
+    q = __double2loint(lo);
+    w1 = x - (lo - 4503599627370496.0);
+    if (q > nbr - 2) { q = nbr - 2; w1 = 1.0; }
     return r2;
 }
 
@@ -1438,9 +1444,9 @@ k_fm_pairs_a(TileArgs a, Tables t, int ntot, Rows rows, const int32_t *__restric
                 if (e0 + u >= n) continue;
                 double ux, uy, uz, rr, w1;
                 int q;
-                const double r2 = fm_pair(t, S.b0, ph, pp[u], ux, uy, uz, rr, q, w1);
+                const double r2 = fm_pair(t, S.b0, ph, pp[u], nbr, ux, uy, uz, rr, q, w1);
                 if (ALL && !(r2 < a.rc2)) continue;
-                const double4 w = ldg4(&t.df4[q]);
+                const double4 w = ldg4(&t.df4[q < t.nr - 1 ? q : t.nr - 1]);
                 const double dp = fma(w.w, w1, w.y);
                 double lam = (gh.x - gg[u].x) * ux + (gh.y - gg[u].y) * uy + (gh.z - gg[u].z) * uz;
                 if (ph.w + pp[u].w > 0.1)
@@ -1533,7 +1539,7 @@ k_fm_pairs_c(TileArgs a, Tables t, int ntot, Rows rows, const int32_t *__restric
                 if (!(hs < jj[u])) continue;             // also the entries past the end (hs itself)
                 double ux, uy, uz, rr, w1;
                 int q;
-                const double r2 = fm_pair(t, S.b0, ph, pp[u], ux, uy, uz, rr, q, w1);
+                const double r2 = fm_pair(t, S.b0, ph, pp[u], nbr, ux, uy, uz, rr, q, w1);
                 if (ALL && !(r2 < a.rc2)) continue;
                 fm_hist(sh, q, nui + nj[u], w1);
             }
@@ -2727,7 +2733,8 @@ int BatchEngine::set_references(const double *fref_xyz, const double *sref) {
 int BatchEngine::force_matching(double wf, double ws, double *loss, double *grads) {
     BCHECK(ready());
     if (!fm_refs) return set_last_error(MOLDY_ERR_ORDER, "set the references first (moldy_gpu_batch_set_references)");
-    const int n = tab.nlookup, nb = n + 1, nbr = tab.nr;
+    const int n = tab.nlookup, nb = n + 1;
+    const int nbr = std::min(nb, std::max(tab.nr, (int)std::ceil((rcut - tab.vp_rmin) * tab.vp_recipstep) + 1));
     if (fm_nb != nb) {
         if (fm_grads) cudaFree(fm_grads);
         fm_grads = nullptr;
