@@ -57,6 +57,16 @@ def test_split_changes_no_bit(gpu_lib, n, ivol, nose, prec):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("fs", [0.5, 0.34, 0.8])
+def test_split_under_the_thermostat_changes_no_bit(gpu_lib, fs, prec):
+    """scalev every second or third step (runs between), and at most steps."""
+    w = wl.make_workload(8, sigma=0.08, temperature=900.0, ivol=0, nbrupdate=7, seed=3, dt_fs=fs)
+    want = _steps(w, prec, 5.0, [23])
+    for split in ([1] * 23, [2, 1, 4, 6, 10]):
+        _same(want, _steps(w, prec, 5.0, split), split)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
 @pytest.mark.parametrize("ivol", [0, 1])
 def test_velocity_verlet_takes_the_same_steps(gpu_lib, ivol, prec):
     """The reference's own loop: velocityverlet, update_therm_avs, relink."""
