@@ -459,6 +459,14 @@ __device__ __forceinline__ double2 tab_emb(const double2 *se, int ne, const Tabl
     return make_double2(a.x * w + b.x * dr, a.y * w + b.y * dr);
 }
 
+// an element of 8 or 16 bytes from global to shared memory, behind the thread's back
+template <typename T>
+__device__ __forceinline__ void copy_async(T *dst, const T *src) {
+    static_assert(sizeof(T) == 8 || sizeof(T) == 16, "cp.async sizes");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(sizeof(T)));
+}
+
 // sum over the L lanes of an atom's group, in every lane of it
 template <int L>
 __device__ __forceinline__ double group_sum(double v) {
@@ -524,7 +532,7 @@ k_run(Params p, Tables t, RunArgs a) {
     constexpr int BD = L >= 8 ? 2 : (!MIXED ? 3 : (L >= 2 ? 5 : 8)), BF = L >= 8 ? 2 : (MIXED ? 4 : 3);
     const bool boxed = p.ivol == 0 || p.ivol == 4;   // the box moves: every step needs its virial
 
-    // the tables
+    // the tables, on their way while the first drift runs
     using Tab = typename std::conditional<MIXED, TabMixed, TabFp64>::type;
     Tab tab;
     double2 *se;
@@ -533,17 +541,19 @@ k_run(Params p, Tables t, RunArgs a) {
         float4 *r4 = reinterpret_cast<float4 *>(dsm);
         float2 *ph = reinterpret_cast<float2 *>(r4 + 2 * (size_t)t.nr);
         se = reinterpret_cast<double2 *>(ph + ((t.nr + 1) & ~1));
-        for (int k = tid; k < 2 * t.nr; k += blockDim.x) r4[k] = __ldg(&t.r4f[k]);
-        for (int k = tid; k < t.nr; k += blockDim.x) ph[k] = __ldg(&t.phi2f[k]);
+        for (int k = tid; k < 2 * t.nr; k += blockDim.x) copy_async(&r4[k], &t.r4f[k]);
+        for (int k = tid; k < t.nr; k += blockDim.x) copy_async(&ph[k], &t.phi2f[k]);
         tab.r4 = r4; tab.phi = ph;
     } else {
         double4 *r4 = reinterpret_cast<double4 *>(dsm);
         double2 *ph = reinterpret_cast<double2 *>(r4 + t.nr);
         se = ph + t.nr;
-        for (int k = tid; k < t.nr; k += blockDim.x) { r4[k] = t.r4[k]; ph[k] = __ldg(&t.phi2[k]); }
+        for (int k = tid; k < 2 * t.nr; k += blockDim.x)
+            copy_async(reinterpret_cast<double2 *>(r4) + k, reinterpret_cast<const double2 *>(t.r4) + k);
+        for (int k = tid; k < t.nr; k += blockDim.x) copy_async(&ph[k], &t.phi2[k]);
         tab.r4 = r4; tab.phi = ph;
     }
-    for (int k = tid; k < ne_emb; k += blockDim.x) se[k] = __ldg(&t.e2[k]);
+    for (int k = tid; k < ne_emb; k += blockDim.x) copy_async(&se[k], &t.e2[k]);
     box_load(s.box, a.box);
     if (tid == 0) s.fail = a.flags[13];       // an earlier run of the call gave up: so does this one
     __syncthreads();
@@ -551,6 +561,10 @@ k_run(Params p, Tables t, RunArgs a) {
 
     unsigned epoch = 0;
     for (int h = a.h0; h <= a.h1; ++h) {
+        if (h == (a.h0 > 0 ? a.h0 : 1)) {     // the first piece that reads them
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+        }
         if (h == 0) {
             // ---- first half-kick and drift of the run's first step (k_drift),
             // with the sums in piece B's grouping
@@ -984,20 +998,19 @@ k_run_therm(Params p, RunArgs a, int lanes, int32_t *__restrict__ ticket) {
     double s3[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) s3[k] = reduce_col(a, 0, kColT + k);
-    if (lane != 0) return;
     BoxState &B = *a.box;
-    double r[kThermoRec], tg[9], tgdot[9], tginv[9], tgid[9], vol;
+    if (lane < 9) {                                   // as warp_therm_prep left them
+        B.tg[lane] = s.tmp[lane]; B.tgdot[lane] = s.tmp[9 + lane]; B.tginv[lane] = s.tmp[18 + lane];
+        B.tgid[lane] = s.box.th_tgid[lane];
+        B.th_tgid[lane] = s.box.th_tgid[lane]; B.th_cof[lane] = s.box.th_cof[lane];
+    }
+    if (lane != 0) return;
+    double r[kThermoRec];
     step_record(p, s.box.b0, s.box.b1, s3, s.box.pe, r);
     if (a.rec)
         for (int k = 0; k < kThermoRec; ++k) a.rec[(size_t)kThermoRec * (size_t)a.rec0 + k] = r[k];
     B.ke = r[0]; B.te = r[2]; B.h = r[3]; B.th = r[4]; B.vol = r[5]; B.s1 = r[6]; B.s2 = r[7]; B.s3 = r[8];
     B.temp = r[9]; B.boxke = r[10];
-    therm_box(p, s.box.b0, s.box.b1, tg, tgdot, tginv, tgid, vol);
-    for (int k = 0; k < 9; ++k) {
-        B.tg[k] = tg[k]; B.tgdot[k] = tgdot[k]; B.tginv[k] = tginv[k];
-        B.tgid[k] = s.box.th_tgid[k];
-        B.th_tgid[k] = s.box.th_tgid[k]; B.th_cof[k] = s.box.th_cof[k];
-    }
     if (s.box.status) B.status = s.box.status;
 }
 
