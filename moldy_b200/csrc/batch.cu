@@ -2313,6 +2313,7 @@ int BatchEngine::layout() {
     BCUDA(cudaStreamSynchronize(stream), "layout");
     list_cut = rcut;
     layout_due = false;
+    rows_refused = false;               // the device may have room for them by now
     return MOLDY_OK;
 }
 
