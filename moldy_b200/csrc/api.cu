@@ -818,8 +818,9 @@ int Engine::ensure_active_capacity(int min_pair, int min_mid, int min_out) {
 int Engine::velocityverlet(moldy_force_out *out) {
     CHECK(check_ready());
     bool rb = false;
+    // rows that grow are rebuilt before they are used: before run_length asks
+    CHECK(ensure_active_capacity(0));
     if (runs_apply() && run_length(1) > 0) {   // the sums of md_steps' step
-        CHECK(ensure_active_capacity(0));
         CHECK(queue_run(1, false, nullptr, 0, true, false));
         ntc_ = ntc_ + 1 == ntcm_ ? 0 : ntc_ + 1;
         CHECK(fetch_force_out(out));
@@ -999,9 +1000,10 @@ int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
         bool rb = false;
         // consecutive steps of a small system that need no half-list build, up
         // to and including one that is followed by a relink or scalev: one launch
+        // (rows that grow are rebuilt before they are used: before run_length asks)
+        CHECK(ensure_active_capacity(0));
         const int run = runs ? run_length(nsteps - k) : 0;
         if (run > 0) {
-            CHECK(ensure_active_capacity(0));
             const int first = k;
             k += run - 1;
             const bool scalev = advance_run(run, &ntcs[first]);
@@ -1026,7 +1028,6 @@ int Engine::md_steps(int nsteps, moldy_thermo *thermo) {
             if (ordinary && !graph_failed && !step_graph) {
                 // capture one ordinary step; the host-side state it changes is
                 // put back, and advanced below for every replay
-                CHECK(ensure_active_capacity(0));
                 const int ntc0 = ntc_, kin0 = kin_blocks, tb0 = therm_blocks;
                 double *tr0 = therm_rec;
                 const bool skip0 = skip_rho, dirty0 = mid_dirty_;
