@@ -467,6 +467,9 @@ __device__ __forceinline__ void copy_async(T *dst, const T *src) {
                  "n"(sizeof(T)));
 }
 
+// waits for this thread's copies
+__device__ __forceinline__ void copies_arrived() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // sum over the L lanes of an atom's group, in every lane of it
 template <int L>
 __device__ __forceinline__ double group_sum(double v) {
@@ -557,12 +560,15 @@ k_run(Params p, Tables t, RunArgs a) {
     box_load(s.box, a.box);
     if (tid == 0) s.fail = a.flags[13];       // an earlier run of the call gave up: so does this one
     __syncthreads();
-    if (s.fail) return;
+    if (s.fail) {
+        copies_arrived();                     // no block ends with copies on their way
+        return;
+    }
 
     unsigned epoch = 0;
     for (int h = a.h0; h <= a.h1; ++h) {
         if (h == (a.h0 > 0 ? a.h0 : 1)) {     // the first piece that reads them
-            asm volatile("cp.async.wait_all;" ::: "memory");
+            copies_arrived();
             __syncthreads();
         }
         if (h == 0) {
@@ -587,7 +593,10 @@ k_run(Params p, Tables t, RunArgs a) {
             }
             warp_columns<6>(s, kB_K, k6);
             warp_column_max(s, kB_Max, d2);
-            if (!end_piece(a, s, epoch, 0x3f80u, false, 1)) return;   // step 0's buffer is 0
+            if (!end_piece(a, s, epoch, 0x3f80u, false, 1)) {   // step 0's buffer is 0
+                copies_arrived();
+                return;
+            }
             continue;
         }
         if (h == 2 * a.m + 1) {
