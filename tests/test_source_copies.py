@@ -13,7 +13,8 @@ def test_run_kernel_waits_for_its_copies_before_it_ends():
     i = re.search(r"^[^\n;/]*\bk_run\(", src, re.M).start()
     body = re.sub(r"//[^\n]*", "", src[i:src.index("\n}\n", i)])
     drift = body.index("if (h == 0) {")
-    upto = body[:body.index("continue;", drift)]
+    end = body.index("if (h == 2 * a.m + 1) {", drift)       # the next piece
+    upto = body[:end]
     returns = [m.start() for m in re.finditer(r"\breturn;", upto)]
     assert len(returns) >= 2
     for r in returns:
