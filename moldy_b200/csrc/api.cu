@@ -882,7 +882,8 @@ int Engine::run_length(int left) const {
 
 // Whether this engine's ordinary steps are taken by runs.  Then all of them
 // are, a single step and velocityverlet's too, and so are all sums of
-// update_therm_avs: how steps are split into calls changes no bit.  scalev ends a
+// update_therm_avs: how steps are split into calls changes no bit (but for a
+// launched step that builds rows which grew between two calls).  scalev ends a
 // run, and a run of one step is slower than the launched step (2500 K with
 // scalev every step, mixed: 16,000 atoms 72 against 65 us, 71,874 98 against 79),
 // so with the thermostat on runs are left to time steps of half a femtosecond
